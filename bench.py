@@ -896,7 +896,10 @@ def run_ours(a, rank, world, local_rank):
     # ---- roofline: the dominant sweep kernel, CUDA-event timed on the solver's stream
     # sweeps per inner iteration -- BiCGSTAB: A SpMM x2, G SpMM x5, x/r/p, s; COCG: q = A p with p.q,
     # T = G r with T.T, z = G^T T (the plain G kernel on the G^T records), r update, x/p update
-    per_iter = {0: 2, 1: 5, 2: 1, 3: 1} if a.inner == "bicgstab" else {4: 1, 5: 1, 1: 1, 6: 1, 7: 1}
+    # (a SpMM pinned on the command line); by default COCG's three fused sweeps
+    pinned = a.no_autotune and (a.spmm_vec or a.spmm_kind)
+    per_iter = ({0: 2, 1: 5, 2: 1, 3: 1} if a.inner == "bicgstab" else
+                {4: 1, 5: 1, 1: 1, 6: 1, 7: 1} if pinned else {8: 1, 9: 1, 10: 1})
     shp = solver.spmm_shape()
     sv, sk = shp["vec"] or 4, shp["kind"]
     gk = 0 if sk == 4 else sk                       # kind 4 pairs the harmonics of A only
@@ -905,7 +908,9 @@ def run_ours(a, rank, world, local_rank):
     names = {0: a0, 1: f"k_spmm<float,{sv},0,OpG32,{gk}> (FSAI apply)",
              2: "k_update_xrp<float>", 3: "k_update_s<float>",
              4: a1, 5: f"k_spmm<float,{sv},3,OpG32,{gk}> (T = G r, T.T)",
-             6: "k_update_r<float>", 7: "k_update_px<float>"}
+             6: "k_update_r<float>", 7: "k_update_px<float>",
+             8: "k_fsweep<4,0> (q = A p, p.q)", 9: "k_fsweep<4,1> (T -= alpha G q, T.T)",
+             10: "k_fsweep<4,2> (x += alpha p, p = G^T T + beta p)"}
     prof = {q: solver.profile_kernel(q, 5) for q in per_iter}
     dom = max(prof, key=lambda q: prof[q][0] * per_iter[q])
     pk = json.load(open(ROOT / "MEASURED_PEAKS.json")) if (ROOT / "MEASURED_PEAKS.json").exists() else {}
@@ -915,6 +920,8 @@ def run_ours(a, rank, world, local_rank):
     # shape on the 20,497-node, 32-harmonic ellipsoid, scaled to this launch by nodes x harmonics
     # (the records and vectors all scale with both)
     captured = {0: 659.7e6, 1: 716.4e6, 4: 804.8e6, 5: 797.1e6, 6: 966.3e6, 7: 1626.1e6}
+    # the fused sweeps: captured at 47,034 nodes, 32 harmonics, 32 sources (scaled to 64 of the case above)
+    captured.update({q: b * 2 * 20497 / 47034 for q, b in {8: 779.6e6, 9: 1309.8e6, 10: 2067.6e6}.items()})
     traffic = traffic_bytes = None
     if dom in captured and a.workload == "ellipsoid":
         traffic_bytes = captured[dom] * (mesh.nn * len(solver.harmonics)) / (20497 * 32)

@@ -1622,6 +1622,28 @@ __global__ void k_omega(int nf, double dfc, const int32_t *__restrict__ harm, do
   }
 }
 
+// sums of K and M over the pattern and max K_ii / M_ii: the scale of the spectrum of (K, M)
+__global__ void k_spectrum(const int32_t *__restrict__ rowptr, const int32_t *__restrict__ col,
+                           const double *__restrict__ K, const double *__restrict__ M, int64_t n, double *out) {
+  double sk = 0.0, sm = 0.0, mx = 0.0;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    for (int p = rowptr[i]; p < rowptr[i + 1]; ++p) {
+      sk += K[p];
+      sm += M[p];
+      if (col[p] == i && M[p] > 0.0) mx = fmax(mx, K[p] / M[p]);
+    }
+  for (int off = 16; off > 0; off >>= 1) {
+    sk += __shfl_xor_sync(0xffffffffu, sk, off);
+    sm += __shfl_xor_sync(0xffffffffu, sm, off);
+    mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(out, sk);
+    atomicAdd(out + 1, sm);
+    atomicMax((unsigned long long *)(out + 2), (unsigned long long)__double_as_longlong(fmax(mx, 0.0)));
+  }
+}
+
 // ------------------------------------------------------------ host side
 inline unsigned g1(int64_t n, int bs) { return (unsigned)std::min<int64_t>(ceil_div(n, bs), 1 << 30); }
 
@@ -1809,6 +1831,7 @@ int ensure_workspace(SolverPlan *S, int prec, int nvec = NVEC_ALL) {
   const size_t esz = prec == DGP_PREC_FP64 ? sizeof(double2) : sizeof(float2);
   const size_t vb = esz * (size_t)C * S->n;
   if (S->ws_prec != prec) {
+    S->drop_fused();
     for (auto &g : S->graph)
       if (g) {
         cudaGraphExecDestroy(g);
@@ -2253,7 +2276,20 @@ void launch_residual(SolverPlan *S, int ns, const double *d_X, const double *d_B
 
 }  // namespace
 
+void SolverPlan::drop_fused() {
+  for (auto &g : fgraph)
+    if (g) {
+      cudaGraphExecDestroy(g);
+      g = nullptr;
+    }
+  for (int &i : fgraph_iters) i = 0;
+  for (auto &v : fvec) v.release();
+  fscal.release();
+  fctl.release();
+}
+
 SolverPlan::~SolverPlan() {
+  drop_fused();
   for (auto &g : graph)
     if (g) cudaGraphExecDestroy(g);
   for (auto &e : poll_ev)
@@ -2300,6 +2336,8 @@ int solver_build(SolverPlan *S, const int32_t *d_rowptr, const int32_t *d_col, i
   S->nf = nf;
   S->ns_max = ns_max;
   S->nsp = pad_sources(ns_max);
+  S->fnsp = (ns_max + 3) / 4 * 4;
+  S->h_harm = hl;
   S->dfc = dfc;
   if (opts) S->opts = *opts; else dgp_solve_opts_default(&S->opts);
   DGP_TRY(S->rowptr.alloc(sizeof(int32_t) * (n + 1)));
@@ -2322,7 +2360,22 @@ int solver_build(SolverPlan *S, const int32_t *d_rowptr, const int32_t *d_col, i
   DGP_TRY(S->GT64.alloc(sizeof(double2) * gcount));
   DGP_TRY(S->RecG32.alloc(sizeof(Rec32) * gcount));
   DGP_TRY(S->RecGT32.alloc(sizeof(Rec32) * gcount));
-  DGP_CUDA(cudaMallocHost(&S->h_ctl, 2 * sizeof(Ctl)));  // two mirrors (run_iterations' pipelined polls)
+  // two mirrors (run_iterations' pipelined polls); the fused solve's control block fits too
+  DGP_CUDA(cudaMallocHost(&S->h_ctl, std::max<size_t>(512, 2 * sizeof(Ctl))));
+  {
+    DevBuf sums;
+    double hs[3] = {0, 0, 0};
+    DGP_TRY(sums.alloc(sizeof(hs)));
+    DGP_CUDA(cudaMemsetAsync(sums.p, 0, sizeof(hs), st));
+    k_spectrum<<<(unsigned)std::min<int64_t>(ceil_div(n, 256), 592), 256, 0, st>>>(
+        S->rowptr.as<int32_t>(), S->col.as<int32_t>(), d_K, d_M, n, sums.as<double>());
+    DGP_CHECK_LAUNCH();
+    DGP_CUDA(cudaMemcpyAsync(hs, sums.p, sizeof(hs), cudaMemcpyDeviceToHost, st));
+    DGP_CUDA(cudaStreamSynchronize(st));
+    S->lam_hi = std::isfinite(hs[2]) && hs[2] > 0 ? hs[2] : 1.0;
+    S->lam_lo = hs[1] > 0 && std::isfinite(hs[0]) && hs[0] > 0 ? hs[0] / hs[1] : S->lam_hi;
+    S->lam_lo = std::min(S->lam_hi, std::max(S->lam_lo, 1e-6 * S->lam_hi));
+  }
   DGP_TRY(tiled_setup(S, st));
   return solver_update(S, d_K, d_M, st);
 }
@@ -2462,18 +2515,22 @@ int solver_solve(SolverPlan *S, const double *d_B, const int32_t *d_nodes, const
   }
   dgp_solve_report local{};
   dgp_solve_report *r = rep ? rep : &local;
+  const bool fused = o.precision == DGP_PREC_MIXED && !S->unfused;
   const int rc = o.precision == DGP_PREC_FP64 ? solve_fp64(S, d_B, d_nodes, d_w, d_fpsf, d_X, ns, o, r, st)
-                                              : solve_mixed(S, d_B, d_nodes, d_w, d_fpsf, d_X, ns, o, r, st);
+                 : fused ? solve_fused(S, d_B, d_nodes, d_w, d_fpsf, d_X, ns, o, r, st)
+                         : solve_mixed(S, d_B, d_nodes, d_w, d_fpsf, d_X, ns, o, r, st);
   if (rc != DGP_OK && rc != DGP_ERR_NOT_CONVERGED) return rc;
   // per-column statuses for the caller (harmonic-major, ns columns per harmonic)
-  std::vector<int> hs((size_t)S->ws_cols);
-  DGP_CUDA(cudaMemcpyAsync(hs.data(), S->status.p, sizeof(int) * S->ws_cols, cudaMemcpyDeviceToHost, st));
+  const int nsp = fused ? S->fnsp : S->nsp;
+  std::vector<int> hs((size_t)S->nf * nsp);
+  DGP_CUDA(cudaMemcpyAsync(hs.data(), fused ? (const void *)fused_status(S) : S->status.p, sizeof(int) * hs.size(),
+                           cudaMemcpyDeviceToHost, st));
   DGP_CUDA(cudaStreamSynchronize(st));
   int bad = 0;
   std::vector<int> out((size_t)S->nf * ns);
   for (int k = 0; k < S->nf; ++k)
     for (int s = 0; s < ns; ++s) {
-      int v = hs[(size_t)k * S->nsp + s];
+      int v = hs[(size_t)k * nsp + s];
       if (v == DGP_COL_ZERO_RHS) v = DGP_COL_CONVERGED;  // x = 0 solves b = 0 exactly
       out[(size_t)k * ns + s] = v;
       bad += v != DGP_COL_CONVERGED;
@@ -2524,8 +2581,10 @@ void profile_launch(int which, const SolverPlan *S, const OpA32 &A, const OpG32 
 // workspace (same shapes and launch configuration as inside the solve) with
 // CUDA events on `st`, and returns its algorithmic bytes per launch.
 int solver_profile(SolverPlan *S, int which, int reps, float *ms, double *bytes, cudaStream_t st) {
-  DGP_REQUIRE(S->ws_prec == DGP_PREC_MIXED, "profile: run a mixed-precision solve first");
-  DGP_REQUIRE(reps >= 1 && which >= 0 && which <= 7, "profile: bad arguments");
+  DGP_REQUIRE(reps >= 1 && which >= 0 && which <= 10, "profile: bad arguments");
+  DGP_REQUIRE(S->ws_prec == DGP_PREC_MIXED || S->fscal.p, "profile: run a mixed-precision solve first");
+  if (which >= 8) return fused_profile(S, which - 8, reps, ms, bytes, st);
+  DGP_TRY(ensure_workspace(S, DGP_PREC_MIXED, NVEC_COCG));
   if (which == 2 || which == 3) DGP_TRY(ensure_workspace(S, DGP_PREC_MIXED, NVEC_ALL));  // BiCGSTAB updates
   Vecs<float> V = vec_views<float>(S);
   Work W = work_views(S);
@@ -2761,6 +2820,10 @@ int solver_autotune(SolverPlan *S, int32_t *tiled_out, int32_t *vec_out, int32_t
   for (int &gi : S->graph_iters) gi = 0;
   DGP_CUDA(cudaMemsetAsync(W.cols.acc, 0, sizeof(double2) * W.cols.C * NACC, st));
   DGP_CUDA(cudaStreamSynchronize(st));
+  if (!S->unfused) {  // the next mixed solve runs on the fused sweeps and their own workspace
+    for (auto &v : S->vec) v.release();
+    S->ws_prec = -1;
+  }
   if (tiled_out) *tiled_out = bt;
   if (vec_out) *vec_out = bv;
   if (rows_out) *rows_out = br;
@@ -2778,6 +2841,7 @@ int solver_set_spmm(SolverPlan *S, int32_t tiled, int32_t vec, int32_t rows) {
                 "set_spmm: rows must be 0 (default), 32, 64, 128 or 256");
   }
   S->tiled = tiled;
+  S->unfused = tiled || vec != 0;  // a shape asked for by name: the sweeps it names
   if (!tiled) {
     S->tune_vec = vec;
     S->tune_rows = vec ? rows : 0;
@@ -2794,6 +2858,7 @@ int solver_set_spmm(SolverPlan *S, int32_t tiled, int32_t vec, int32_t rows) {
 int solver_set_spmm_kind(SolverPlan *S, int32_t kind) {
   DGP_REQUIRE(kind >= 0 && kind <= 4, "set_spmm_kind: kind must be 0, 1, 2, 3 or 4");
   S->tune_kind = kind;
+  S->unfused = 1;
   for (auto &g : S->graph)
     if (g) {
       cudaGraphExecDestroy(g);

@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 #include "dgp_common.cuh"
 
 namespace dgp {
@@ -108,8 +110,32 @@ struct SolverPlan {
   TiledPlan tA, tG, tGT;
   int32_t tiled_ok = 0, tiled = 0;
   int64_t bytes = 0;
+  // ---- fused COCG (cocg.cu): the mixed solve unless a gather or tiled SpMM was asked for by name
+  int32_t unfused = 0;
+  int32_t fnsp = 0;              // columns per harmonic, padded to a multiple of 4
+  std::vector<int32_t> h_harm;   // harmonic index of each batch slot
+  double lam_lo = 0, lam_hi = 0; // 1^T K 1 / 1^T M 1 and max K_ii / M_ii at plan creation
+  DevBuf fvec[4], fscal, fctl;   // x, p, q (also the right-hand side), T; per-column state; control block
+  cudaGraphExec_t fgraph[2] = {nullptr, nullptr};  // host-polled, device-driven
+  int fgraph_iters[2] = {0, 0};
+  struct Level {                 // harmonics solved together, and the combinations they start from
+    std::vector<int32_t> members, solved, idx;  // idx: positions in `solved`, `terms` per member
+    std::vector<double> coef;    // (re, im) of `terms` coefficients per member
+    int terms = 0;
+    size_t off_mem = 0, off_idx = 0, off_solved = 0, off_coef = 0;
+  };
+  std::vector<Level> levels;
+  int levels_first = -1;
+  DevBuf lev_int, lev_coef;
+  void drop_fused();             // releases the fused workspace (another precision takes its place)
   ~SolverPlan();
 };
+
+// the mixed COCG solve on fused sweeps; statuses of its last solve ([nf][fnsp], device)
+int solve_fused(SolverPlan *S, const double *d_B, const int32_t *d_nodes, const double *d_w, const double *d_fpsf,
+                double *d_X, int ns, const dgp_solve_opts &o, dgp_solve_report *rep, cudaStream_t st);
+const int *fused_status(SolverPlan *S);
+int fused_profile(SolverPlan *S, int which, int reps, float *ms, double *bytes, cudaStream_t st);
 
 // h_harm: host list of the nf harmonic indices the plan solves (NULL = 0 .. nf-1)
 int solver_build(SolverPlan *S, const int32_t *d_rowptr, const int32_t *d_col, int64_t n, int64_t nnz,

@@ -251,7 +251,9 @@ int dgp_solver_memory(dgp_solver_t solver, int64_t *bytes);
  * the plan, and the tiled SpMM (32-row blocks whose
  * halo rows are staged in shared memory) when it fits -- on the plan's own
  * workspace (allocating it if needed), and keeps the fastest for later
- * solves.  Outputs (each may be NULL): 1 if the tiled SpMM won, the best
+ * solves on these sweeps: BiCGSTAB inner solves, and COCG ones once a SpMM
+ * has been set by name (dgp_solver_set_spmm, _set_spmm_kind); by default COCG
+ * runs on its fused sweeps, which have one shape.  Outputs (each may be NULL): 1 if the tiled SpMM won, the best
  * gather lane width and rows per block, and the winner's time for the seven
  * launches in ms.  Synchronises the stream.  No reference counterpart (the
  * reference's launch shapes are fixed, smv_CUDA.cu:57-82). */
@@ -332,7 +334,9 @@ int dgp_solve_sources(dgp_solver_t solver, const int32_t *d_nodes,
  * workspace with CUDA events on `stream` (which: 0 = t = A z SpMM,
  * 1 = G p SpMM, 2 = BiCGSTAB x/r/p update, 3 = h/s update, 4 = q = A p SpMM
  * with p.q, 5 = T = G r SpMM with T.T, 6 = COCG r update, 7 = COCG x/p
- * update) and returns the average
+ * update; the three sweeps of the default fused COCG iteration: 8 = q = A p
+ * with p.q, 9 = T -= alpha G q with T.T, 10 = x += alpha p, p = G^T T +
+ * beta p) and returns the average
  * milliseconds per launch and the kernel's algorithmic bytes per launch.
  * Needs a prior DGP_PREC_MIXED solve; overwrites workspace vectors. */
 int dgp_solver_profile_kernel(dgp_solver_t solver, int32_t which, int32_t reps,
