@@ -5,18 +5,17 @@
 // symmetric positive definite, i.e. a Cholesky factorisation and two triangular solves).
 //
 // H is row-major [n][ldh]; its lower triangle is read and overwritten by L (H = L L^T); the
-// strict upper triangle is not touched.  Right-looking, 1536-column outer panels of 128-column
-// steps:
+// strict upper triangle is not touched.  Right-looking, outer panels of 1024 or 1536 columns
+// (outer_width) in 128-column steps:
 //
-//   for each step k (columns [k0, k0 + 128)) of the outer panel [o0, o0 + 1536):
+//   for each step k (columns [k0, k0 + 128)) of the outer panel:
 //     k_potrf_tile   the 128 x 128 diagonal block: L_kk in place, and inv(L_kk) into a scratch
-//                    table (one CTA, block in shared memory: 32-column steps, a warp factors the
-//                    32 x 32 diagonal, all warps solve and update the rest; the inverse by
-//                    32-blocks)
-//     k_dgemm_nt     panel: L_ik = A_ik inv(L_kk)^T for the rows below (in place: a CTA owns
-//                    whole 128-row strips of the panel)
-//     k_dgemm_nt     update of the outer panel's remaining columns: A_il -= L_ik L_lk^T
-//   k_dgemm_nt       trailing update of the rest, depth 1536: A_il -= sum over the outer panel
+//                    table (one CTA, block in shared memory, 8-column steps)
+//     k_strip        the panel's rows below: L_ik = A_ik inv(L_kk)^T in place, a CTA per 32 rows;
+//                    then the next diagonal block's update
+//     k_dgemm_nt     update of the outer panel's remaining columns: A_il -= L_ik L_lk^T, and the
+//                    rows below the panel
+//   k_dgemm_nt       trailing update of the rest, as deep as the panel is wide
 //
 // k_dgemm_nt: C = beta C + alpha A B^T with A, B row-major (K contiguous); 128 x 64 CTA tiles,
 // two CTAs per SM, 256 threads (8 warps of 32 x 32), K in stages of 16 doubles moved by cp.async
@@ -55,10 +54,6 @@ constexpr int gemm_smem(int gbn) {
                                                                                : GBM * (gbn + 1));
 }
 constexpr int GV = 256;          // k per CTA of the solves' off-diagonal partial sums
-#ifndef DGP_CHOL_NBO
-#define DGP_CHOL_NBO 1536
-#endif
-constexpr int64_t NBO = DGP_CHOL_NBO;  // outer panel width: depth of the trailing update GEMM
 
 __device__ inline uint32_t su32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -266,91 +261,161 @@ __global__ void __launch_bounds__(GTHREADS, GBN == 64 ? 2 : 1) k_dgemm_nt(Gemm g
   }
 }
 
+// Row strips of the step chain, depth 128 (a block with rows below it is a whole one), one CTA per
+// 32 rows:
+//   UPD = false   L = A inv(L_kk)^T in place for the outer panel's rows below the diagonal block
+//   UPD = true    C -= A A^T on the lower triangle of the next diagonal block (C rows = A rows)
+// Both sit between two diagonal blocks, so their latency counts, not their rate: a 128 x 128 tile
+// of depth 128 is 15 us of one SM's FP64 tensor pipe, a 32-row strip a quarter of that.  The
+// strip is loaded whole, the other operand in 32-column chunks through two buffers (108 KB: fits
+// beside a trailing-update CTA).  8 warps of 16 rows x 32 columns; a warp skips the chunks and
+// columns that the triangles leave empty.  Step chain per block at n = 10,240: 27 + 20 -> 9 + 8 us.
+constexpr int SR = 32, SK = 32, SLD = SK + 4, SALD = CB + 4;
+constexpr int STRIP_SMEM = (int)sizeof(double) * (SR * SALD + 2 * CB * SLD);
+struct Strip {
+  double *A;            // M strip rows of 128 columns; overwritten when !UPD
+  int64_t lda;
+  const double *B;      // N rows of 128 columns
+  int64_t ldb;
+  double *C;            // UPD: the updated block
+  int M, N;
+};
+template <int V, bool UPD> __global__ void __launch_bounds__(256) k_strip(Strip g) {
+  extern __shared__ __align__(16) double ssm[];
+  double *As = ssm, *Bs = ssm + SR * SALD;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gid = lane >> 2, tig = lane & 3;
+  const int r0 = blockIdx.x * SR, m0 = 16 * (warp & 1), n0 = 32 * (warp >> 1);
+  constexpr int E = V / 8;
+  constexpr int nk = CB / SK;
+  // columns this strip needs: all N, or (UPD) those on or left of its last row
+  const int ncol = UPD ? min(g.N, r0 + SR) : g.N;
+  for (int e = tid; e < SR * (CB / E); e += 256) {
+    const int row = e / (CB / E), kc = (e % (CB / E)) * E;
+    const bool ok = r0 + row < g.M;
+    cp_async<V>(As + row * SALD + kc, ok ? g.A + (int64_t)(r0 + row) * g.lda + kc : g.A, ok);
+  }
+  auto load_b = [&](int c, int slot) {
+    double *dst = Bs + slot * CB * SLD;
+    for (int e = tid; e < CB * (SK / E); e += 256) {
+      const int row = e / (SK / E), kc = (e % (SK / E)) * E, k = c * SK + kc;
+      const bool ok = row < ncol;
+      cp_async<V>(dst + row * SLD + kc, ok ? g.B + (int64_t)row * g.ldb + k : g.B, ok);
+    }
+  };
+  load_b(0, 0);
+  cp_commit();
+  load_b(1, 1);
+  cp_commit();
+  double acc[4][4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) acc[j][q] = 0.0;
+  for (int c = 0; c < nk; ++c) {
+    cp_wait<1>();
+    __syncthreads();
+    // inv(L)[n][k] = 0 for k > n: chunk c meets columns n0 .. n0 + 31 only if c * 32 <= n0 + 31
+    const bool use = n0 < ncol && (UPD || c * SK <= n0 + 31);
+    if (use) {
+      const double *b_ = Bs + (c & 1) * CB * SLD;
+#pragma unroll
+      for (int k4 = 0; k4 < SK; k4 += 4) {
+        const double a0 = As[(m0 + gid) * SALD + c * SK + k4 + tig], a1 = As[(m0 + gid + 8) * SALD + c * SK + k4 + tig];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) mma_f64(acc[j], a0, a1, b_[(n0 + 8 * j + gid) * SLD + k4 + tig]);
+      }
+    }
+    __syncthreads();
+    if (c + 2 < nk) load_b(c + 2, c & 1);
+    cp_commit();
+  }
+  cp_wait<0>();
+  // (the strip was read whole before the first chunk: writing it in place is safe)
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int r = r0 + m0 + gid + 8 * (q >> 1), c = n0 + 8 * j + 2 * tig + (q & 1);
+      if (r >= g.M || c >= g.N) continue;
+      if (!UPD) g.A[(int64_t)r * g.lda + c] = acc[j][q];
+      else if (c <= r) g.C[(int64_t)r * g.lda + c] -= acc[j][q];
+    }
+}
+
 // Factor the nb x nb diagonal block at (k0, k0) in place (lower) and write inv(L) (row-major,
 // nb x nb, zero above the diagonal) to Linv.  One CTA of 256 threads; the block sits in shared
 // memory with rows padded to 129 doubles, rows and columns past nb set to the identity (which
 // the factorisation leaves alone).  The strict upper triangle of the shared tile collects
-// X = inv(L) transposed ([c][i] holds X[i][c]); dinv[c] = 1 / L[c][c].  Four 32-column steps:
-//   1. warp 0 factors the 32 x 32 diagonal block D, one row per lane in registers (a column per
-//      step: the pivot by shuffle, its reciprocal square root, the column scaled and passed
-//      through shared memory, the rank-1 update of the lanes' rows)
-//   2. the rows below by forward substitution, one row per thread: L_rD = A_rD L_D^-T
-//   3. the trailing lower triangle: A -= L_rD L_cD^T in 4 x 4 register tiles
-// then the four diagonal inverses X_II (a warp each, one column per lane) and the off-diagonal
-// blocks of X by their distance d = I - J below the diagonal:
-//   T = sum_{K = J .. I-1} L_IK X_KJ,   X_IJ = -X_II T   (a column of T per group of lanes).
+// X = inv(L) transposed ([c][i] holds X[i][c]); dinv[c] = 1 / L[c][c].
+//
+// What bounds it is the chain of 128 dependent pivots on one SM.  Sixteen 8-column steps:
+//   1. each of the first 128 threads factors the 8 x 8 diagonal block by itself, in registers: the
+//      pivots' reciprocal square roots follow each other without any exchange between threads;
+//      then it solves its own row against it (one row per thread)
+//   2. all warps update the rest of the lower triangle in 8 x 8 tiles on the FP64 tensor cores
+// (32-column steps, a warp on each 32 x 32 diagonal with its columns passed through shared memory:
+// 87 us per block, 560 cycles a pivot; now 48 us, half of it the pivots' chain at 190 cycles each.)  The inverse: the
+// 8 x 8 diagonal inverses, one column per thread, then pairs of blocks of 8, 16, 32, 64 are joined,
+// X_21 = -X_22 (L_21 X_11), on the tensor cores too.  Rows are 132 doubles apart: a half-warp's
+// 4 x 4 operand fragment touches all 32 banks.
 // err |= 1 on a non-positive or non-finite pivot.
-constexpr int PT = 128, PLD = 129, PTHREADS = 256;
-// One level of the off-diagonal blocks of X = inv(L) in the shared tile of k_potrf_tile (X[i][c]
-// kept at [c][i]), the 4 - D block pairs (J, I = J + D):
-//   A. T = sum_{K=J}^{I-1} L_IK X_KJ, a TR x TC register tile per thread (rows i of block I,
-//      columns c of block J), written where X_IJ goes ([c][32I + i], which nothing at this level
-//      reads); X[k][c] is L[c][k] above c, dinv[c] on it, zero below
-//   B. X_IJ = -X_II T, one column c per thread, T's column in registers and X_II[i][m] (at
-//      [32I + m][32I + i]) read as a broadcast
-template <int D, int TR, int TC>
-__device__ inline void inv_level(double *L, const double *dinv) {
-  constexpr int TPP = (32 / TR) * (32 / TC), NP = 4 - D;      // tiles per pair, pairs
-  static_assert(NP * TPP <= PTHREADS, "one tile per thread");
-  const int tid = threadIdx.x;
-  if (tid < NP * TPP) {
-    const int J = tid / TPP, rem = tid % TPP, I = J + D;
-    const int i0 = 32 * I + (rem / (32 / TC)) * TR, c0 = 32 * J + (rem % (32 / TC)) * TC;
-    double acc[TR][TC];
+constexpr int PT = 128, PLD = 132, PTHREADS = 256;
+// D += A B for one 8 x 8 x 4 tile: a = A[g][t], b = B[t][g], d = {D[g][2t], D[g][2t+1]}
+__device__ inline void mma_884(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(d[0]), "+d"(d[1]) : "d"(a), "d"(b));
+}
+// Joins the inverses of the blocks of S into those of 2 S: T = L_21 X_11 (kept where X_21 goes),
+// X_21 = -X_22 T.  Each warp takes one 8-row strip of one pair's block, its S / 8 tiles together:
+// an m8n8k4's result is ~100 cycles away, so the tiles' products are issued side by side.
+template <int S> __device__ __forceinline__ void join_inverse(double *L, const double *dinv) {
+  constexpr int TS = S / 8;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+  const int b1 = 2 * S * (warp / TS), b2 = b1 + S, i0 = b2 + 8 * (warp % TS);
+  double acc[TS][2];
 #pragma unroll
-    for (int u = 0; u < TR; ++u)
+  for (int u = 0; u < TS; ++u) acc[u][0] = acc[u][1] = 0.0;
+#pragma unroll 2
+  for (int k = b1; k < b2; k += 4) {
+    const int kk = k + tig;
+    const double a = L[(i0 + gid) * PLD + kk];
 #pragma unroll
-      for (int v = 0; v < TC; ++v) acc[u][v] = 0.0;
-#pragma unroll 4
-    for (int k = 32 * J; k < 32 * I; ++k) {
-      double lr[TR], xc[TC];
-#pragma unroll
-      for (int u = 0; u < TR; ++u) lr[u] = L[(i0 + u) * PLD + k];
-#pragma unroll
-      for (int v = 0; v < TC; ++v) {
-        const int c = c0 + v;
-        const double up = L[c * PLD + k];
-        xc[v] = k > c ? up : (k == c ? dinv[c] : 0.0);
+    for (int u = 0; u < TS; ++u)
+      if (k >= b1 + 8 * u) {                                 // X_11[k][c] = 0 for k < c
+        const int c = b1 + 8 * u + gid;
+        const double up = L[c * PLD + kk];
+        mma_884(acc[u], a, kk > c ? up : (kk == c ? dinv[c] : 0.0));
       }
+  }
 #pragma unroll
-      for (int u = 0; u < TR; ++u)
-#pragma unroll
-        for (int v = 0; v < TC; ++v) acc[u][v] += lr[u] * xc[v];
-    }
-#pragma unroll
-    for (int u = 0; u < TR; ++u)
-#pragma unroll
-      for (int v = 0; v < TC; ++v) L[(c0 + v) * PLD + i0 + u] = acc[u][v];
+  for (int u = 0; u < TS; ++u) {
+    L[(b1 + 8 * u + 2 * tig) * PLD + i0 + gid] = acc[u][0];
+    L[(b1 + 8 * u + 2 * tig + 1) * PLD + i0 + gid] = acc[u][1];
+    acc[u][0] = acc[u][1] = 0.0;
   }
   __syncthreads();
-  if (tid < NP * 32) {
-    const int J = tid >> 5, I = J + D, c = 32 * J + (tid & 31), b = 32 * I;
-    double t[32];
+#pragma unroll 2
+  for (int m = b2; m < i0 + 8; m += 4) {                     // X_22[i][m] = 0 for m > i
+    const int mm = m + tig, i = i0 + gid;
+    const double up = L[mm * PLD + i], a = mm < i ? up : (mm == i ? dinv[i] : 0.0);
 #pragma unroll
-    for (int m = 0; m < 32; ++m) t[m] = L[c * PLD + b + m];
+    for (int u = 0; u < TS; ++u) mma_884(acc[u], a, L[(b1 + 8 * u + gid) * PLD + mm]);
+  }
+  __syncthreads();
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      double x0 = dinv[b + i] * t[i], x1 = 0.0;
-#pragma unroll
-      for (int m = 0; m + 1 < i; m += 2) {
-        x0 += L[(b + m) * PLD + b + i] * t[m];
-        x1 += L[(b + m + 1) * PLD + b + i] * t[m + 1];
-      }
-      if (i & 1) x0 += L[(b + i - 1) * PLD + b + i] * t[i - 1];
-      L[c * PLD + b + i] = -(x0 + x1);
-    }
+  for (int u = 0; u < TS; ++u) {
+    L[(b1 + 8 * u + 2 * tig) * PLD + i0 + gid] = -acc[u][0];
+    L[(b1 + 8 * u + 2 * tig + 1) * PLD + i0 + gid] = -acc[u][1];
   }
   __syncthreads();
 }
-constexpr size_t POT_SMEM = sizeof(double) * ((size_t)PT * PLD + PT);   // 130 KB: fits beside a GEMM CTA
+constexpr size_t POT_SMEM = sizeof(double) * ((size_t)PT * PLD + PT);   // 133 KB: fits beside a GEMM CTA
 __global__ void __launch_bounds__(PTHREADS, 1) k_potrf_tile(double *__restrict__ H, int64_t ldh, int64_t k0, int nb,
                                                            double *__restrict__ Linv, int *err) {
   extern __shared__ double L[];                      // [PT][PLD], then dinv[PT]
   double *dinv = L + PT * PLD;
-  __shared__ __align__(16) double colj[32];
   __shared__ int bad;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr unsigned FULL = 0xffffffffu;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gid = lane >> 2, tig = lane & 3;
   if (tid == 0) bad = 0;
   // the lower triangle (16 loads in flight per thread); the identity past nb; zero above
   constexpr int PER = PT * PT / PTHREADS;
@@ -369,126 +434,114 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_potrf_tile(double *__restrict__
     }
   }
   __syncthreads();
-  for (int j0 = 0; j0 < PT; j0 += 32) {
-    // 1. D = L_D L_D^T with row lane of D in lane's registers (loops unrolled: every register
-    //    index is a constant)
-    if (warp == 0) {
-      double a[32];
-      double *row = L + (j0 + lane) * PLD + j0;            // row lane of D
+  constexpr int W = 8;
+  for (int j0 = 0; j0 < PT; j0 += W) {
+    if (tid < PT) {
+      double d[W][W], inv[W];
 #pragma unroll
-      for (int q = 0; q < 32; ++q) a[q] = q <= lane ? row[q] : 0.0;
+      for (int i = 0; i < W; ++i)
+#pragma unroll
+        for (int j = 0; j <= i; ++j) d[i][j] = L[(j0 + i) * PLD + j0 + j];
+      const int r = tid;
+      double a[W];
+      const bool below = r >= j0 + W;
+#pragma unroll
+      for (int j = 0; j < W; j += 2) {
+        const double2 v = *reinterpret_cast<const double2 *>(L + r * PLD + j0 + j);
+        a[j] = v.x;
+        a[j + 1] = v.y;
+      }
       bool lbad = false;
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        double d = __shfl_sync(FULL, a[j], j);
-        if (!(d > 0.0) || !isfinite(d)) {                  // the same d in every lane
+      for (int j = 0; j < W; ++j) {
+        double p = d[j][j];
+        if (!(p > 0.0) || !isfinite(p)) {
           lbad = true;
-          d = 1.0;
+          p = 1.0;
         }
-        const double inv = rsqrt(d), s = d * inv;
-        a[j] = lane == j ? s : (lane > j ? a[j] * inv : 0.0);
-        if (lane == 0) dinv[j0 + j] = inv;
-        const double aj = a[j];
-        colj[lane] = aj;                                   // column j of L_D, read back as a broadcast
-        __syncwarp();
+        inv[j] = rsqrt(p);
+        d[j][j] = p * inv[j];
 #pragma unroll
-        for (int q = j + 1; q < 32; ++q)
-          if (lane >= q) a[q] -= aj * colj[q];             // colj[q] = L[q][j]
-        __syncwarp();                                      // colj is rewritten at the next step
+        for (int i = j + 1; i < W; ++i) d[i][j] *= inv[j];
+        a[j] *= inv[j];
+#pragma unroll
+        for (int q = j + 1; q < W; ++q) {
+#pragma unroll
+          for (int i = q; i < W; ++i) d[i][q] = fma(-d[i][j], d[q][j], d[i][q]);
+          a[q] = fma(-a[j], d[q][j], a[q]);
+        }
+      }
+      if (lbad && tid == 0) bad = 1;
+      asm volatile("bar.sync 1, 128;" ::: "memory");  // every thread has read the diagonal block
+      if (below) {
+#pragma unroll
+        for (int j = 0; j < W; j += 2)
+          *reinterpret_cast<double2 *>(L + r * PLD + j0 + j) = make_double2(a[j], a[j + 1]);
       }
 #pragma unroll
-      for (int q = 0; q < 32; ++q)
-        if (q <= lane) row[q] = a[q];                      // L[lane][q]
-      if (lbad && lane == 0) bad = 1;
-      __syncwarp();
+      for (int i = 0; i < W; ++i)
+        if (r == j0 + i) {
+#pragma unroll
+          for (int j = 0; j <= i; ++j) L[r * PLD + j0 + j] = d[i][j];
+          dinv[j0 + i] = inv[i];
+        }
     }
     __syncthreads();
-    const int t0 = j0 + 32, nr = PT - t0;
-    if (nr == 0) break;
-    // 2. rows below by substitution, one row per thread:
-    //    L[r][j0 + c] = (A[r][j0 + c] - sum_{k<c} L[r][j0 + k] L[j0 + c][j0 + k]) / L[j0 + c][j0 + c]
-    if (tid < nr) {
-      const int r = t0 + tid;
-      double a[32];
+    // the trailing lower triangle [t0, PT): 8 x 8 tiles (ti >= tj), depth 8, four per warp at a time
+    const int t0 = j0 + W, T = (PT - t0) / 8, ntile = T * (T + 1) / 2;
+    int ti = 0, tj = warp;
+    for (int t = warp; t < ntile; t += 32) {
+      double d[4][2], a[4][2], b[4][2];
+      double *cp[4];
 #pragma unroll
-      for (int k = 0; k < 32; ++k) a[k] = L[r * PLD + j0 + k];
+      for (int u = 0; u < 4; ++u) {
+        while (tj > ti) tj -= ++ti;                          // tile number t + 8 u
+        const bool in = t + 8 * u < ntile;
+        const int ra = t0 + 8 * (in ? ti : 0) + gid, ca = t0 + 8 * (in ? tj : 0);
+        cp[u] = L + ra * PLD + ca + 2 * tig;
+        const double2 cv = *reinterpret_cast<const double2 *>(cp[u]);
+        d[u][0] = cv.x;
+        d[u][1] = cv.y;
 #pragma unroll
-      for (int c = 0; c < 32; ++c) {
-        const double l = a[c] * dinv[j0 + c];
-        a[c] = l;
-#pragma unroll
-        for (int q = c + 1; q < 32; ++q) a[q] -= l * L[(j0 + q) * PLD + j0 + c];
-      }
-#pragma unroll
-      for (int k = 0; k < 32; ++k) L[r * PLD + j0 + k] = a[k];
-    }
-    __syncthreads();
-    // 3. trailing lower triangle of rows/columns [t0, PT): 4 x 4 tiles (ti >= tj)
-    {
-      const int T = nr / 4, ntile = T * (T + 1) / 2;
-      for (int t = tid; t < ntile; t += PTHREADS) {
-        int ti = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
-        while (ti * (ti + 1) / 2 > t) --ti;
-        while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
-        const int tj = t - ti * (ti + 1) / 2;
-        const int r0 = t0 + 4 * ti, c0 = t0 + 4 * tj;
-        double acc[4][4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-          for (int v = 0; v < 4; ++v) acc[u][v] = 0.0;
-#pragma unroll 8
-        for (int q = 0; q < 32; ++q) {
-          double lr[4], lc[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            lr[u] = L[(r0 + u) * PLD + j0 + q];
-            lc[u] = L[(c0 + u) * PLD + j0 + q];
-          }
-#pragma unroll
-          for (int u = 0; u < 4; ++u)
-#pragma unroll
-            for (int v = 0; v < 4; ++v) acc[u][v] += lr[u] * lc[v];
+        for (int h = 0; h < 2; ++h) {
+          a[u][h] = -L[ra * PLD + j0 + 4 * h + tig];
+          b[u][h] = L[(ca + gid) * PLD + j0 + 4 * h + tig];
         }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-          for (int v = 0; v < 4; ++v)
-            if (c0 + v <= r0 + u) L[(r0 + u) * PLD + c0 + v] -= acc[u][v];
+        tj += 8;
       }
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) mma_884(d[u], a[u][h], b[u][h]);
+      // (diagonal tiles: the entries above the diagonal are free until the inverse is built)
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (t + 8 * u < ntile) *reinterpret_cast<double2 *>(cp[u]) = make_double2(d[u][0], d[u][1]);
     }
     __syncthreads();
   }
-  // the four 32 x 32 diagonal inverses X_II, warp I each
-  if (warp < 4) {
-    const int j0 = 32 * warp;
-    double *row = L + (j0 + lane) * PLD + j0;
-    // column c = lane of X_D: X[i][c] = (delta_ic - sum_{m<i} L[i][m] X[m][c]) / L[i][i]
-    // (X[m][c] = 0 for m < c; two partial sums halve the dependent chain), kept at [c][i]
-    double x[32];
+  if (bad && tid == 0) atomicOr(err, 1);
+  // the 8 x 8 diagonal inverses: column c of its block per thread,
+  // X[i][c] = (delta_ic - sum_{m<i} L[i][m] X[m][c]) / L[i][i]
+  if (tid < PT) {
+    const int b = tid & ~(W - 1), c = tid & (W - 1);
+    double x[W];
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      const double *li = L + (j0 + i) * PLD + j0;
-      double t0 = i == lane ? 1.0 : 0.0, t1 = 0.0;
+    for (int i = 0; i < W; ++i) {
+      double t = i == c ? 1.0 : 0.0;
 #pragma unroll
-      for (int m = 0; m + 1 < i; m += 2) {
-        t0 -= li[m] * x[m];
-        t1 -= li[m + 1] * x[m + 1];
-      }
-      if (i & 1) t0 -= li[i - 1] * x[i - 1];
-      x[i] = i >= lane ? (t0 + t1) * dinv[j0 + i] : 0.0;
+      for (int m = 0; m < i; ++m) t = fma(-L[(b + i) * PLD + b + m], x[m], t);
+      x[i] = i >= c ? t * dinv[b + i] : 0.0;
     }
 #pragma unroll
-    for (int i = 0; i < 32; ++i)
-      if (i > lane) row[i] = x[i];
+    for (int i = 0; i < W; ++i)
+      if (i > c) L[tid * PLD + b + i] = x[i];
   }
   __syncthreads();
-  if (bad && tid == 0) atomicOr(err, 1);
-  // the off-diagonal blocks of X by distance D = I - J (level D reads only the diagonal inverses
-  // and the levels below it)
-  inv_level<1, 4, 4>(L, dinv);
-  inv_level<2, 4, 2>(L, dinv);
-  inv_level<3, 2, 2>(L, dinv);
+  join_inverse<8>(L, dinv);
+  join_inverse<16>(L, dinv);
+  join_inverse<32>(L, dinv);
+  join_inverse<64>(L, dinv);
   // L back to H, inv(L) to Linv
 #pragma unroll 16
   for (int u = 0; u < PER; ++u) {
@@ -496,10 +549,11 @@ __global__ void __launch_bounds__(PTHREADS, 1) k_potrf_tile(double *__restrict__
     if (r < nb && c <= r) H[(k0 + r) * ldh + k0 + c] = L[r * PLD + c];
   }
   if (nb == PT) {
+    // (lanes 8 columns x 4 rows: the transposed reads meet two to a bank)
 #pragma unroll 16
     for (int u = 0; u < PER; ++u) {
-      const int e = tid + u * PTHREADS, i = e >> 7, c = e & (PT - 1);
-      Linv[e] = c > i ? 0.0 : (c == i ? dinv[i] : L[c * PLD + i]);
+      const int q = warp + 8 * u, i = 4 * (q >> 4) + (lane >> 3), c = 8 * (q & 15) + (lane & 7);
+      Linv[i * PT + c] = c > i ? 0.0 : (c == i ? dinv[i] : L[c * PLD + i]);
     }
   } else {
     for (int e = tid; e < nb * nb; e += PTHREADS) {
@@ -854,6 +908,27 @@ int gemm_nt(const Gemm &g, cudaStream_t st) {
   return a16 ? gemm_launch<16, 64, false>(g, st) : gemm_launch<8, 64, false>(g, st);
 }
 
+// Outer panel width, the depth of the trailing updates.  Wide panels make those GEMMs deep, narrow
+// ones shorten the chain in front of each.  384 / 512 / 768 / 1024 / 1536 / 2048 columns, ms:
+// n = 3,333: 4.8 / 4.7 / 4.7 / 4.7 / 5.1 / 4.8; n = 10,240: 19.0 / 18.6 / 18.4 / 18.3 / 19.4 / 19.6;
+// n = 22,971: 153 / 149 / 144 / 142 / 141 / 142.  Up to 1536 one panel is the whole matrix.
+int64_t outer_width(int64_t n) { return n <= 1536 || n >= 16384 ? 1536 : 1024; }
+
+// a launch of the strip kernel; 16-byte copies when every row start is 16-byte aligned
+template <bool UPD> int strip_launch(const Strip &g, cudaStream_t st) {
+  const bool a16 = ((uintptr_t)g.A % 16 == 0) && ((uintptr_t)g.B % 16 == 0) && g.lda % 2 == 0 && g.ldb % 2 == 0;
+  const unsigned grid = (unsigned)ceil_div(g.M, SR);
+  if (a16) {
+    DGP_TRY(allow_dyn_smem(k_strip<16, UPD>, STRIP_SMEM));
+    k_strip<16, UPD><<<grid, 256, STRIP_SMEM, st>>>(g);
+  } else {
+    DGP_TRY(allow_dyn_smem(k_strip<8, UPD>, STRIP_SMEM));
+    k_strip<8, UPD><<<grid, 256, STRIP_SMEM, st>>>(g);
+  }
+  DGP_CHECK_LAUNCH();
+  return DGP_OK;
+}
+
 // The four streams and eight events of the lookahead; the destructor waits for every stream, so
 // that an early error return never frees buffers that queued kernels still use.
 struct LookaheadStreams {
@@ -889,7 +964,7 @@ int cholesky_solve_many_run(double *H, int64_t n, int64_t ldh, double *x, int32_
   DGP_REQUIRE(nrhs >= 1 && ldx >= n, "cholesky: need nrhs >= 1 and ldx >= n");
   DGP_REQUIRE(nrhs <= 65535, "cholesky: at most 65535 right-hand sides");
   DGP_REQUIRE(ceil_div(n, (int64_t)GVB) <= INT32_MAX, "cholesky: n too large for the solve grid");
-  const int64_t nblk = ceil_div(n, CB);
+  const int64_t nblk = ceil_div(n, CB), NBO = outer_width(n);
   DevBuf linv, errb, acc, flags;
   DGP_TRY(linv.alloc(sizeof(double) * (size_t)nblk * CB * CB));
   DGP_TRY(errb.alloc(sizeof(int)));
@@ -968,18 +1043,16 @@ int cholesky_solve_many_run(double *H, int64_t n, int64_t ldh, double *x, int32_
         side_pending = false;
       }
       // L_ik = A_ik inv(L_kk)^T for the outer panel's rows below the block (in place, one CTA per
-      // 128-row strip)
-      const Gemm p{H + kend * ldh + k0, ldh, Lb, nb, H + kend * ldh + k0, ldh, w, nb, nb, 1.0, 0.0, 0, 0};
-      DGP_TRY(gemm_nt(p, sf));
+      // 32-row strip)
+      double *below_rows = H + kend * ldh + k0;
+      DGP_TRY(strip_launch<false>(Strip{below_rows, ldh, Lb, CB, nullptr, (int)w, CB}, sf));
       ++launches;
       // the next diagonal block's update, then its factorisation at once on sf; the rest of the
       // step's update of the outer panel's remaining columns on ss beside it
       const int nb2 = (int)std::min<int64_t>(CB, w);
       const int64_t k2 = kend + nb2, w2 = oend - k2;
       DGP_CUDA(cudaEventRecord(ls.step, sf));
-      const Gemm a1{H + kend * ldh + k0, ldh, H + kend * ldh + k0, ldh, H + kend * ldh + kend, ldh, nb2, nb2, nb,
-                    -1.0, 1.0, 1, 0};
-      DGP_TRY(gemm_nt(a1, sf));
+      DGP_TRY(strip_launch<true>(Strip{below_rows, ldh, below_rows, ldh, H + kend * ldh + kend, nb2, nb2}, sf));
       k_potrf_tile<<<1, PTHREADS, pot_smem, sf>>>(H, ldh, kend, nb2, Li + (b + 1) * CB * CB, errb.as<int>());
       DGP_CHECK_LAUNCH();
       launches += 2;

@@ -182,18 +182,107 @@ __global__ void __launch_bounds__(128, 1) k_syrk_tc(const __grid_constant__ CUte
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TN) : "memory");
 }
 
-// Js = sqrt(W) Jt split into bf16 hi + lo, zero-padded to [nvp][nmp]; exact
-// FP64 diagonal d[v] = sum_m W_m Jt[v][m]^2
-__global__ void k_split(const float *__restrict__ Jt, const double *__restrict__ W, int64_t nv, int64_t nm,
-                        int64_t nvp, int64_t nmp, __nv_bfloat16 *hi, __nv_bfloat16 *lo) {
-  int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= nvp * nmp) return;
-  int64_t v = t / nmp, m = t % nmp;
-  float x = 0.f;
-  if (v < nv && m < nm) x = Jt[v * nm + m] * (W ? (float)sqrt(W[m]) : 1.f);
-  __nv_bfloat16 h = __float2bfloat16_rn(x);
-  hi[t] = h;
-  lo[t] = __float2bfloat16_rn(x - __bfloat162float(h));
+// bf16 hi + lo of x
+__device__ inline void split_bf16(float x, __nv_bfloat16 &h, __nv_bfloat16 &l) {
+  h = __float2bfloat16_rn(x);
+  l = __float2bfloat16_rn(x - __bfloat162float(h));
+}
+
+// sw[m] = (float)sqrt(W[m]) (1 without weights): the square root once per measurement, not per entry
+__global__ void k_sqrt_weights(const double *__restrict__ W, int64_t nm, float *sw) {
+  const int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (m < nm) sw[m] = W ? (float)sqrt(W[m]) : 1.f;
+}
+
+// Js = sqrt(W) Jt split into bf16 hi + lo, zero-padded to [nvp][nmp] (nmp a multiple of 64).  HBM
+// bound (4 bytes in, 4 out per entry): 8 entries per thread, 16-byte stores; VECIN: 16-byte loads
+// (rows 16-byte aligned).  One entry per thread with an FP64 square root each: 0.91 ms at
+// 10,240 x 22,971; now 0.31.
+template <bool VECIN>
+__global__ void __launch_bounds__(256) k_split(const float *__restrict__ Jt, const float *__restrict__ sw, int64_t nv,
+                                               int64_t nm, int64_t nmp, __nv_bfloat16 *hi, __nv_bfloat16 *lo) {
+  const int64_t v = blockIdx.y;
+  const int64_t m0 = (blockIdx.x * (int64_t)256 + threadIdx.x) * 8;
+  if (m0 >= nmp) return;
+  float x[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) x[u] = 0.f;
+  if (v < nv) {
+    const float *row = Jt + v * nm;
+    if (VECIN && m0 + 8 <= nm) {
+#pragma unroll
+      for (int u = 0; u < 8; u += 4) {
+        const float4 a = __ldg(reinterpret_cast<const float4 *>(row + m0 + u));
+        const float4 b = __ldg(reinterpret_cast<const float4 *>(sw + m0 + u));
+        x[u] = a.x * b.x;
+        x[u + 1] = a.y * b.y;
+        x[u + 2] = a.z * b.z;
+        x[u + 3] = a.w * b.w;
+      }
+    } else {
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (m0 + u < nm) x[u] = row[m0 + u] * sw[m0 + u];
+    }
+  }
+  __align__(16) __nv_bfloat16 h[8], l[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) split_bf16(x[u], h[u], l[u]);
+  *reinterpret_cast<uint4 *>(hi + v * nmp + m0) = *reinterpret_cast<const uint4 *>(h);
+  *reinterpret_cast<uint4 *>(lo + v * nmp + m0) = *reinterpret_cast<const uint4 *>(l);
+}
+
+// J_w = W^1/2 J, i.e. Jt transposed and scaled, split into bf16 hi + lo [nmp][nvp] (both multiples
+// of 64, zero past nm and nv), with the FP64 partial sums of each J_w row's squares over a block's
+// 64 unknowns in part [nvp / 64][nmp].  One read of Jt instead of a transpose to FP32, its split and
+// its row norms (0.73 + 0.91 + 0.23 ms at 10,240 x 22,971; now 0.36).
+__global__ void __launch_bounds__(256) k_split_transposed(const float *__restrict__ Jt, const float *__restrict__ sw,
+                                                          int64_t nv, int64_t nm, int64_t nvp, int64_t nmp,
+                                                          __nv_bfloat16 *hi, __nv_bfloat16 *lo, double *part) {
+  __shared__ float t[64][65];                                  // [unknown][measurement]
+  const int64_t m0 = (int64_t)blockIdx.x * 64, v0 = (int64_t)blockIdx.y * 64;
+  const int tid = threadIdx.x;
+#pragma unroll 4
+  for (int e = tid; e < 64 * 64; e += 256) {
+    const int r = e >> 6, c = e & 63;
+    const int64_t v = v0 + r, m = m0 + c;
+    t[r][c] = v < nv && m < nm ? __ldg(Jt + v * nm + m) * __ldg(sw + m) : 0.f;
+  }
+  __syncthreads();
+  // four threads per measurement row, 16 unknowns each: 32-byte runs of hi and lo
+  const int r = tid >> 2, c0 = (tid & 3) * 16;
+  __align__(16) __nv_bfloat16 h[16], l[16];
+  double s = 0.0;
+#pragma unroll
+  for (int u = 0; u < 16; ++u) {
+    const float x = t[c0 + u][r];
+    split_bf16(x, h[u], l[u]);
+    s = fma((double)x, (double)x, s);
+  }
+  const int64_t o = (m0 + r) * nvp + v0 + c0;
+#pragma unroll
+  for (int u = 0; u < 16; u += 8) {
+    *reinterpret_cast<uint4 *>(hi + o + u) = *reinterpret_cast<const uint4 *>(h + u);
+    *reinterpret_cast<uint4 *>(lo + o + u) = *reinterpret_cast<const uint4 *>(l + u);
+  }
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  if ((tid & 3) == 0) part[(int64_t)blockIdx.y * nmp + m0 + r] = s;
+}
+// diag[m] = sum over the blocks' partial sums, 8 threads per measurement in a fixed order
+__global__ void __launch_bounds__(256) k_sum_parts(const double *__restrict__ part, int64_t nblk, int64_t nmp,
+                                                   int64_t nm, double *diag) {
+  __shared__ double t[8][32];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  const int64_t m = blockIdx.x * (int64_t)32 + x;
+  double s = 0.0;
+  if (m < nm) {
+#pragma unroll 8
+    for (int64_t b = y; b < nblk; b += 8) s += part[b * nmp + m];
+  }
+  t[y][x] = s;
+  __syncthreads();
+  if (y == 0 && m < nm) diag[m] = ((t[0][x] + t[1][x]) + (t[2][x] + t[3][x])) + ((t[4][x] + t[5][x]) + (t[6][x] + t[7][x]));
 }
 
 __global__ void k_check_weights(const double *__restrict__ W, int64_t nm, int *err) {
@@ -201,8 +290,9 @@ __global__ void k_check_weights(const double *__restrict__ W, int64_t nm, int *e
   if (m < nm && !(W[m] >= 0.0 && isfinite(W[m]))) atomicOr(err, 16);
 }
 
+// diag[v] = sum_m W_m J_mv^2, rhs[v] = sum_m W_m J_mv y_m (FP64); dmax (zeroed): the largest diag
 __global__ void k_row_dots(const float *__restrict__ Jt, const double *__restrict__ W, const double *__restrict__ y,
-                           int64_t nv, int64_t nm, double *diag, double *rhs) {
+                           int64_t nv, int64_t nm, double *diag, double *rhs, double *dmax) {
   __shared__ double sd[256], sr[256];
   for (int64_t v = blockIdx.x; v < nv; v += gridDim.x) {
     double d = 0, r = 0;
@@ -224,22 +314,19 @@ __global__ void k_row_dots(const float *__restrict__ Jt, const double *__restric
     if (threadIdx.x == 0) {
       diag[v] = sd[0];
       if (rhs) rhs[v] = sr[0];
+      // (non-negative doubles order like their bits; a NaN does not enter the maximum)
+      if (dmax && sd[0] > 0.0)
+        atomicMax((unsigned long long *)dmax, (unsigned long long)__double_as_longlong(sd[0]));
     }
     __syncthreads();
   }
 }
 
-// H_ii = d_i + lam * (mode 0: max_j d_j, the tik_inv rule; mode 1: d_i; mode 2: 1)
-__global__ void k_damp(double *H, int64_t ldh, const double *__restrict__ diag, int64_t nv, double lam, int mode) {
-  __shared__ double smax;
-  if (threadIdx.x == 0) {
-    double m = 0;
-    for (int64_t i = 0; i < nv; ++i) m = fmax(m, diag[i]);
-    smax = m;
-  }
-  __syncthreads();
-  for (int64_t i = threadIdx.x; i < nv; i += blockDim.x)
-    H[i * ldh + i] = diag[i] + lam * (mode == 0 ? smax : mode == 1 ? diag[i] : 1.0);
+// H_ii = d_i + lam * (mode 0: dmax, the tik_inv rule; mode 1: d_i; mode 2: 1)
+__global__ void k_damp(double *H, int64_t ldh, const double *__restrict__ diag, int64_t nv, double lam, int mode,
+                       const double *__restrict__ dmax) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < nv) H[i * ldh + i] = diag[i] + lam * (mode == 0 ? *dmax : mode == 1 ? diag[i] : 1.0);
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 get_encode() {
@@ -282,6 +369,28 @@ int check_weights(const double *W, int64_t nm, int *errb, const char *who, cudaS
 
 }  // namespace
 
+namespace {
+// H (lower triangle) = (hi + lo)(hi + lo)^T without lo lo^T, operands [np][kp]; then the damped diagonal
+int gram_split(const __nv_bfloat16 *hi, const __nv_bfloat16 *lo, int64_t n, int64_t np, int64_t kp, double *H,
+               int64_t ldh, const double *diag, double lam, int mode, const double *dmax, int *errb, cudaStream_t st) {
+  CUtensorMap mhi, mlo;
+  DGP_TRY(make_map(&mhi, (void *)hi, np, kp));
+  DGP_TRY(make_map(&mlo, (void *)lo, np, kp));
+  DGP_TRY(allow_dyn_smem(k_syrk_tc, SYRK_SMEM));
+  const int64_t T = np / TM;
+  k_syrk_tc<<<(unsigned)(T * (T + 1) / 2), 128, SYRK_SMEM, st>>>(mhi, mlo, (int)(kp / TK), n, H, ldh, errb);
+  DGP_CHECK_LAUNCH();
+  k_damp<<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(H, ldh, diag, n, lam, mode, dmax);
+  DGP_CHECK_LAUNCH();
+  int herr = 0;
+  DGP_CUDA(cudaMemcpyAsync(&herr, errb, sizeof(int), cudaMemcpyDeviceToHost, st));
+  DGP_CUDA(cudaStreamSynchronize(st));
+  if (herr) return fail(DGP_ERR_CUDA, "normal_eq: tensor-core pipeline wait timed out (error flags " +
+                                          std::to_string(herr) + ")");
+  return DGP_OK;
+}
+}  // namespace
+
 int normal_eq_run(const float *Jt, int64_t nv, int64_t nm, const double *W, const double *y, double lam, int mode,
                   double *H, int64_t ldh, double *rhs, cudaStream_t st) {
   DGP_REQUIRE(Jt && H, "normal_eq: null pointer");
@@ -290,54 +399,34 @@ int normal_eq_run(const float *Jt, int64_t nv, int64_t nm, const double *W, cons
               "normal_eq: damping mode is 0 (lam*max diag), 1 (lam*diag) or 2 (lam)");
   const int64_t nvp = ceil_div(nv, TM) * TM, nmp = ceil_div(nm, TK) * TK;
   DGP_REQUIRE(nmp < (int64_t)INT32_MAX && nvp < (int64_t)INT32_MAX, "normal_eq: sizes exceed TMA coordinates");
-  DevBuf hi, lo, diag, errb;
+  DevBuf hi, lo, diag, errb, sw;
   DGP_TRY(hi.alloc(sizeof(__nv_bfloat16) * (size_t)nvp * nmp));
   DGP_TRY(lo.alloc(sizeof(__nv_bfloat16) * (size_t)nvp * nmp));
-  DGP_TRY(diag.alloc(sizeof(double) * nv));
+  DGP_TRY(diag.alloc(sizeof(double) * (nv + 1)));
+  DGP_TRY(sw.alloc(sizeof(float) * nmp));
   DGP_TRY(errb.alloc(sizeof(int)));
+  double *dmax = diag.as<double>() + nv;
   DGP_CUDA(cudaMemsetAsync(errb.p, 0, sizeof(int), st));
+  DGP_CUDA(cudaMemsetAsync(dmax, 0, sizeof(double), st));
   if (W) DGP_TRY(check_weights(W, nm, errb.as<int>(), "normal_eq", st));
-  k_split<<<(unsigned)ceil_div(nvp * nmp, 256), 256, 0, st>>>(Jt, W, nv, nm, nvp, nmp, hi.as<__nv_bfloat16>(),
-                                                               lo.as<__nv_bfloat16>());
+  k_sqrt_weights<<<(unsigned)ceil_div(nm, 256), 256, 0, st>>>(W, nm, sw.as<float>());
   DGP_CHECK_LAUNCH();
-  k_row_dots<<<(unsigned)std::min<int64_t>(nv, 4096), 256, 0, st>>>(Jt, W, y, nv, nm, diag.as<double>(), rhs);
+  const bool vecin = (uintptr_t)Jt % 16 == 0 && nm % 4 == 0;
+  for (int64_t v0 = 0; v0 < nvp; v0 += 65535) {  // (grid rows)
+    const dim3 g((unsigned)ceil_div(nmp, 2048), (unsigned)std::min<int64_t>(65535, nvp - v0));
+    __nv_bfloat16 *h = hi.as<__nv_bfloat16>() + v0 * nmp, *l = lo.as<__nv_bfloat16>() + v0 * nmp;
+    if (vecin) k_split<true><<<g, 256, 0, st>>>(Jt + v0 * nm, sw.as<float>(), nv - v0, nm, nmp, h, l);
+    else k_split<false><<<g, 256, 0, st>>>(Jt + v0 * nm, sw.as<float>(), nv - v0, nm, nmp, h, l);
+    DGP_CHECK_LAUNCH();
+  }
+  k_row_dots<<<(unsigned)std::min<int64_t>(nv, 4096), 256, 0, st>>>(Jt, W, y, nv, nm, diag.as<double>(), rhs, dmax);
   DGP_CHECK_LAUNCH();
-  CUtensorMap mhi, mlo;
-  DGP_TRY(make_map(&mhi, hi.p, nvp, nmp));
-  DGP_TRY(make_map(&mlo, lo.p, nvp, nmp));
-  DGP_CUDA(cudaFuncSetAttribute(k_syrk_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, SYRK_SMEM));
-  const int64_t T = nvp / TM;
-  const int64_t tiles = T * (T + 1) / 2;
-  k_syrk_tc<<<(unsigned)tiles, 128, SYRK_SMEM, st>>>(mhi, mlo, (int)(nmp / TK), nv, H, ldh, errb.as<int>());
-  DGP_CHECK_LAUNCH();
-  k_damp<<<1, 256, 0, st>>>(H, ldh, diag.as<double>(), nv, lam, mode);
-  DGP_CHECK_LAUNCH();
-  int herr = 0;
-  DGP_CUDA(cudaMemcpyAsync(&herr, errb.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-  DGP_CUDA(cudaStreamSynchronize(st));
-  if (herr) return fail(DGP_ERR_CUDA, "normal_eq: tensor-core pipeline wait timed out (error flags " +
-                                          std::to_string(herr) + ")");
-  return DGP_OK;
+  return gram_split(hi.as<__nv_bfloat16>(), lo.as<__nv_bfloat16>(), nv, nvp, nmp, H, ldh, diag.as<double>(), lam, mode,
+                    dmax, errb.as<int>(), st);
 }
 
 // ----------------------------------------------------- tik_inv update
 namespace {
-
-// Jw[m][v] = sqrt(W[m]) Jt[v][m]: 32 x 32 tiles through shared memory
-__global__ void k_scale_transpose(const float *__restrict__ Jt, const double *__restrict__ W, int64_t nv, int64_t nm,
-                                  float *__restrict__ Jw) {
-  __shared__ float t[32][33];
-  const int64_t v0 = (int64_t)blockIdx.y * 32, m0 = (int64_t)blockIdx.x * 32;
-  for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-    const int64_t v = v0 + r, m = m0 + threadIdx.x;
-    t[r][threadIdx.x] = (v < nv && m < nm) ? Jt[v * nm + m] : 0.f;
-  }
-  __syncthreads();
-  for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-    const int64_t m = m0 + r, v = v0 + threadIdx.x;
-    if (m < nm && v < nv) Jw[m * nv + v] = (W ? (float)sqrt(W[m]) : 1.f) * t[threadIdx.x][r];
-  }
-}
 
 // out[m] = sqrt(W[m]) in[m]
 __global__ void k_scale_sqrtw(const double *in, const double *__restrict__ W, int64_t nm, double *out) {
@@ -391,7 +480,7 @@ int times_jt_run(const double *A, int64_t na, int64_t nv, const float *Jt, int64
 int row_dots_run(const float *Jt, int64_t nv, int64_t nm, const double *W, const double *y, double *diag, double *rhs,
                  cudaStream_t st) {
   DGP_REQUIRE(Jt && diag && nv > 0 && nm > 0, "row_dots: bad arguments");
-  k_row_dots<<<(unsigned)std::min<int64_t>(nv, 4096), 256, 0, st>>>(Jt, W, y, nv, nm, diag, rhs);
+  k_row_dots<<<(unsigned)std::min<int64_t>(nv, 4096), 256, 0, st>>>(Jt, W, y, nv, nm, diag, rhs, nullptr);
   DGP_CHECK_LAUNCH();
   return DGP_OK;
 }
@@ -415,30 +504,38 @@ int lm_update_run(const float *Jt, int64_t nv, int64_t nm, const double *W, cons
     DGP_TRY(normal_eq_run(Jt, nv, nm, W, y, lam, 0, H.as<double>(), ldh, x, st));
     return cholesky_solve_run(H.as<double>(), nv, ldh, x, st);
   }
-  DevBuf diag, Jw, G, z, errb;
-  if (W) {
-    DGP_TRY(errb.alloc(sizeof(int)));
-    DGP_CUDA(cudaMemsetAsync(errb.p, 0, sizeof(int), st));
-    DGP_TRY(check_weights(W, nm, errb.as<int>(), "lm_update", st));
-  }
-  DGP_TRY(diag.alloc(sizeof(double) * nv));
-  DGP_TRY(Jw.alloc(sizeof(float) * (size_t)nm * nv));
+  const int64_t nmp = ceil_div(nm, TM) * TM, nvp = ceil_div(nv, TK) * TK;
+  DGP_REQUIRE(nmp < (int64_t)INT32_MAX && nvp < (int64_t)INT32_MAX, "lm_update: sizes exceed TMA coordinates");
+  DGP_REQUIRE(nvp / 64 <= 65535, "lm_update: too many unknowns for the transpose grid");
+  DevBuf diag, hi, lo, G, z, errb, sw, part;
+  DGP_TRY(errb.alloc(sizeof(int)));
+  DGP_CUDA(cudaMemsetAsync(errb.p, 0, sizeof(int), st));
+  if (W) DGP_TRY(check_weights(W, nm, errb.as<int>(), "lm_update", st));
+  const int64_t nd = std::max(nv, nm);
+  DGP_TRY(diag.alloc(sizeof(double) * (nd + 1)));
+  DGP_TRY(hi.alloc(sizeof(__nv_bfloat16) * (size_t)nmp * nvp));
+  DGP_TRY(lo.alloc(sizeof(__nv_bfloat16) * (size_t)nmp * nvp));
+  DGP_TRY(part.alloc(sizeof(double) * (size_t)(nvp / 64) * nmp));
+  DGP_TRY(sw.alloc(sizeof(float) * nmp));
   const int64_t ldg = nm + (nm & 1);
   DGP_TRY(G.alloc(sizeof(double) * (size_t)nm * ldg));
   DGP_TRY(z.alloc(sizeof(double) * nm));
-  DGP_TRY(row_dots_run(Jt, nv, nm, W, nullptr, diag.as<double>(), nullptr, st));
-  std::vector<double> hd((size_t)nv);
-  DGP_CUDA(cudaMemcpyAsync(hd.data(), diag.p, sizeof(double) * nv, cudaMemcpyDeviceToHost, st));
-  DGP_CUDA(cudaStreamSynchronize(st));
-  double dmax = 0.0;
-  for (double d : hd) dmax = std::max(dmax, d);
-  const double mu = lam * dmax;
-  dim3 tb(32, 8), tg((unsigned)ceil_div(nm, 32), (unsigned)ceil_div(nv, 32));
-  DGP_REQUIRE(tg.y <= 65535u, "lm_update: too many unknowns for the transpose grid");
-  k_scale_transpose<<<tg, tb, 0, st>>>(Jt, W, nv, nm, Jw.as<float>());
+  double *dmax = diag.as<double>() + nd;
+  DGP_CUDA(cudaMemsetAsync(dmax, 0, sizeof(double), st));
+  // mu = lam max_i (J^T W J)_ii
+  k_row_dots<<<(unsigned)std::min<int64_t>(nv, 4096), 256, 0, st>>>(Jt, W, nullptr, nv, nm, diag.as<double>(), nullptr,
+                                                                    dmax);
+  DGP_CHECK_LAUNCH();
+  k_sqrt_weights<<<(unsigned)ceil_div(nm, 256), 256, 0, st>>>(W, nm, sw.as<float>());
+  DGP_CHECK_LAUNCH();
+  k_split_transposed<<<dim3((unsigned)(nmp / 64), (unsigned)(nvp / 64)), 256, 0, st>>>(
+      Jt, sw.as<float>(), nv, nm, nvp, nmp, hi.as<__nv_bfloat16>(), lo.as<__nv_bfloat16>(), part.as<double>());
+  DGP_CHECK_LAUNCH();
+  k_sum_parts<<<(unsigned)ceil_div(nm, 32), 256, 0, st>>>(part.as<double>(), nvp / 64, nmp, nm, diag.as<double>());
   DGP_CHECK_LAUNCH();
   // G = J_w J_w^T + mu I: the split-BF16 Gram kernel on J_w (rows = measurements)
-  DGP_TRY(normal_eq_run(Jw.as<float>(), nm, nv, nullptr, nullptr, mu, 2, G.as<double>(), ldg, nullptr, st));
+  DGP_TRY(gram_split(hi.as<__nv_bfloat16>(), lo.as<__nv_bfloat16>(), nm, nmp, nvp, G.as<double>(), ldg,
+                     diag.as<double>(), lam, 0, dmax, errb.as<int>(), st));
   k_scale_sqrtw<<<(unsigned)ceil_div(nm, 256), 256, 0, st>>>(y, W, nm, z.as<double>());
   DGP_CHECK_LAUNCH();
   DGP_TRY(cholesky_solve_run(G.as<double>(), nm, ldg, z.as<double>(), st));
