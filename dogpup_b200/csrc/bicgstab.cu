@@ -1689,9 +1689,9 @@ int tiled_build(TiledPlan *T, const int32_t *d_rowptr, const int32_t *d_col, int
   T->nblk = nblk;
   T->hmax = hmax;
   T->zmax = zmax;
-  DGP_TRY(T->hptr.alloc(sizeof(int32_t) * hptr.size()));
-  DGP_TRY(T->hcols.alloc(sizeof(int32_t) * std::max<size_t>(1, hcols.size())));
-  DGP_TRY(T->lcol.alloc(sizeof(int32_t) * std::max<int64_t>(1, nnz)));
+  DGP_TRY(T->hptr.alloc_plan(sizeof(int32_t) * hptr.size()));
+  DGP_TRY(T->hcols.alloc_plan(sizeof(int32_t) * std::max<size_t>(1, hcols.size())));
+  DGP_TRY(T->lcol.alloc_plan(sizeof(int32_t) * std::max<int64_t>(1, nnz)));
   DGP_CUDA(cudaMemcpyAsync(T->hptr.p, hptr.data(), sizeof(int32_t) * hptr.size(), cudaMemcpyHostToDevice, st));
   DGP_CUDA(cudaMemcpyAsync(T->hcols.p, hcols.data(), sizeof(int32_t) * hcols.size(), cudaMemcpyHostToDevice, st));
   DGP_CUDA(cudaMemcpyAsync(T->lcol.p, lcol.data(), sizeof(int32_t) * nnz, cudaMemcpyHostToDevice, st));
@@ -1748,8 +1748,17 @@ void tspmm(const SolverPlan *S, int what, const float2 *X, float2 *Y, const floa
   }
 }
 
-// builds the three halo plans and sets the kernels' shared-memory limits; tiled_ok = 1 when they fit
+// rec[t].pad = lcol[t % nnz]: the halo positions the tiled SpMM reads
+__global__ void k_set_halo(Rec32 *rec, const int32_t *__restrict__ lcol, int64_t nnz, int64_t tot) {
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (t < tot) rec[t].pad = __int_as_float(lcol[t % nnz]);
+}
+
+// builds the three halo plans and sets the kernels' shared-memory limits; tiled_ok = 1 when they
+// fit.  Done when the tiled SpMM is first asked for: the halo lists are sorted on the host from
+// copies of the patterns, which was most of a plan's creation time.
 int tiled_setup(SolverPlan *S, cudaStream_t st) {
+  if (S->tiled_built) return DGP_OK;
   DGP_TRY(tiled_build(&S->tA, S->rowptr.as<int32_t>(), S->col.as<int32_t>(), S->n, S->nnz, TILE_RB, st));
   DGP_TRY(tiled_build(&S->tG, S->P.rowptr.as<int32_t>(), S->P.col.as<int32_t>(), S->n, S->nnzG, TILE_RB, st));
   DGP_TRY(tiled_build(&S->tGT, S->P.rowptrT.as<int32_t>(), S->P.colT.as<int32_t>(), S->n, S->nnzG, TILE_RB, st));
@@ -1757,8 +1766,15 @@ int tiled_setup(SolverPlan *S, cudaStream_t st) {
   size_t need = 0;
   for (const TiledPlan *T : {&S->tA, &S->tG, &S->tGT})
     for (int m = 0; m < 3; ++m) need = std::max(need, tile_smem(*T, sw, m));
+  S->tiled_built = 1;
   S->tiled_ok = need <= TILE_SMEM_MAX && S->nsp % sw == 0;
   if (!S->tiled_ok) return DGP_OK;
+  const int64_t ng = S->nnzG * S->nf;
+  k_set_halo<<<g1(S->nnz, 256), 256, 0, st>>>(S->RecA32.as<Rec32>(), S->tA.lcol.as<int32_t>(), S->nnz, S->nnz);
+  k_set_halo<<<g1(ng, 256), 256, 0, st>>>(S->RecG32.as<Rec32>(), S->tG.lcol.as<int32_t>(), S->nnzG, ng);
+  k_set_halo<<<g1(ng, 256), 256, 0, st>>>(S->RecGT32.as<Rec32>(), S->tGT.lcol.as<int32_t>(), S->nnzG, ng);
+  count_launches(2);
+  DGP_CHECK_LAUNCH();
   auto attrs = [&](auto w) {
     constexpr int W_ = decltype(w)::value;
     int rc = tspmm_attrs<W_, OpA32>({&S->tA});
@@ -1839,15 +1855,16 @@ int ensure_workspace(SolverPlan *S, int prec, int nvec = NVEC_ALL) {
       }
     for (int &gi : S->graph_iters) gi = 0;
     for (auto &v : S->vec) v.release();
-    DGP_TRY(S->scal.alloc(scal_bytes(C)));
-    DGP_TRY(S->status.alloc(sizeof(int) * C));
-    DGP_TRY(S->ctl.alloc(sizeof(Ctl)));
-    DGP_CUDA(cudaMemset(S->scal.p, 0, scal_bytes(C)));
+    DGP_TRY(S->scal.alloc_plan(scal_bytes(C)));
+    DGP_TRY(S->status.alloc_plan(sizeof(int) * C));
+    DGP_TRY(S->ctl.alloc_plan(sizeof(Ctl)));
+    DGP_CUDA(cudaMemsetAsync(S->scal.p, 0, scal_bytes(C), cudaStreamPerThread));
+    DGP_CUDA(cudaStreamSynchronize(cudaStreamPerThread));
     S->ws_prec = prec;
     S->ws_cols = C;
   }
   for (int q = 0; q < nvec; ++q)
-    if (!S->vec[q].p) DGP_TRY(S->vec[q].alloc(vb));
+    if (!S->vec[q].p) DGP_TRY(S->vec[q].alloc_plan(vb));
   return DGP_OK;
 }
 
@@ -2289,6 +2306,7 @@ void SolverPlan::drop_fused() {
 }
 
 SolverPlan::~SolverPlan() {
+  if (busy) cudaDeviceSynchronize();  // a call that ended early may have left work on the buffers
   drop_fused();
   for (auto &g : graph)
     if (g) cudaGraphExecDestroy(g);
@@ -2297,13 +2315,25 @@ SolverPlan::~SolverPlan() {
   if (h_ctl) cudaFreeHost(h_ctl);
 }
 
+// One call on a plan.  Every call ends with its stream waited for; one that does not get there (an
+// error) leaves the plan marked, and the device is waited for before its buffers move or go.
+struct PlanCall {
+  SolverPlan *S;
+  explicit PlanCall(SolverPlan *s) : S(s) {
+    if (S->busy) cudaDeviceSynchronize();
+    S->busy = 1;
+  }
+  void done() { S->busy = 0; }
+};
+
 int solver_update(SolverPlan *S, const double *d_K, const double *d_M, cudaStream_t st) {
+  PlanCall call(S);
   const int64_t nnz = S->nnz;
   k_cvt_km<<<g1(nnz, 256), 256, 0, st>>>(d_K, d_M, S->col.as<int32_t>(), nnz, S->KM64.as<double2>(),
                                           S->RecA32.as<Rec32>(), S->tA.lcol.as<int32_t>());
   DGP_CHECK_LAUNCH();
   // FSAI of tril(K + i*k*dfc*M) for every harmonic (scratch kept in the plan: no allocation per update)
-  if (!S->dfcM.p) DGP_TRY(S->dfcM.alloc(sizeof(double) * nnz));
+  if (!S->dfcM.p) DGP_TRY(S->dfcM.alloc_plan(sizeof(double) * nnz));
   k_dfc_m<<<g1(nnz, 256), 256, 0, st>>>(d_M, S->dfc, nnz, S->dfcM.as<double>());
   DGP_CHECK_LAUNCH();
   DGP_TRY(fsai_factor_run(S->rowptr.as<int32_t>(), S->col.as<int32_t>(), d_K, S->dfcM.as<double>(), S->n,
@@ -2316,6 +2346,7 @@ int solver_update(SolverPlan *S, const double *d_K, const double *d_M, cudaStrea
                                                        S->tGT.lcol.as<int32_t>());
   DGP_CHECK_LAUNCH();
   DGP_CUDA(cudaStreamSynchronize(st));
+  call.done();
   return DGP_OK;
 }
 
@@ -2331,6 +2362,7 @@ int solver_build(SolverPlan *S, const int32_t *d_rowptr, const int32_t *d_col, i
   DGP_REQUIRE(ns_max >= 1 && ns_max <= 128, "solver: 1 <= ns_max <= 128 sources per harmonic");
   DGP_REQUIRE(nnz < INT32_MAX && n < (1 << 24), "solver: nnz must fit int32 and n < 2^24");
   DGP_TRY(csr_in_range(d_rowptr, d_col, n, n, nnz, 0, "solver: pattern", st));
+  S->busy = 1;  // (until solver_update below takes over)
   S->n = n;
   S->nnz = nnz;
   S->nf = nf;
@@ -2340,14 +2372,14 @@ int solver_build(SolverPlan *S, const int32_t *d_rowptr, const int32_t *d_col, i
   S->h_harm = hl;
   S->dfc = dfc;
   if (opts) S->opts = *opts; else dgp_solve_opts_default(&S->opts);
-  DGP_TRY(S->rowptr.alloc(sizeof(int32_t) * (n + 1)));
-  DGP_TRY(S->col.alloc(sizeof(int32_t) * nnz));
+  DGP_TRY(S->rowptr.alloc_plan(sizeof(int32_t) * (n + 1)));
+  DGP_TRY(S->col.alloc_plan(sizeof(int32_t) * nnz));
   DGP_CUDA(cudaMemcpyAsync(S->rowptr.p, d_rowptr, sizeof(int32_t) * (n + 1), cudaMemcpyDeviceToDevice, st));
   DGP_CUDA(cudaMemcpyAsync(S->col.p, d_col, sizeof(int32_t) * nnz, cudaMemcpyDeviceToDevice, st));
-  DGP_TRY(S->KM64.alloc(sizeof(double2) * nnz));
-  DGP_TRY(S->RecA32.alloc(sizeof(Rec32) * nnz));
-  DGP_TRY(S->omega.alloc((sizeof(double) + sizeof(float)) * nf));
-  DGP_TRY(S->harm.alloc(sizeof(int32_t) * nf));
+  DGP_TRY(S->KM64.alloc_plan(sizeof(double2) * nnz));
+  DGP_TRY(S->RecA32.alloc_plan(sizeof(Rec32) * nnz));
+  DGP_TRY(S->omega.alloc_plan((sizeof(double) + sizeof(float)) * nf));
+  DGP_TRY(S->harm.alloc_plan(sizeof(int32_t) * nf));
   DGP_CUDA(cudaMemcpyAsync(S->harm.p, hl.data(), sizeof(int32_t) * nf, cudaMemcpyHostToDevice, st));
   k_omega<<<g1(nf, 128), 128, 0, st>>>(nf, dfc, S->harm.as<int32_t>(), S->omega.as<double>(),
                                         (float *)(S->omega.as<char>() + sizeof(double) * nf));
@@ -2356,16 +2388,16 @@ int solver_build(SolverPlan *S, const int32_t *d_rowptr, const int32_t *d_col, i
                              S->opts.fsai_cap, st));
   S->nnzG = S->P.nnzG;
   const size_t gcount = (size_t)S->nnzG * nf;
-  DGP_TRY(S->G64.alloc(sizeof(double2) * gcount));
-  DGP_TRY(S->GT64.alloc(sizeof(double2) * gcount));
-  DGP_TRY(S->RecG32.alloc(sizeof(Rec32) * gcount));
-  DGP_TRY(S->RecGT32.alloc(sizeof(Rec32) * gcount));
+  DGP_TRY(S->G64.alloc_plan(sizeof(double2) * gcount));
+  DGP_TRY(S->GT64.alloc_plan(sizeof(double2) * gcount));
+  DGP_TRY(S->RecG32.alloc_plan(sizeof(Rec32) * gcount));
+  DGP_TRY(S->RecGT32.alloc_plan(sizeof(Rec32) * gcount));
   // two mirrors (run_iterations' pipelined polls); the fused solve's control block fits too
   DGP_CUDA(cudaMallocHost(&S->h_ctl, std::max<size_t>(512, 2 * sizeof(Ctl))));
   {
-    DevBuf sums;
+    ScratchBuf sums;
     double hs[3] = {0, 0, 0};
-    DGP_TRY(sums.alloc(sizeof(hs)));
+    DGP_TRY(sums.alloc(sizeof(hs), st));
     DGP_CUDA(cudaMemsetAsync(sums.p, 0, sizeof(hs), st));
     k_spectrum<<<(unsigned)std::min<int64_t>(ceil_div(n, 256), 592), 256, 0, st>>>(
         S->rowptr.as<int32_t>(), S->col.as<int32_t>(), d_K, d_M, n, sums.as<double>());
@@ -2376,7 +2408,7 @@ int solver_build(SolverPlan *S, const int32_t *d_rowptr, const int32_t *d_col, i
     S->lam_lo = hs[1] > 0 && std::isfinite(hs[0]) && hs[0] > 0 ? hs[0] / hs[1] : S->lam_hi;
     S->lam_lo = std::min(S->lam_hi, std::max(S->lam_lo, 1e-6 * S->lam_hi));
   }
-  DGP_TRY(tiled_setup(S, st));
+  S->busy = 0;
   return solver_update(S, d_K, d_M, st);
 }
 
@@ -2503,15 +2535,19 @@ int solver_solve(SolverPlan *S, const double *d_B, const int32_t *d_nodes, const
   DGP_REQUIRE(o.precision == DGP_PREC_FP64 || o.precision == DGP_PREC_MIXED || o.precision == DGP_PREC_MIXED_BICGSTAB,
               "solve: unknown precision");
   if (o.check_every < 1) o.check_every = 1;
+  PlanCall call(S);
   if (d_nodes) {
-    if (!S->node_flag.p) DGP_TRY(S->node_flag.alloc(sizeof(int)));
+    if (!S->node_flag.p) DGP_TRY(S->node_flag.alloc_plan(sizeof(int)));
     DGP_CUDA(cudaMemsetAsync(S->node_flag.p, 0, sizeof(int), st));
     k_check_nodes<<<g1(4 * ns, 128), 128, 0, st>>>(d_nodes, ns, S->n, S->node_flag.as<int>());
     DGP_CHECK_LAUNCH();
     int hb = 0;
     DGP_CUDA(cudaMemcpyAsync(&hb, S->node_flag.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     DGP_CUDA(cudaStreamSynchronize(st));
-    if (hb) return fail(DGP_ERR_ARG, "solve: source node index out of range");
+    if (hb) {
+      call.done();
+      return fail(DGP_ERR_ARG, "solve: source node index out of range");
+    }
   }
   dgp_solve_report local{};
   dgp_solve_report *r = rep ? rep : &local;
@@ -2539,6 +2575,7 @@ int solver_solve(SolverPlan *S, const double *d_B, const int32_t *d_nodes, const
   if (r->d_status)
     DGP_CUDA(cudaMemcpyAsync(r->d_status, out.data(), sizeof(int) * out.size(), cudaMemcpyHostToDevice, st));
   DGP_CUDA(cudaStreamSynchronize(st));
+  call.done();
   // any column that missed tol -- maxit, a breakdown or a non-finite value -- makes the call NOT_CONVERGED
   if (rc == DGP_ERR_NOT_CONVERGED || bad > 0)
     return fail(DGP_ERR_NOT_CONVERGED, "solve: " + std::to_string(bad) + " of " + std::to_string(out.size()) +
@@ -2583,14 +2620,19 @@ void profile_launch(int which, const SolverPlan *S, const OpA32 &A, const OpG32 
 int solver_profile(SolverPlan *S, int which, int reps, float *ms, double *bytes, cudaStream_t st) {
   DGP_REQUIRE(reps >= 1 && which >= 0 && which <= 10, "profile: bad arguments");
   DGP_REQUIRE(S->ws_prec == DGP_PREC_MIXED || S->fscal.p, "profile: run a mixed-precision solve first");
-  if (which >= 8) return fused_profile(S, which - 8, reps, ms, bytes, st);
+  PlanCall call(S);
+  if (which >= 8) {
+    DGP_TRY(fused_profile(S, which - 8, reps, ms, bytes, st));
+    call.done();
+    return DGP_OK;
+  }
   DGP_TRY(ensure_workspace(S, DGP_PREC_MIXED, NVEC_COCG));
   if (which == 2 || which == 3) DGP_TRY(ensure_workspace(S, DGP_PREC_MIXED, NVEC_ALL));  // BiCGSTAB updates
   Vecs<float> V = vec_views<float>(S);
   Work W = work_views(S);
   W.cols.hact = nullptr;  // timing / checking runs sweep every harmonic
-  DevBuf dctl;
-  DGP_TRY(dctl.alloc(sizeof(Ctl)));
+  ScratchBuf dctl;
+  DGP_TRY(dctl.alloc(sizeof(Ctl), st));
   Ctl hc{};
   hc.state = ST_RUNNING;
   hc.maxit = 1 << 30;
@@ -2639,6 +2681,7 @@ int solver_profile(SolverPlan *S, int which, int reps, float *ms, double *bytes,
   DGP_CUDA(cudaMemsetAsync(W.cols.acc, 0, sizeof(double2) * W.cols.C * NACC, st));
   DGP_CUDA(cudaStreamSynchronize(st));
   *ms = t / reps;
+  call.done();
   return DGP_OK;
 }
 
@@ -2709,12 +2752,14 @@ __global__ void k_maxdiff(const float2 *__restrict__ a, const float2 *__restrict
 // contents are scratch here (every solve re-initialises them).
 int solver_autotune(SolverPlan *S, int32_t *tiled_out, int32_t *vec_out, int32_t *rows_out, float *ms_out,
                     cudaStream_t st) {
+  PlanCall call(S);
+  DGP_TRY(tiled_setup(S, st));
   DGP_TRY(ensure_workspace(S, DGP_PREC_MIXED, NVEC_COCG));
   Vecs<float> V = vec_views<float>(S);
   Work W = work_views(S);
   W.cols.hact = nullptr;  // timing / checking runs sweep every harmonic
-  DevBuf dctl;
-  DGP_TRY(dctl.alloc(sizeof(Ctl)));
+  ScratchBuf dctl;
+  DGP_TRY(dctl.alloc(sizeof(Ctl), st));
   Ctl hc{};
   hc.state = ST_RUNNING;
   hc.maxit = 1 << 30;
@@ -2824,6 +2869,7 @@ int solver_autotune(SolverPlan *S, int32_t *tiled_out, int32_t *vec_out, int32_t
     for (auto &v : S->vec) v.release();
     S->ws_prec = -1;
   }
+  call.done();
   if (tiled_out) *tiled_out = bt;
   if (vec_out) *vec_out = bv;
   if (rows_out) *rows_out = br;
@@ -2833,6 +2879,8 @@ int solver_autotune(SolverPlan *S, int32_t *tiled_out, int32_t *vec_out, int32_t
 
 int solver_set_spmm(SolverPlan *S, int32_t tiled, int32_t vec, int32_t rows) {
   DGP_REQUIRE(tiled == 0 || tiled == 1, "set_spmm: tiled must be 0 or 1");
+  if (tiled) DGP_TRY(tiled_setup(S, cudaStreamPerThread));
+  if (tiled) DGP_CUDA(cudaStreamSynchronize(cudaStreamPerThread));
   DGP_REQUIRE(!tiled || S->tiled_ok, "set_spmm: the tiled SpMM does not fit this plan's shared memory");
   if (!tiled && vec != 0) {
     DGP_REQUIRE((vec == 2 || vec == 4 || vec == 8) && vec <= S->nsp && S->nsp / vec <= 32,
@@ -2892,14 +2940,16 @@ int solver_set_dot_rows(SolverPlan *S, int32_t mult) {
 // only the summation order differs).
 int solver_check_spmm(SolverPlan *S, double *max_rel, cudaStream_t st) {
   DGP_REQUIRE(max_rel, "check_spmm: null output");
+  PlanCall call(S);
+  DGP_TRY(tiled_setup(S, st));
   DGP_REQUIRE(S->tiled_ok, "check_spmm: the tiled SpMM does not fit this plan");
   DGP_TRY(ensure_workspace(S, DGP_PREC_MIXED, NVEC_COCG));
   Vecs<float> V = vec_views<float>(S);
   Work W = work_views(S);
   W.cols.hact = nullptr;  // timing / checking runs sweep every harmonic
-  DevBuf dctl, dm;
-  DGP_TRY(dctl.alloc(sizeof(Ctl)));
-  DGP_TRY(dm.alloc(2 * sizeof(unsigned)));
+  ScratchBuf dctl, dm;
+  DGP_TRY(dctl.alloc(sizeof(Ctl), st));
+  DGP_TRY(dm.alloc(2 * sizeof(unsigned), st));
   Ctl hc{};
   hc.state = ST_RUNNING;
   hc.maxit = 1 << 30;
@@ -2937,6 +2987,7 @@ int solver_check_spmm(SolverPlan *S, double *max_rel, cudaStream_t st) {
   count_launches(3 * 3 + 1);
   DGP_CHECK_LAUNCH();
   *max_rel = worst;
+  call.done();
   return DGP_OK;
 }
 

@@ -1,11 +1,14 @@
 // C ABI of libdogpup_b200: argument checks, error reporting, plan handles.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <atomic>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <string>
+#include <type_traits>
 
 #include "dgp_common.cuh"
 #include "dgp_internal.h"
@@ -36,24 +39,168 @@ int cuda_fail(cudaError_t e, const char *what, const char *file, int line) {
   return e == cudaErrorMemoryAllocation ? DGP_ERR_NOMEM : DGP_ERR_CUDA;
 }
 
-int DevBuf::alloc(size_t n) {
-  release();
+namespace {
+
+// driver entry points fetched through the runtime (no link against libcuda)
+struct Driver {
+  CUresult (*ctx_current)(CUcontext *) = nullptr;
+  CUresult (*ctx_id)(CUcontext, unsigned long long *) = nullptr;
+  CUresult (*primary_retain)(CUcontext *, CUdevice) = nullptr;
+  CUresult (*primary_release)(CUdevice) = nullptr;
+};
+const Driver &driver() {
+  static Driver d;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    auto get = [](const char *name, auto *fn) {
+      void *p = nullptr;
+      cudaDriverEntryPointQueryResult q;
+      if (cudaGetDriverEntryPointByVersion(name, &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+          q == cudaDriverEntryPointSuccess)
+        *fn = reinterpret_cast<std::remove_pointer_t<decltype(fn)>>(p);
+      else
+        cudaGetLastError();
+    };
+    get("cuCtxGetCurrent", &d.ctx_current);
+    get("cuCtxGetId", &d.ctx_id);
+    get("cuDevicePrimaryCtxRetain", &d.primary_retain);
+    get("cuDevicePrimaryCtxRelease", &d.primary_release);
+  });
+  return d;
+}
+
+constexpr int kMaxDev = 64;
+struct PoolEntry {
+  unsigned long long ctx = 0;  // context the pools were made in (0: none yet)
+  cudaMemPool_t pool[2] = {nullptr, nullptr};  // scratch, plans
+};
+std::mutex g_pool_mutex;
+PoolEntry g_pools[kMaxDev];
+
+cudaMemPool_t make_pool(int dev) {
+  const Driver &d = driver();
+  CUcontext cur = nullptr, prim = nullptr;
+  if (!d.primary_retain || !d.primary_release || d.ctx_current(&cur) != CUDA_SUCCESS) return nullptr;
+  if (d.primary_retain(&prim, dev) != CUDA_SUCCESS) return nullptr;
+  d.primary_release(dev);
+  if (prim != cur) return nullptr;  // a context of the application's own: plain allocations
+  int ok = 0;
+  if (cudaDeviceGetAttribute(&ok, cudaDevAttrMemoryPoolsSupported, dev) != cudaSuccess || !ok) return nullptr;
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.handleTypes = cudaMemHandleTypeNone;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  cudaMemPool_t pool = nullptr;
+  size_t free_b = 0, total = 0;
+  if (cudaMemGetInfo(&free_b, &total) != cudaSuccess || cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  uint64_t keep = total / 64;
+  cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  return pool;
+}
+
+}  // namespace
+
+unsigned long long context_id() {
+  const Driver &d = driver();
+  CUcontext c = nullptr;
+  unsigned long long id = 0;
+  if (!d.ctx_current || !d.ctx_id || d.ctx_current(&c) != CUDA_SUCCESS || !c || d.ctx_id(c, &id) != CUDA_SUCCESS)
+    return 0;
+  return id;
+}
+
+cudaMemPool_t device_pool(bool plans) {
+  const unsigned long long id = context_id();
+  int dev = 0;
+  if (!id || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) return nullptr;
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  PoolEntry &e = g_pools[dev];
+  if (e.ctx != id) {  // first use, or the context was reset: its pool went with it
+    e.ctx = id;
+    for (auto &p : e.pool) p = make_pool(dev);
+  }
+  return e.pool[plans ? 1 : 0];
+}
+
+void trim_pools() {
+  for (bool plans : {false, true}) {
+    cudaMemPool_t pool = device_pool(plans);
+    if (!pool) continue;
+    cudaDeviceSynchronize();
+    cudaMemPoolTrimTo(pool, 0);
+  }
+}
+
+// which: 0 cudaMalloc, 1 the scratch pool, 2 the plan pool, in the order of st; sets *pooled
+static int device_alloc(void **p, size_t n, cudaStream_t st, int which, bool *pooled) {
   if (n == 0) n = 16;
-  cudaError_t e = cudaMalloc(&p, n);
   g_device_allocs.fetch_add(1, std::memory_order_relaxed);
+  *pooled = false;
+  if (which) {
+    cudaMemPool_t pool = device_pool(which == 2);
+    if (pool) {
+      if (cudaMallocFromPoolAsync(p, n, pool, st) == cudaSuccess) {
+        *pooled = true;
+        return DGP_OK;
+      }
+      cudaGetLastError();
+    }
+  }
+  cudaError_t e = cudaMalloc(p, n);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    trim_pools();
+    e = cudaMalloc(p, n);
+  }
   if (e != cudaSuccess) {
-    p = nullptr;
+    *p = nullptr;
     cudaGetLastError();
     char buf[160];
     std::snprintf(buf, sizeof buf, "device allocation of %zu bytes failed: %s", n, cudaGetErrorString(e));
     return fail(DGP_ERR_NOMEM, buf);
   }
-  bytes = n;
+  return DGP_OK;
+}
+
+int ScratchBuf::alloc(size_t n, cudaStream_t stream) {
+  release();
+  st = stream;
+  return device_alloc(&p, n, stream, 1, &pooled);
+}
+
+void ScratchBuf::release() {
+  if (p) {
+    if (pooled) cudaFreeAsync(p, st);
+    else cudaFree(p);
+  }
+  p = nullptr;
+}
+
+int DevBuf::alloc(size_t n) {
+  release();
+  DGP_TRY(device_alloc(&p, n, nullptr, 0, &pooled));
+  bytes = n ? n : 16;
+  return DGP_OK;
+}
+
+int DevBuf::alloc_plan(size_t n) {
+  release();
+  DGP_TRY(device_alloc(&p, n, cudaStreamPerThread, 2, &pooled));
+  bytes = n ? n : 16;
+  // any stream may use it from here on
+  if (pooled) DGP_CUDA(cudaStreamSynchronize(cudaStreamPerThread));
   return DGP_OK;
 }
 
 void DevBuf::release() {
-  if (p) cudaFree(p);
+  if (p) {
+    if (pooled) cudaFreeAsync(p, cudaStreamPerThread);
+    else cudaFree(p);
+  }
   p = nullptr;
   bytes = 0;
 }

@@ -37,8 +37,27 @@ __global__ void k_rowptr_ok(const int32_t *__restrict__ rowptr, int64_t nrows, i
   }
 }
 
-int read_flag(const DevBuf &err, cudaStream_t st, int *h) {
-  DGP_CUDA(cudaMemcpyAsync(h, err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+// columns of a CSR pattern whose row pointer k_rowptr_ok passed (nothing is read otherwise): err[1] =
+// entries; *err |= 8 unless that is nnz (nnz >= 0), |= 16 without a column array, |= 1 as k_ids_in_range
+__global__ void k_csr_cols(const int32_t *__restrict__ rowptr, const int32_t *__restrict__ col, int64_t nrows,
+                           int64_t ncols, int64_t nnz, int *err) {
+  if (*(volatile int *)err & (2 | 4)) return;
+  const int64_t last = rowptr[nrows];
+  if (blockIdx.x == 0 && threadIdx.x == 0) err[1] = (int)last;
+  if (nnz >= 0 && last != nnz) {
+    if (threadIdx.x == 0) atomicOr(err, 8);
+    return;
+  }
+  if (!col) {
+    if (last > 0 && threadIdx.x == 0) atomicOr(err, 16);
+    return;
+  }
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < last; i += (int64_t)gridDim.x * blockDim.x)
+    if (col[i] < 0 || col[i] >= ncols) atomicOr(err, 1);
+}
+
+int read_flag(const ScratchBuf &err, cudaStream_t st, int *h, int n = 1) {
+  DGP_CUDA(cudaMemcpyAsync(h, err.p, sizeof(int) * n, cudaMemcpyDeviceToHost, st));
   DGP_CUDA(cudaStreamSynchronize(st));
   return DGP_OK;
 }
@@ -48,8 +67,8 @@ int read_flag(const DevBuf &err, cudaStream_t st, int *h) {
 int ids_in_range(const int32_t *d_ids, int64_t count, int64_t limit, const char *who, cudaStream_t st) {
   if (count <= 0) return DGP_OK;
   DGP_REQUIRE(d_ids, std::string(who) + ": null index array");
-  DevBuf err;
-  DGP_TRY(err.alloc(sizeof(int)));
+  ScratchBuf err;
+  DGP_TRY(err.alloc(sizeof(int), st));
   DGP_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), st));
   k_ids_in_range<<<check_grid(count), CHECK_NT, 0, st>>>(d_ids, count, limit, err.as<int>());
   DGP_CHECK_LAUNCH();
@@ -62,29 +81,25 @@ int ids_in_range(const int32_t *d_ids, int64_t count, int64_t limit, const char 
 int csr_in_range(const int32_t *d_rowptr, const int32_t *d_col, int64_t nrows, int64_t ncols, int64_t nnz,
                  int64_t max_row, const char *who, cudaStream_t st) {
   DGP_REQUIRE(d_rowptr && nrows > 0, std::string(who) + ": empty or null CSR row pointer");
-  DevBuf err;
-  DGP_TRY(err.alloc(sizeof(int)));
-  DGP_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), st));
+  // both checks on the device, one read of their outcome
+  ScratchBuf err;
+  DGP_TRY(err.alloc(2 * sizeof(int), st));
+  DGP_CUDA(cudaMemsetAsync(err.p, 0, 2 * sizeof(int), st));
   k_rowptr_ok<<<check_grid(nrows), CHECK_NT, 0, st>>>(d_rowptr, nrows, max_row, err.as<int>());
   DGP_CHECK_LAUNCH();
-  int h = 0;
-  DGP_TRY(read_flag(err, st, &h));
-  if (h & 2) return fail(DGP_ERR_MESH, std::string(who) + ": CSR row pointer must start at 0 and not decrease");
-  if (h & 4)
-    return fail(DGP_ERR_MESH, std::string(who) + ": a CSR row holds more than " + std::to_string(max_row) + " entries");
-  int32_t last = 0;
-  DGP_CUDA(cudaMemcpyAsync(&last, d_rowptr + nrows, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-  DGP_CUDA(cudaStreamSynchronize(st));
-  if (nnz >= 0 && last != nnz)
-    return fail(DGP_ERR_MESH, std::string(who) + ": CSR row pointer ends at " + std::to_string(last) +
-                                  ", not at nnz = " + std::to_string(nnz));
-  if (last == 0) return DGP_OK;
-  DGP_REQUIRE(d_col, std::string(who) + ": null CSR column array");
-  DGP_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), st));
-  k_ids_in_range<<<check_grid(last), CHECK_NT, 0, st>>>(d_col, last, ncols, err.as<int>());
+  k_csr_cols<<<check_grid(nnz >= 0 ? nnz : 8 * nrows), CHECK_NT, 0, st>>>(d_rowptr, d_col, nrows, ncols, nnz,
+                                                                         err.as<int>());
   DGP_CHECK_LAUNCH();
-  DGP_TRY(read_flag(err, st, &h));
-  if (h) return fail(DGP_ERR_MESH, std::string(who) + ": CSR column index out of range");
+  int h[2] = {0, 0};
+  DGP_TRY(read_flag(err, st, h, 2));
+  if (h[0] & 2) return fail(DGP_ERR_MESH, std::string(who) + ": CSR row pointer must start at 0 and not decrease");
+  if (h[0] & 4)
+    return fail(DGP_ERR_MESH, std::string(who) + ": a CSR row holds more than " + std::to_string(max_row) + " entries");
+  if (h[0] & 8)
+    return fail(DGP_ERR_MESH, std::string(who) + ": CSR row pointer ends at " + std::to_string(h[1]) +
+                                  ", not at nnz = " + std::to_string(nnz));
+  if (h[0] & 16) return fail(DGP_ERR_ARG, std::string(who) + ": null CSR column array");
+  if (h[0] & 1) return fail(DGP_ERR_MESH, std::string(who) + ": CSR column index out of range");
   return DGP_OK;
 }
 

@@ -33,6 +33,8 @@
 // diagonal product.
 #include <algorithm>
 #include <cmath>
+#include <memory>
+#include <mutex>
 #include <vector>
 
 #include "dgp_common.cuh"
@@ -946,13 +948,67 @@ struct LookaheadStreams {
       DGP_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     return DGP_OK;
   }
-  ~LookaheadStreams() {
+  void wait() const {
     for (cudaStream_t q : {f, s, b, r})
       if (q) cudaStreamSynchronize(q);
+  }
+  ~LookaheadStreams() {
+    wait();
     for (cudaEvent_t e : {fork, panel, rest, join, step, side, diag, below})
       if (e) cudaEventDestroy(e);
     for (cudaStream_t q : {f, s, b, r})
       if (q) cudaStreamDestroy(q);
+  }
+};
+
+// A set of streams on loan for one call: creating and destroying them took 0.5 ms of each.  At most
+// four idle sets are kept; a set made in a context that has been reset since is dropped (its
+// handles went with the context).
+struct StreamLoan {
+  struct Idle {
+    unsigned long long ctx;
+    std::unique_ptr<LookaheadStreams> set;
+  };
+  static std::mutex &mutex() {
+    static std::mutex m;
+    return m;
+  }
+  static std::vector<Idle> &idle() {
+    static auto *v = new std::vector<Idle>;  // (never destroyed: the driver may be gone by then)
+    return *v;
+  }
+  unsigned long long ctx = 0;
+  std::unique_ptr<LookaheadStreams> set;
+  bool clean = false;
+  int take() {
+    ctx = context_id();
+    if (ctx) {
+      std::lock_guard<std::mutex> lock(mutex());
+      auto &v = idle();
+      for (size_t i = 0; i < v.size(); ++i)
+        if (v[i].ctx == ctx) {
+          set = std::move(v[i].set);
+          v.erase(v.begin() + i);
+          return DGP_OK;
+        }
+    }
+    set = std::make_unique<LookaheadStreams>();
+    return set->create();
+  }
+  ~StreamLoan() {
+    if (!set) return;
+    if (!clean || !ctx) return;  // an error left work queued: the set's destructor waits for it
+    std::lock_guard<std::mutex> lock(mutex());
+    auto &v = idle();
+    if (v.size() >= 4) {
+      if (v.front().ctx != ctx) {
+        v.front().set.release();
+        v.erase(v.begin());
+      } else {
+        return;
+      }
+    }
+    v.push_back(Idle{ctx, std::move(set)});
   }
 };
 
@@ -965,11 +1021,11 @@ int cholesky_solve_many_run(double *H, int64_t n, int64_t ldh, double *x, int32_
   DGP_REQUIRE(nrhs <= 65535, "cholesky: at most 65535 right-hand sides");
   DGP_REQUIRE(ceil_div(n, (int64_t)GVB) <= INT32_MAX, "cholesky: n too large for the solve grid");
   const int64_t nblk = ceil_div(n, CB), NBO = outer_width(n);
-  DevBuf linv, errb, acc, flags;
-  DGP_TRY(linv.alloc(sizeof(double) * (size_t)nblk * CB * CB));
-  DGP_TRY(errb.alloc(sizeof(int)));
-  DGP_TRY(acc.alloc(sizeof(double) * (size_t)CB * nrhs));
-  DGP_TRY(flags.alloc(sizeof(uint32_t) * 2 * (size_t)nblk));
+  ScratchBuf linv, errb, acc, flags;
+  DGP_TRY(linv.alloc(sizeof(double) * (size_t)nblk * CB * CB, st));
+  DGP_TRY(errb.alloc(sizeof(int), st));
+  DGP_TRY(acc.alloc(sizeof(double) * (size_t)CB * nrhs, st));
+  DGP_TRY(flags.alloc(sizeof(uint32_t) * 2 * (size_t)nblk, st));
   DGP_CUDA(cudaMemsetAsync(errb.p, 0, sizeof(int), st));
   DGP_CUDA(cudaMemsetAsync(flags.p, 0, sizeof(uint32_t) * 2 * (size_t)nblk, st));
   DGP_CUDA(cudaMemsetAsync(acc.p, 0, sizeof(double) * (size_t)CB * nrhs, st));
@@ -992,8 +1048,9 @@ int cholesky_solve_many_run(double *H, int64_t n, int64_t ldh, double *x, int32_
   //              R_{p-1}, which updates the same entries)
   //   sr:  R_p   the lower triangle of [nend, n)^2 -= Q Q^T  (after F_p)
   // so F_{p+1} runs while R_p does, and the trailing GEMMs keep the outer panel width as depth.
-  LookaheadStreams ls;
-  DGP_TRY(ls.create());
+  StreamLoan loan;
+  DGP_TRY(loan.take());
+  LookaheadStreams &ls = *loan.set;
   DGP_CUDA(cudaEventRecord(ls.fork, st));
   DGP_CUDA(cudaStreamWaitEvent(ls.f, ls.fork, 0));
   DGP_CUDA(cudaStreamWaitEvent(ls.s, ls.fork, 0));
@@ -1137,6 +1194,7 @@ int cholesky_solve_many_run(double *H, int64_t n, int64_t ldh, double *x, int32_
   int herr = 0;
   DGP_CUDA(cudaMemcpyAsync(&herr, errb.p, sizeof(int), cudaMemcpyDeviceToHost, st));
   DGP_CUDA(cudaStreamSynchronize(st));
+  loan.clean = true;  // every stream has joined st
   if (herr & 1) return fail(DGP_ERR_ARG, "cholesky: matrix is not positive definite");
   if (herr & 2) return fail(DGP_ERR_CUDA, "cholesky: a wait of the chained solve gave up");
   return DGP_OK;

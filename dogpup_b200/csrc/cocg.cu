@@ -806,12 +806,13 @@ int fused_setup(SolverPlan *S, FWork *out) {
     for (auto &v : S->vec) v.release();
     S->ws_prec = -1;
     const size_t vb = sizeof(float2) * (size_t)S->nf * S->n * nsp;
-    for (int i = 0; i < 4; ++i) DGP_TRY(S->fvec[i].alloc(vb));
-    DGP_TRY(S->fctl.alloc(sizeof(FCtl)));
+    for (int i = 0; i < 4; ++i) DGP_TRY(S->fvec[i].alloc_plan(vb));
+    DGP_TRY(S->fctl.alloc_plan(sizeof(FCtl)));
     const size_t sb = fscal_bytes((int64_t)S->nf * nsp, S->nf);
-    DGP_TRY(S->fscal.alloc(sb));
-    DGP_CUDA(cudaMemset(S->fscal.p, 0, sb));
-    DGP_CUDA(cudaMemset(S->fctl.p, 0, sizeof(FCtl)));
+    DGP_TRY(S->fscal.alloc_plan(sb));
+    DGP_CUDA(cudaMemsetAsync(S->fscal.p, 0, sb, cudaStreamPerThread));
+    DGP_CUDA(cudaMemsetAsync(S->fctl.p, 0, sizeof(FCtl), cudaStreamPerThread));
+    DGP_CUDA(cudaStreamSynchronize(cudaStreamPerThread));
   }
   FWork w = fwork(S);
   w.vec = vec;
@@ -1127,8 +1128,8 @@ int upload_levels(SolverPlan *S, cudaStream_t st) {
     std::copy(L.solved.begin(), L.solved.end(), hi.begin() + L.off_solved);
     std::copy(L.coef.begin(), L.coef.end(), hd.begin() + L.off_coef);
   }
-  DGP_TRY(S->lev_int.alloc(sizeof(int32_t) * hi.size()));
-  DGP_TRY(S->lev_coef.alloc(sizeof(double) * hd.size()));
+  DGP_TRY(S->lev_int.alloc_plan(sizeof(int32_t) * hi.size()));
+  DGP_TRY(S->lev_coef.alloc_plan(sizeof(double) * hd.size()));
   DGP_CUDA(cudaMemcpyAsync(S->lev_int.p, hi.data(), sizeof(int32_t) * hi.size(), cudaMemcpyHostToDevice, st));
   DGP_CUDA(cudaMemcpyAsync(S->lev_coef.p, hd.data(), sizeof(double) * hd.size(), cudaMemcpyHostToDevice, st));
   DGP_CUDA(cudaStreamSynchronize(st));

@@ -108,7 +108,8 @@ struct SolverPlan {
   int32_t tune_dot = 0;  // rows per block of the FP32 dot-product sweeps, as a multiple of tune_rows (0: 4)
   // tiled SpMM (halo rows staged in shared memory) for A, G and G^T; tiled = 1 selects it
   TiledPlan tA, tG, tGT;
-  int32_t tiled_ok = 0, tiled = 0;
+  int32_t tiled_built = 0, tiled_ok = 0, tiled = 0;
+  int32_t busy = 0;  // a call is running, or ended early with work possibly still queued
   int64_t bytes = 0;
   // ---- fused COCG (cocg.cu): the mixed solve unless a gather or tiled SpMM was asked for by name
   int32_t unfused = 0;

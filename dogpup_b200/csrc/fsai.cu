@@ -189,16 +189,16 @@ int fsai_pattern_rows(const int32_t *d_rowptr, const int32_t *d_col, const doubl
                       int32_t *h_mmax, cudaStream_t st) {
   DGP_REQUIRE(n > 0 && cap >= 1 && cap <= 32, "fsai pattern: need n > 0 and 1 <= cap <= 32");
   const int bs = 256;
-  DevBuf cnt, flag, tmp;
-  DGP_TRY(cnt.alloc(sizeof(int32_t) * (n + 1)));
-  DGP_TRY(flag.alloc(2 * sizeof(int)));
+  ScratchBuf cnt, flag, tmp;
+  DGP_TRY(cnt.alloc(sizeof(int32_t) * (n + 1), st));
+  DGP_TRY(flag.alloc(2 * sizeof(int), st));
   DGP_CUDA(cudaMemsetAsync(flag.p, 0, 2 * sizeof(int), st));
   DGP_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(int32_t) * (n + 1), st));
   k_pattern_count<<<grid1(n, bs), bs, 0, st>>>(d_rowptr, d_col, n, cap, cnt.as<int32_t>(), flag.as<int>());
   DGP_CHECK_LAUNCH();
   size_t tb = 0;
   DGP_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt.as<int32_t>(), d_rowptrG, (int)(n + 1), st));
-  DGP_TRY(tmp.alloc(tb));
+  DGP_TRY(tmp.alloc(tb, st));
   DGP_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, tb, cnt.as<int32_t>(), d_rowptrG, (int)(n + 1), st));
   k_max_row<<<grid1(n, bs), bs, 0, st>>>(d_rowptrG, n, flag.as<int>() + 1);
   DGP_CHECK_LAUNCH();
@@ -241,13 +241,13 @@ int fsai_factor_run(const int32_t *d_rowptr, const int32_t *d_col, const double 
 int fsai_pattern_build(FsaiPattern *P, const int32_t *d_rowptr, const int32_t *d_col, const double *d_K,
                        const double *d_M, double dfc, int64_t n, int32_t cap, cudaStream_t st) {
   P->n = n;
-  DGP_TRY(P->rowptr.alloc(sizeof(int32_t) * (n + 1)));
+  DGP_TRY(P->rowptr.alloc_plan(sizeof(int32_t) * (n + 1)));
   int32_t nnzG = 0, mmax = 0;
   DGP_TRY(fsai_pattern_rows(d_rowptr, d_col, d_K, d_M, dfc, n, cap, P->rowptr.as<int32_t>(), nullptr, &nnzG,
                             &mmax, st));
   P->nnzG = nnzG;
   P->mmax = mmax;
-  DGP_TRY(P->col.alloc(sizeof(int32_t) * nnzG));
+  DGP_TRY(P->col.alloc_plan(sizeof(int32_t) * nnzG));
   DGP_TRY(fsai_pattern_rows(d_rowptr, d_col, d_K, d_M, dfc, n, cap, P->rowptr.as<int32_t>(), P->col.as<int32_t>(),
                             nullptr, nullptr, st));
   return fsai_transpose_pattern(P, st);
@@ -255,20 +255,20 @@ int fsai_pattern_build(FsaiPattern *P, const int32_t *d_rowptr, const int32_t *d
 
 int fsai_transpose_pattern(FsaiPattern *P, cudaStream_t st) {
   const int64_t n = P->n, nnz = P->nnzG;
-  DevBuf k0, k1, s0, tmp;
-  DGP_TRY(k0.alloc(sizeof(uint64_t) * nnz));
-  DGP_TRY(k1.alloc(sizeof(uint64_t) * nnz));
-  DGP_TRY(s0.alloc(sizeof(int32_t) * nnz));
-  DGP_TRY(P->permT.alloc(sizeof(int32_t) * nnz));
-  DGP_TRY(P->rowptrT.alloc(sizeof(int32_t) * (n + 1)));
-  DGP_TRY(P->colT.alloc(sizeof(int32_t) * nnz));
+  ScratchBuf k0, k1, s0, tmp;
+  DGP_TRY(k0.alloc(sizeof(uint64_t) * nnz, st));
+  DGP_TRY(k1.alloc(sizeof(uint64_t) * nnz, st));
+  DGP_TRY(s0.alloc(sizeof(int32_t) * nnz, st));
+  DGP_TRY(P->permT.alloc_plan(sizeof(int32_t) * nnz));
+  DGP_TRY(P->rowptrT.alloc_plan(sizeof(int32_t) * (n + 1)));
+  DGP_TRY(P->colT.alloc_plan(sizeof(int32_t) * nnz));
   k_transpose_keys<<<grid1(n, 256), 256, 0, st>>>(P->rowptr.as<int32_t>(), P->col.as<int32_t>(), n,
                                                  k0.as<uint64_t>(), s0.as<int32_t>());
   DGP_CHECK_LAUNCH();
   size_t tb = 0;
   DGP_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, k0.as<uint64_t>(), k1.as<uint64_t>(), s0.as<int32_t>(),
                                            P->permT.as<int32_t>(), (int)nnz, 0, 64, st));
-  DGP_TRY(tmp.alloc(tb));
+  DGP_TRY(tmp.alloc(tb, st));
   DGP_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tb, k0.as<uint64_t>(), k1.as<uint64_t>(), s0.as<int32_t>(),
                                            P->permT.as<int32_t>(), (int)nnz, 0, 64, st));
   k_transpose_fill<<<grid1(nnz, 256), 256, 0, st>>>(k1.as<uint64_t>(), nnz, n, P->rowptrT.as<int32_t>(),
@@ -284,8 +284,8 @@ int fsai_factor_full(const int32_t *d_rowptr, const int32_t *d_col, const double
   DGP_REQUIRE(n > 0 && nf > 0, "fsai_factor: sizes must be positive");
   DGP_TRY(csr_in_range(d_rowptr, d_col, n, n, -1, 0, "fsai_factor: A", st));
   DGP_TRY(csr_in_range(d_rowptrG, d_colG, n, n, -1, 0, "fsai_factor: G pattern", st));
-  DevBuf m, im;
-  DGP_TRY(m.alloc(sizeof(int)));
+  ScratchBuf m, im;
+  DGP_TRY(m.alloc(sizeof(int), st));
   DGP_CUDA(cudaMemsetAsync(m.p, 0, sizeof(int), st));
   k_max_row<<<grid1(n, 256), 256, 0, st>>>(d_rowptrG, n, m.as<int>());
   DGP_CHECK_LAUNCH();
@@ -295,7 +295,7 @@ int fsai_factor_full(const int32_t *d_rowptr, const int32_t *d_col, const double
   DGP_CUDA(cudaMemcpyAsync(&nnzA, d_rowptr + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
   DGP_CUDA(cudaStreamSynchronize(st));
   // Im A = (df/c) * M, formed like the reference before the factor (dMesh.m:1241)
-  DGP_TRY(im.alloc(sizeof(double) * (size_t)nnzA));
+  DGP_TRY(im.alloc(sizeof(double) * (size_t)nnzA, st));
   k_scale<<<grid1(nnzA, 256), 256, 0, st>>>(d_M, dfc, nnzA, im.as<double>());
   DGP_CHECK_LAUNCH();
   DGP_TRY(fsai_factor_run(d_rowptr, d_col, d_K, im.as<double>(), n, d_rowptrG, d_colG, hm, nf, d_G, 1, nnzG, st));

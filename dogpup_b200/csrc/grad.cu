@@ -85,10 +85,10 @@ int tg_adjoint_rhs(const int32_t *d_det_nodes, const double *d_det_w, int32_t nd
     std::vector<int32_t> fill(rowp.begin(), rowp.end() - 1);
     for (int m = 0; m < nm; ++m) idx[fill[hl[2 * m]]++] = m;
   }
-  DevBuf ws;
+  ScratchBuf ws;
   const size_t coef_bytes = sizeof(double2) * (size_t)nm * nf;
   const size_t meta = sizeof(int32_t) * ((size_t)ns + 1 + nm) + sizeof(int);
-  DGP_TRY(ws.alloc(coef_bytes + meta));
+  DGP_TRY(ws.alloc(coef_bytes + meta, st));
   double2 *c = ws.as<double2>();
   int32_t *d_rowp = (int32_t *)((char *)ws.p + coef_bytes);
   int32_t *d_idx = d_rowp + ns + 1;

@@ -891,9 +891,9 @@ int jacobian_run(int mode, const int32_t *prow, const int32_t *pcol, const doubl
     DGP_REQUIRE(pcol && pval, "jacobian: null basis column or value array");
     DGP_TRY(csr_in_range(prow, pcol, nv, nn, -1, PMAX, "jacobian basis", st));
   }
-  DevBuf ctab, finv, chat;
-  DGP_TRY(ctab.alloc(sizeof(float2) * (size_t)std::max(1, ng) * nf));
-  DGP_TRY(finv.alloc(sizeof(double2) * nf));
+  ScratchBuf ctab, finv, chat;
+  DGP_TRY(ctab.alloc(sizeof(float2) * (size_t)std::max(1, ng) * nf, st));
+  DGP_TRY(finv.alloc(sizeof(double2) * nf, st));
   int nt_ = std::max(ng * nf, nf);
   k_ctab<<<(unsigned)ceil_div(nt_, 256), 256, 0, st>>>((const double2 *)gate, (const double2 *)fpsf, mode == 1 ? 0 : ng,
                                                         nf, nt, ctab.as<float2>(), finv.as<double2>());
@@ -906,8 +906,8 @@ int jacobian_run(int mode, const int32_t *prow, const int32_t *pcol, const doubl
   if (tc_fits && g_jacobian_engine != 1) {
     // tensor cores: one persistent warp-specialised CTA per SM
     const int dense = !links_dense ? 0 : (!rytov && nd % 4 == 0 && nm % 4 == 0) ? 2 : 1;
-    DevBuf flag;
-    DGP_TRY(flag.alloc(sizeof(int)));
+    ScratchBuf flag;
+    DGP_TRY(flag.alloc(sizeof(int), st));
     DGP_CUDA(cudaMemsetAsync(flag.p, 0, sizeof(int), st));
     DGP_TRY(allow_dyn_smem(k_jacobian_tg_tc, smem_tc));
     const int gtc = (int)std::min<int64_t>(nv, (int64_t)sm_count());
@@ -925,8 +925,8 @@ int jacobian_run(int mode, const int32_t *prow, const int32_t *pcol, const doubl
     const int ngc = ng <= 8 ? 8 : ng <= 16 ? 16 : ng <= 24 ? 24 : 32;
     // measurements per thread: 4 while the accumulators fit two blocks per SM (<= 16 gates), else 2
     const int mt = (nm > 2 * JBS && ngc <= 16) ? 4 : nm > JBS ? 2 : 1;
-    DevBuf ckg;
-    DGP_TRY(ckg.alloc(sizeof(float2) * (size_t)nf * ngc));
+    ScratchBuf ckg;
+    DGP_TRY(ckg.alloc(sizeof(float2) * (size_t)nf * ngc, st));
     k_ctab_kg<<<(unsigned)ceil_div((int64_t)nf * ngc, 256), 256, 0, st>>>(ctab.as<float2>(), ng, nf, ngc,
                                                                           ckg.as<float2>());
     DGP_CHECK_LAUNCH();
@@ -956,15 +956,15 @@ int jacobian_run(int mode, const int32_t *prow, const int32_t *pcol, const doubl
     k_jacobian_complex<<<grid, JBS, smem, st>>>(a, finv.as<double2>(), (double2 *)out);
   } else {
     DGP_REQUIRE(gin, "jacobian vjp: null upstream gradient");
-    DGP_TRY(chat.alloc(sizeof(float2) * (size_t)nm * nf));
+    DGP_TRY(chat.alloc(sizeof(float2) * (size_t)nm * nf, st));
     k_chat<<<(unsigned)ceil_div((int64_t)nm * nf, 256), 256, 0, st>>>(gin, ctab.as<float2>(), rytov, nm, ng, nf,
                                                                       chat.as<float2>());
     DGP_CHECK_LAUNCH();
     if (g_jacobian_engine != 1 && ns <= 32 && nd <= 32 && nm <= 4096) {
       // tensor cores: per-harmonic complex GEMM over voxel tiles
-      DevBuf btab, flag;
-      DGP_TRY(btab.alloc((size_t)nf * 2 * VT_B));
-      DGP_TRY(flag.alloc(sizeof(int)));
+      ScratchBuf btab, flag;
+      DGP_TRY(btab.alloc((size_t)nf * 2 * VT_B, st));
+      DGP_TRY(flag.alloc(sizeof(int), st));
       DGP_CUDA(cudaMemsetAsync(flag.p, 0, sizeof(int), st));
       k_vjp_btab<<<(unsigned)ceil_div((int64_t)nf * 1024, 256), 256, 0, st>>>(chat.as<float2>(), link, nm, nf,
                                                                               btab.as<unsigned char>());

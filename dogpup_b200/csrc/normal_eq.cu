@@ -399,12 +399,12 @@ int normal_eq_run(const float *Jt, int64_t nv, int64_t nm, const double *W, cons
               "normal_eq: damping mode is 0 (lam*max diag), 1 (lam*diag) or 2 (lam)");
   const int64_t nvp = ceil_div(nv, TM) * TM, nmp = ceil_div(nm, TK) * TK;
   DGP_REQUIRE(nmp < (int64_t)INT32_MAX && nvp < (int64_t)INT32_MAX, "normal_eq: sizes exceed TMA coordinates");
-  DevBuf hi, lo, diag, errb, sw;
-  DGP_TRY(hi.alloc(sizeof(__nv_bfloat16) * (size_t)nvp * nmp));
-  DGP_TRY(lo.alloc(sizeof(__nv_bfloat16) * (size_t)nvp * nmp));
-  DGP_TRY(diag.alloc(sizeof(double) * (nv + 1)));
-  DGP_TRY(sw.alloc(sizeof(float) * nmp));
-  DGP_TRY(errb.alloc(sizeof(int)));
+  ScratchBuf hi, lo, diag, errb, sw;
+  DGP_TRY(hi.alloc(sizeof(__nv_bfloat16) * (size_t)nvp * nmp, st));
+  DGP_TRY(lo.alloc(sizeof(__nv_bfloat16) * (size_t)nvp * nmp, st));
+  DGP_TRY(diag.alloc(sizeof(double) * (nv + 1), st));
+  DGP_TRY(sw.alloc(sizeof(float) * nmp, st));
+  DGP_TRY(errb.alloc(sizeof(int), st));
   double *dmax = diag.as<double>() + nv;
   DGP_CUDA(cudaMemsetAsync(errb.p, 0, sizeof(int), st));
   DGP_CUDA(cudaMemsetAsync(dmax, 0, sizeof(double), st));
@@ -499,27 +499,27 @@ int lm_update_run(const float *Jt, int64_t nv, int64_t nm, const double *W, cons
     // an even leading dimension keeps every row 16-byte aligned: the Cholesky's GEMMs then move
     // their operands with 16-byte copies
     const int64_t ldh = nv + (nv & 1);
-    DevBuf H;
-    DGP_TRY(H.alloc(sizeof(double) * (size_t)nv * ldh));
+    ScratchBuf H;
+    DGP_TRY(H.alloc(sizeof(double) * (size_t)nv * ldh, st));
     DGP_TRY(normal_eq_run(Jt, nv, nm, W, y, lam, 0, H.as<double>(), ldh, x, st));
     return cholesky_solve_run(H.as<double>(), nv, ldh, x, st);
   }
   const int64_t nmp = ceil_div(nm, TM) * TM, nvp = ceil_div(nv, TK) * TK;
   DGP_REQUIRE(nmp < (int64_t)INT32_MAX && nvp < (int64_t)INT32_MAX, "lm_update: sizes exceed TMA coordinates");
   DGP_REQUIRE(nvp / 64 <= 65535, "lm_update: too many unknowns for the transpose grid");
-  DevBuf diag, hi, lo, G, z, errb, sw, part;
-  DGP_TRY(errb.alloc(sizeof(int)));
+  ScratchBuf diag, hi, lo, G, z, errb, sw, part;
+  DGP_TRY(errb.alloc(sizeof(int), st));
   DGP_CUDA(cudaMemsetAsync(errb.p, 0, sizeof(int), st));
   if (W) DGP_TRY(check_weights(W, nm, errb.as<int>(), "lm_update", st));
   const int64_t nd = std::max(nv, nm);
-  DGP_TRY(diag.alloc(sizeof(double) * (nd + 1)));
-  DGP_TRY(hi.alloc(sizeof(__nv_bfloat16) * (size_t)nmp * nvp));
-  DGP_TRY(lo.alloc(sizeof(__nv_bfloat16) * (size_t)nmp * nvp));
-  DGP_TRY(part.alloc(sizeof(double) * (size_t)(nvp / 64) * nmp));
-  DGP_TRY(sw.alloc(sizeof(float) * nmp));
+  DGP_TRY(diag.alloc(sizeof(double) * (nd + 1), st));
+  DGP_TRY(hi.alloc(sizeof(__nv_bfloat16) * (size_t)nmp * nvp, st));
+  DGP_TRY(lo.alloc(sizeof(__nv_bfloat16) * (size_t)nmp * nvp, st));
+  DGP_TRY(part.alloc(sizeof(double) * (size_t)(nvp / 64) * nmp, st));
+  DGP_TRY(sw.alloc(sizeof(float) * nmp, st));
   const int64_t ldg = nm + (nm & 1);
-  DGP_TRY(G.alloc(sizeof(double) * (size_t)nm * ldg));
-  DGP_TRY(z.alloc(sizeof(double) * nm));
+  DGP_TRY(G.alloc(sizeof(double) * (size_t)nm * ldg, st));
+  DGP_TRY(z.alloc(sizeof(double) * nm, st));
   double *dmax = diag.as<double>() + nd;
   DGP_CUDA(cudaMemsetAsync(dmax, 0, sizeof(double), st));
   // mu = lam max_i (J^T W J)_ii

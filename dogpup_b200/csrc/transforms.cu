@@ -147,8 +147,8 @@ int meas_run(const int32_t *dn, const double *dw, int nd, const int32_t *link, i
              int ns, double *data, cudaStream_t st) {
   DGP_REQUIRE(dn && dw && link && phi && data, "meas: null pointer");
   DGP_REQUIRE(nm > 0 && n > 0 && nf > 0 && ns > 0, "meas: sizes must be positive");
-  DevBuf flag;
-  DGP_TRY(flag.alloc(sizeof(int)));
+  ScratchBuf flag;
+  DGP_TRY(flag.alloc(sizeof(int), st));
   DGP_CUDA(cudaMemsetAsync(flag.p, 0, sizeof(int), st));
   k_meas<<<g1((int64_t)nm * nf, 128), 128, 0, st>>>(dn, dw, nd, link, nm, (const double2 *)phi, n, nf, ns,
                                                      (double2 *)data, flag.as<int>());

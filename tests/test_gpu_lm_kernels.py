@@ -53,3 +53,41 @@ def test_cholesky_wide_panels(n):
     check(lib.dgp_cholesky_solve(_v(H), n, n, _v(x), None))
     S = torch.tril(H0) + torch.tril(H0, -1).T
     assert float((S @ x - b).norm() / b.norm()) < 1e-9
+
+
+def test_lm_update_from_several_host_threads():
+    """Calls on their own streams share the library's scratch memory and Cholesky streams: each gives what
+    it gives alone, bit for bit (no atomics in its sums)."""
+    import threading
+    import torch
+    from dogpup_b200._lib import lib
+    sizes = [(300, 700), (900, 400), (513, 2100), (1700, 1600)]
+    g = torch.Generator(device="cuda").manual_seed(5)
+    data = [(torch.randn((nv, nm), generator=g, device="cuda"),
+             torch.randn(nm, generator=g, dtype=torch.float64, device="cuda")) for nv, nm in sizes]
+
+    def call(i, x, stream):
+        J, y = data[i]
+        return lib.dgp_lm_update(_v(J), J.shape[0], J.shape[1], None, _v(y), 0.2, _v(x), 0, None, stream)
+
+    alone = [torch.empty(nv, dtype=torch.float64, device="cuda") for nv, _ in sizes]
+    for i, x in enumerate(alone):
+        assert call(i, x, None) == 0
+    torch.cuda.synchronize()
+    out = [[torch.empty_like(x) for _ in range(4)] for x in alone]
+    rcs = []
+
+    def work(i):
+        s = torch.cuda.Stream()
+        for x in out[i]:
+            rcs.append(call(i, x, s.cuda_stream))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(sizes))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert rcs == [0] * 16
+    for a, xs in zip(alone, out):
+        assert all(torch.equal(a, x) for x in xs)
