@@ -1394,17 +1394,6 @@ __global__ void __launch_bounds__(1024) k_stage_init(Cols c, Ctl *ctl, int nsp, 
   }
 }
 
-// final statuses: active columns below tol are converged, the rest hit maxit
-__global__ void __launch_bounds__(1024) k_stage_final(Cols c, Ctl *ctl) {
-  const double tol = ctl->tol;
-  for (int64_t j = threadIdx.x; j < c.C; j += blockDim.x) {
-    if (c.status[j] == DGP_COL_MAXIT || c.active[j]) {
-      c.status[j] = (c.err[j] < tol || (ctl->reason == 0 && ctl->stop_rule == DGP_STOP_MAX_ALL))
-                        ? DGP_COL_CONVERGED : DGP_COL_MAXIT;
-    }
-  }
-}
-
 // mixed precision: a column's status is decided by its FP64 residual
 __global__ void k_status_outer(Cols c, const double *__restrict__ outer_err, double tol, int nsp, int ns) {
   int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -1415,48 +1404,6 @@ __global__ void k_status_outer(Cols c, const double *__restrict__ outer_err, dou
   if (st == DGP_COL_BREAKDOWN_RHO || st == DGP_COL_BREAKDOWN_OMEGA || st == DGP_COL_NONFINITE) return;
   if (st == DGP_COL_ZERO_RHS) return;
   c.status[j] = outer_err[j] < tol ? DGP_COL_CONVERGED : DGP_COL_MAXIT;
-}
-
-// ------------------------------------------------ user layout <-> workspace
-// dst[k][i][s] (nsp) = (T) src[k][i][s] (ns), zero padding
-template <class R>
-__global__ void k_pack(int64_t n, int nf, int nsp, int ns, const double2 *__restrict__ src,
-                       typename CT<R>::C *__restrict__ dst) {
-  const int64_t tot = (int64_t)nf * n * nsp;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
-    const int s = (int)(e % nsp);
-    const int64_t ki = e / nsp;
-    double2 v = s < ns ? src[ki * ns + s] : make_double2(0, 0);
-    dst[e] = cvt<R>(v);
-  }
-}
-
-template <class R>
-__global__ void k_unpack(int64_t n, int nf, int nsp, int ns, const typename CT<R>::C *__restrict__ src,
-                         double2 *__restrict__ dst) {
-  const int64_t tot = (int64_t)nf * n * ns;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
-    const int s = (int)(e % ns);
-    const int64_t ki = e / ns;
-    dst[e] = d2(src[ki * nsp + s]);
-  }
-}
-
-// point-source right-hand sides (dMesh.m:124-129): b[k][node][s] = w * fpsf[k]
-template <class R>
-__global__ void k_sources(int64_t n, int nf, int nsp, int ns, const int32_t *__restrict__ nodes,
-                          const double *__restrict__ w, const double2 *__restrict__ fpsf,
-                          typename CT<R>::C *__restrict__ b) {
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= (int64_t)nf * ns) return;
-  const int k = (int)(t / ns), s = (int)(t % ns);
-  for (int l = 0; l < 4; ++l) {
-    const int32_t nd = nodes[4 * s + l];
-    if (nd < 0 || nd >= n) continue;  // rejected on the host before the solve
-    // the reference assigns (not accumulates) the 4 weights of a tet's distinct nodes
-    double2 v = make_double2(w[4 * s + l] * fpsf[k].x, w[4 * s + l] * fpsf[k].y);
-    b[((int64_t)k * n + nd) * nsp + s] = cvt<R>(v);
-  }
 }
 
 __global__ void k_check_nodes(const int32_t *__restrict__ nodes, int ns, int64_t n, int *bad) {
@@ -1847,14 +1794,7 @@ int ensure_workspace(SolverPlan *S, int prec, int nvec = NVEC_ALL) {
   const size_t esz = prec == DGP_PREC_FP64 ? sizeof(double2) : sizeof(float2);
   const size_t vb = esz * (size_t)C * S->n;
   if (S->ws_prec != prec) {
-    S->drop_fused();
-    for (auto &g : S->graph)
-      if (g) {
-        cudaGraphExecDestroy(g);
-        g = nullptr;
-      }
-    for (int &gi : S->graph_iters) gi = 0;
-    for (auto &v : S->vec) v.release();
+    S->drop_workspaces();
     DGP_TRY(S->scal.alloc_plan(scal_bytes(C)));
     DGP_TRY(S->status.alloc_plan(sizeof(int) * C));
     DGP_TRY(S->ctl.alloc_plan(sizeof(Ctl)));
@@ -2064,13 +2004,6 @@ int enqueue_for(SolverPlan *S, const Vecs<R> &V, const Work &W, cudaStream_t st,
     OpA32 A{rp, S->RecA32.as<Rec32>(), (const float *)(S->omega.as<char>() + sizeof(double) * S->nf)};
     OpG32 G{S->P.rowptr.as<int32_t>(), S->RecG32.as<Rec32>(), S->nnzG};
     OpG32 GT{S->P.rowptrT.as<int32_t>(), S->RecGT32.as<Rec32>(), S->nnzG};
-    if (what == ENQ_COCG) enqueue_cocg<R, VS, VD>(S, A, G, GT, V, W, st);
-    else if (what == ENQ_COCG_START) enqueue_cocg_start<R, VS, VD>(S, G, GT, V, W, st);
-    else enqueue_iteration<R, VS, VD>(S, A, G, GT, V, W, st);
-  } else {
-    OpA64 A{rp, S->col.as<int32_t>(), S->KM64.as<double2>(), S->omega.as<double>()};
-    OpG64 G{S->P.rowptr.as<int32_t>(), S->P.col.as<int32_t>(), S->G64.as<double2>(), S->nnzG};
-    OpG64 GT{S->P.rowptrT.as<int32_t>(), S->P.colT.as<int32_t>(), S->GT64.as<double2>(), S->nnzG};
     if (what == ENQ_COCG) enqueue_cocg<R, VS, VD>(S, A, G, GT, V, W, st);
     else if (what == ENQ_COCG_START) enqueue_cocg_start<R, VS, VD>(S, G, GT, V, W, st);
     else enqueue_iteration<R, VS, VD>(S, A, G, GT, V, W, st);
@@ -2293,23 +2226,25 @@ void launch_residual(SolverPlan *S, int ns, const double *d_X, const double *d_B
 
 }  // namespace
 
-void SolverPlan::drop_fused() {
-  for (auto &g : fgraph)
-    if (g) {
-      cudaGraphExecDestroy(g);
-      g = nullptr;
+void SolverPlan::drop_workspaces() {
+  for (cudaGraphExec_t *g : {graph, graph + 1, graph + 2, graph + 3, graph + 4, graph + 5, fgraph, fgraph + 1, dgraph,
+                             dgraph + 1})
+    if (*g) {
+      cudaGraphExecDestroy(*g);
+      *g = nullptr;
     }
+  for (int &i : graph_iters) i = 0;
   for (int &i : fgraph_iters) i = 0;
+  for (auto &v : vec) v.release();
   for (auto &v : fvec) v.release();
-  fscal.release();
-  fctl.release();
+  for (auto &v : dvec) v.release();
+  for (DevBuf *b : {&fscal, &dscal, &dpart, &fctl}) b->release();
+  ws_prec = -1;
 }
 
 SolverPlan::~SolverPlan() {
   if (busy) cudaDeviceSynchronize();  // a call that ended early may have left work on the buffers
-  drop_fused();
-  for (auto &g : graph)
-    if (g) cudaGraphExecDestroy(g);
+  drop_workspaces();
   for (auto &e : poll_ev)
     if (e) cudaEventDestroy(e);
   if (h_ctl) cudaFreeHost(h_ctl);
@@ -2412,53 +2347,6 @@ int solver_build(SolverPlan *S, const int32_t *d_rowptr, const int32_t *d_col, i
   return solver_update(S, d_K, d_M, st);
 }
 
-// FP64 reference-semantics solve (DGP_PREC_FP64)
-static int solve_fp64(SolverPlan *S, const double *d_B, const int32_t *d_nodes, const double *d_w,
-                      const double *d_fpsf, double *d_X, int ns, const dgp_solve_opts &o, dgp_solve_report *rep,
-                      cudaStream_t st) {
-  DGP_TRY(ensure_workspace(S, DGP_PREC_FP64));
-  Work W = work_views(S);
-  Vecs<double> V = vec_views<double>(S);
-  const int vec = vec_for(S, false);
-  const Layouts LL = layouts_for(S, vec);
-  const size_t vbytes = sizeof(double2) * (size_t)S->ws_cols * S->n;
-  // b -> r (workspace layout)
-  if (d_B) {
-    k_pack<double><<<g1((int64_t)S->ws_cols * S->n, 256), 256, 0, st>>>(S->n, S->nf, S->nsp, ns,
-                                                                         (const double2 *)d_B, V.r);
-  } else {
-    DGP_CUDA(cudaMemsetAsync(V.r, 0, vbytes, st));
-    k_sources<double><<<g1((int64_t)S->nf * ns, 128), 128, 0, st>>>(S->n, S->nf, S->nsp, ns, d_nodes, d_w,
-                                                                      (const double2 *)d_fpsf, V.r);
-  }
-  DGP_CHECK_LAUNCH();
-  DGP_TRY(set_ctl(W.ctl, o.tol, o.maxit, o.stop_rule, st, S->h_ctl));
-  launch_init<double, VU>(layouts_for(S, VU).Ld, V, W, st);
-  DGP_CHECK_LAUNCH();
-  k_stage_init<<<1, 1024, 0, st>>>(W.cols, W.ctl, S->nsp, ns);
-  DGP_CHECK_LAUNCH();
-  int iters = 0;
-  DGP_TRY(run_iterations<double>(S, V, W, o.check_every, o.maxit, st, &iters));
-  k_stage_final<<<1, 1024, 0, st>>>(W.cols, W.ctl);
-  DGP_CHECK_LAUNCH();
-  k_unpack<double><<<g1((int64_t)S->nf * S->n * ns, 256), 256, 0, st>>>(S->n, S->nf, S->nsp, ns, V.x,
-                                                                          (double2 *)d_X);
-  DGP_CHECK_LAUNCH();
-  // true FP64 residual of the returned solution, for the report (||b|| = ||r0|| since x0 = 0)
-  DGP_CUDA(cudaMemcpyAsync(W.bnorm, W.cols.err0, sizeof(double) * W.cols.C, cudaMemcpyDeviceToDevice, st));
-  DGP_CUDA(cudaMemsetAsync(W.cols.acc + ACC_NR * W.cols.C, 0, sizeof(double2) * W.cols.C, st));
-  launch_residual(S, ns, d_X, d_B, d_nodes, d_w, d_fpsf, (float2 *)V.T1, W, st);
-  k_outer_norms<<<1, 1024, 0, st>>>(W.cols, W.bnorm, W.outer_err, W.ctl, 1, S->nsp, ns);
-  DGP_CHECK_LAUNCH();
-  Ctl hc;
-  DGP_CUDA(cudaMemcpyAsync(&hc, W.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
-  DGP_CUDA(cudaStreamSynchronize(st));
-  rep->iterations = iters;
-  rep->refinements = 0;
-  rep->max_rel_residual = hc.max_err;
-  return hc.reason == 1 ? DGP_ERR_NOT_CONVERGED : DGP_OK;
-}
-
 // mixed precision: complex-FP32 inner solves (COCG, or BiCGSTAB for DGP_PREC_MIXED_BICGSTAB)
 // inside FP64 iterative refinement
 static int solve_mixed(SolverPlan *S, const double *d_B, const int32_t *d_nodes, const double *d_w,
@@ -2551,22 +2439,23 @@ int solver_solve(SolverPlan *S, const double *d_B, const int32_t *d_nodes, const
   }
   dgp_solve_report local{};
   dgp_solve_report *r = rep ? rep : &local;
-  const bool fused = o.precision == DGP_PREC_MIXED && !S->unfused;
-  const int rc = o.precision == DGP_PREC_FP64 ? solve_fp64(S, d_B, d_nodes, d_w, d_fpsf, d_X, ns, o, r, st)
+  const bool fp64 = o.precision == DGP_PREC_FP64, fused = o.precision == DGP_PREC_MIXED && !S->unfused;
+  const int rc = fp64 ? solve_fp64(S, d_B, d_nodes, d_w, d_fpsf, d_X, ns, o, r, st)
                  : fused ? solve_fused(S, d_B, d_nodes, d_w, d_fpsf, d_X, ns, o, r, st)
                          : solve_mixed(S, d_B, d_nodes, d_w, d_fpsf, d_X, ns, o, r, st);
   if (rc != DGP_OK && rc != DGP_ERR_NOT_CONVERGED) return rc;
   // per-column statuses for the caller (harmonic-major, ns columns per harmonic)
-  const int nsp = fused ? S->fnsp : S->nsp;
+  const int nsp = fp64 || fused ? S->fnsp : S->nsp;
+  const int *d_st = fp64 || fused ? S->last_status : S->status.as<int>();
   std::vector<int> hs((size_t)S->nf * nsp);
-  DGP_CUDA(cudaMemcpyAsync(hs.data(), fused ? (const void *)fused_status(S) : S->status.p, sizeof(int) * hs.size(),
-                           cudaMemcpyDeviceToHost, st));
+  DGP_CUDA(cudaMemcpyAsync(hs.data(), d_st, sizeof(int) * hs.size(), cudaMemcpyDeviceToHost, st));
   DGP_CUDA(cudaStreamSynchronize(st));
   int bad = 0;
   std::vector<int> out((size_t)S->nf * ns);
   for (int k = 0; k < S->nf; ++k)
     for (int s = 0; s < ns; ++s) {
       int v = hs[(size_t)k * nsp + s];
+      if (v == DGP_COL_NONFINITE) r->max_rel_residual = INFINITY;
       if (v == DGP_COL_ZERO_RHS) v = DGP_COL_CONVERGED;  // x = 0 solves b = 0 exactly
       out[(size_t)k * ns + s] = v;
       bad += v != DGP_COL_CONVERGED;

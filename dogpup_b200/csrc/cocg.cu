@@ -35,49 +35,14 @@
 
 #include "dgp_common.cuh"
 #include "dgp_internal.h"
-#include "sweep.cuh"
+#include "fused.cuh"
 
 namespace dgp {
 
 namespace {
 
-using namespace sweep;
-
-constexpr double TINY = 1e-290;  // smallest right-hand-side norm that is scaled to 1
-
 enum { ST_RUNNING = 0, ST_DONE = 2 };
 enum { F_A = 0, F_G = 1, F_GT = 2, F_G0 = 3, F_GT0 = 4 };
-
-struct FCtl {
-  int state, iters, maxit, na, nr, n_active, ctas, loops;
-  int stall_since, reason;
-  unsigned long long err_bits, max_err_bits;
-  double max_err, stall_ref;
-};
-
-struct FCols {  // per-column state, C = nf * nsp columns
-  int64_t C;
-  int nsp;
-  double *bnorm, *oerr, *tolc, *t0, *acc;  // acc: [3][C]
-  double2 *rho;
-  float2 *alpha, *beta;
-  int *act, *status;            // act: 1 iterating, 2 its last x update is pending, 0 done
-  int *hact, *list, *rlist, *cnt, *mem;  // [nf] active flag, active harmonics, the round's harmonics, steps done, level members
-};
-
-// max of non-negative doubles (their bits order like integers)
-__device__ __forceinline__ void max_bits(unsigned long long *dst, double v) {
-  atomicMax(dst, (unsigned long long)__double_as_longlong(v));
-}
-
-__device__ __forceinline__ double2 load_acc(FCols &c, int64_t j, int q) {
-  double *p = c.acc + q * c.C + j;
-  const double v = __ldcg(p);
-  *p = 0.0;
-  return make_double2(v, 0.0);
-}
-
-__device__ __forceinline__ bool finite2(double2 a) { return isfinite(a.x) && isfinite(a.y); }
 
 // scalars of column j once its harmonic has finished a sweep
 template <int MODE> __device__ void column_scalars(FCols &c, FCtl *ctl, int64_t j) {
@@ -146,27 +111,7 @@ struct FSweep {
 
 // after the third sweep, by the last block: next iteration's list, stop tests
 __device__ void end_iteration(const FSweep &a, FCtl *ctl) {
-  __shared__ int s_cnt, s_warp[WARPS];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) s_cnt = 0;
-  __syncthreads();
-  const int na = ctl->na;
-  for (int q0 = 0; q0 < na; q0 += BS) {  // stable compaction, BS entries at a time (in place: only shrinks)
-    const int q = q0 + threadIdx.x;
-    const int k = q < na ? a.c.list[q] : 0;
-    const bool keep = q < na && __ldcg(a.c.hact + k) != 0;
-    const unsigned m = __ballot_sync(0xffffffffu, keep);
-    if (lane == 0) s_warp[warp] = __popc(m);
-    __syncthreads();
-    int at = s_cnt + __popc(m & ((1u << lane) - 1u));
-    for (int w = 0; w < warp; ++w) at += s_warp[w];
-    if (q < na) a.c.hact[k] = 0;
-    if (keep) a.c.list[at] = k;
-    __syncthreads();
-    if (threadIdx.x == 0)
-      for (int w = 0; w < WARPS; ++w) s_cnt += s_warp[w];
-    __syncthreads();
-  }
+  const int s_cnt = compact_active(a.c, ctl->na);
   if (threadIdx.x == 0) {
     const double e = __longlong_as_double((long long)__ldcg(&ctl->err_bits));
     ctl->err_bits = 0ull;
@@ -343,7 +288,7 @@ template <int VEC, int MODE> __global__ void __launch_bounds__(BS, 2) k_fsweep(c
       for (int v = 0; v < VEC; ++v)
 #pragma unroll
         for (int q = 0; q < NQ; ++q) d[v][q] = (double)part[v][q];
-      warp_add<VEC, NQ, false>(g, lane, sub, rsub, d, slots + warp * g.nsp * NQ);
+      warp_add<VEC, NQ, VEC>(g, lane, sub, rsub, d, slots + warp * g.nsp * NQ);
     }
     done += s1 - s0;
   }
@@ -386,150 +331,6 @@ __global__ void k_fbnorm(FCols c, int nf, int ns, const double *__restrict__ w, 
   c.bnorm[j] = r;
   c.oerr[j] = r > 0.0 || !(r == r) ? 1.0 : 0.0;
   c.status[j] = isfinite(r) ? DGP_COL_ZERO_RHS : DGP_COL_NONFINITE;
-}
-
-struct FResid {
-  Geo g;                    // FP64 mapping: column v * lpr + sub
-  int ns, mode;             // mode 0: |b| only; 1: write scaled residual, oerr
-  const int32_t *rowptr, *col;
-  const double2 *KM;
-  const double *omega;
-  const double2 *X, *B;     // [nf][n][ns]; X NULL: zero
-  const int32_t *snodes;
-  const double *sw;
-  const double2 *fpsf;
-  float2 *r32;              // [nf][n][nsp]
-  FCols c;
-  FCtl *ctl;
-  const int *list;
-  int nlist;
-};
-
-// FP64 residual b - A_k X of the listed harmonics, written as FP32 scaled by 1 / |b|, with its
-// norm relative to |b| per column; b is dense or the point sources formed on the fly.
-template <int VEC> __global__ void __launch_bounds__(BS) k_fresid(const FResid a) {
-  const Geo &g = a.g;
-  extern __shared__ __align__(16) unsigned char sm[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int sub = lane % g.lpr, rsub = lane / g.lpr;
-  unsigned char *wbuf = sm + (size_t)warp * 2 * g.cap * 20;
-  double *swt = reinterpret_cast<double *>(sm + (size_t)WARPS * 2 * g.cap * 20 + 128);  // [nsp][4]
-  double *slots = swt + 4 * g.nsp;                                                // [WARPS][nsp]
-  int *sn = reinterpret_cast<int *>(slots + WARPS * g.nsp);                       // [nsp][4]
-  __shared__ int s_last;
-  for (int t = threadIdx.x; t < WARPS * g.nsp; t += BS) slots[t] = 0.0;
-  for (int t = threadIdx.x; t < 4 * g.nsp; t += BS) {
-    const bool ok = a.snodes && t / 4 < a.ns;
-    sn[t] = ok ? a.snodes[t] : -1;
-    swt[t] = ok ? a.sw[t] : 0.0;
-  }
-  __syncthreads();
-  const int per = g.steps;
-  const int csz = (int)max((int64_t)1, min((int64_t)CHUNK, (int64_t)a.nlist * per / gridDim.x));
-  const int nch = (per + csz - 1) / csz;
-  const int64_t total = (int64_t)a.nlist * nch;
-  int nv = 0;
-#pragma unroll
-  for (int v = 0; v < VEC; ++v) nv += v * g.lpr + sub < a.ns;
-  int ai = -1, k = 0, done = 0;
-  double sc[VEC];
-  auto flush = [&]() {
-    __syncthreads();
-    for (int t = threadIdx.x; t < g.nsp; t += BS) {
-      double x = 0.0;
-#pragma unroll
-      for (int w = 0; w < WARPS; ++w) {
-        x += slots[w * g.nsp + t];
-        slots[w * g.nsp + t] = 0.0;
-      }
-      atomicAdd(a.c.acc + (int64_t)k * g.nsp + t, x);
-    }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      const int old = atomicAdd(a.c.cnt + k, done);
-      s_last = old + done == per;
-      if (s_last) a.c.cnt[k] = 0;
-      __threadfence();
-    }
-    __syncthreads();
-    if (s_last) {
-      FCols c = a.c;
-      for (int t = threadIdx.x; t < g.nsp; t += BS) {
-        const int64_t j = (int64_t)k * g.nsp + t;
-        const double r = sqrt(load_acc(c, j, 0).x);
-        if (a.mode == 0) {
-          c.bnorm[j] = t < a.ns ? r : 0.0;
-          c.oerr[j] = t < a.ns && !(r == 0.0) ? 1.0 : 0.0;
-          c.status[j] = t < a.ns && !isfinite(r) ? DGP_COL_NONFINITE : DGP_COL_ZERO_RHS;
-        } else if (t < a.ns && c.bnorm[j] > 0.0 && isfinite(c.bnorm[j])) {
-          c.oerr[j] = r;  // (rows are scaled by 1 / |b|)
-          max_bits(&a.ctl->max_err_bits, isfinite(r) ? r : INFINITY);
-        }
-      }
-    }
-    __syncthreads();
-  };
-  for (int64_t ch = blockIdx.x; ch < total; ch += gridDim.x) {
-    const int na_i = (int)(ch / nch), s0 = (int)(ch - (int64_t)na_i * nch) * csz, s1 = min(per, s0 + csz);
-    if (na_i != ai) {
-      if (ai >= 0) flush();
-      ai = na_i;
-      k = a.list[ai];
-      done = 0;
-#pragma unroll
-      for (int v = 0; v < VEC; ++v) {
-        const double b = a.mode ? a.c.bnorm[(int64_t)k * g.nsp + v * g.lpr + sub] : 1.0;
-        sc[v] = a.mode == 0 ? 1.0 : (b > 0.0 && isfinite(b)) ? 1.0 / fmax(b, TINY) : 0.0;
-      }
-    }
-    const Src<double> src{a.KM, a.col};
-    const double2 fk = a.fpsf ? a.fpsf[k] : make_double2(0.0, 0.0);
-    double part[VEC][1];
-#pragma unroll
-    for (int v = 0; v < VEC; ++v) part[v][0] = 0.0;
-    const double2 *X = a.X ? a.X + (int64_t)k * g.n * a.ns + sub : nullptr;
-    auto finish = [&](int i, bool valid, double2(&y)[VEC]) {
-      if (!valid) return;
-#pragma unroll
-      for (int v = 0; v < VEC; ++v) {
-        const int s = v * g.lpr + sub;
-        double2 r = make_double2(0.0, 0.0);
-        if (s < a.ns) {
-          if (a.B) {
-            r = a.B[((int64_t)k * g.n + i) * a.ns + s];
-          } else {
-            const int4 nd = *reinterpret_cast<const int4 *>(sn + 4 * s);
-            double wt = 0.0;
-            if (nd.x == i) wt = swt[4 * s];
-            if (nd.y == i) wt = swt[4 * s + 1];
-            if (nd.z == i) wt = swt[4 * s + 2];
-            if (nd.w == i) wt = swt[4 * s + 3];
-            r = make_double2(wt * fk.x, wt * fk.y);
-          }
-          r = make_double2((r.x - y[v].x) * sc[v], (r.y - y[v].y) * sc[v]);
-          if (sc[v] == 0.0) r = make_double2(0.0, 0.0);  // zero or non-finite right-hand side
-        }
-        part[v][0] = fma(r.x, r.x, fma(r.y, r.y, part[v][0]));
-        if (a.mode) a.r32[((int64_t)k * g.n + i) * g.nsp + s] = make_float2((float)r.x, (float)r.y);
-      }
-    };
-    if (X) {
-      rows<double, VEC>(g, a.rowptr, src, a.omega[k], X, a.ns, s0, s1, wbuf, lane, warp, rsub, nv > 0, nv,
-                              [](int, bool) {}, finish);
-    } else {
-      for (int step = s0; step < s1; ++step) {
-        const int i = (step * WARPS + warp) * g.rpw + rsub;
-        double2 y[VEC];
-#pragma unroll
-        for (int v = 0; v < VEC; ++v) y[v] = make_double2(0.0, 0.0);
-        finish(i, rsub < g.rpw && i < g.n, y);
-      }
-    }
-    warp_add<VEC, 1, true>(g, lane, sub, rsub, part, slots + warp * g.nsp);
-    done += s1 - s0;
-  }
-  if (ai >= 0) flush();
 }
 
 // Start of a round: columns still above tol are active, with their own relative target -- the
@@ -796,15 +597,7 @@ int fused_setup(SolverPlan *S, FWork *out) {
   const int nsp = S->fnsp;
   const int vec = nsp <= 8 ? 2 : 4;  // (at least two lanes per row: full warps down to 4 columns)
   if (!S->fscal.p) {
-    // the other precisions' vectors are dropped, as they drop these (one workspace per plan)
-    for (auto &g : S->graph)
-      if (g) {
-        cudaGraphExecDestroy(g);
-        g = nullptr;
-      }
-    for (int &gi : S->graph_iters) gi = 0;
-    for (auto &v : S->vec) v.release();
-    S->ws_prec = -1;
+    S->drop_workspaces();
     const size_t vb = sizeof(float2) * (size_t)S->nf * S->n * nsp;
     for (int i = 0; i < 4; ++i) DGP_TRY(S->fvec[i].alloc_plan(vb));
     DGP_TRY(S->fctl.alloc_plan(sizeof(FCtl)));
@@ -818,12 +611,24 @@ int fused_setup(SolverPlan *S, FWork *out) {
   w.vec = vec;
     w.g = make_geo<float>(S->n, S->nf, nsp, vec, 16);
   w.g64 = make_geo<double>(S->n, S->nf, nsp, vec, 16);
-  for (int m = 0; m < 5; ++m) {
-    const int nq = m == F_A ? 2 : (m == F_G || m == F_G0) ? 3 : 0;
-    w.sm[m] = stage_bytes<float>(w.g) + 16 * (size_t)nsp + 8 * (size_t)WARPS * nsp * nq;
+  SolverPlan::Shape &sh = S->shape32;
+  if (!sh.set) {
+    for (int m = 0; m < 5; ++m) {
+      const int nq = m == F_A ? 2 : (m == F_G || m == F_G0) ? 3 : 0;
+      w.sm[m] = stage_bytes<float>(w.g) + 16 * (size_t)nsp + 8 * (size_t)WARPS * nsp * nq;
+    }
+    w.sm64 = stage_bytes<double>(w.g64) + (size_t)nsp * (4 * 8 + WARPS * 8 + 4 * 4);
+    DGP_TRY(vec == 2 ? sweep_grids<2>(w, S->nf) : sweep_grids<4>(w, S->nf));
+    std::copy(w.grid, w.grid + 5, sh.grid);
+    std::copy(w.sm, w.sm + 5, sh.sm);
+    sh.grid[5] = w.grid64;
+    sh.sm[5] = w.sm64;
+    sh.set = true;
   }
-  w.sm64 = stage_bytes<double>(w.g64) + (size_t)nsp * (4 * 8 + WARPS * 8 + 4 * 4);
-  DGP_TRY(vec == 2 ? sweep_grids<2>(w, S->nf) : sweep_grids<4>(w, S->nf));
+  std::copy(sh.grid, sh.grid + 5, w.grid);
+  std::copy(sh.sm, sh.sm + 5, w.sm);
+  w.grid64 = sh.grid[5];
+  w.sm64 = sh.sm[5];
   *out = w;
   return DGP_OK;
 }
@@ -1151,6 +956,7 @@ int solve_fused(SolverPlan *S, const double *d_B, const int32_t *d_nodes, const 
                 double *d_X, int ns, const dgp_solve_opts &o, dgp_solve_report *rep, cudaStream_t st) {
   FWork w;
   DGP_TRY(fused_setup(S, &w));
+  S->last_status = w.c.status;
   const int first = first_level(S, d_nodes != nullptr);
   if (S->levels.empty() || S->levels_first != first) {
     plan_levels(S, first);
@@ -1239,8 +1045,6 @@ int solve_fused(SolverPlan *S, const double *d_B, const int32_t *d_nodes, const 
   rep->max_rel_residual = worst;
   return status;
 }
-
-const int *fused_status(SolverPlan *S) { return fwork(S).c.status; }
 
 // Times one sweep of the fused iteration (which: 0 A, 1 G, 2 G^T) on the plan's workspace with all
 // harmonics and columns active, CUDA events on st; its algorithmic bytes per launch.

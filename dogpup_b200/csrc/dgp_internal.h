@@ -128,14 +128,32 @@ struct SolverPlan {
   std::vector<Level> levels;
   int levels_first = -1;
   DevBuf lev_int, lev_coef;
-  void drop_fused();             // releases the fused workspace (another precision takes its place)
+  // ---- FP64 BiCGSTAB on fused sweeps (bicg64.cu)
+  DevBuf dvec[9], dscal, dpart;  // vectors; per-column state; chunks' partial sums
+  struct LoopKey {               // what a captured loop depends on besides the workspace
+    double tol = 0;
+    int stop_rule = -1, body = 0;
+    bool operator==(const LoopKey &o) const { return tol == o.tol && stop_rule == o.stop_rule && body == o.body; }
+  };
+  cudaGraphExec_t dgraph[2] = {nullptr, nullptr};  // host-polled, device-driven
+  LoopKey dgraph_key[2];
+  struct Shape {                 // grids and shared memory of a solve's kernels, asked for once per plan
+    bool set = false;
+    int grid[8] = {};
+    size_t sm[8] = {};
+  };
+  Shape shape32, shape64;
+  const int *last_status = nullptr;  // statuses of the last solve ([nf][fnsp], device)
+  void drop_workspaces();        // one solve's workspace at a time: frees the others'
   ~SolverPlan();
 };
 
-// the mixed COCG solve on fused sweeps; statuses of its last solve ([nf][fnsp], device)
+// the mixed COCG solve on fused sweeps
 int solve_fused(SolverPlan *S, const double *d_B, const int32_t *d_nodes, const double *d_w, const double *d_fpsf,
                 double *d_X, int ns, const dgp_solve_opts &o, dgp_solve_report *rep, cudaStream_t st);
-const int *fused_status(SolverPlan *S);
+// the FP64 solve (the reference's BiCGSTAB)
+int solve_fp64(SolverPlan *S, const double *d_B, const int32_t *d_nodes, const double *d_w, const double *d_fpsf,
+               double *d_X, int ns, const dgp_solve_opts &o, dgp_solve_report *rep, cudaStream_t st);
 int fused_profile(SolverPlan *S, int which, int reps, float *ms, double *bytes, cudaStream_t st);
 
 // h_harm: host list of the nf harmonic indices the plan solves (NULL = 0 .. nf-1)

@@ -140,8 +140,8 @@ template <int VEC> __device__ __forceinline__ void stw(float2 *p, const float2 (
 
 // One row's product y = sum (a + i w b) x, accumulated as sum a x and sum b x.  FP32: two packed
 // FMAs per complex value and nonzero (half the instructions of the four scalar ones).
-template <class R, int VEC> struct Acc;
-template <int VEC> struct Acc<float, VEC> {
+template <class R, int VEC, bool PAD = false> struct Acc;
+template <int VEC> struct Acc<float, VEC, false> {
   float2 s[VEC], t[VEC];
   struct Nz {
     float a, b;
@@ -175,8 +175,28 @@ template <int VEC> struct Acc<float, VEC> {
     for (int v = 0; v < VEC; ++v) y[v] = make_float2(fmaf(-w, t[v].y, s[v].x), fmaf(w, t[v].x, s[v].y));
   }
 };
-// FP64: columns q * lpr + sub of a row (any row stride), nv of them exist
-template <int VEC> struct Acc<double, VEC> {
+// FP64.  PAD: chunks of two consecutive complex values (32 bytes), chunk q of a lane at q * lpr chunks
+// after its first; else columns q * lpr + sub of a row (any row stride), nv of them exist.
+template <int VEC> __device__ __forceinline__ void ld_pad(const double2 *p, int lpr, double2 (&c)[VEC]) {
+#pragma unroll
+  for (int q = 0; q < VEC; q += 2)
+    asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];"
+        : "=d"(c[q].x), "=d"(c[q].y), "=d"(c[q + 1].x), "=d"(c[q + 1].y) : "l"(p + q * lpr));
+}
+template <int VEC> __device__ __forceinline__ void ldw_pad(const double2 *p, int lpr, double2 (&c)[VEC]) {
+#pragma unroll
+  for (int q = 0; q < VEC; q += 2)
+    asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];"
+                 : "=d"(c[q].x), "=d"(c[q].y), "=d"(c[q + 1].x), "=d"(c[q + 1].y) : "l"(p + q * lpr) : "memory");
+}
+template <int VEC> __device__ __forceinline__ void stw_pad(double2 *p, int lpr, const double2 (&c)[VEC]) {
+#pragma unroll
+  for (int q = 0; q < VEC; q += 2)
+    asm volatile("st.global.v4.f64 [%0], {%1,%2,%3,%4};" ::"l"(p + q * lpr), "d"(c[q].x), "d"(c[q].y), "d"(c[q + 1].x),
+                 "d"(c[q + 1].y)
+                 : "memory");
+}
+template <int VEC, bool PAD> struct Acc<double, VEC, PAD> {
   double2 s[VEC];
   double w;
   struct Nz {
@@ -198,8 +218,12 @@ template <int VEC> struct Acc<double, VEC> {
     const int j = *reinterpret_cast<const int *>(buf + 16 * cap + 4 * p);
     z.a = make_double2(r.x, w * r.y);
     const double2 *x = reinterpret_cast<const double2 *>(X + (int64_t)j * xb);
+    if constexpr (PAD) {
+      ld_pad<VEC>(x, cs, z.x);
+    } else {
 #pragma unroll
-    for (int v = 0; v < VEC; ++v) z.x[v] = v < nv ? __ldg(x + v * cs) : make_double2(0.0, 0.0);
+      for (int v = 0; v < VEC; ++v) z.x[v] = v < nv ? __ldg(x + v * cs) : make_double2(0.0, 0.0);
+    }
   }
   __device__ __forceinline__ void add(const Nz &z) {
 #pragma unroll
@@ -217,7 +241,7 @@ template <int VEC> struct Acc<double, VEC> {
 // gather of row i (its loads overlap it), post(i, valid, y) after.  wbuf: the warp's two staging
 // buffers.  Control flow is warp-uniform (the warp's longest row sets the trip counts, shorter
 // rows are predicated); lanes past the last row have valid = false.
-template <class R, int VEC, class Pre, class Post>
+template <class R, int VEC, bool PAD = false, class Pre, class Post>
 __device__ __forceinline__ void rows(const Geo &g, const int32_t *__restrict__ rowptr, const Src<R> &src, const R om,
                                      const typename Tr<R>::C *__restrict__ X, const int xs, const int s0, const int s1,
                                      unsigned char *wbuf, const int lane, const int warp, const int rsub,
@@ -256,12 +280,12 @@ __device__ __forceinline__ void rows(const Geo &g, const int32_t *__restrict__ r
       cp_wait<0>();
     }
     __syncwarp();
-    Acc<R, VEC> acc;
+    Acc<R, VEC, PAD> acc;
     acc.clear();
     if constexpr (sizeof(R) == 8) acc.w = om;
-    typename Acc<R, VEC>::Nz z[UNR];
+    typename Acc<R, VEC, PAD>::Nz z[UNR];
 #pragma unroll
-    for (int u = 0; u < UNR; ++u) Acc<R, VEC>::clear(z[u]);
+    for (int u = 0; u < UNR; ++u) Acc<R, VEC, PAD>::clear(z[u]);
     for (int c0 = p0;;) {
       const int p = max(b, c0) - c0;
       const int cnt = (valid && live) ? min(e, c0 + g.cap) - c0 - p : 0;
@@ -299,13 +323,13 @@ __device__ __forceinline__ void rows(const Geo &g, const int32_t *__restrict__ r
 }
 
 // Adds the rpw lanes' values of each column into the warp's slots [nsp][NQ] (FP64).
-// column of a lane's value c: VEC * sub + c (FP32) or c * lpr + sub (strided)
-template <int VEC, int NQ, bool STRIDED>
+// E: consecutive columns per chunk of a lane (FP32: VEC, FP64: 2 padded, 1 strided).
+template <int VEC, int NQ, int E>
 __device__ __forceinline__ void warp_add(const Geo &g, int lane, int sub, int rsub, double (&v)[VEC][NQ], double *slot) {
   constexpr unsigned ALL = 0xffffffffu;
 #pragma unroll
   for (int c = 0; c < VEC; ++c) {
-    const int col = STRIDED ? c * g.lpr + sub : VEC * sub + c;
+    const int col = E * ((c / E) * g.lpr + sub) + c % E;
 #pragma unroll
     for (int q = 0; q < NQ; ++q) {
       double x = rsub < g.rpw ? v[c][q] : 0.0;
