@@ -21,8 +21,9 @@
 // all harmonics and optodes into shared memory once (FP64 sums, stored as
 // complex FP32), then each thread owns measurements m and accumulates all NG
 // gates in registers; consecutive threads write consecutive m (coalesced).
-// The time-gated form (k_jacobian_tg) blocks MT measurements per thread so that
-// each gate coefficient read from shared memory feeds MT complex products.
+// The time-gated form on the CUDA cores projects the fields in a pass of its own
+// (k_project) and blocks MT measurements per thread so that each gate coefficient
+// read from shared memory feeds MT complex products (k_jacobian_tg).
 #include <algorithm>
 #include <type_traits>
 #include <vector>
@@ -102,76 +103,166 @@ __global__ void __launch_bounds__(JBS) k_jacobian_complex(JArgs a, const double2
   }
 }
 
-// Time-gated Jacobian with register blocking: a thread owns MT measurements (m = m0 + j*JBS)
-// and all NGC (>= ng, zero-padded) gates of each; per harmonic it forms the MT products
-// a_k(m) once and reads the gate coefficients C[k][0..NGC) as 128-bit shared loads, each
-// used for MT complex products (the DFT over harmonics is 2*MT*NGC FMAs per harmonic).
-template <int MT, int NGC>
-__global__ void __launch_bounds__(JBS) k_jacobian_tg(JArgs a, const float2 *__restrict__ Ckg /*[nf][NGC]*/,
-                                                     const double *__restrict__ rytov, float *__restrict__ Jtg) {
-  extern __shared__ float2 sh[];
-  float2 *Ps = sh;                         // [nf][ns]
-  float2 *Pd = Ps + a.nf * a.ns;           // [nf][nd]
-  // [nf][NGC], read as float4: start at an even float2 offset (16-byte aligned)
-  float2 *Cs = Pd + a.nf * a.nd + ((a.nf * (a.ns + a.nd)) & 1);
-  for (int t = threadIdx.x; t < a.nf * NGC; t += blockDim.x) Cs[t] = Ckg[t];
-  for (int64_t v = blockIdx.x; v < a.nv; v += gridDim.x) {
-    __syncthreads();
-    stage_field(a, v, a.phi, a.ns, Ps);
-    stage_field(a, v, a.phiA, a.nd, Pd);
-    __syncthreads();
-    const double wv = a.w ? a.w[v] : 1.0;
-    for (int m0 = 0; m0 < a.nm; m0 += JBS * MT) {
-      int sj[MT], dj[MT];
-#pragma unroll
-      for (int j = 0; j < MT; ++j) {
-        const int m = m0 + j * JBS + threadIdx.x;
-        const bool ok = m < a.nm;
-        sj[j] = ok ? a.link[2 * m] : 0;
-        dj[j] = ok ? a.link[2 * m + 1] : 0;
+// The basis fields of voxels [v0, v0 + gridDim.x), FP64 sums rounded to complex FP32 as stage_field
+// rounds them: F[v - v0][k (ns + nd) ..] = (P phi)_k then (P phiA)_k of voxel v, one run per voxel.
+// A pass of its own, many small blocks deep: gathered inside the Jacobian kernel (two blocks per SM)
+// the four nodes' rows were a serial latency of ~60 us per voxel.  Several neighbouring voxels per
+// block (shared rows from L1) measured the same (2) or slower (4, 8, 16).
+__global__ void __launch_bounds__(JBS) k_project(JArgs a, int64_t v0, int64_t per, float2 *__restrict__ F) {
+  __shared__ int32_t s_node[PMAX];
+  __shared__ double s_w[PMAX];
+  __shared__ int s_np;
+  const int64_t v = v0 + blockIdx.x;
+  if (threadIdx.x == 0) {
+    if (a.prow) {
+      const int b = a.prow[v], e = min(a.prow[v + 1], b + PMAX);
+      s_np = e - b;
+      for (int q = b; q < e; ++q) {
+        s_node[q - b] = a.pcol[q];
+        s_w[q - b] = a.pval[q];
       }
-      float acc[MT][NGC];
+    } else {
+      s_np = 1;
+      s_node[0] = (int32_t)v;
+      s_w[0] = 1.0;
+    }
+  }
+  __syncthreads();
+  const int np = s_np;
+  float2 *out = F + (int64_t)blockIdx.x * per;
+  // harmonics over the warps' groups of 32 / 16 / 8 lanes, optodes over the lanes of a group
 #pragma unroll
-      for (int j = 0; j < MT; ++j)
-#pragma unroll
-        for (int g = 0; g < NGC; ++g) acc[j][g] = 0.f;
-#pragma unroll 1
-      for (int k = 0; k < a.nf; ++k) {
-        float ar[MT], ai[MT];
-#pragma unroll
-        for (int j = 0; j < MT; ++j) {
-          const float2 x = Ps[k * a.ns + sj[j]], y = Pd[k * a.nd + dj[j]];
-          ar[j] = x.x * y.x - x.y * y.y;
-          ai[j] = x.x * y.y + x.y * y.x;
+  for (int f = 0; f < 2; ++f) {
+    const int cnt = f ? a.nd : a.ns;
+    const double2 *__restrict__ x = f ? a.phiA : a.phi;
+    const int lw = cnt > 16 ? 32 : cnt > 8 ? 16 : 8;
+    const int o0 = threadIdx.x % lw, k0 = threadIdx.x / lw, kst = JBS / lw;
+    for (int o = o0; o < cnt; o += lw)
+#pragma unroll 4
+      for (int k = k0; k < a.nf; k += kst) {
+        const double2 *row = x + (int64_t)k * a.nn * cnt + o;
+        double2 acc = make_double2(0.0, 0.0);
+        for (int q = 0; q < np; ++q) {
+          const double2 z = __ldg(row + (int64_t)s_node[q] * cnt);
+          acc.x += s_w[q] * z.x;
+          acc.y += s_w[q] * z.y;
         }
-        const float4 *c4 = reinterpret_cast<const float4 *>(Cs + k * NGC);
+        out[k * (a.ns + a.nd) + (f ? a.ns : 0) + o] = make_float2((float)acc.x, (float)acc.y);
+      }
+  }
+}
+
+// Time-gated Jacobian on the CUDA cores (voxel bases, more than 32 optodes or 64 harmonics): voxels
+// [v0, v0 + nvc) from their projected fields F.  Persistent blocks; the next voxels' fields come by
+// cp.async while the current ones are used.  A thread owns MT measurements of one voxel (tpv threads
+// per voxel, JBS / tpv voxels per pass) and all NGC (>= ng, zero-padded) gates of each: per harmonic
+// it forms the MT products a_k(m) once and reads the gate table as 128-bit shared loads
+// (Re C of two gates, -Im C of two gates), each feeding MT pairs of packed FMAs.
+// Bound by issue slots and latency at the two blocks per SM that the accumulators leave (FP32 pipe
+// 48 %, issue 50 %, LDS pipe 42 %).  21,360 voxels x 1,024 links x 32 harmonics x 10 gates: 4.85 ms
+// with the fields gathered in this kernel, gates padded to 16 and scalar FMAs; now 0.44 (projection)
+// + 1.24 ms.  Two links per thread (more blocks), blocks of 128 threads, two harmonics per 128-bit
+// load from rows by optode, and a division by precomputed reciprocals were no faster (1.24 to 1.47).
+template <int MT, int NGC>
+__global__ void __launch_bounds__(JBS) k_jacobian_tg(JArgs a, const float2 *__restrict__ F, int64_t per, int64_t v0,
+                                                     int nvc, int tpv, int nbuf,
+                                                     const float4 *__restrict__ Ckg /*[nf][NGC/2]*/,
+                                                     const float *__restrict__ ryt /*[ng][nm]*/,
+                                                     float *__restrict__ Jtg) {
+  constexpr int G2 = NGC / 2;
+  extern __shared__ __align__(16) float2 sh[];
+  const int vpb = JBS / tpv, tid = threadIdx.x;
+  const int64_t tile = per * vpb;                        // (per is even: voxels stay 16-byte aligned)
+  float4 *Cs = reinterpret_cast<float4 *>(sh + nbuf * tile);
+  for (int t = tid; t < a.nf * G2; t += JBS) Cs[t] = Ckg[t];
+  const int ntile = (nvc + vpb - 1) / vpb, st = a.ns + a.nd;
+  auto fetch = [&](int t, int buf) {
+    const int64_t n16 = min((int64_t)vpb, (int64_t)nvc - (int64_t)t * vpb) * per / 2;
+    const float2 *src = F + (int64_t)t * tile;
+    for (int64_t e = tid; e < n16; e += JBS) tc::cp_async16(sh + buf * tile + 2 * e, src + 2 * e, true);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  const int vv = tid / tpv, lt = tid % tpv;
+  const bool once = a.nm <= tpv * MT;                    // the same links for every voxel
+  int sj[MT], dj[MT];
+  auto links = [&](int m0) {
 #pragma unroll
-        for (int g2 = 0; g2 < NGC / 2; ++g2) {
-          const float4 c = c4[g2];  // (C[k][2 g2], C[k][2 g2 + 1])
+    for (int j = 0; j < MT; ++j) {
+      const int m = m0 + j * tpv;
+      sj[j] = m < a.nm ? a.link[2 * m] : 0;
+      dj[j] = a.ns + (m < a.nm ? a.link[2 * m + 1] : 0);
+    }
+  };
+  links(lt);
+  int buf = 0;
+  if ((int)blockIdx.x < ntile) fetch(blockIdx.x, 0);
+  for (int t = blockIdx.x; t < ntile; t += gridDim.x, buf ^= nbuf - 1) {
+    const bool more = t + (int)gridDim.x < ntile;
+    if (nbuf > 1 && more) {
+      fetch(t + gridDim.x, buf ^ 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    const int64_t vl = (int64_t)t * vpb + vv;
+    if (vl < nvc) {
+      const float2 *fields = sh + buf * tile + vv * per;
+      const int64_t v = v0 + vl;
+      const float wf = (float)(a.w ? a.w[v] : 1.0);
+      for (int m0 = lt; m0 < a.nm; m0 += tpv * MT) {
+        if (!once) links(m0);
+        float2 acc[MT][G2];
+#pragma unroll
+        for (int j = 0; j < MT; ++j)
+#pragma unroll
+          for (int g = 0; g < G2; ++g) acc[j][g] = make_float2(0.f, 0.f);
+        const float2 *fk = fields;
+        const float4 *ck = Cs;
+#pragma unroll 1
+        for (int k = 0; k < a.nf; ++k, fk += st, ck += G2) {
+          float2 ar[MT], ai[MT];
 #pragma unroll
           for (int j = 0; j < MT; ++j) {
-            acc[j][2 * g2] = fmaf(c.x, ar[j], fmaf(-c.y, ai[j], acc[j][2 * g2]));
-            acc[j][2 * g2 + 1] = fmaf(c.z, ar[j], fmaf(-c.w, ai[j], acc[j][2 * g2 + 1]));
+            const float2 x = fk[sj[j]], y = fk[dj[j]];
+            const float re = x.x * y.x - x.y * y.y, im = x.x * y.y + x.y * y.x;
+            ar[j] = make_float2(re, re);
+            ai[j] = make_float2(im, im);
+          }
+#pragma unroll
+          for (int g = 0; g < G2; ++g) {
+            const float4 c = ck[g];
+            const float2 cr = make_float2(c.x, c.y), ci = make_float2(c.z, c.w);
+#pragma unroll
+            for (int j = 0; j < MT; ++j) acc[j][g] = __ffma2_rn(cr, ar[j], __ffma2_rn(ci, ai[j], acc[j][g]));
           }
         }
-      }
-      // epilogue in FP32 (the output precision): w_v scaling and the Rytov division
-      const float wf = (float)wv;
+        // epilogue in FP32 (the output precision): w_v scaling and the Rytov division
 #pragma unroll
-      for (int j = 0; j < MT; ++j) {
-        const int m = m0 + j * JBS + threadIdx.x;
-        if (m >= a.nm) continue;
+        for (int j = 0; j < MT; ++j) {
+          const int m = m0 + j * tpv;
+          if (m >= a.nm) continue;
+          float *out = Jtg + (int64_t)v * a.ng * a.nm + m;
+          const float *r = ryt + m;
 #pragma unroll
-        for (int g = 0; g < NGC; ++g) {
-          if (g < a.ng) {
-            float val = wf * acc[j][g];
-            if (rytov) val = val / (float)rytov[(int64_t)m * a.ng + g];
-            Jtg[((int64_t)v * a.ng + g) * a.nm + m] = val;
-          }
+          for (int g = 0; g < NGC; ++g)
+            if (g < a.ng) {
+              float val = wf * (g % 2 ? acc[j][g / 2].y : acc[j][g / 2].x);
+              if (ryt) val = val / r[(int64_t)g * a.nm];
+              out[(int64_t)g * a.nm] = val;
+            }
         }
       }
     }
+    __syncthreads();  // the buffer is refilled: with the next tile or the one after it
+    if (nbuf == 1 && more) fetch(t + gridDim.x, 0);
   }
+}
+
+// ryt[g][m] = (float)rytov[m][g]: the divisor as the epilogue reads it, consecutive over m
+__global__ void k_rytov_t(const double *__restrict__ rytov, int nm, int ng, float *ryt) {
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (t < (int64_t)nm * ng) ryt[(t % ng) * nm + t / ng] = (float)rytov[t];
 }
 
 // ------------------------------------------------------------------------------------------
@@ -791,12 +882,13 @@ __global__ void __launch_bounds__(JBS) k_jacobian_vjp(JArgs a, const float2 *__r
   }
 }
 
-// Ckg[k][g] = C[g][k] for g < ng, 0 for ng <= g < ngc (the register-blocked kernel's layout)
-__global__ void k_ctab_kg(const float2 *__restrict__ C, int ng, int nf, int ngc, float2 *Ckg) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nf * ngc) return;
-  const int k = t / ngc, g = t % ngc;
-  Ckg[t] = g < ng ? C[g * nf + k] : make_float2(0.f, 0.f);
+// Ckg[k][g / 2] = (Re C of gates g, g + 1; -Im C of them), zero past ng
+__global__ void k_ctab_kg(const float2 *__restrict__ C, int ng, int nf, int ngc, float4 *Ckg) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, g2 = ngc / 2;
+  if (t >= nf * g2) return;
+  const int k = t / g2, g = 2 * (t % g2);
+  const float2 z = make_float2(0.f, 0.f), c0 = g < ng ? C[g * nf + k] : z, c1 = g + 1 < ng ? C[(g + 1) * nf + k] : z;
+  Ckg[t] = make_float4(c0.x, c1.x, -c0.y, -c1.y);
 }
 
 // C[g,k] = -2 Nt h_k conj(gate[g,k]) / fpsf[k]; also -1/fpsf[k] for the FD form
@@ -921,37 +1013,83 @@ int jacobian_run(int mode, const int32_t *prow, const int32_t *pcol, const doubl
     return DGP_OK;
   }
   if (mode == 0) {
-    // register-blocked TG kernel: gates padded to 8/16/24/32, MT measurements per thread
-    const int ngc = ng <= 8 ? 8 : ng <= 16 ? 16 : ng <= 24 ? 24 : 32;
-    // measurements per thread: 4 while the accumulators fit two blocks per SM (<= 16 gates), else 2
+    // gates padded to an even count that has an instance
+    int ngc = 32;
+    for (int c : {24, 20, 16, 12, 10, 8, 4})
+      if (ng <= c) ngc = c;
+    // measurements per thread: 4 while the accumulators leave room for two blocks per SM, else 2;
+    // below 256 links one each and several voxels per block
     const int mt = (nm > 2 * JBS && ngc <= 16) ? 4 : nm > JBS ? 2 : 1;
-    ScratchBuf ckg;
-    DGP_TRY(ckg.alloc(sizeof(float2) * (size_t)nf * ngc, st));
-    k_ctab_kg<<<(unsigned)ceil_div((int64_t)nf * ngc, 256), 256, 0, st>>>(ctab.as<float2>(), ng, nf, ngc,
-                                                                          ckg.as<float2>());
+    int tpv = JBS;
+    while (mt == 1 && tpv > 32 && tpv / 2 >= nm) tpv /= 2;
+    const int64_t per = ((int64_t)nf * (ns + nd) + 1) & ~1ll;  // even: voxels stay 16-byte aligned
+    const size_t smem_c = sizeof(float4) * (size_t)nf * (ngc / 2);
+    const auto smem_of = [&](int t, int b) { return sizeof(float2) * b * per * (JBS / t) + smem_c; };
+    DGP_REQUIRE(sizeof(float2) * (size_t)nf * (ns + nd + 8 * ceil_div(ng, 8)) + 8 <= 200 * 1024,
+                "jacobian: NF*(NS+ND+NG) too large for one block's shared memory");
+    while (tpv < JBS && smem_of(tpv, 2) > 100 * 1024) tpv *= 2;
+    // two buffers of fields, one where two don't fit
+    const int nbuf = smem_of(tpv, 2) <= 200 * 1024 ? 2 : 1;
+    const size_t smem_tg = smem_of(tpv, nbuf);
+    // projected fields in chunks that stay in L2 between the two kernels
+    int64_t chunk = std::min<int64_t>(nv, std::max<int64_t>(1, ((int64_t)96 << 20) / (8 * per)));
+    ScratchBuf ckg, fields, ryt;
+    DGP_TRY(ckg.alloc(sizeof(float4) * (size_t)nf * (ngc / 2), st));
+    int frc = fields.alloc(sizeof(float2) * (size_t)chunk * per, st);
+    while (frc != DGP_OK && chunk > 64) {  // a nearly full device: smaller chunks
+      chunk /= 4;
+      frc = fields.alloc(sizeof(float2) * (size_t)chunk * per, st);
+    }
+    DGP_TRY(frc);
+    if (rytov) {
+      DGP_TRY(ryt.alloc(sizeof(float) * (size_t)nm * ng, st));
+      k_rytov_t<<<(unsigned)ceil_div((int64_t)nm * ng, 256), 256, 0, st>>>(rytov, nm, ng, ryt.as<float>());
+      DGP_CHECK_LAUNCH();
+    }
+    k_ctab_kg<<<(unsigned)ceil_div((int64_t)nf * (ngc / 2), 256), 256, 0, st>>>(ctab.as<float2>(), ng, nf, ngc,
+                                                                                ckg.as<float4>());
     DGP_CHECK_LAUNCH();
-    const size_t smem_tg = sizeof(float2) * ((size_t)nf * (ns + nd) + 1 + (size_t)nf * ngc);
-    DGP_REQUIRE(smem_tg <= 200 * 1024, "jacobian: NF*(NS+ND+NG) too large for one block's shared memory");
     int arc = DGP_OK;
     auto go = [&](auto mtc, auto ngcc) {
       constexpr int MT_ = decltype(mtc)::value, NGC_ = decltype(ngcc)::value;
       arc = allow_dyn_smem(k_jacobian_tg<MT_, NGC_>, smem_tg);
-      if (arc == DGP_OK) k_jacobian_tg<MT_, NGC_><<<grid, JBS, smem_tg, st>>>(a, ckg.as<float2>(), rytov, (float *)out);
+      int occ = 0;
+      if (arc == DGP_OK &&
+          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_jacobian_tg<MT_, NGC_>, JBS, smem_tg) != cudaSuccess)
+        arc = cuda_fail(cudaGetLastError(), "jacobian occupancy", __FILE__, __LINE__);
+      for (int64_t v0 = 0; v0 < nv && arc == DGP_OK; v0 += chunk) {
+        const int nvc = (int)std::min<int64_t>(chunk, nv - v0);
+        k_project<<<nvc, JBS, 0, st>>>(a, v0, per, fields.as<float2>());
+        const int gt = (int)std::min<int64_t>(ceil_div(nvc, JBS / tpv), (int64_t)std::max(1, occ) * sm_count());
+        k_jacobian_tg<MT_, NGC_><<<gt, JBS, smem_tg, st>>>(a, fields.as<float2>(), per, v0, nvc, tpv, nbuf,
+                                                           ckg.as<float4>(), rytov ? ryt.as<float>() : nullptr,
+                                                           (float *)out);
+        count_launches(2);
+      }
     };
     auto by_ngc = [&](auto mtc) {
+      constexpr int MT_ = decltype(mtc)::value;
       switch (ngc) {
+        case 4: go(mtc, std::integral_constant<int, 4>()); break;
         case 8: go(mtc, std::integral_constant<int, 8>()); break;
+        case 10: go(mtc, std::integral_constant<int, 10>()); break;
+        case 12: go(mtc, std::integral_constant<int, 12>()); break;
         case 16: go(mtc, std::integral_constant<int, 16>()); break;
-        case 24: go(mtc, std::integral_constant<int, 24>()); break;
-        default: go(mtc, std::integral_constant<int, 32>()); break;
+        default:
+          if constexpr (MT_ < 4) {
+            if (ngc == 20) go(mtc, std::integral_constant<int, 20>());
+            else if (ngc == 24) go(mtc, std::integral_constant<int, 24>());
+            else go(mtc, std::integral_constant<int, 32>());
+          }
       }
     };
     if (mt == 4) by_ngc(std::integral_constant<int, 4>());
     else if (mt == 2) by_ngc(std::integral_constant<int, 2>());
     else by_ngc(std::integral_constant<int, 1>());
     DGP_TRY(arc);
-    DGP_CHECK_LAUNCH();
-    DGP_CUDA(cudaStreamSynchronize(st));  // ckg is released on return
+    DGP_CUDA(cudaGetLastError());
+    DGP_CUDA(cudaStreamSynchronize(st));
+    return DGP_OK;
   } else if (mode == 1) {
     k_jacobian_complex<<<grid, JBS, smem, st>>>(a, finv.as<double2>(), (double2 *)out);
   } else {

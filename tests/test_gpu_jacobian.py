@@ -271,3 +271,50 @@ def test_vjp_from_several_host_threads(jac_case):
     assert not errors, errors
     for k in args:
         assert rel(results[k].numpy(), alone[k].numpy()) < 1e-12, k
+
+
+@pytest.mark.parametrize("ns,nd,nf,ng,nm,nv,rows", [
+    (3, 4, 5, 1, 7, 1, "four"),          # one voxel, a quarter-block of links
+    (40, 7, 33, 10, 280, 301, "any"),    # more than 32 optodes; rows of 0 to 8 entries
+    (5, 37, 9, 12, 513, 97, "four"),     # four links per thread, one in the last pass
+    (9, 9, 3, 11, 33, 1000, "four"),     # several voxels per block, odd gate count
+    (17, 16, 66, 32, 272, 64, "nodal"),  # more than 64 harmonics, all gates
+    (64, 64, 120, 20, 1500, 40, "any"),  # fields of one voxel fill most of a block's shared memory
+    (12000, 3001, 1, 2, 300, 9, "four"),  # ... at one harmonic, an odd count
+])
+@pytest.mark.parametrize("use_rytov", [False, True])
+def test_tg_jacobian_projected_fields(ns, nd, nf, ng, nm, nv, rows, use_rytov):
+    """CUDA-core TG Jacobian against 64-bit sums, for random fields, bases and (repeated) links.
+    Each term is rounded at most five times and added in FP32, so an entry is off by at most
+    (2 nf + 8) eps / 2 of the sum of its terms' magnitudes."""
+    import scipy.sparse as sp
+    import torch
+    from dogpup_b200 import api
+    rng = np.random.default_rng(ns + nf)
+    nn = nv if rows == "nodal" else 83
+    cn = lambda *s: rng.standard_normal(s) + 1j * rng.standard_normal(s)
+    phi, phiA, fpsf, gates = cn(nf, nn, ns), cn(nf, nn, nd), cn(nf), cn(ng, nf)
+    link = np.stack([rng.integers(0, ns, nm), rng.integers(0, nd, nm)], 1).astype(np.int32)
+    wts = rng.uniform(0.5, 2.0, nv)
+    if rows == "nodal":
+        P = sp.identity(nn, format="csr")
+        basis = api.Basis(None, wts, nn=nn)
+    else:
+        cnt = np.full(nv, 4) if rows == "four" else rng.integers(0, 9, nv)
+        col = np.concatenate([rng.choice(nn, c, replace=False) for c in cnt]).astype(np.int32)
+        P = sp.csr_matrix((rng.uniform(0.1, 1.0, col.size), col, np.concatenate([[0], np.cumsum(cnt)])), shape=(nv, nn))
+        basis = api.Basis(P, wts)
+    ryt = rng.uniform(0.5, 2.0, (nm, ng))
+    cu = lambda x: torch.as_tensor(x, device="cuda")
+    J = api.jacobian_tg(basis, cu(phi), cu(phiA), cu(fpsf), cu(link), cu(gates), 64,
+                        data_tg=cu(ryt) if use_rytov else None)
+    h = np.where(np.arange(nf) == 0, 0.5, 1.0)
+    C = -2.0 * 64 * h * np.conj(gates) / fpsf                                     # [ng, nf]
+    J0, mag = np.zeros((nv, ng, nm)), np.zeros((nv, ng, nm))
+    for k in range(nf):
+        a = (P @ phi[k])[:, link[:, 0]] * (P @ phiA[k])[:, link[:, 1]]           # [nv, nm]
+        J0 += np.real(C[None, :, k, None] * a[:, None, :])
+        mag += np.abs(C[None, :, k, None]) * np.abs(a[:, None, :])
+    scale = wts[:, None, None] / (ryt.T[None] if use_rytov else 1.0)
+    err = np.abs(J.cpu().numpy() - scale * J0)
+    assert (err <= (2 * nf + 8) * 2.0 ** -24 * np.sqrt(2) * scale * mag).all()
