@@ -79,58 +79,19 @@ __device__ void stage_field(const JArgs &a, int64_t v, const double2 *__restrict
   }
 }
 
-// Complex Jacobian J[v][k][m] (double2 [nv][nf][nm]): one block per voxel, threads over m.
-__global__ void __launch_bounds__(JBS) k_jacobian_complex(JArgs a, const double2 *__restrict__ fpsf_inv,
-                                                          double2 *__restrict__ Jfd) {
-  extern __shared__ float2 sh[];
-  float2 *Ps = sh;                         // [nf][ns]
-  float2 *Pd = Ps + a.nf * a.ns;           // [nf][nd]
-  for (int64_t v = blockIdx.x; v < a.nv; v += gridDim.x) {
-    __syncthreads();
-    stage_field(a, v, a.phi, a.ns, Ps);
-    stage_field(a, v, a.phiA, a.nd, Pd);
-    __syncthreads();
-    const double wv = a.w ? a.w[v] : 1.0;
-    for (int m = threadIdx.x; m < a.nm; m += blockDim.x) {
-      const int s = a.link[2 * m], d = a.link[2 * m + 1];
-      for (int k = 0; k < a.nf; ++k) {
-        float2 x = Ps[k * a.ns + s], y = Pd[k * a.nd + d];
-        double2 p = make_double2((double)x.x * y.x - (double)x.y * y.y, (double)x.x * y.y + (double)x.y * y.x);
-        double2 r = cmul(p, fpsf_inv[k]);  // -1 / s_fpsf[k]
-        Jfd[((int64_t)v * a.nf + k) * a.nm + m] = make_double2(wv * r.x, wv * r.y);
-      }
-    }
-  }
-}
-
-// The basis fields of voxels [v0, v0 + gridDim.x), FP64 sums rounded to complex FP32 as stage_field
-// rounds them: F[v - v0][k (ns + nd) ..] = (P phi)_k then (P phiA)_k of voxel v, one run per voxel.
-// A pass of its own, many small blocks deep: gathered inside the Jacobian kernel (two blocks per SM)
-// the four nodes' rows were a serial latency of ~60 us per voxel.  Several neighbouring voxels per
-// block (shared rows from L1) measured the same (2) or slower (4, 8, 16).
-__global__ void __launch_bounds__(JBS) k_project(JArgs a, int64_t v0, int64_t per, float2 *__restrict__ F) {
+// The basis fields of one voxel by a block: put(k, o, z), o over the sources' (P phi)_k, then the
+// detectors' (P phiA)_k; FP64 sums rounded to complex FP32, as stage_field rounds them.  Harmonics go
+// over the warps' groups of 32 / 16 / 8 lanes, optodes over the lanes of a group, so that a row of a
+// node is read in one go; the loads of four nodes and several harmonics are in flight together.
+template <class PUT> __device__ __forceinline__ void project_voxel(const JArgs &a, int64_t v, PUT put) {
   __shared__ int32_t s_node[PMAX];
   __shared__ double s_w[PMAX];
-  __shared__ int s_np;
-  const int64_t v = v0 + blockIdx.x;
-  if (threadIdx.x == 0) {
-    if (a.prow) {
-      const int b = a.prow[v], e = min(a.prow[v + 1], b + PMAX);
-      s_np = e - b;
-      for (int q = b; q < e; ++q) {
-        s_node[q - b] = a.pcol[q];
-        s_w[q - b] = a.pval[q];
-      }
-    } else {
-      s_np = 1;
-      s_node[0] = (int32_t)v;
-      s_w[0] = 1.0;
-    }
+  const int b = a.prow ? a.prow[v] : 0, np = a.prow ? min(a.prow[v + 1] - b, PMAX) : 1;
+  if (threadIdx.x < np) {
+    s_node[threadIdx.x] = a.prow ? a.pcol[b + threadIdx.x] : (int32_t)v;
+    s_w[threadIdx.x] = a.prow ? a.pval[b + threadIdx.x] : 1.0;
   }
   __syncthreads();
-  const int np = s_np;
-  float2 *out = F + (int64_t)blockIdx.x * per;
-  // harmonics over the warps' groups of 32 / 16 / 8 lanes, optodes over the lanes of a group
 #pragma unroll
   for (int f = 0; f < 2; ++f) {
     const int cnt = f ? a.nd : a.ns;
@@ -142,14 +103,51 @@ __global__ void __launch_bounds__(JBS) k_project(JArgs a, int64_t v0, int64_t pe
       for (int k = k0; k < a.nf; k += kst) {
         const double2 *row = x + (int64_t)k * a.nn * cnt + o;
         double2 acc = make_double2(0.0, 0.0);
+#pragma unroll 4
         for (int q = 0; q < np; ++q) {
           const double2 z = __ldg(row + (int64_t)s_node[q] * cnt);
           acc.x += s_w[q] * z.x;
           acc.y += s_w[q] * z.y;
         }
-        out[k * (a.ns + a.nd) + (f ? a.ns : 0) + o] = make_float2((float)acc.x, (float)acc.y);
+        put(k, (f ? a.ns : 0) + o, make_float2((float)acc.x, (float)acc.y));
       }
   }
+}
+
+// Complex Jacobian J[v][k][m] (double2 [nv][nf][nm]): one block per voxel, threads over m.  Bound by
+// writing J; many blocks per SM cover the gathers of one with the stores of others.  Fields kept as
+// FP64 (converted once per voxel instead of once per link) measured the same.  3,990 voxels x 240
+// links x 32 harmonics: 247 us with the gathers node after node and a division per element, 131 now.
+__global__ void __launch_bounds__(JBS) k_jacobian_complex(JArgs a, const double2 *__restrict__ fpsf_inv,
+                                                          double2 *__restrict__ Jfd) {
+  extern __shared__ float2 sh[];           // [nf][ns + nd]
+  const int st = a.ns + a.nd;
+  for (int64_t v = blockIdx.x; v < a.nv; v += gridDim.x) {
+    __syncthreads();
+    project_voxel(a, v, [&](int k, int o, float2 z) { sh[k * st + o] = z; });
+    __syncthreads();
+    const double wv = a.w ? a.w[v] : 1.0;
+    for (int m = threadIdx.x; m < a.nm; m += JBS) {
+      const float2 *x = sh + a.link[2 * m], *y = sh + a.ns + a.link[2 * m + 1];
+      double2 *out = Jfd + v * a.nf * a.nm + m;
+#pragma unroll 4
+      for (int k = 0; k < a.nf; ++k, x += st, y += st, out += a.nm) {
+        const double2 p = cmul(make_double2((double)x->x, (double)x->y), make_double2((double)y->x, (double)y->y));
+        const double2 r = cmul(p, fpsf_inv[k]);  // -1 / s_fpsf[k]
+        *out = make_double2(wv * r.x, wv * r.y);
+      }
+    }
+  }
+}
+
+// The projected fields of voxels [v0, v0 + gridDim.x): F[v - v0][k (ns + nd) + o], one run of `per`
+// per voxel.  A pass of its own, many small blocks deep: gathered inside the time-gated kernel (two
+// blocks per SM) the four nodes' rows were a serial latency of ~60 us per voxel.  Several
+// neighbouring voxels per block (shared rows from L1) measured the same (2) or slower (4, 8, 16).
+__global__ void __launch_bounds__(JBS) k_project(JArgs a, int64_t v0, int64_t per, float2 *__restrict__ F) {
+  float2 *out = F + (int64_t)blockIdx.x * per;
+  const int st = a.ns + a.nd;
+  project_voxel(a, v0 + blockIdx.x, [&](int k, int o, float2 z) { out[k * st + o] = z; });
 }
 
 // Time-gated Jacobian on the CUDA cores (voxel bases, more than 32 optodes or 64 harmonics): voxels
@@ -990,7 +988,6 @@ int jacobian_run(int mode, const int32_t *prow, const int32_t *pcol, const doubl
   k_ctab<<<(unsigned)ceil_div(nt_, 256), 256, 0, st>>>((const double2 *)gate, (const double2 *)fpsf, mode == 1 ? 0 : ng,
                                                         nf, nt, ctab.as<float2>(), finv.as<double2>());
   DGP_CHECK_LAUNCH();
-  if (mode == 1) DGP_TRY(allow_dyn_smem(k_jacobian_complex, smem));
   const T2Layout tl = t2_layout(nf, std::max(1, ng));
   const size_t smem_tc = tl.bytes + 1024;
   // (+ 1 KB of the kernel's own static shared memory)
@@ -1091,7 +1088,9 @@ int jacobian_run(int mode, const int32_t *prow, const int32_t *pcol, const doubl
     DGP_CUDA(cudaStreamSynchronize(st));
     return DGP_OK;
   } else if (mode == 1) {
-    k_jacobian_complex<<<grid, JBS, smem, st>>>(a, finv.as<double2>(), (double2 *)out);
+    DGP_TRY(allow_dyn_smem(k_jacobian_complex, smem));
+    k_jacobian_complex<<<(unsigned)std::min<int64_t>(nv, INT32_MAX), JBS, smem, st>>>(a, finv.as<double2>(),
+                                                                                      (double2 *)out);
   } else {
     DGP_REQUIRE(gin, "jacobian vjp: null upstream gradient");
     DGP_TRY(chat.alloc(sizeof(float2) * (size_t)nm * nf, st));
