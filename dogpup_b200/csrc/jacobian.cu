@@ -79,8 +79,8 @@ __device__ void stage_field(const JArgs &a, int64_t v, const double2 *__restrict
   }
 }
 
-// The basis fields of one voxel by a block: put(k, o, z), o over the sources' (P phi)_k, then the
-// detectors' (P phiA)_k; FP64 sums rounded to complex FP32, as stage_field rounds them.  Harmonics go
+// The basis fields of one voxel by a block, FP64: put(k, o, z), o over the sources' (P phi)_k, then
+// the detectors' (P phiA)_k.  Harmonics go
 // over the warps' groups of 32 / 16 / 8 lanes, optodes over the lanes of a group, so that a row of a
 // node is read in one go; the loads of four nodes and several harmonics are in flight together.
 template <class PUT> __device__ __forceinline__ void project_voxel(const JArgs &a, int64_t v, PUT put) {
@@ -109,7 +109,7 @@ template <class PUT> __device__ __forceinline__ void project_voxel(const JArgs &
           acc.x += s_w[q] * z.x;
           acc.y += s_w[q] * z.y;
         }
-        put(k, (f ? a.ns : 0) + o, make_float2((float)acc.x, (float)acc.y));
+        put(k, (f ? a.ns : 0) + o, acc);
       }
   }
 }
@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(JBS) k_jacobian_complex(JArgs a, const double2
   const int st = a.ns + a.nd;
   for (int64_t v = blockIdx.x; v < a.nv; v += gridDim.x) {
     __syncthreads();
-    project_voxel(a, v, [&](int k, int o, float2 z) { sh[k * st + o] = z; });
+    project_voxel(a, v, [&](int k, int o, double2 z) { sh[k * st + o] = make_float2((float)z.x, (float)z.y); });
     __syncthreads();
     const double wv = a.w ? a.w[v] : 1.0;
     for (int m = threadIdx.x; m < a.nm; m += JBS) {
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(JBS) k_jacobian_complex(JArgs a, const double2
 __global__ void __launch_bounds__(JBS) k_project(JArgs a, int64_t v0, int64_t per, float2 *__restrict__ F) {
   float2 *out = F + (int64_t)blockIdx.x * per;
   const int st = a.ns + a.nd;
-  project_voxel(a, v0 + blockIdx.x, [&](int k, int o, float2 z) { out[k * st + o] = z; });
+  project_voxel(a, v0 + blockIdx.x, [&](int k, int o, double2 z) { out[k * st + o] = make_float2((float)z.x, (float)z.y); });
 }
 
 // Time-gated Jacobian on the CUDA cores (voxel bases, more than 32 optodes or 64 harmonics): voxels
@@ -675,18 +675,30 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
 // The per-harmonic operand B'_k = the real embedding of Chat_k^T is built once per call in
 // global memory, already split and swizzled (k_vjp_btab), and copied into shared memory.
 //
-// CTA = 256 threads over a tile of 128 voxels, looping over the harmonics: the threads convert
-// this tile's (P phiA)_k rows to the split A' operand (coalesced FP64 loads), thread 0 issues the
-// 24 MMAs, and in the epilogue each warp reads its 32 voxel rows x 32 columns of Y_k from tensor
-// memory, dots them with (P phi)_k read from global memory and accumulates in FP64.  96 KB of
-// shared memory: two CTAs per SM overlap one's loads with the other's MMAs and epilogue.
-constexpr int VT_THREADS = 256;
+// Persistent CTA (one per SM), warp-specialised; the (tile of 128 voxels, harmonic) pairs are dealt out
+// in equal contiguous runs, so that neither the last wave nor a small mesh leaves SMs idle; a tile that
+// two or more CTAs share is added up by k_vjp_join in a fixed order.  Per pair:
+//   warps 8-11  copy the tile's rows of phiA, then of phi (FP64, 64 KB each) by cp.async into a ring
+//               of three slabs, row r's 16-byte element o at o ^ (r % 32): rows are written and
+//               columns read without bank conflicts
+//   warp 13     copies B'_k (32 KB, one bulk copy) once the MMAs are done with the previous one
+//   warps 4-7   thread = voxel row: FP64 -> FP32 -> (hi, lo) into one of two A' stages in tensor memory
+//   warp 12     one thread issues the 24 MMAs into one of two accumulators
+//   warps 0-3   thread = voxel row: dots Y_k with phi from the slab, in FP64
+// Bound by HBM: every field value is read once, NF (NS + ND) 16 bytes per voxel.  101,898 nodes x 64
+// optodes x 64 harmonics (6.7 GB): 4.34 ms with two CTAs per SM that loaded, converted, multiplied and
+// reduced one after the other (phi by 16-byte loads 512 bytes apart), 1.20 ms now.
+// A voxel basis is projected, chunk by chunk, into slabs of the same layout (k_project_slabs).
 constexpr int VT_ROWS = 128;                       // voxels per tile (MMA M)
 constexpr int VT_NP = 64;                          // N' = 2 x 32 sources
 constexpr int VT_KP = 64;                          // K' = 2 x 32 detectors
-constexpr int VT_A = VT_ROWS * VT_KP * 4;          // 32 KB: 128 rows x 64 fp32 (two 128-byte atoms)
 constexpr int VT_B = VT_NP * VT_KP * 4;            // 16 KB
-constexpr int VT_SMEM = 2 * VT_A + 2 * VT_B + 1024;
+constexpr int VT_EPI = 4, VT_CONV = 4, VT_LOAD = 4;
+constexpr int VT_THREADS = 32 * (VT_EPI + VT_CONV + VT_LOAD + 2);
+constexpr int VT_NSLAB = 3;
+constexpr int VT_SLAB = VT_ROWS * 32 * 16;         // 64 KB
+constexpr int VT_SMEM = VT_NSLAB * VT_SLAB + 2 * VT_B + 1024;
+constexpr uint32_t VT_ACOL = 128;                  // first A' column: two accumulators of 64 come before
 constexpr uint32_t VT_IDESC = tc::idesc(2, 2, VT_ROWS, VT_NP);
 
 // K-major split operand image: element (row, j) of a [rows][64] fp32 tile stored as two 128-byte
@@ -697,19 +709,37 @@ __host__ __device__ inline uint32_t kmaj64(uint32_t row, uint32_t j, uint32_t ro
 
 // Btab[k] = (hi, lo) images of B'_k [64 rows n'][64 K'] (16 KB each), from Chat [nm][nf]:
 //   B'[2s][2d] = Re C, B'[2s][2d+1] = -Im C, B'[2s+1][2d] = Im C, B'[2s+1][2d+1] = Re C,
-// C = Chat_k[s][d]; one thread per (k, s, d).
-__global__ void k_vjp_btab(const float2 *__restrict__ Chat, const int32_t *__restrict__ link, int nm, int nf,
-                           unsigned char *__restrict__ Btab) {
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+// C = Chat_k[s][d]; one thread per (k, s, d).  The links (nm <= 4096) are searched in shared memory,
+// four per read: 69 us with a scan of the table in global memory per entry (1,024 links x 64), 25 now.
+__global__ void __launch_bounds__(256) k_vjp_btab(const float2 *__restrict__ Chat, const int32_t *__restrict__ link,
+                                                  int nm, int nf, unsigned char *__restrict__ Btab) {
+  __shared__ int4 s_link[1024];
+  int *sl = reinterpret_cast<int *>(s_link);
+  const int nm4 = (nm + 3) / 4;
+  for (int m = threadIdx.x; m < 4 * nm4; m += 256) sl[m] = m < nm ? 32 * link[2 * m] + link[2 * m + 1] : -1;
+  __syncthreads();
+  const int64_t t = blockIdx.x * (int64_t)256 + threadIdx.x;
   if (t >= (int64_t)nf * 32 * 32) return;
-  const int k = (int)(t / 1024), s = (int)(t / 32 % 32), d = (int)(t % 32);
+  const int k = (int)(t / 1024), s = (int)(t / 32 % 32), d = (int)(t % 32), me = 32 * s + d;
   float2 c = make_float2(0.f, 0.f);
-  for (int m = 0; m < nm; ++m)  // link tables are small (nm <= 1024 here): a scan per entry
-    if (link[2 * m] == s && link[2 * m + 1] == d) {
-      const float2 x = Chat[(int64_t)m * nf + k];
-      c.x += x.x;
-      c.y += x.y;
-    }
+  auto add = [&](int m) {
+    const float2 x = Chat[(int64_t)m * nf + k];
+    c.x += x.x;
+    c.y += x.y;
+  };
+  int hit = -1;  // added when the next one is found, or at the end: one read per warp if links are unique
+  auto found = [&](int m) {
+    if (hit >= 0) add(hit);
+    hit = m;
+  };
+  for (int q = 0; q < nm4; ++q) {
+    const int4 l = s_link[q];
+    if (l.x == me) found(4 * q);
+    if (l.y == me) found(4 * q + 1);
+    if (l.z == me) found(4 * q + 2);
+    if (l.w == me) found(4 * q + 3);
+  }
+  if (hit >= 0) add(hit);
   unsigned char *hi = Btab + (size_t)k * 2 * VT_B, *lo = hi + VT_B;
   const float v[2][2] = {{c.x, -c.y}, {c.y, c.x}};
 #pragma unroll
@@ -723,108 +753,233 @@ __global__ void k_vjp_btab(const float2 *__restrict__ Chat, const int32_t *__res
     }
 }
 
-// (P f)_k[v][o] for o < cnt optodes of field f [nf][nn][cnt], FP64
-__device__ inline double2 basis_field(const JArgs &a, int64_t v, int k, int o, const double2 *__restrict__ f, int cnt) {
-  if (!a.prow) return f[((int64_t)k * a.nn + v) * cnt + o];
-  double2 acc = make_double2(0.0, 0.0);
-  const int b = a.prow[v], e = min(a.prow[v + 1], b + PMAX);
-  for (int q = b; q < e; ++q) {
-    const double2 x = f[((int64_t)k * a.nn + a.pcol[q]) * cnt + o];
-    acc.x += a.pval[q] * x.x;
-    acc.y += a.pval[q] * x.y;
-  }
-  return acc;
+// (P phi)_k and (P phiA)_k of voxels [v0, v0 + gridDim.x), FP64, as [nf][gridDim.x][ns] and [nd]
+__global__ void __launch_bounds__(JBS) k_project_slabs(JArgs a, int64_t v0, double2 *__restrict__ phi,
+                                                       double2 *__restrict__ phiA) {
+  const int64_t n = gridDim.x, v = blockIdx.x;
+  project_voxel(a, v0 + v, [&](int k, int o, double2 z) {
+    if (o < a.ns) phi[(k * n + v) * a.ns + o] = z;
+    else phiA[(k * n + v) * a.nd + o - a.ns] = z;
+  });
 }
 
-__global__ void __launch_bounds__(VT_THREADS, 2) k_jacobian_vjp_tc(JArgs a, const unsigned char *__restrict__ Btab,
-                                                                  double *__restrict__ vjp, int *err) {
+// first of CTA c's (tile, harmonic) pairs
+__device__ inline int64_t vt_first(int64_t pairs, int64_t c, int64_t ctas) { return c * pairs / ctas; }
+
+__global__ void __launch_bounds__(VT_THREADS, 1) k_jacobian_vjp_tc(JArgs a, const unsigned char *__restrict__ Btab,
+                                                                  double *__restrict__ vjp, double *__restrict__ part,
+                                                                  int *err) {
   extern __shared__ __align__(1024) unsigned char vt_raw[];
-  __shared__ __align__(8) uint64_t bar_mma;
+  __shared__ __align__(8) uint64_t full[VT_NSLAB], empty[VT_NSLAB], afull[2], aempty[2], cfull[2], cempty[2];
+  __shared__ __align__(8) uint64_t bfull, bempty, done;
   __shared__ uint32_t tmem_slot;
-  __shared__ double part[VT_THREADS];
+  __shared__ int abort_flag;
   unsigned char *sm = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(vt_raw) + 1023) & ~uintptr_t(1023));
-  unsigned char *Ahi = sm, *Alo = sm + VT_A, *Bhi = sm + 2 * VT_A, *Blo = Bhi + VT_B;
+  unsigned char *B = sm, *slabs = sm + 2 * VT_B;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  constexpr unsigned FULL = 0xffffffffu;
+  volatile int *abort_v = &abort_flag;
   if (tid == 0) {
-    tc::mbar_init(&bar_mma, 1);
+    for (int i = 0; i < VT_NSLAB; ++i) {
+      tc::mbar_init(&full[i], 32 * VT_LOAD);           // one cp.async arrival per copying thread
+      tc::mbar_init(&empty[i], 4);                     // one arrival per reading warp
+    }
+    for (int i = 0; i < 2; ++i) {
+      tc::mbar_init(&afull[i], VT_CONV);
+      tc::mbar_init(&aempty[i], 1);
+      tc::mbar_init(&cfull[i], 1);
+      tc::mbar_init(&cempty[i], VT_EPI);
+    }
+    tc::mbar_init(&bfull, 1);
+    tc::mbar_init(&bempty, 1);
+    tc::mbar_init(&done, 1);
+    abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 0) tc::tmem_alloc(&tmem_slot, VT_NP);
+  if (warp == VT_EPI + VT_CONV + VT_LOAD) tc::tmem_alloc(&tmem_slot, 512);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = tmem_slot;
-  const int quad = warp & 3, chalf = warp >> 2;    // TMEM lanes 32 quad.., columns 32 chalf.. (sources 16 chalf..)
-  uint32_t phase = 0;
+  const int64_t pairs = (a.nv + VT_ROWS - 1) / VT_ROWS * a.nf;
+  const int64_t u0 = vt_first(pairs, blockIdx.x, gridDim.x);
+  const int n = (int)(vt_first(pairs, blockIdx.x + 1, gridDim.x) - u0);  // this CTA's pairs
+  int tile = (int)(u0 / a.nf), k = (int)(u0 % a.nf);
   bool ok = true;
-  for (int64_t v0 = (int64_t)blockIdx.x * VT_ROWS; v0 < a.nv && ok; v0 += (int64_t)gridDim.x * VT_ROWS) {
-    const int64_t vr = v0 + 32 * quad + lane;      // this thread's voxel row in the epilogue
-    double acc = 0.0;
-    for (int k = 0; k < a.nf && ok; ++k) {
-      // A' = split real embedding of (P phiA)_k for the tile's voxels: element (row, d) -> K' 2d, 2d+1
-      for (int e = tid; e < VT_ROWS * 32; e += VT_THREADS) {
-        const int row = e >> 5, d = e & 31;
-        const int64_t v = v0 + row;
-        double2 x = make_double2(0.0, 0.0);
-        if (v < a.nv && d < a.nd) x = basis_field(a, v, k, d, a.phiA, a.nd);
-        const float xr = (float)x.x, xi = (float)x.y;
-        const float hr = tc::to_tf32(xr), hi_ = tc::to_tf32(xi);
-        const uint32_t off = kmaj64(row, 2 * d, VT_ROWS);
-        *reinterpret_cast<float2 *>(Ahi + off) = make_float2(hr, hi_);
-        *reinterpret_cast<float2 *>(Alo + off) = make_float2(tc::to_tf32(xr - hr), tc::to_tf32(xi - hi_));
-      }
-      // B'_k: a straight copy of its (hi, lo) images
-      {
-        const uint4 *src = reinterpret_cast<const uint4 *>(Btab + (size_t)k * 2 * VT_B);
-        uint4 *dst = reinterpret_cast<uint4 *>(Bhi);
-        for (int e = tid; e < 2 * VT_B / 16; e += VT_THREADS) dst[e] = __ldg(src + e);
-      }
-      tc::fence_async_smem();
-      tc::fence_before_sync();
-      __syncthreads();
-      if (tid == 0) {
-        tc::fence_after_sync();
-        const uint32_t ah = tc::smem_u32(Ahi), al = tc::smem_u32(Alo), bh = tc::smem_u32(Bhi), bl = tc::smem_u32(Blo);
-#pragma unroll
-        for (int kk = 0; kk < VT_KP / 8; ++kk) {       // K = 8 tf32 per MMA; 4 per 128-byte atom
-          const uint32_t oa = (kk >> 2) * VT_ROWS * 128u + 32u * (kk & 3);
-          const uint32_t ob = (kk >> 2) * VT_NP * 128u + 32u * (kk & 3);
-          tc::umma_tf32<VT_IDESC>(tmem, tc::sdesc_k_sw128(ah + oa), tc::sdesc_k_sw128(bh + ob), kk ? 1u : 0u);
-          tc::umma_tf32<VT_IDESC>(tmem, tc::sdesc_k_sw128(ah + oa), tc::sdesc_k_sw128(bl + ob), 1u);
-          tc::umma_tf32<VT_IDESC>(tmem, tc::sdesc_k_sw128(al + oa), tc::sdesc_k_sw128(bh + ob), 1u);
-        }
-        tc::umma_commit(&bar_mma);
-      }
-      bool w = tc::mbar_wait(&bar_mma, phase);
-      phase ^= 1u;
-      if (!w) atomicOr(err, 1);
-      w = __all_sync(0xffffffffu, w);
+
+  if (warp < VT_EPI) {
+    // ---------------------------------------------------------------- Y_k . phi, FP64
+    const int row = 32 * warp + lane, first = tile;
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    int from = k;                                        // first harmonic of this tile that is summed here
+    for (int i = 0; i < n; ++i) {
+      if (__any_sync(FULL, *abort_v != 0)) break;
+      const int j = 2 * i + 1, slot = j % VT_NSLAB, cs = i & 1;
+      ok = __all_sync(FULL, tc::mbar_wait(&cfull[cs], (i >> 1) & 1)) &&
+           __all_sync(FULL, tc::mbar_wait(&full[slot], (j / VT_NSLAB) & 1));
+      if (!ok) break;
       tc::fence_after_sync();
-      if (w) {
-        uint32_t y[32];                                // Y_k[vr][s], s = 16 chalf + i: (re, im) pairs
-        tc::tmem_ld32(tmem + ((uint32_t)(32 * quad) << 16) + 32u * chalf, y);
-        if (vr < a.nv) {
+      const unsigned char *sr = slabs + slot * VT_SLAB + row * 512;
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const int sidx = 16 * chalf + i;
-            if (sidx < a.ns) {
-              const double2 p = basis_field(a, vr, k, sidx, a.phi, a.ns);
-              acc += p.x * (double)__uint_as_float(y[2 * i]) - p.y * (double)__uint_as_float(y[2 * i + 1]);
-            }
+      for (int h = 0; h < 2; ++h) {
+        uint32_t y[32];                                  // sources 16 h ..: (re, im) pairs
+        tc::tmem_ld32(tmem + ((uint32_t)(32 * warp) << 16) + 64u * cs + 32u * h, y);
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+          const int s = 16 * h + q;
+          if (s < a.ns) {
+            const double2 p = *reinterpret_cast<const double2 *>(sr + ((s ^ lane) << 4));
+            acc[q & 3] += p.x * (double)__uint_as_float(y[2 * q]) - p.y * (double)__uint_as_float(y[2 * q + 1]);
           }
         }
       }
       tc::fence_before_sync();
-      ok = __syncthreads_and(w);                       // operands and accumulator are free again
+      __syncwarp();
+      if (lane == 0) {
+        tc::mbar_arrive(&cempty[cs]);
+        tc::mbar_arrive(&empty[slot]);
+      }
+      if (++k == a.nf || i + 1 == n) {
+        const double tot = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+        const int64_t v = (int64_t)tile * VT_ROWS + row;
+        if (from == 0 && k == a.nf) {
+          if (v < a.nv) vjp[v] = (a.w ? a.w[v] : 1.0) * tot;
+        } else {
+          part[(2 * blockIdx.x + (tile == first ? 0 : 1)) * VT_ROWS + row] = tot;
+        }
+        acc[0] = acc[1] = acc[2] = acc[3] = 0.0;
+        k = from = 0;
+        ++tile;
+      }
     }
-    part[tid] = acc;
-    __syncthreads();
-    if (chalf == 0 && vr < a.nv && ok) vjp[vr] = (a.w ? a.w[vr] : 1.0) * (part[tid] + part[tid + 128]);
-    __syncthreads();
+  } else if (warp < VT_EPI + VT_CONV) {
+    // ---------------------------------------------------------------- A' = split FP32 of phiA, into tensor memory
+    const int row = 32 * (warp & 3) + lane;
+    const uint32_t dst0 = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + VT_ACOL;
+    for (int i = 0; i < n; ++i) {
+      if (__any_sync(FULL, *abort_v != 0)) break;
+      const int j = 2 * i, slot = j % VT_NSLAB, as = i & 1;
+      ok = __all_sync(FULL, tc::mbar_wait(&full[slot], (j / VT_NSLAB) & 1)) &&
+           (i < 2 || __all_sync(FULL, tc::mbar_wait(&aempty[as], ((i >> 1) - 1) & 1)));
+      if (!ok) break;
+      tc::fence_after_sync();
+      const unsigned char *sr = slabs + slot * VT_SLAB + row * 512;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {                      // detectors 4 c ..: columns 8 c .. of hi, of lo
+        float hi[8], lo[8];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const double2 x = *reinterpret_cast<const double2 *>(sr + (((4 * c + q) ^ lane) << 4));
+          const float xr = (float)x.x, xi = (float)x.y;
+          hi[2 * q] = tc::to_tf32(xr);
+          hi[2 * q + 1] = tc::to_tf32(xi);
+          lo[2 * q] = tc::to_tf32(xr - hi[2 * q]);
+          lo[2 * q + 1] = tc::to_tf32(xi - hi[2 * q + 1]);
+        }
+        tc::tmem_st8(dst0 + 128u * as + 8u * c, hi);
+        tc::tmem_st8(dst0 + 128u * as + 64u + 8u * c, lo);
+      }
+      tc::tmem_wait_st();
+      tc::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) {
+        tc::mbar_arrive(&afull[as]);
+        tc::mbar_arrive(&empty[slot]);
+      }
+    }
+  } else if (warp < VT_EPI + VT_CONV + VT_LOAD) {
+    // ---------------------------------------------------------------- field rows into the ring
+    const int w = warp - VT_EPI - VT_CONV;
+    for (int j = 0; j < 2 * n && ok; ++j) {
+      if (__any_sync(FULL, *abort_v != 0)) break;
+      const int slot = j % VT_NSLAB;
+      if (j >= VT_NSLAB) ok = __all_sync(FULL, tc::mbar_wait(&empty[slot], (j / VT_NSLAB - 1) & 1));
+      if (!ok) break;
+      const int cnt = j & 1 ? a.ns : a.nd;
+      const double2 *f = j & 1 ? a.phi : a.phiA;
+      const int64_t v0 = (int64_t)tile * VT_ROWS + w;
+      const double2 *src = f + ((int64_t)k * a.nn + v0) * cnt + lane;
+      unsigned char *dst = slabs + slot * VT_SLAB + w * 512;
+#pragma unroll 8
+      for (int rr = 0; rr < VT_ROWS / VT_LOAD; ++rr) {   // row w + 4 rr, element = lane
+        const bool in = lane < cnt && v0 + VT_LOAD * rr < a.nv;
+        tc::cp_async16(dst + rr * (VT_LOAD * 512) + ((lane ^ ((w + VT_LOAD * rr) & 31)) << 4),
+                       in ? src + (int64_t)VT_LOAD * rr * cnt : f, in);
+      }
+      tc::cp_async_arrive(&full[slot]);
+      if ((j & 1) && ++k == a.nf) {
+        k = 0;
+        ++tile;
+      }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  } else if (warp == VT_EPI + VT_CONV + VT_LOAD) {
+    // ---------------------------------------------------------------- MMA issue (one thread)
+    if (lane == 0) {
+      const uint64_t bh0 = tc::sdesc_k_sw128(tc::smem_u32(B)), bl0 = tc::sdesc_k_sw128(tc::smem_u32(B + VT_B));
+      for (int i = 0; i < n && ok && !*abort_v; ++i) {
+        const int st = i & 1;
+        ok = (i < 2 || tc::mbar_wait(&cempty[st], ((i >> 1) - 1) & 1)) && tc::mbar_wait(&bfull, i & 1) &&
+             tc::mbar_wait(&afull[st], (i >> 1) & 1);
+        if (!ok) break;
+        tc::fence_after_sync();
+        const uint32_t d = tmem + 64u * st, ah = tmem + VT_ACOL + 128u * st, al = ah + 64u;
+#pragma unroll
+        for (int kk = 0; kk < VT_KP / 8; ++kk) {         // K = 8 tf32 per MMA; 4 per 128-byte atom of B'
+          const uint64_t ob = (uint64_t)((kk >> 2) * VT_NP * 128 / 16 + 2 * (kk & 3));
+          tc::umma_tf32_ts<VT_IDESC>(d, ah + 8u * kk, bh0 + ob, kk ? 1u : 0u);
+          tc::umma_tf32_ts<VT_IDESC>(d, ah + 8u * kk, bl0 + ob, 1u);
+          tc::umma_tf32_ts<VT_IDESC>(d, al + 8u * kk, bh0 + ob, 1u);
+        }
+        tc::umma_commit(&bempty);
+        tc::umma_commit(&aempty[st]);
+        tc::umma_commit(&cfull[st]);
+      }
+      tc::umma_commit(&done);                            // arrives once every MMA issued has completed
+      if (!tc::mbar_wait(&done, 0)) ok = false;
+    }
+    __syncwarp();
+  } else if (lane == 0) {
+    // ---------------------------------------------------------------- B'_k
+    int i = 0;
+    for (; i < n && !*abort_v; ++i) {
+      if (i > 0) ok = tc::mbar_wait(&bempty, (i - 1) & 1);
+      if (!ok) break;
+      tc::mbar_expect_tx(&bfull, 2 * VT_B);
+      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                       tc::smem_u32(B)),
+                   "l"(Btab + (size_t)k * 2 * VT_B), "r"(2 * VT_B), "r"(tc::smem_u32(&bfull))
+                   : "memory");
+      if (++k == a.nf) k = 0;
+    }
+    if (i > 0 && !tc::mbar_wait(&bfull, (i - 1) & 1)) ok = false;  // no copy is left in flight
+  }
+  if (!ok) {
+    atomicOr(err, 1);
+    *abort_v = 1;
   }
   tc::fence_before_sync();
   __syncthreads();
-  if (warp == 0) tc::tmem_free(tmem, VT_NP);
+  if (warp == VT_EPI + VT_CONV + VT_LOAD) tc::tmem_free(tmem, 512);
+}
+
+// tiles whose harmonics several CTAs summed: their parts in the order of the CTAs
+__global__ void k_vjp_join(int64_t nv, int nf, int ctas, const double *__restrict__ part, const double *__restrict__ w,
+                           double *__restrict__ vjp) {
+  const int64_t pairs = (nv + VT_ROWS - 1) / VT_ROWS * nf, ub = (int64_t)blockIdx.x * nf, ue = ub + nf;
+  int c = (int)(ub * ctas / pairs);
+  while (vt_first(pairs, c + 1, ctas) <= ub) ++c;
+  while (vt_first(pairs, c, ctas) > ub) --c;
+  if (vt_first(pairs, c + 1, ctas) >= ue) return;        // one CTA had them all
+  const int64_t v = (int64_t)blockIdx.x * VT_ROWS + threadIdx.x;
+  if (v >= nv) return;
+  double tot = 0.0;
+  for (; c < ctas && vt_first(pairs, c, ctas) < ue; ++c) {
+    const int64_t b = vt_first(pairs, c, ctas);
+    if (vt_first(pairs, c + 1, ctas) == b) continue;
+    tot += part[(2 * c + (b / nf == blockIdx.x ? 0 : 1)) * VT_ROWS + threadIdx.x];
+  }
+  vjp[v] = (w ? w[v] : 1.0) * tot;
 }
 
 // Vector-Jacobian product out[v] = w_v sum_m sum_k Re(Chat[m,k] a_k(m)) for VB voxels per block
@@ -928,13 +1083,25 @@ int launch_common(JArgs &a, size_t &smem, int &grid) {
   return DGP_OK;
 }
 
+// Projected fields of as many of `chunk` voxels, `bytes` each, as stay in L2 (126 MB) between the kernel
+// that writes them and the one that reads them; fewer on a nearly full device.
+int alloc_chunk(ScratchBuf &buf, int64_t &chunk, size_t bytes, cudaStream_t st) {
+  chunk = std::min<int64_t>(chunk, std::max<int64_t>(1, ((int64_t)96 << 20) / (int64_t)bytes));
+  int rc = buf.alloc(bytes * chunk, st);
+  while (rc != DGP_OK && chunk > 64) {
+    chunk /= 4;
+    rc = buf.alloc(bytes * chunk, st);
+  }
+  return rc;
+}
+
 }  // namespace
 
 // 0 (default) and 2: the tensor cores where the shapes fit (TG Jacobian: nodal basis, unique
 //   links, up to 32 sources and detectors, shared memory for the operand rings; vjp: up to 32
 //   sources and detectors), else the CUDA cores.  Measured at the sensitivity configuration
 //   (100k voxels, 32 x 32 optodes, 64 harmonics, 20 gates, one B200): TG Jacobian 11.9 ms
-//   against 20.0 ms, vjp 5.2 ms against 16.4 ms.
+//   against 20.0 ms, vjp 1.2 ms against 16.4 ms.
 // 1: both on the CUDA cores (cross-checks, timing)
 static int g_jacobian_engine = 0;
 
@@ -1028,16 +1195,10 @@ int jacobian_run(int mode, const int32_t *prow, const int32_t *pcol, const doubl
     // two buffers of fields, one where two don't fit
     const int nbuf = smem_of(tpv, 2) <= 200 * 1024 ? 2 : 1;
     const size_t smem_tg = smem_of(tpv, nbuf);
-    // projected fields in chunks that stay in L2 between the two kernels
-    int64_t chunk = std::min<int64_t>(nv, std::max<int64_t>(1, ((int64_t)96 << 20) / (8 * per)));
     ScratchBuf ckg, fields, ryt;
     DGP_TRY(ckg.alloc(sizeof(float4) * (size_t)nf * (ngc / 2), st));
-    int frc = fields.alloc(sizeof(float2) * (size_t)chunk * per, st);
-    while (frc != DGP_OK && chunk > 64) {  // a nearly full device: smaller chunks
-      chunk /= 4;
-      frc = fields.alloc(sizeof(float2) * (size_t)chunk * per, st);
-    }
-    DGP_TRY(frc);
+    int64_t chunk = nv;
+    DGP_TRY(alloc_chunk(fields, chunk, sizeof(float2) * per, st));
     if (rytov) {
       DGP_TRY(ryt.alloc(sizeof(float) * (size_t)nm * ng, st));
       k_rytov_t<<<(unsigned)ceil_div((int64_t)nm * ng, 256), 256, 0, st>>>(rytov, nm, ng, ryt.as<float>());
@@ -1098,18 +1259,38 @@ int jacobian_run(int mode, const int32_t *prow, const int32_t *pcol, const doubl
                                                                       chat.as<float2>());
     DGP_CHECK_LAUNCH();
     if (g_jacobian_engine != 1 && ns <= 32 && nd <= 32 && nm <= 4096) {
-      // tensor cores: per-harmonic complex GEMM over voxel tiles
-      ScratchBuf btab, flag;
+      // tensor cores: per-harmonic complex GEMM over voxel tiles; a voxel basis chunk by chunk through
+      // projected fields that stay in L2 between the two kernels
+      const int64_t per = (int64_t)nf * (ns + nd);
+      int64_t chunk = nv;
+      ScratchBuf btab, flag, part, fields;
       DGP_TRY(btab.alloc((size_t)nf * 2 * VT_B, st));
       DGP_TRY(flag.alloc(sizeof(int), st));
+      DGP_TRY(part.alloc(sizeof(double) * 2 * VT_ROWS * (size_t)sm_count(), st));
+      if (prow) DGP_TRY(alloc_chunk(fields, chunk, sizeof(double2) * per, st));
       DGP_CUDA(cudaMemsetAsync(flag.p, 0, sizeof(int), st));
       k_vjp_btab<<<(unsigned)ceil_div((int64_t)nf * 1024, 256), 256, 0, st>>>(chat.as<float2>(), link, nm, nf,
                                                                               btab.as<unsigned char>());
       DGP_CHECK_LAUNCH();
-      DGP_CUDA(cudaFuncSetAttribute(k_jacobian_vjp_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, VT_SMEM));
-      const int gv = (int)std::min<int64_t>(ceil_div(nv, VT_ROWS), (int64_t)sm_count() * 2);
-      k_jacobian_vjp_tc<<<gv, VT_THREADS, VT_SMEM, st>>>(a, btab.as<unsigned char>(), (double *)out, flag.as<int>());
-      DGP_CHECK_LAUNCH();
+      DGP_TRY(allow_dyn_smem(k_jacobian_vjp_tc, VT_SMEM));
+      for (int64_t v0 = 0; v0 < nv; v0 += chunk) {
+        JArgs b = a;
+        b.nv = std::min(chunk, nv - v0);
+        if (prow) {
+          double2 *f = fields.as<double2>(), *fA = f + b.nv * nf * ns;
+          k_project_slabs<<<(unsigned)b.nv, JBS, 0, st>>>(a, v0, f, fA);
+          DGP_CHECK_LAUNCH();
+          b.phi = f, b.phiA = fA, b.nn = b.nv;
+          if (w) b.w = w + v0;
+        }
+        const int64_t tiles = ceil_div(b.nv, VT_ROWS);
+        const int gv = (int)std::min<int64_t>(tiles * nf, sm_count());
+        k_jacobian_vjp_tc<<<gv, VT_THREADS, VT_SMEM, st>>>(b, btab.as<unsigned char>(), (double *)out + v0,
+                                                           part.as<double>(), flag.as<int>());
+        DGP_CHECK_LAUNCH();
+        k_vjp_join<<<(unsigned)tiles, VT_ROWS, 0, st>>>(b.nv, nf, gv, part.as<double>(), b.w, (double *)out + v0);
+        DGP_CHECK_LAUNCH();
+      }
       int h = 0;
       DGP_CUDA(cudaMemcpyAsync(&h, flag.p, sizeof(int), cudaMemcpyDeviceToHost, st));
       DGP_CUDA(cudaStreamSynchronize(st));

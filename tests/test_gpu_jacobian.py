@@ -318,3 +318,48 @@ def test_tg_jacobian_projected_fields(ns, nd, nf, ng, nm, nv, rows, use_rytov):
     scale = wts[:, None, None] / (ryt.T[None] if use_rytov else 1.0)
     err = np.abs(J.cpu().numpy() - scale * J0)
     assert (err <= (2 * nf + 8) * 2.0 ** -24 * np.sqrt(2) * scale * mag).all()
+
+
+@pytest.mark.parametrize("ns,nd,nf,ng,nm,nv,rows", [
+    (1, 1, 1, 1, 1, 1, "nodal"),           # one pair of a tile and a harmonic
+    (32, 32, 64, 20, 1024, 129, "nodal"),  # two tiles, each shared by many blocks
+    (7, 5, 3, 4, 40, 40001, "nodal"),      # more tiles than blocks, a block's run inside several tiles
+    (32, 17, 9, 32, 4096, 1000, "four"),   # the longest link list, repeated pairs
+    (5, 32, 70, 2, 150, 257, "any"),       # more than 64 harmonics; rows of 0 to 8 entries
+    (32, 32, 64, 3, 700, 3333, "any"),     # projected in several chunks
+])
+def test_vjp_tensor_core_tiles(ns, nd, nf, ng, nm, nv, rows):
+    """Tensor-core vjp against 64-bit sums for random fields, bases and links.  A partial sum over the
+    detectors is the FP32 accumulation of 3 x 64 truncated products, operands rounded to 2^-24: off by
+    at most 200 x 2^-23 of the sum of its terms' magnitudes (times sqrt 2, complex)."""
+    import scipy.sparse as sp
+    import torch
+    from dogpup_b200 import api
+    rng = np.random.default_rng(nv)
+    nn = nv if rows == "nodal" else 91
+    cn = lambda *s: rng.standard_normal(s) + 1j * rng.standard_normal(s)
+    phi, phiA, fpsf, gates = cn(nf, nn, ns), cn(nf, nn, nd), cn(nf), cn(ng, nf)
+    link = np.stack([rng.integers(0, ns, nm), rng.integers(0, nd, nm)], 1).astype(np.int32)
+    wts, gin = rng.uniform(0.5, 2.0, nv), rng.standard_normal((nm, ng))
+    if rows == "nodal":
+        P = sp.identity(nn, format="csr")
+        basis = api.Basis(None, wts, nn=nn)
+    else:
+        cnt = np.full(nv, 4) if rows == "four" else rng.integers(0, 9, nv)
+        col = np.concatenate([rng.choice(nn, c, replace=False) for c in cnt]).astype(np.int32)
+        P = sp.csr_matrix((rng.uniform(0.1, 1.0, col.size), col, np.concatenate([[0], np.cumsum(cnt)])), shape=(nv, nn))
+        basis = api.Basis(P, wts)
+    cu = lambda x: torch.as_tensor(x, device="cuda")
+    v = api.jacobian_tg_vjp(basis, cu(phi), cu(phiA), cu(fpsf), cu(link), cu(gates), 64, cu(gin))
+    C = -128.0 * np.where(np.arange(nf) == 0, 0.5, 1.0) * np.conj(gates) / fpsf      # [ng, nf]
+    ch, cm = gin @ C, np.abs(gin) @ np.abs(C)                                        # [nm, nf]
+    v0, mag = np.zeros(nv), np.zeros(nv)
+    for k in range(nf):
+        M, A = np.zeros((ns, nd), complex), np.zeros((ns, nd))
+        np.add.at(M, (link[:, 0], link[:, 1]), ch[:, k])
+        np.add.at(A, (link[:, 0], link[:, 1]), cm[:, k])
+        x, y = P @ phi[k], P @ phiA[k]
+        v0 += np.real((x * (y @ M.T)).sum(1))
+        mag += (np.abs(x) * (np.abs(y) @ A.T)).sum(1)
+    err = np.abs(v.cpu().numpy() - wts * v0)
+    assert (err <= 200 * 2.0 ** -23 * np.sqrt(2) * wts * mag).all()
