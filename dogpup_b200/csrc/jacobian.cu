@@ -147,7 +147,8 @@ __global__ void __launch_bounds__(JBS) k_jacobian_complex(JArgs a, const double2
 __global__ void __launch_bounds__(JBS) k_project(JArgs a, int64_t v0, int64_t per, float2 *__restrict__ F) {
   float2 *out = F + (int64_t)blockIdx.x * per;
   const int st = a.ns + a.nd;
-  project_voxel(a, v0 + blockIdx.x, [&](int k, int o, double2 z) { out[k * st + o] = make_float2((float)z.x, (float)z.y); });
+  project_voxel(a, v0 + blockIdx.x,
+                [&](int k, int o, double2 z) { out[k * st + o] = make_float2((float)z.x, (float)z.y); });
 }
 
 // Time-gated Jacobian on the CUDA cores (voxel bases, more than 32 optodes or 64 harmonics): voxels
@@ -287,28 +288,37 @@ __global__ void k_rytov_t(const double *__restrict__ rytov, int nm, int ng, floa
 // written to shared memory and read back by every MMA: ~100 KB per stage), so here:
 //   - the A' stages go from the builders' registers straight into tensor memory (tcgen05.st;
 //     warp 4+q writes lanes 32q.. = the rows of gate 4t+q) and the MMAs read A' from there;
-//   - the fields of the next voxel are copied into shared memory by cp.async while the current
-//     one is built (completion counted on an mbarrier), and each builder keeps its source
-//     fields in registers for the whole voxel.
+//   - four feeder warps read the next voxel's fields straight into registers and leave them in
+//     shared memory as the readers want them: complex FP32 for the builders, B'' for the MMAs
+//     (with builders that copied and converted the FP64 rows themselves, leaving out either took 9
+//     to 13 % off the kernel's time);
+//   - a row of J (a gate's NS x ND entries) is put together in shared memory, 16-byte pieces in an
+//     order that spreads the banks, and leaves as one bulk copy, or through the Rytov division in
+//     consecutive 16-byte stores.
 //
 // Persistent CTA (one per SM), warp-specialised, all hand-offs through mbarriers:
 //   warps 0-3   epilogue: per tile, tensor memory -> hi + lo halves, w_v (and Rytov) -> J
 //               (warp q reads accumulator lanes 32q.. = gate 4t+q of tile t, lane = source)
-//   warps 4-11  builders: field copies, A' stages tile by tile (lane = source, warp = gate
-//               within the tile x harmonic half)
-//   warp 12     one thread issues the MMAs (tile by tile: every chunk of a tile, after which
+//   warps 4-19  builders: A' stages tile by tile (lane = source, warp = gate within the tile x
+//               harmonic quarter of a chunk)
+//   warp 20     one thread issues the MMAs (tile by tile: every chunk of a tile, after which
 //               its accumulator is complete); tensor-memory allocation
-//   warps 13-14 B'' of each voxel as soon as its fields are staged (lane = detector), ahead of
-//               the MMAs that need it
+//   warps 21-24 feeders: sources and B'' of each voxel, ahead of the builders and MMAs that need
+//               them (lane = optode)
+// Bound by the chain of build, hand-over and MMAs through the three stages that tensor memory has
+// room for: without the MMAs the kernel takes 5.1 ms of its 7.4, without the builders' stores 6.6,
+// with half the MMAs 6.1.  101,880 nodes x 1,024 links x 64 harmonics x 20 gates: 7.8 ms with eight
+// builder warps that also staged the fields, 7.4 now; 20,000 nodes with Rytov 10.1 -> 2.8 ms (FP64
+// divisors read and rows written 4 bytes at a time before).  Six stages of one chunk (8.1 to 9.2 ms:
+// the cost per stage is the hand-over) and two builder groups on alternate stages (8.7) were slower.
 // Tensor memory: 2 accumulator slots of 64 columns (a tile's slot is released as soon as the
 // epilogue has read it), then 3 A' stages of two chunks each (128 columns: hi 0-63, lo 64-127),
 // so the MMA thread waits once per 16 MMAs (an mbarrier wait right after a burst of MMAs costs
 // a few hundred cycles on B200).  Every mbarrier
 // wait is bounded: a timeout sets err, raises the abort flag that every role polls, and the
 // MMA thread waits (bounded) for all of its MMAs before the tensor memory is freed.
-constexpr int T2_EPI = 4, T2_BLD = 8, T2_BB = 2;    // epilogue, A' builder, B'' builder warps
-constexpr int T2_THREADS = 32 * (T2_EPI + T2_BLD + 1 + T2_BB);
-constexpr int T2_BT = 32 * T2_BLD;                 // builder threads
+constexpr int T2_EPI = 4, T2_BLD = 16, T2_FD = 4;   // epilogue, A' builder, feeder warps
+constexpr int T2_THREADS = 32 * (T2_EPI + T2_BLD + 1 + T2_FD);
 constexpr int T2_NSLOT = 2;                        // accumulator slots (64 columns each)
 constexpr int T2_NST = 3;                          // A' stages in tensor memory (2 chunks, 128 columns each)
 constexpr uint32_t T2_ACOL = 64u * T2_NSLOT;       // first A' column
@@ -316,8 +326,7 @@ constexpr int T2_BCH = 2 * 32 * 128;               // one chunk of B'': 32 hi ro
 constexpr uint32_t T2_IDESC = tc::idesc(2, 2, 128, 64);
 
 struct T2Layout {
-  uint32_t b_off, f_off, c_off, l_off, bytes;      // shared memory, from the 1 KB-aligned base
-  uint32_t fbuf;                                   // bytes of one voxel's staged fields
+  uint32_t b_off, f_off, c_off, l_off, o_off, bytes;  // shared memory, from the 1 KB-aligned base
   int nch, ntile, nkp;
 };
 
@@ -326,26 +335,13 @@ __host__ __device__ inline T2Layout t2_layout(int nf, int ng) {
   L.nch = (nf + 15) / 16;
   L.ntile = (ng + 3) / 4;
   L.nkp = 16 * L.nch;
-  L.fbuf = (uint32_t)(2 * 32 * 16 * L.nkp);                      // [2 fields][NKP][32] complex FP64
   L.b_off = 0;
-  L.f_off = L.b_off + 2 * L.nch * T2_BCH;                        // two voxels' staged fields
-  L.c_off = L.f_off + 2 * L.fbuf;                                // gate table [4 NTILE][NKP] float2
+  L.f_off = L.b_off + 2 * L.nch * T2_BCH;                        // two voxels' source fields [NKP][32] float2
+  L.c_off = L.f_off + 2 * (uint32_t)(32 * 8 * L.nkp);            // gate table [4 NTILE][NKP] float2
   L.l_off = L.c_off + (uint32_t)(8 * 4 * L.ntile * L.nkp);        // link lookup [32][32] int
-  L.bytes = L.l_off + 4 * 32 * 32;
+  L.o_off = L.l_off + 4 * 32 * 32;                               // a gate's output row per epilogue warp
+  L.bytes = L.o_off + 4096 * T2_EPI;
   return L;
-}
-
-// cp.async copies of voxel v's fields into a staging buffer [2][NKP][32] (source, then detector;
-// zero past NF and past the optode counts): builder thread bt copies elements bt + 256 q
-__device__ inline void t2_stage_fields(const JArgs &a, int64_t v, int nkp, unsigned char *dst, int bt) {
-  const int per = nkp * 32;
-  for (int e = bt; e < 2 * per; e += T2_BT) {
-    const bool det = e >= per;
-    const int r = det ? e - per : e, k = r >> 5, o = r & 31, cnt = det ? a.nd : a.ns;
-    const double2 *f = det ? a.phiA : a.phi;
-    const bool ok = o < cnt && k < a.nf;
-    tc::cp_async16(dst + 16 * (size_t)e, ok ? f + ((int64_t)k * a.nn + v) * cnt + o : f, ok);
-  }
 }
 
 // x -> (tf32(x), tf32(x - tf32(x))) for 4 values, stored as 16-byte chunks of the hi and lo images
@@ -360,11 +356,17 @@ __device__ inline void st_split4(unsigned char *hi, unsigned char *lo, uint32_t 
   *reinterpret_cast<float4 *>(lo + off) = make_float4(l[0], l[1], l[2], l[3]);
 }
 
+__device__ inline void swap_if(bool p, float4 &x, float4 &y) {
+  const float4 t = x;
+  x = p ? y : x;
+  y = p ? t : y;
+}
+
 __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const float2 *__restrict__ C /*[ng][nf]*/,
-                                                                 const double *__restrict__ rytov, int dense,
+                                                                 const float *__restrict__ ryt /*[ng][nm]*/, int dense,
                                                                  float *__restrict__ Jtg, int *err) {
   extern __shared__ __align__(1024) unsigned char t2_raw[];
-  __shared__ __align__(8) uint64_t full[T2_NST], empty[T2_NST], bfull[2], bempty[2], fready[2], fdone[2];
+  __shared__ __align__(8) uint64_t full[T2_NST], empty[T2_NST], bfull[2], bempty[2], sfull[2], sempty[2];
   __shared__ __align__(8) uint64_t tfull[T2_NSLOT], tempty[T2_NSLOT], done;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
@@ -382,10 +384,10 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
       tc::mbar_init(&empty[i], 1);
     }
     for (int b = 0; b < 2; ++b) {
-      tc::mbar_init(&bfull[b], T2_BB);
+      tc::mbar_init(&bfull[b], T2_FD);
       tc::mbar_init(&bempty[b], 1);
-      tc::mbar_init(&fready[b], T2_BT);                // one cp.async arrival per builder thread
-      tc::mbar_init(&fdone[b], T2_BLD + T2_BB);        // readers of a staged voxel's fields
+      tc::mbar_init(&sfull[b], T2_FD);
+      tc::mbar_init(&sempty[b], T2_BLD);
     }
     for (int q = 0; q < T2_NSLOT; ++q) {
       tc::mbar_init(&tfull[q], 1);
@@ -467,32 +469,41 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
     }
     __syncwarp();
   } else if (warp > T2_EPI + T2_BLD) {
-    // ---------------------------------------------------------------- B'' builders
-    // Voxel i's detector operand into buffer i % 2 as soon as its fields are staged (fready) and
-    // the MMAs of voxel i - 2 are done with the buffer (bempty): warp w takes the 8-harmonic
-    // blocks p = w, w + 2, .. (chunk p / 2, half p % 2), lane = detector.
+    // ---------------------------------------------------------------- feeders
+    // Voxel i's fields into buffers i % 2 once the builders (sempty) and the MMAs (bempty) of voxel
+    // i - 2 are done with them: warp w takes the 8-harmonic blocks p = w, w + 4, .., lane = optode.
+    // Sources as complex FP32 [harmonic][32], detectors as B'' (chunk p / 2, half p % 2).
     const int w = warp - (T2_EPI + T2_BLD + 1);
-    unsigned char *fst = sm + L.f_off;
     int i = 0;
     bool fail = false;
+    auto buffers_free = [&](int i) {
+      const int b = i & 1;
+      return i < 2 || (__all_sync(FULL, tc::mbar_wait(&sempty[b], ((i >> 1) - 1) & 1)) &&
+                       __all_sync(FULL, tc::mbar_wait(&bempty[b], ((i >> 1) - 1) & 1)));
+    };
     for (int64_t v = blockIdx.x; v < a.nv; v += gridDim.x, ++i) {
       if (__any_sync(FULL, *abort_v != 0)) break;
       const int bj = i & 1;
-      if (!__all_sync(FULL, tc::mbar_wait(&fready[bj], (i >> 1) & 1)) ||
-          (i >= 2 && !__all_sync(FULL, tc::mbar_wait(&bempty[bj], ((i >> 1) - 1) & 1)))) {
-        fail = true;
-        break;
-      }
-      const double2 *fd = reinterpret_cast<const double2 *>(fst + bj * L.fbuf) + L.nkp * 32;
+      bool free = w < 2 * L.nch || buffers_free(i);      // (a warp without a block keeps step)
       unsigned char *bb = sm + L.b_off + bj * L.nch * T2_BCH;
-      for (int p = w; p < 2 * L.nch; p += T2_BB) {
+      float2 *fs = reinterpret_cast<float2 *>(sm + L.f_off) + bj * 32 * L.nkp + lane;
+      for (int p = w; p < 2 * L.nch; p += T2_FD) {
+        double2 x[8];
+        const double2 *py = a.phiA + ((int64_t)(8 * p) * a.nn + v) * a.nd + lane;
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          x[q] = 8 * p + q < a.nf && lane < a.nd ? __ldg(py + (int64_t)q * a.nn * a.nd) : make_double2(0.0, 0.0);
+        if (p == w && !(free = buffers_free(i))) break;  // (the first loads are under way)
         float re[8], im[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-          const double2 y = fd[(8 * p + q) * 32 + lane];
-          re[q] = (float)y.x;
-          im[q] = (float)y.y;
+          re[q] = (float)x[q].x;
+          im[q] = (float)x[q].y;
         }
+        const double2 *px = a.phi + ((int64_t)(8 * p) * a.nn + v) * a.ns + lane;
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          x[q] = 8 * p + q < a.nf && lane < a.ns ? __ldg(px + (int64_t)q * a.nn * a.ns) : make_double2(0.0, 0.0);
         unsigned char *bh = bb + (p >> 1) * T2_BCH;
         const float r0[4] = {re[0], re[1], re[2], re[3]}, r1[4] = {re[4], re[5], re[6], re[7]};
         const float i0[4] = {im[0], im[1], im[2], im[3]}, i1[4] = {im[4], im[5], im[6], im[7]};
@@ -501,12 +512,18 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
         st_split4(bh, bh + 4096, tc::sw128_chunk(lane, 2 * h + 1), r1);
         st_split4(bh, bh + 4096, tc::sw128_chunk(lane, 4 + 2 * h + 0), i0);
         st_split4(bh, bh + 4096, tc::sw128_chunk(lane, 4 + 2 * h + 1), i1);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) fs[32 * (8 * p + q)] = make_float2((float)x[q].x, (float)x[q].y);
+      }
+      if (!free) {
+        fail = true;
+        break;
       }
       tc::fence_async_smem();                            // B'' -> async proxy
       __syncwarp();
       if (lane == 0) {
+        tc::mbar_arrive(&sfull[bj]);
         tc::mbar_arrive(&bfull[bj]);
-        tc::mbar_arrive(&fdone[bj]);
       }
     }
     if (fail && lane == 0) {
@@ -515,46 +532,31 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
     }
   } else if (warp >= T2_EPI) {
     // ---------------------------------------------------------------- builders
-    // Per voxel i (staging buffer i % 2): copy voxel i+1's fields into the other buffer once
-    // every reader of voxel i-1's is done with them (fdone), wait for voxel i's copies (fready),
-    // read this thread's source fields into registers (harmonics 16 c + 8 half + j), then build
-    // the A' stages tile by tile into tensor memory.  Waits are warp-uniform.
-    const int bt = tid - 32 * T2_EPI, bw = bt >> 5, gl = bw & 3, half = bw >> 2, s = lane;
-    unsigned char *fst = sm + L.f_off;
-    int64_t v = blockIdx.x;
-    if (v < a.nv) t2_stage_fields(a, v, L.nkp, fst, bt);
-    tc::cp_async_arrive(&fready[0]);
+    // Per voxel i: read this thread's source fields into registers (harmonics 16 c + 4 part + j),
+    // then build the A' stages tile by tile into tensor memory.  Waits are warp-uniform.
+    const int bw = warp - T2_EPI, gl = bw & 3, part = bw >> 2, s = lane;
     uint32_t st_idx = 0;
     int i = 0;
     bool fail = false;
-    for (; v < a.nv && !fail; v += gridDim.x, ++i) {
+    for (int64_t v = blockIdx.x; v < a.nv && !fail; v += gridDim.x, ++i) {
       if (__any_sync(FULL, *abort_v != 0)) break;
       const int buf = i & 1;
-      const int64_t vn = v + gridDim.x;
-      if (vn < a.nv) {
-        if (i >= 1 && !__all_sync(FULL, tc::mbar_wait(&fdone[buf ^ 1], ((i - 1) >> 1) & 1))) {
-          fail = true;
-          break;
-        }
-        t2_stage_fields(a, vn, L.nkp, fst + (buf ^ 1) * L.fbuf, bt);
-        tc::cp_async_arrive(&fready[buf ^ 1]);
-      }
-      if (!__all_sync(FULL, tc::mbar_wait(&fready[buf], (i >> 1) & 1))) {
+      if (!__all_sync(FULL, tc::mbar_wait(&sfull[buf], (i >> 1) & 1))) {
         fail = true;
         break;
       }
-      const double2 *fs = reinterpret_cast<const double2 *>(fst + buf * L.fbuf);
-      float pr[4][8], pi[4][8];
+      const float2 *fs = reinterpret_cast<const float2 *>(sm + L.f_off) + buf * 32 * L.nkp + s;
+      float pr[4][4], pi[4][4];
 #pragma unroll
       for (int c = 0; c < 4; ++c)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const double2 y = c < L.nch ? fs[(16 * c + 8 * half + j) * 32 + s] : make_double2(0.0, 0.0);
-          pr[c][j] = (float)y.x;
-          pi[c][j] = (float)y.y;
+        for (int j = 0; j < 4; ++j) {
+          const float2 y = c < L.nch ? fs[32 * (16 * c + 4 * part + j)] : make_float2(0.f, 0.f);
+          pr[c][j] = y.x;
+          pi[c][j] = y.y;
         }
       __syncwarp();
-      if (lane == 0) tc::mbar_arrive(&fdone[buf]);
+      if (lane == 0) tc::mbar_arrive(&sempty[buf]);
       for (int t = 0; t < L.ntile && !fail; ++t) {
 #pragma unroll
         for (int c0 = 0; c0 < 4; c0 += 2) {             // a stage = chunks c0, c0 + 1
@@ -569,10 +571,10 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
           for (int cc = 0; cc < 2; ++cc) {
             const int c = c0 + cc;
             if (c >= L.nch) break;
-            const float2 *cg = Ct + (4 * t + gl) * L.nkp + 16 * c + 8 * half;
-            float hr[8], lr[8], hm[8], lm[8];
+            const float2 *cg = Ct + (4 * t + gl) * L.nkp + 16 * c + 4 * part;
+            float hr[4], lr[4], hm[4], lm[4];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
+            for (int j = 0; j < 4; ++j) {
               const float2 q = cg[j];
               const float qr = q.x * pr[c][j] - q.y * pi[c][j], qi = -(q.x * pi[c][j] + q.y * pr[c][j]);
               // hi = x with the 13 low mantissa bits cleared (a TF32 value), lo = x - hi (exact);
@@ -582,13 +584,13 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
               hm[j] = __uint_as_float(__float_as_uint(qi) & 0xffffe000u);
               lm[j] = qi - hm[j];
             }
-            // row gl * 32 + s = lane s of this warp's quadrant; chunk cc of the stage: K' = 8 half + j
-            // (real), 16 + 8 half + j (imaginary); lo 64 columns after hi
-            const uint32_t tq = tmem + ((uint32_t)(32 * gl) << 16) + T2_ACOL + 128u * si + 32u * cc + 8u * half;
-            tc::tmem_st8(tq, hr);
-            tc::tmem_st8(tq + 16u, hm);
-            tc::tmem_st8(tq + 64u, lr);
-            tc::tmem_st8(tq + 80u, lm);
+            // row gl * 32 + s = lane s of this warp's quadrant; chunk cc of the stage: K' = 4 part + j
+            // (real), 16 + 4 part + j (imaginary); lo 64 columns after hi
+            const uint32_t tq = tmem + ((uint32_t)(32 * gl) << 16) + T2_ACOL + 128u * si + 32u * cc + 4u * part;
+            tc::tmem_st(tq, hr);
+            tc::tmem_st(tq + 16u, hm);
+            tc::tmem_st(tq + 64u, lr);
+            tc::tmem_st(tq + 80u, lm);
           }
           tc::tmem_wait_st();                            // the stores have landed, then
           tc::fence_before_sync();                       // ordered before the arrival
@@ -598,7 +600,6 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
         }
       }
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");    // no copy outlives the kernel
     if (fail && lane == 0) {
       atomicOr(err, 8);
       *abort_v = 1;
@@ -606,6 +607,7 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
   } else {
     // ---------------------------------------------------------------- epilogue
     const int gl = warp, s = lane;
+    unsigned char *ob = sm + L.o_off + 4096 * warp;
     uint32_t tl_idx = 0;
     bool ok = true;
     for (int64_t v = blockIdx.x; v < a.nv && ok; v += gridDim.x) {
@@ -622,40 +624,78 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
           break;
         }
         tc::fence_after_sync();
-        uint32_t r[32], q[32];
-        const uint32_t ta = tmem + ((uint32_t)(32 * warp) << 16) + 64u * slot;
-        tc::tmem_ld32(ta, r);                            // (A_hi + A_lo) B_hi
-        tc::tmem_ld32(ta + 32u, q);                      // (A_hi + A_lo) B_lo
-        tc::fence_before_sync();
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&tempty[slot]);
         const int g = 4 * t + gl;
-        if (g >= a.ng || s >= a.ns) continue;
         float *row = Jtg + ((int64_t)v * a.ng + g) * a.nm;
-        if (dense == 2) {                                // m = s nd + d, nd and nm multiples of 4
-          float4 *dst = reinterpret_cast<float4 *>(row + s * a.nd);
+        if (dense == 2) {                                // the row's last copy has left the buffer
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+          __syncwarp();
+        }
 #pragma unroll
-          for (int d4 = 0; d4 < 8; ++d4)
-            if (4 * d4 < a.nd) {
-              const int d = 4 * d4;
-              dst[d4] = make_float4(wv * (__uint_as_float(r[d]) + __uint_as_float(q[d])),
-                                    wv * (__uint_as_float(r[d + 1]) + __uint_as_float(q[d + 1])),
-                                    wv * (__uint_as_float(r[d + 2]) + __uint_as_float(q[d + 2])),
-                                    wv * (__uint_as_float(r[d + 3]) + __uint_as_float(q[d + 3])));
-            }
-        } else {
-#pragma unroll
-          for (int d = 0; d < 32; ++d) {
-            if (d >= a.nd) break;
-            const int m = dense ? s * a.nd + d : lk[s * 32 + d];
-            if (m < 0) continue;
-            float val = wv * (__uint_as_float(r[d]) + __uint_as_float(q[d]));
-            if (rytov) val = val / (float)rytov[(int64_t)m * a.ng + g];
-            row[m] = val;
+        for (int h = 0; h < 2; ++h) {                    // detectors 16 h ..
+          uint32_t r[16], q[16];
+          const uint32_t ta = tmem + ((uint32_t)(32 * warp) << 16) + 64u * slot + 16u * h;
+          tc::tmem_ld16(ta, r);                          // (A_hi + A_lo) B_hi
+          tc::tmem_ld16(ta + 32u, q);                    // (A_hi + A_lo) B_lo
+          if (h == 1) {
+            tc::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&tempty[slot]);
           }
+          if (dense == 2) {                              // m = s nd + d, nd a multiple of 4
+            float4 x[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              x[i] = make_float4(wv * (__uint_as_float(r[4 * i]) + __uint_as_float(q[4 * i])),
+                                 wv * (__uint_as_float(r[4 * i + 1]) + __uint_as_float(q[4 * i + 1])),
+                                 wv * (__uint_as_float(r[4 * i + 2]) + __uint_as_float(q[4 * i + 2])),
+                                 wv * (__uint_as_float(r[4 * i + 3]) + __uint_as_float(q[4 * i + 3])));
+            // lane s stores its four 16-byte pieces in the order i ^ (s % 4): rows are 128 bytes apart
+            swap_if(lane & 1, x[0], x[1]);
+            swap_if(lane & 1, x[2], x[3]);
+            swap_if(lane & 2, x[0], x[2]);
+            swap_if(lane & 2, x[1], x[3]);
+            if (s < a.ns)
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const int d = 16 * h + 4 * (i ^ (lane & 3));
+                if (d < a.nd) *reinterpret_cast<float4 *>(ob + 4 * (s * a.nd + d)) = x[i];
+              }
+          } else if (g < a.ng && s < a.ns) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              const int d = 16 * h + i;
+              if (d >= a.nd) break;
+              const int m = dense ? s * a.nd + d : lk[s * 32 + d];
+              if (m < 0) continue;
+              float val = wv * (__uint_as_float(r[i]) + __uint_as_float(q[i]));
+              if (ryt) val = val / ryt[(int64_t)g * a.nm + m];
+              row[m] = val;
+            }
+          }
+          __syncwarp();                                  // converged again for the next load
+        }
+        if (dense == 2 && g < a.ng) {
+          if (ryt) {
+            for (int m = 4 * lane; m < a.nm; m += 128) {
+              float4 x = *reinterpret_cast<const float4 *>(ob + 4 * m);
+              const float4 y = __ldg(reinterpret_cast<const float4 *>(ryt + (int64_t)g * a.nm + m));
+              x.x /= y.x, x.y /= y.y, x.z /= y.z, x.w /= y.w;
+              *reinterpret_cast<float4 *>(row + m) = x;
+            }
+          } else {
+            tc::fence_async_smem();
+            __syncwarp();
+            if (lane == 0)
+              asm volatile(
+                  "cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n\tcp.async.bulk.commit_group;" ::"l"(row),
+                  "r"(tc::smem_u32(ob)), "r"(4 * a.nm)
+                  : "memory");
+          }
+          __syncwarp();
         }
       }
     }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // no copy outlives the kernel
   }
   tc::fence_before_sync();
   __syncthreads();
@@ -876,8 +916,8 @@ __global__ void __launch_bounds__(VT_THREADS, 1) k_jacobian_vjp_tc(JArgs a, cons
           lo[2 * q] = tc::to_tf32(xr - hi[2 * q]);
           lo[2 * q + 1] = tc::to_tf32(xi - hi[2 * q + 1]);
         }
-        tc::tmem_st8(dst0 + 128u * as + 8u * c, hi);
-        tc::tmem_st8(dst0 + 128u * as + 64u + 8u * c, lo);
+        tc::tmem_st(dst0 + 128u * as + 8u * c, hi);
+        tc::tmem_st(dst0 + 128u * as + 64u + 8u * c, lo);
       }
       tc::tmem_wait_st();
       tc::fence_before_sync();
@@ -1100,8 +1140,8 @@ int alloc_chunk(ScratchBuf &buf, int64_t &chunk, size_t bytes, cudaStream_t st) 
 // 0 (default) and 2: the tensor cores where the shapes fit (TG Jacobian: nodal basis, unique
 //   links, up to 32 sources and detectors, shared memory for the operand rings; vjp: up to 32
 //   sources and detectors), else the CUDA cores.  Measured at the sensitivity configuration
-//   (100k voxels, 32 x 32 optodes, 64 harmonics, 20 gates, one B200): TG Jacobian 11.9 ms
-//   against 20.0 ms, vjp 1.2 ms against 16.4 ms.
+//   (100k voxels, 32 x 32 optodes, 64 harmonics, 20 gates, one B200): TG Jacobian 7.4 ms
+//   against 17.1 ms, vjp 1.3 ms against 16.5 ms.
 // 1: both on the CUDA cores (cross-checks, timing)
 static int g_jacobian_engine = 0;
 
@@ -1155,19 +1195,25 @@ int jacobian_run(int mode, const int32_t *prow, const int32_t *pcol, const doubl
   k_ctab<<<(unsigned)ceil_div(nt_, 256), 256, 0, st>>>((const double2 *)gate, (const double2 *)fpsf, mode == 1 ? 0 : ng,
                                                         nf, nt, ctab.as<float2>(), finv.as<double2>());
   DGP_CHECK_LAUNCH();
+  ScratchBuf ryt;  // FP32 Rytov divisors [ng][nm] of the time-gated forms
+  if (mode == 0 && rytov) {
+    DGP_TRY(ryt.alloc(sizeof(float) * (size_t)nm * ng, st));
+    k_rytov_t<<<(unsigned)ceil_div((int64_t)nm * ng, 256), 256, 0, st>>>(rytov, nm, ng, ryt.as<float>());
+    DGP_CHECK_LAUNCH();
+  }
   const T2Layout tl = t2_layout(nf, std::max(1, ng));
   const size_t smem_tc = tl.bytes + 1024;
   // (+ 1 KB of the kernel's own static shared memory)
   const bool tc_fits = mode == 0 && !prow && links_unique && nf <= 64 && smem_tc + 1024 <= 227 * 1024;
   if (tc_fits && g_jacobian_engine != 1) {
     // tensor cores: one persistent warp-specialised CTA per SM
-    const int dense = !links_dense ? 0 : (!rytov && nd % 4 == 0 && nm % 4 == 0) ? 2 : 1;
+    const int dense = !links_dense ? 0 : (nd % 4 == 0 && (uintptr_t)out % 16 == 0) ? 2 : 1;
     ScratchBuf flag;
     DGP_TRY(flag.alloc(sizeof(int), st));
     DGP_CUDA(cudaMemsetAsync(flag.p, 0, sizeof(int), st));
     DGP_TRY(allow_dyn_smem(k_jacobian_tg_tc, smem_tc));
     const int gtc = (int)std::min<int64_t>(nv, (int64_t)sm_count());
-    k_jacobian_tg_tc<<<gtc, T2_THREADS, smem_tc, st>>>(a, ctab.as<float2>(), rytov, dense, (float *)out,
+    k_jacobian_tg_tc<<<gtc, T2_THREADS, smem_tc, st>>>(a, ctab.as<float2>(), ryt.as<float>(), dense, (float *)out,
                                                        flag.as<int>());
     DGP_CHECK_LAUNCH();
     int h = 0;
@@ -1195,15 +1241,10 @@ int jacobian_run(int mode, const int32_t *prow, const int32_t *pcol, const doubl
     // two buffers of fields, one where two don't fit
     const int nbuf = smem_of(tpv, 2) <= 200 * 1024 ? 2 : 1;
     const size_t smem_tg = smem_of(tpv, nbuf);
-    ScratchBuf ckg, fields, ryt;
+    ScratchBuf ckg, fields;
     DGP_TRY(ckg.alloc(sizeof(float4) * (size_t)nf * (ngc / 2), st));
     int64_t chunk = nv;
     DGP_TRY(alloc_chunk(fields, chunk, sizeof(float2) * per, st));
-    if (rytov) {
-      DGP_TRY(ryt.alloc(sizeof(float) * (size_t)nm * ng, st));
-      k_rytov_t<<<(unsigned)ceil_div((int64_t)nm * ng, 256), 256, 0, st>>>(rytov, nm, ng, ryt.as<float>());
-      DGP_CHECK_LAUNCH();
-    }
     k_ctab_kg<<<(unsigned)ceil_div((int64_t)nf * (ngc / 2), 256), 256, 0, st>>>(ctab.as<float2>(), ng, nf, ngc,
                                                                                 ckg.as<float4>());
     DGP_CHECK_LAUNCH();

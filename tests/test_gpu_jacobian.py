@@ -363,3 +363,33 @@ def test_vjp_tensor_core_tiles(ns, nd, nf, ng, nm, nv, rows):
         mag += (np.abs(x) * (np.abs(y) @ A.T)).sum(1)
     err = np.abs(v.cpu().numpy() - wts * v0)
     assert (err <= 200 * 2.0 ** -23 * np.sqrt(2) * wts * mag).all()
+
+
+@pytest.mark.parametrize("use_rytov", [False, True])
+@pytest.mark.parametrize("ns,nd,nf,ng,nn", [
+    (32, 32, 64, 20, 300),  # full tiles, more voxels than blocks
+    (5, 8, 1, 1, 1),        # one harmonic block, one voxel
+    (7, 12, 33, 32, 149),   # a third chunk, all gates
+    (32, 4, 16, 5, 40),     # one 16-byte piece per source
+    (9, 6, 24, 7, 150),     # rows that are no multiple of 16 bytes
+])
+def test_tg_jacobian_tensor_core_rows(ns, nd, nf, ng, nn, use_rytov):
+    """Tensor-core TG Jacobian of all source-detector pairs against 64-bit sums.  An entry is the FP32
+    accumulation of 3 x 128 truncated products at most, operands rounded to 2^-22: off by at most
+    400 x 2^-23 of the sum of its terms' magnitudes (times sqrt 2, complex)."""
+    import torch
+    from dogpup_b200 import api
+    rng = np.random.default_rng(ns * nd)
+    cn = lambda *s: rng.standard_normal(s) + 1j * rng.standard_normal(s)
+    phi, phiA, fpsf, gates = cn(nf, nn, ns), cn(nf, nn, nd), cn(nf), cn(ng, nf)
+    link = np.stack(np.divmod(np.arange(ns * nd), nd), 1).astype(np.int32)
+    wts, ryt = rng.uniform(0.5, 2.0, nn), rng.uniform(0.5, 2.0, (ns * nd, ng))
+    cu = lambda x: torch.as_tensor(x, device="cuda")
+    J = api.jacobian_tg(api.Basis(None, wts, nn=nn), cu(phi), cu(phiA), cu(fpsf), cu(link), cu(gates), 64,
+                        data_tg=cu(ryt) if use_rytov else None)
+    C = -128.0 * np.where(np.arange(nf) == 0, 0.5, 1.0) * np.conj(gates) / fpsf
+    a = (phi[:, :, :, None] * phiA[:, :, None, :]).reshape(nf, nn, ns * nd)
+    J0 = np.real(np.einsum("gk,kvm->vgm", C, a))
+    mag = np.einsum("gk,kvm->vgm", np.abs(C), np.abs(a))
+    scale = wts[:, None, None] / (ryt.T[None] if use_rytov else 1.0)
+    assert (np.abs(J.cpu().numpy() - scale * J0) <= 400 * 2.0 ** -23 * np.sqrt(2) * scale * mag).all()
