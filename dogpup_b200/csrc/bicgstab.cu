@@ -1,13 +1,14 @@
-// Batched FSAI-preconditioned BiCGSTAB (and COCG) over every source x harmonic.
+// Solver plans, and the unfused solvers over every source x harmonic: FSAI-preconditioned BiCGSTAB
+// in complex FP32 (DGP_PREC_MIXED_BICGSTAB), COCG at a launch shape that was set by hand, and the
+// batched SpMM they run on.  The default solves are in cocg.cu (mixed) and bicg64.cu (FP64).
 //
 // Replaces gpuBicstab_FSAIP + fluGPU (DOGPUP/dMesh.m:1238-1348).  The
 // reference runs the iteration from MATLAB: 7 mex mat-vec calls per
 // iteration, each re-copying A, x and the index arrays to fresh device
 // arrays, about 20 gpuArray BLAS-1 launches and 4 device-wide waits.  Here
-// one iteration is 10 sweep kernels + 5 single-block scalar kernels,
+// one BiCGSTAB iteration is 10 sweep kernels + 5 single-block scalar kernels,
 // captured once in a CUDA graph and replayed; convergence is decided on the
-// device (FP64 dot products and norms) and polled by the host every
-// `check_every` iterations.
+// device (FP64 dot products and norms).
 //
 // Arithmetic follows the reference: bilinear (unconjugated) dots r^0.v,
 // r^0.r and (G t).(G s), (G t).(G t); alph = (v.r^0)/rho0 (its reciprocal
@@ -28,8 +29,8 @@
 // Mixed precision: a complex-FP32 inner solve runs on the current FP64
 // residual; the FP64 solution is updated and the FP64 residual b - A x is
 // recomputed (FP64 K, M) with FP64 norms, until the maximum relative FP64
-// residual is below tol (iterative refinement).  The inner solver is COCG
-// (DGP_PREC_MIXED): A_k = K + i w_k M and the FSAI preconditioner G^T G are
+// residual is below tol (iterative refinement).  With COCG as the inner
+// solver: A_k = K + i w_k M and the FSAI preconditioner G^T G are
 // complex symmetric, so conjugate-orthogonal CG with bilinear dots applies;
 // it costs one A and one G^T G application per iteration (9 launches)
 // against BiCGSTAB's two of each (15 launches), for ~1.1x the iterations on

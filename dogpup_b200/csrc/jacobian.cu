@@ -725,7 +725,7 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
 //   warps 4-7   thread = voxel row: FP64 -> FP32 -> (hi, lo) into one of two A' stages in tensor memory
 //   warp 12     one thread issues the 24 MMAs into one of two accumulators
 //   warps 0-3   thread = voxel row: dots Y_k with phi from the slab, in FP64
-// Bound by HBM: every field value is read once, NF (NS + ND) 16 bytes per voxel.  101,898 nodes x 64
+// Bound by HBM: every field value is read once, NF (NS + ND) 16 bytes per voxel.  101,880 nodes x 64
 // optodes x 64 harmonics (6.7 GB): 4.34 ms with two CTAs per SM that loaded, converted, multiplied and
 // reduced one after the other (phi by 16-byte loads 512 bytes apart), 1.20 ms now.
 // A voxel basis is projected, chunk by chunk, into slabs of the same layout (k_project_slabs).
