@@ -343,10 +343,16 @@ __global__ void k_gather_slots(const int32_t *__restrict__ cstart, const int32_t
 // absorption block vol sum_q w_q N_v N_i N_j, and the stiffness block
 // vol (grad N_i . grad N_j) d(ksum)/dp with ksum = sum_q w_q sum_l N_l kappa_l,
 // d(ksum)/dmua_v = d(ksum)/dmusp_v = -3 kappa_v^2 sum_q w_q N_v(x_q)
-// (kappa = 1/(3(mua + musp)), dMesh.m:74, :85).  One warp per element, lanes
-// over sources, all harmonics; the per-vertex sums leave by one FP64 atomic
-// per vertex and output.  Robin and M blocks do not depend on mua or musp.
-__global__ void __launch_bounds__(256) k_elem_grad(const double *__restrict__ node, const int32_t *__restrict__ elem,
+// (kappa = 1/(3(mua + musp)), dMesh.m:74, :85).  One warp per element, lanes over the harmonics'
+// sources in a row; the per-vertex sums leave by one FP64 atomic per vertex and output.  Robin and M
+// blocks do not depend on mua or musp.
+// Per sample the vertex pairs' products alone are summed, Re(lam_i phi_j + lam_j phi_i) and the same
+// of the differences from vertex 0 (whose gradients' products carry no cancellation); quadrature and
+// geometry are applied to the sums: 50 FP64 multiply-adds instead of 170.  Bound by the gathers of
+// eight rows per element and harmonic from L2.  14,040 nodes x 16 sources x 32 harmonics: 1.25 ms
+// with lanes over one harmonic's sources (half of them idle here), 0.45 now at three blocks per SM
+// (0.57 at two; 0.67 at four, where the accumulators spill).
+__global__ void __launch_bounds__(256, 3) k_elem_grad(const double *__restrict__ node, const int32_t *__restrict__ elem,
                                                    int64_t ne, const double2 *__restrict__ phi,
                                                    const double2 *__restrict__ lam, int64_t n, int nf, int ns,
                                                    const double *__restrict__ mua, const double *__restrict__ musp,
@@ -367,47 +373,73 @@ __global__ void __launch_bounds__(256) k_elem_grad(const double *__restrict__ no
     double kap = 1.0 / (3.0 * (mua[v[l]] + musp[v[l]]));
     dk[l] = -3.0 * kap * kap * cv * G.vol;
   }
-  double acc_a[4] = {0, 0, 0, 0}, acc_k = 0.0;
-  for (int k = 0; k < nf; ++k) {
+  // W[ij] = sum Re(lam_i phi_j + lam_j phi_i) (i < j), Re(lam_i phi_i) (i = j); E the same of the
+  // differences of vertices 1, 2, 3 from vertex 0
+  double W[10], E[6];
+#pragma unroll
+  for (int q = 0; q < 10; ++q) W[q] = 0.0;
+#pragma unroll
+  for (int q = 0; q < 6; ++q) E[q] = 0.0;
+  int k = lane / ns, s = lane % ns;
+  const int dk_ = 32 / ns, ds = 32 % ns;
+  for (; k < nf;) {
     const int64_t base = (int64_t)k * n;
-    for (int s = lane; s < ns; s += 32) {
-      double2 f[4], a[4];
+    double2 f[4], a[4];
 #pragma unroll
-      for (int l = 0; l < 4; ++l) {
-        f[l] = phi[(base + v[l]) * ns + s];
-        a[l] = lam[(base + v[l]) * ns + s];
-      }
-      // absorption: sum_q w_q N_v(x_q) Re(lam(x_q) phi(x_q))
-#pragma unroll
-      for (int q = 0; q < 5; ++q) {
-        double fr = 0, fi = 0, ar = 0, ai = 0;
-#pragma unroll
-        for (int l = 0; l < 4; ++l) {
-          fr += c_tq[l][q] * f[l].x;
-          fi += c_tq[l][q] * f[l].y;
-          ar += c_tq[l][q] * a[l].x;
-          ai += c_tq[l][q] * a[l].y;
-        }
-        const double pr = c_tw[q] * (ar * fr - ai * fi);
-#pragma unroll
-        for (int l = 0; l < 4; ++l) acc_a[l] += c_tq[l][q] * pr;
-      }
-      // stiffness: Re(grad lam . grad phi), shared by all four vertices
-      double dot = 0.0;
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        double lr = 0, li = 0, pr = 0, pi = 0;
-#pragma unroll
-        for (int l = 0; l < 4; ++l) {
-          lr += G.g[l][d] * a[l].x;
-          li += G.g[l][d] * a[l].y;
-          pr += G.g[l][d] * f[l].x;
-          pi += G.g[l][d] * f[l].y;
-        }
-        dot += lr * pr - li * pi;
-      }
-      acc_k += dot;
+    for (int l = 0; l < 4; ++l) {
+      f[l] = __ldg(phi + (base + v[l]) * ns + s);
+      a[l] = __ldg(lam + (base + v[l]) * ns + s);
     }
+    k += dk_;
+    if ((s += ds) >= ns) {
+      s -= ns;
+      ++k;
+    }
+    int w = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      W[w] += a[i].x * f[i].x - a[i].y * f[i].y;
+      ++w;
+#pragma unroll
+      for (int j = i + 1; j < 4; ++j, ++w)
+        W[w] += (a[i].x * f[j].x - a[i].y * f[j].y) + (a[j].x * f[i].x - a[j].y * f[i].y);
+    }
+#pragma unroll
+    for (int l = 1; l < 4; ++l) {
+      f[l] = csub(f[l], f[0]);
+      a[l] = csub(a[l], a[0]);
+    }
+    w = 0;
+#pragma unroll
+    for (int i = 1; i < 4; ++i) {
+      E[w] += a[i].x * f[i].x - a[i].y * f[i].y;
+      ++w;
+#pragma unroll
+      for (int j = i + 1; j < 4; ++j, ++w)
+        E[w] += (a[i].x * f[j].x - a[i].y * f[j].y) + (a[j].x * f[i].x - a[j].y * f[i].y);
+    }
+  }
+  // absorption: sum_q w_q N_v(x_q) Re(lam(x_q) phi(x_q)); stiffness: Re(grad lam . grad phi), shared by
+  // all four vertices
+  double acc_a[4] = {0, 0, 0, 0}, acc_k = 0.0;
+#pragma unroll
+  for (int q = 0; q < 5; ++q) {
+    double pr = 0.0;
+    int w = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = i; j < 4; ++j, ++w) pr += c_tq[i][q] * c_tq[j][q] * W[w];
+#pragma unroll
+    for (int l = 0; l < 4; ++l) acc_a[l] += c_tw[q] * c_tq[l][q] * pr;
+  }
+  {
+    int w = 0;
+#pragma unroll
+    for (int i = 1; i < 4; ++i)
+#pragma unroll
+      for (int j = i; j < 4; ++j, ++w)
+        acc_k += (G.g[i][0] * G.g[j][0] + G.g[i][1] * G.g[j][1] + G.g[i][2] * G.g[j][2]) * E[w];
   }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {

@@ -194,3 +194,22 @@ def test_device_autograd_mixed_precision(dev_case):
         (model(mua, dev_case["musp"]) * dev_case["g"]).sum().backward()
         out.append(mua.grad.cpu().numpy())
     assert np.abs(out[1] - out[0]).max() <= 1e-4 * np.abs(out[0]).max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ns,nf", [(1, 1), (1, 40), (3, 5), (5, 13), (31, 3), (32, 2), (33, 3), (64, 1), (70, 2)])
+@pytest.mark.parametrize("rough", [1.0, 1e-3])
+def test_element_gradient_over_source_counts(dev_case, ns, nf, rough):
+    """The element kernel for source counts around a warp's width, on rough fields and on nearly constant
+    ones (whose gradients are small differences), against the oracle on the same fields."""
+    import torch
+    from dogpup_b200 import api
+    mesh, rng = dev_case["mesh"], np.random.default_rng(ns)
+    field = lambda: 1.0 + rough * (rng.standard_normal((nf, mesh.nn, ns)) + 1j * rng.standard_normal((nf, mesh.nn, ns)))
+    phi, lam = field(), field()
+    gm, gs = api.fem_adjoint_grad(mesh.fem, dev_case["mua"], dev_case["musp"], torch.as_tensor(phi, device="cuda"),
+                                  torch.as_tensor(lam, device="cuda"))
+    gm0, gs0 = grad.adjoint_grad(mesh.node_host, mesh.elem_host, _oracle_geo(mesh), dev_case["w"]["mua"],
+                                 dev_case["w"]["musp"], np.transpose(phi, (1, 2, 0)), np.transpose(lam, (1, 2, 0)))
+    assert np.abs(gm.cpu().numpy() - gm0).max() <= 1e-11 * np.abs(gm0).max()
+    assert np.abs(gs.cpu().numpy() - gs0).max() <= 1e-11 * np.abs(gs0).max()
