@@ -97,7 +97,7 @@ cudaMemPool_t make_pool(int dev) {
     cudaGetLastError();
     return nullptr;
   }
-  uint64_t keep = total / 32;
+  uint64_t keep = total / 64;
   cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
   return pool;
 }

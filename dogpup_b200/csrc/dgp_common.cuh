@@ -60,11 +60,9 @@ template <class K> inline int allow_dyn_smem(K *kernel, size_t bytes) {
 // context, or pools unsupported; callers then allocate with cudaMalloc): per-call scratch, and plan
 // buffers.  A call then pays neither for mapping and unmapping memory nor for the device-wide wait
 // of cudaFree (an LM update at 3,333 x 7,001 spent up to 20 of its 25 ms there).  Each pool keeps at
-// most 1/32 of the device's memory when idle (at 1/64 a batch of meshes on four streams gave memory
-// back after each run, and the next query of the free memory waited 10 to 90 ms for it); what is
-// above goes back at the next synchronisation, and all of it when an allocation fails (trim_pools).
-// Two pools, because the bound counts memory in use: one large plan would leave nothing for the
-// scratch.
+// most 1/64 of the device's memory when idle; what is above goes back at the next synchronisation,
+// and all of it when an allocation fails (trim_pools).  Two pools, because the bound counts memory
+// in use: one large plan would leave nothing for the scratch.
 cudaMemPool_t device_pool(bool plans);
 void trim_pools();
 // id of the current context, unique for the process's lifetime (0: no context is current)
