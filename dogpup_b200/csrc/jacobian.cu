@@ -306,9 +306,9 @@ __global__ void k_rytov_t(const double *__restrict__ rytov, int nm, int ng, floa
 //   warps 21-24 feeders: sources and B'' of each voxel, ahead of the builders and MMAs that need
 //               them (lane = optode)
 // Bound by the chain of build, hand-over and MMAs through the three stages that tensor memory has
-// room for: without the MMAs the kernel takes 5.1 ms of its 7.4, without the builders' stores 6.6,
+// room for: at 7.4 ms, without the MMAs the kernel took 5.1, without the builders' stores 6.6,
 // with half the MMAs 6.1.  101,880 nodes x 1,024 links x 64 harmonics x 20 gates: 7.8 ms with eight
-// builder warps that also staged the fields, 7.4 now; 20,000 nodes with Rytov 10.1 -> 2.8 ms (FP64
+// builder warps that also staged the fields, 7.0 now; 20,000 nodes with Rytov 10.1 -> 2.7 ms (FP64
 // divisors read and rows written 4 bytes at a time before).  Six stages of one chunk (8.1 to 9.2 ms:
 // the cost per stage is the hand-over) and two builder groups on alternate stages (8.7) were slower.
 // Tensor memory: 2 accumulator slots of 64 columns (a tile's slot is released as soon as the
@@ -339,8 +339,8 @@ __host__ __device__ inline T2Layout t2_layout(int nf, int ng) {
   L.f_off = L.b_off + 2 * L.nch * T2_BCH;                        // two voxels' source fields [NKP][32] float2
   L.c_off = L.f_off + 2 * (uint32_t)(32 * 8 * L.nkp);            // gate table [4 NTILE][NKP] float2
   L.l_off = L.c_off + (uint32_t)(8 * 4 * L.ntile * L.nkp);        // link lookup [32][32] int
-  L.o_off = L.l_off + 4 * 32 * 32;                               // a gate's output row per epilogue warp
-  L.bytes = L.o_off + 4096 * T2_EPI;
+  L.o_off = L.l_off + 4 * 32 * 32;                               // two output rows per epilogue warp
+  L.bytes = L.o_off + 2 * 4096 * T2_EPI;
   return L;
 }
 
@@ -471,8 +471,11 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
   } else if (warp > T2_EPI + T2_BLD) {
     // ---------------------------------------------------------------- feeders
     // Voxel i's fields into buffers i % 2 once the builders (sempty) and the MMAs (bempty) of voxel
-    // i - 2 are done with them: warp w takes the 8-harmonic blocks p = w, w + 4, .., lane = optode.
-    // Sources as complex FP32 [harmonic][32], detectors as B'' (chunk p / 2, half p % 2).
+    // i - 2 are done with them: warp w takes the groups of 4 harmonics p = w, w + 4, .., lane = optode,
+    // both fields' loads in flight together (a group per warp for up to 16 harmonics: with 8 harmonics
+    // at a time and one field after the other, two load latencies per voxel made 45,155 nodes x 20 links x
+    // 13 harmonics x 7 gates slower than builders that staged the fields a voxel ahead: 1.06 ms).
+    // Sources as complex FP32 [harmonic][32], detectors as B'' (chunk p / 4, quarter p % 4).
     const int w = warp - (T2_EPI + T2_BLD + 1);
     int i = 0;
     bool fail = false;
@@ -484,36 +487,30 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
     for (int64_t v = blockIdx.x; v < a.nv; v += gridDim.x, ++i) {
       if (__any_sync(FULL, *abort_v != 0)) break;
       const int bj = i & 1;
-      bool free = w < 2 * L.nch || buffers_free(i);      // (a warp without a block keeps step)
+      bool free = true;
       unsigned char *bb = sm + L.b_off + bj * L.nch * T2_BCH;
       float2 *fs = reinterpret_cast<float2 *>(sm + L.f_off) + bj * 32 * L.nkp + lane;
-      for (int p = w; p < 2 * L.nch; p += T2_FD) {
-        double2 x[8];
-        const double2 *py = a.phiA + ((int64_t)(8 * p) * a.nn + v) * a.nd + lane;
+      for (int p = w; p < 4 * L.nch; p += T2_FD) {
+        double2 x[4], y[4];
+        const double2 *px = a.phi + ((int64_t)(4 * p) * a.nn + v) * a.ns + lane;
+        const double2 *py = a.phiA + ((int64_t)(4 * p) * a.nn + v) * a.nd + lane;
 #pragma unroll
-        for (int q = 0; q < 8; ++q)
-          x[q] = 8 * p + q < a.nf && lane < a.nd ? __ldg(py + (int64_t)q * a.nn * a.nd) : make_double2(0.0, 0.0);
-        if (p == w && !(free = buffers_free(i))) break;  // (the first loads are under way)
-        float re[8], im[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          re[q] = (float)x[q].x;
-          im[q] = (float)x[q].y;
+        for (int q = 0; q < 4; ++q) {
+          const bool in = 4 * p + q < a.nf;
+          x[q] = in && lane < a.ns ? __ldg(px + (int64_t)q * a.nn * a.ns) : make_double2(0.0, 0.0);
+          y[q] = in && lane < a.nd ? __ldg(py + (int64_t)q * a.nn * a.nd) : make_double2(0.0, 0.0);
         }
-        const double2 *px = a.phi + ((int64_t)(8 * p) * a.nn + v) * a.ns + lane;
+        if (p == w && !(free = buffers_free(i))) break;  // (the first loads are under way)
+        float re[4], im[4];
 #pragma unroll
-        for (int q = 0; q < 8; ++q)
-          x[q] = 8 * p + q < a.nf && lane < a.ns ? __ldg(px + (int64_t)q * a.nn * a.ns) : make_double2(0.0, 0.0);
-        unsigned char *bh = bb + (p >> 1) * T2_BCH;
-        const float r0[4] = {re[0], re[1], re[2], re[3]}, r1[4] = {re[4], re[5], re[6], re[7]};
-        const float i0[4] = {im[0], im[1], im[2], im[3]}, i1[4] = {im[4], im[5], im[6], im[7]};
-        const int h = p & 1;                             // hi rows 0-31, lo rows 32-63
-        st_split4(bh, bh + 4096, tc::sw128_chunk(lane, 2 * h + 0), r0);
-        st_split4(bh, bh + 4096, tc::sw128_chunk(lane, 2 * h + 1), r1);
-        st_split4(bh, bh + 4096, tc::sw128_chunk(lane, 4 + 2 * h + 0), i0);
-        st_split4(bh, bh + 4096, tc::sw128_chunk(lane, 4 + 2 * h + 1), i1);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) fs[32 * (8 * p + q)] = make_float2((float)x[q].x, (float)x[q].y);
+        for (int q = 0; q < 4; ++q) {
+          fs[32 * (4 * p + q)] = make_float2((float)x[q].x, (float)x[q].y);
+          re[q] = (float)y[q].x;
+          im[q] = (float)y[q].y;
+        }
+        unsigned char *bh = bb + (p >> 2) * T2_BCH;      // hi rows 0-31, lo rows 32-63
+        st_split4(bh, bh + 4096, tc::sw128_chunk(lane, p & 3), re);
+        st_split4(bh, bh + 4096, tc::sw128_chunk(lane, 4 + (p & 3)), im);
       }
       if (!free) {
         fail = true;
@@ -606,8 +603,7 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
     }
   } else {
     // ---------------------------------------------------------------- epilogue
-    const int gl = warp, s = lane;
-    unsigned char *ob = sm + L.o_off + 4096 * warp;
+    const int gl = warp, s = lane, last = a.nd > 16 ? 1 : 0;
     uint32_t tl_idx = 0;
     bool ok = true;
     for (int64_t v = blockIdx.x; v < a.nv && ok; v += gridDim.x) {
@@ -626,17 +622,19 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
         tc::fence_after_sync();
         const int g = 4 * t + gl;
         float *row = Jtg + ((int64_t)v * a.ng + g) * a.nm;
-        if (dense == 2) {                                // the row's last copy has left the buffer
-          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        unsigned char *ob = sm + L.o_off + 4096 * (2 * warp + (tl_idx & 1u));
+        if (dense == 2) {                                // the copy before the last has left this buffer
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
           __syncwarp();
         }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {                    // detectors 16 h ..
+          if (h > last) break;
           uint32_t r[16], q[16];
           const uint32_t ta = tmem + ((uint32_t)(32 * warp) << 16) + 64u * slot + 16u * h;
           tc::tmem_ld16(ta, r);                          // (A_hi + A_lo) B_hi
           tc::tmem_ld16(ta + 32u, q);                    // (A_hi + A_lo) B_lo
-          if (h == 1) {
+          if (h == last) {
             tc::fence_before_sync();
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(&tempty[slot]);
@@ -686,13 +684,14 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
             tc::fence_async_smem();
             __syncwarp();
             if (lane == 0)
-              asm volatile(
-                  "cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n\tcp.async.bulk.commit_group;" ::"l"(row),
-                  "r"(tc::smem_u32(ob)), "r"(4 * a.nm)
-                  : "memory");
+              asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(row),
+                           "r"(tc::smem_u32(ob)), "r"(4 * a.nm)
+                           : "memory");
           }
           __syncwarp();
         }
+        // a group per tile, empty or not: the wait above counts them
+        if (dense == 2 && lane == 0) asm volatile("cp.async.bulk.commit_group;" ::: "memory");
       }
     }
     if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // no copy outlives the kernel
@@ -1140,7 +1139,7 @@ int alloc_chunk(ScratchBuf &buf, int64_t &chunk, size_t bytes, cudaStream_t st) 
 // 0 (default) and 2: the tensor cores where the shapes fit (TG Jacobian: nodal basis, unique
 //   links, up to 32 sources and detectors, shared memory for the operand rings; vjp: up to 32
 //   sources and detectors), else the CUDA cores.  Measured at the sensitivity configuration
-//   (100k voxels, 32 x 32 optodes, 64 harmonics, 20 gates, one B200): TG Jacobian 7.4 ms
+//   (100k voxels, 32 x 32 optodes, 64 harmonics, 20 gates, one B200): TG Jacobian 7.0 ms
 //   against 17.1 ms, vjp 1.3 ms against 16.5 ms.
 // 1: both on the CUDA cores (cross-checks, timing)
 static int g_jacobian_engine = 0;
