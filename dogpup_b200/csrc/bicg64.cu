@@ -210,7 +210,7 @@ template <int VEC, int MODE> __global__ void __launch_bounds__(BS, 2) k_dsweep(c
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int sub = lane % g.lpr, rsub = lane / g.lpr;
   unsigned char *wbuf = sm + (size_t)warp * 2 * g.cap * 20;
-  double *slots = reinterpret_cast<double *>(sm + (GATHER ? (size_t)WARPS * 2 * g.cap * 20 + 128 : 0));  // [WARPS][nsp][NQ]
+  double *slots = reinterpret_cast<double *>(sm + (GATHER ? stage_bytes<double>(g) : 0));  // [WARPS][nsp][NQ]
   double2 *s_al = reinterpret_cast<double2 *>(slots + WARPS * g.nsp * NQ1), *s_om = s_al + g.nsp;
   double *s_sum = reinterpret_cast<double *>(s_om + g.nsp);  // [BS]
   __shared__ int s_last;

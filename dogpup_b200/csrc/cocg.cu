@@ -150,7 +150,7 @@ template <int VEC, int MODE> __global__ void __launch_bounds__(BS, 2) k_fsweep(c
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int sub = lane % g.lpr, rsub = lane / g.lpr;
   unsigned char *wbuf = sm + (size_t)warp * 2 * g.cap * 16;
-  float2 *s_al = reinterpret_cast<float2 *>(sm + (size_t)WARPS * 2 * g.cap * 16 + 128);
+  float2 *s_al = reinterpret_cast<float2 *>(sm + stage_bytes<float>(g));
   float2 *s_be = s_al + g.nsp;
   double *slots = reinterpret_cast<double *>(s_be + g.nsp);   // [WARPS][nsp][NQ]
   __shared__ int s_last;

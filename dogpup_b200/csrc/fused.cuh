@@ -96,7 +96,7 @@ template <int VEC> __global__ void __launch_bounds__(BS) k_fresid(const FResid a
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int sub = lane % g.lpr, rsub = lane / g.lpr;
   unsigned char *wbuf = sm + (size_t)warp * 2 * g.cap * 20;
-  double *swt = reinterpret_cast<double *>(sm + (size_t)WARPS * 2 * g.cap * 20 + 128);  // [nsp][4]
+  double *swt = reinterpret_cast<double *>(sm + stage_bytes<double>(g));  // [nsp][4]
   double *slots = swt + 4 * g.nsp;                                                // [WARPS][nsp]
   int *sn = reinterpret_cast<int *>(slots + WARPS * g.nsp);                       // [nsp][4]
   __shared__ int s_last;

@@ -67,9 +67,25 @@ template <class R> inline Geo make_geo(int64_t n, int nf, int nsp, int vec, int 
   g.steps = (int)ceil_div(n, (int64_t)WARPS * g.rpw);
   return g;
 }
-template <class R> inline size_t stage_bytes(const Geo &g) {
-  return (size_t)WARPS * 2 * g.cap * Tr<R>::REC + 128;  // + reads past a row's end (unused)
+// two buffers of cap records per warp (a multiple of 16 bytes)
+template <class R> __host__ __device__ inline size_t stage_bytes(const Geo &g) {
+  return (size_t)WARPS * 2 * g.cap * Tr<R>::REC;
 }
+
+// A lane's records [b, e) in the staged window of cap records from c0: the first one's place in the
+// buffer, and how many there are (<= 0: none).
+struct Window {
+  int first, count;
+};
+__host__ __device__ inline Window window(int b, int e, int c0, int cap, bool live) {
+  Window w;
+  w.first = (b > c0 ? b : c0) - c0;
+  w.count = live ? (e < c0 + cap ? e : c0 + cap) - c0 - w.first : 0;
+  return w;
+}
+// Place of the lane's u-th record.  A warp goes as far as its longest row; a lane without a u-th record
+// in this window is given the buffer's first one, so that every place lies below cap.
+__host__ __device__ inline int place(const Window &w, int u) { return u < w.count ? w.first + u : 0; }
 
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
@@ -287,14 +303,14 @@ __device__ __forceinline__ void rows(const Geo &g, const int32_t *__restrict__ r
 #pragma unroll
     for (int u = 0; u < UNR; ++u) Acc<R, VEC, PAD>::clear(z[u]);
     for (int c0 = p0;;) {
-      const int p = max(b, c0) - c0;
-      const int cnt = (valid && live) ? min(e, c0 + g.cap) - c0 - p : 0;
-      const int m = __reduce_max_sync(ALL, cnt);
+      const Window win = window(b, e, c0, g.cap, valid && live);
+      const int m = __reduce_max_sync(ALL, win.count);
       int u0 = 0;
       auto block = [&](auto nu) {
         constexpr int N = decltype(nu)::value;
 #pragma unroll
-        for (int u = 0; u < N; ++u) acc.load(z[u], buf, g.cap, p + u0 + u, Xb, xb, g.lpr, nv, u0 + u < cnt);
+        for (int u = 0; u < N; ++u)
+          acc.load(z[u], buf, g.cap, place(win, u0 + u), Xb, xb, g.lpr, nv, u0 + u < win.count);
 #pragma unroll
         for (int u = 0; u < N; ++u) acc.add(z[u]);
         u0 += N;

@@ -1,0 +1,107 @@
+"""The staged-record windows of the sparse-row sweeps, walked on the host with the functions the kernel
+uses (sweep.cuh): whatever the row lengths, every record a lane reads lies inside its warp's own staging
+buffer, and over the windows each row's records are read once and in order."""
+import shutil
+import subprocess
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+CSRC = Path(__file__).resolve().parent.parent / "dogpup_b200" / "csrc"
+
+PROGRAM = r"""
+#include <algorithm>
+#include <cstdio>
+#include <cstdlib>
+#include <vector>
+#include "sweep.cuh"
+using namespace dgp::sweep;
+
+template <class R> int walk(const std::vector<int> &rp, int nsp) {
+  const int n = (int)rp.size() - 1, vec = nsp <= 8 ? 2 : 4;
+  const Geo g = make_geo<R>(n, 1, nsp, vec, 16);
+  if (stage_bytes<R>(g) < (size_t)WARPS * 2 * g.cap * Tr<R>::REC) return 1;
+  for (int step = 0; step < g.steps; ++step)
+    for (int warp = 0; warp < WARPS; ++warp) {
+      const int r0 = (step * WARPS + warp) * g.rpw;
+      auto bound = [&](int r) { return rp[std::min(r0 + std::min(r, g.rpw), n)]; };
+      const int p0 = bound(0), pe = bound(g.rpw);
+      std::vector<int> next(33);
+      for (int r = 0; r <= g.rpw; ++r) next[r] = bound(r);
+      for (int c0 = p0;;) {
+        int m = 0;
+        for (int lane = 0; lane < 32; ++lane) {
+          const int r = lane / g.lpr;
+          m = std::max(m, window(bound(r), bound(r + 1), c0, g.cap, r < g.rpw && r0 + r < n).count);
+        }
+        for (int lane = 0; lane < 32; ++lane) {
+          const int r = lane / g.lpr;
+          const Window w = window(bound(r), bound(r + 1), c0, g.cap, r < g.rpw && r0 + r < n);
+          for (int u = 0; u < m; ++u) {
+            const int q = place(w, u);
+            if (q < 0 || q >= g.cap) return 2;                         // outside the warp's buffer
+            if (u < w.count) {
+              if (c0 + q >= pe) return 3;                              // not staged
+              if (lane % g.lpr == 0 && c0 + q != next[r]++) return 4;  // skipped or read twice
+            }
+          }
+        }
+        c0 += g.cap;
+        if (c0 >= pe) break;
+      }
+      for (int r = 0; r < g.rpw; ++r)
+        if (next[r] != bound(r + 1)) return 5;
+    }
+  return 0;
+}
+
+int main(int argc, char **argv) {
+  std::vector<int> rp(1, 0);
+  for (int v; std::scanf("%d", &v) == 1;) rp.push_back(rp.back() + v);
+  for (int i = 1; i < argc; ++i) {
+    const int nsp = std::atoi(argv[i]), f = walk<float>(rp, nsp), d = walk<double>(rp, nsp);
+    if (f || d) {
+      std::printf("%d columns: float %d, double %d\n", nsp, f, d);
+      return 1;
+    }
+  }
+  return 0;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def program(tmp_path_factory):
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not Path(nvcc).exists():
+        pytest.skip("no nvcc")
+    d = tmp_path_factory.mktemp("window")
+    src = d / "window.cu"
+    src.write_text(PROGRAM)
+    subprocess.run([nvcc, "-std=c++17", "-O1", "--expt-relaxed-constexpr", "-gencode", "arch=compute_100a,code=sm_100a",
+                    f"-I{CSRC}", f"-I{CSRC.parent.parent / 'include'}", str(src), "-o", str(d / "window")], check=True)
+    return d / "window"
+
+
+def _rows(kind):
+    rng = np.random.default_rng(5)
+    n = 1237
+    r = rng.integers(8, 16, n)
+    if kind == "uniform30":
+        r[:] = 30
+    elif kind == "hubs":
+        r[[0, 7, 130, 131, 600, n - 1]] = [90, 150, 400, 60, 75, 333]
+    elif kind == "empty":
+        r[rng.random(n) < 0.5] = 0
+    elif kind == "one":
+        r[:] = 0
+        r[5] = 1000
+    return r
+
+
+@pytest.mark.parametrize("kind", ["lattice", "uniform30", "hubs", "empty", "one"])
+def test_every_read_stays_in_the_buffer(program, kind):
+    cols = [str(c) for c in (4, 8, 12, 16, 20, 24, 32, 36, 48, 64, 100, 128)]
+    p = subprocess.run([program, *cols], input=" ".join(map(str, _rows(kind))), text=True, capture_output=True)
+    assert p.returncode == 0, p.stdout
