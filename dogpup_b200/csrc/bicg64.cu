@@ -355,8 +355,11 @@ template <int VEC, int MODE> __global__ void __launch_bounds__(BS, 2) k_dsweep(c
               if (a.B) {
                 b[v] = a.B[((int64_t)k * g.n + i) * a.ns + s];
               } else {
-                const int4 nd = __ldg(reinterpret_cast<const int4 *>(a.snodes) + s);
-                int l = nd.w == i ? 3 : nd.z == i ? 2 : nd.y == i ? 1 : nd.x == i ? 0 : -1;
+                const int32_t *nd = a.snodes + 4 * s;  // (the caller's array: no more than 4-byte aligned)
+                int l = -1;
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                  if (__ldg(nd + q) == i) l = q;
                 if (l >= 0) {
                   const double wt = a.sw[4 * s + l];
                   b[v] = make_double2(wt * a.fpsf[k].x, wt * a.fpsf[k].y);

@@ -44,3 +44,24 @@ def test_same_bits_every_time(case, ns, nf):  # noqa: F811
     assert np.array_equal(runs[0][2], runs[1][2]) and np.array_equal(runs[0][2], runs[2][2])
     nodes, w, X, _, _ = runs[0]
     _check(case, nodes, w, X, list(range(nf)), np.ones(nf), [0, nf // 2, nf - 1])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_node_ids_behind_a_header(case, precision):  # noqa: F811
+    """Node ids at a 4-byte offset in their buffer: int32 data needs no wider alignment."""
+    import torch
+    from dogpup_b200 import api
+    m, ns, harm = case["m"], 6, [0, 5]
+    rng = np.random.default_rng(2)
+    nodes = m.elem[rng.choice(m.ne, ns, replace=False)].astype(np.int32)
+    w = rng.random((ns, 4))
+    S = api.Solver(case["fem"].rowptr, case["fem"].col, case["Kd"], case["Md"], DFC, 2, ns, harmonics=harm)
+    for skip in (1, 2, 3):
+        buf = torch.zeros(skip + 4 * ns, dtype=torch.int32, device="cuda")
+        ids = buf[skip:].view(ns, 4)
+        ids.copy_(torch.as_tensor(nodes))
+        X, rep = S.solve_sources(ids, torch.as_tensor(w, device="cuda"),
+                                 torch.ones(2, dtype=torch.complex128, device="cuda"),
+                                 api.make_opts(precision=precision, tol=1e-12 if precision == "fp64" else 1e-11))
+        assert rep.n_not_converged == 0
+        _check(case, nodes, w, X.cpu().numpy(), harm, np.ones(2), range(2))
