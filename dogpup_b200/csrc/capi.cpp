@@ -471,7 +471,7 @@ int dgp_solver_memory(dgp_solver_t s, int64_t *bytes) {
   int64_t b = 0;
   const DevBuf *bufs[] = {&p.rowptr, &p.col, &p.KM64, &p.RecA32, &p.dfcM, &p.omega, &p.G64, &p.GT64, &p.RecG32, &p.RecGT32,
                           &p.P.rowptr, &p.P.col, &p.P.rowptrT, &p.P.colT, &p.P.permT, &p.scal, &p.ctl, &p.status, &p.fscal, &p.dscal, &p.dpart,
-                          &p.lev_int, &p.lev_coef};
+                          &p.levels[0].ints, &p.levels[0].coef, &p.levels[1].ints, &p.levels[1].coef};
   for (auto *d : bufs) b += (int64_t)d->bytes;
   for (auto &v : p.vec) b += (int64_t)v.bytes;
   for (auto &v : p.fvec) b += (int64_t)v.bytes;

@@ -125,9 +125,12 @@ struct SolverPlan {
     int terms = 0;
     size_t off_mem = 0, off_idx = 0, off_solved = 0, off_coef = 0;
   };
-  std::vector<Level> levels;
-  int levels_first = -1;
-  DevBuf lev_int, lev_coef;
+  struct LevelPlan {             // built at the first solve of its kind and kept
+    bool built = false;
+    std::vector<Level> levels;
+    DevBuf ints, coef;
+  };
+  LevelPlan levels[2];           // dense right-hand sides (one level), point sources
   // ---- FP64 BiCGSTAB on fused sweeps (bicg64.cu)
   DevBuf dvec[9], dscal, dpart;  // vectors; per-column state; chunks' partial sums
   struct LoopKey {               // what a captured loop depends on besides the workspace

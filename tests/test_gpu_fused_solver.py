@@ -109,3 +109,31 @@ def test_nonfinite_source_keeps_the_others(case):
     keep = np.arange(ns) != 7
     assert (st[:, 7] == 4).all() and (st[:, keep] == 0).all() and rep.n_not_converged == 16
     _check(case, nodes[keep], w[keep], X.cpu().numpy()[:, :, keep], harm, np.ones(16), [0, 5, 15])
+
+
+def test_forward_and_adjoint_solves_share_a_plan_without_allocating(case):
+    """Point-source and dense solves in turn on one plan, as a gradient step makes them: after one of each
+    the plan holds all it needs, and the results stay the same."""
+    import torch
+    from dogpup_b200 import api
+    from dogpup_b200._lib import lib
+    m, ns, nf = case["m"], 66, 20
+    rng = np.random.default_rng(4)
+    nodes = m.elem[rng.choice(m.ne, ns, replace=False)].astype(np.int32)
+    w = np.full((ns, 4), 0.25)
+    S = api.Solver(case["fem"].rowptr, case["fem"].col, case["Kd"], case["Md"], DFC, nf, ns)
+    src = [torch.as_tensor(a, device="cuda") for a in (nodes, w, np.ones(nf, dtype=complex))]
+    B = torch.zeros((nf, m.nn, ns), dtype=torch.complex128, device="cuda")
+    for s in range(ns):
+        B[:, torch.as_tensor(nodes[s].astype(np.int64), device="cuda"), s] = 0.25
+    opts = api.make_opts(precision="mixed", tol=1e-11)
+    steps = []
+    for _ in range(3):
+        a0 = lib.dgp_device_allocations()
+        X, r = S.solve_sources(*src, opts)
+        Y, q = S.solve(B, opts)
+        assert r.n_not_converged == 0 and q.n_not_converged == 0
+        _check(case, nodes, w, X.cpu().numpy(), range(nf), np.ones(nf), [0, 7, 19])
+        _check(case, nodes, w, Y.cpu().numpy(), range(nf), np.ones(nf), [0, 7, 19])
+        steps.append(lib.dgp_device_allocations() - a0)
+    assert steps[0] > 0 and steps[1:] == [0, 0]
