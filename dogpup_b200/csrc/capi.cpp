@@ -45,6 +45,7 @@ namespace {
 struct Driver {
   CUresult (*ctx_current)(CUcontext *) = nullptr;
   CUresult (*ctx_id)(CUcontext, unsigned long long *) = nullptr;
+  CUresult (*primary_state)(CUdevice, unsigned *, int *) = nullptr;
   CUresult (*primary_retain)(CUcontext *, CUdevice) = nullptr;
   CUresult (*primary_release)(CUdevice) = nullptr;
 };
@@ -63,6 +64,7 @@ const Driver &driver() {
     };
     get("cuCtxGetCurrent", &d.ctx_current);
     get("cuCtxGetId", &d.ctx_id);
+    get("cuDevicePrimaryCtxGetState", &d.primary_state);
     get("cuDevicePrimaryCtxRetain", &d.primary_retain);
     get("cuDevicePrimaryCtxRelease", &d.primary_release);
   });
@@ -70,20 +72,29 @@ const Driver &driver() {
 }
 
 constexpr int kMaxDev = 64;
-struct PoolEntry {
-  unsigned long long ctx = 0;  // context the pools were made in (0: none yet)
+struct DeviceEntry {
+  unsigned long long primary = 0;  // id of the primary context, as last seen (0: not yet)
+  unsigned long long other = 0;    // id last found to belong to another context
+  unsigned long long pools_of = 0; // context the pools were made in (0: none yet)
   cudaMemPool_t pool[2] = {nullptr, nullptr};  // scratch, plans
 };
-std::mutex g_pool_mutex;
-PoolEntry g_pools[kMaxDev];
+std::mutex g_device_mutex;
+DeviceEntry g_devices[kMaxDev];
 
-cudaMemPool_t make_pool(int dev) {
+// whether the current context is dev's primary one (which is not brought up for the question)
+bool is_primary(int dev) {
   const Driver &d = driver();
   CUcontext cur = nullptr, prim = nullptr;
-  if (!d.primary_retain || !d.primary_release || d.ctx_current(&cur) != CUDA_SUCCESS) return nullptr;
-  if (d.primary_retain(&prim, dev) != CUDA_SUCCESS) return nullptr;
+  unsigned flags = 0;
+  int active = 0;
+  if (!d.primary_state || !d.primary_retain || !d.primary_release || d.ctx_current(&cur) != CUDA_SUCCESS) return false;
+  if (d.primary_state(dev, &flags, &active) != CUDA_SUCCESS || !active) return false;
+  if (d.primary_retain(&prim, dev) != CUDA_SUCCESS) return false;
   d.primary_release(dev);
-  if (prim != cur) return nullptr;  // a context of the application's own: plain allocations
+  return prim == cur;
+}
+
+cudaMemPool_t make_pool(int dev) {
   int ok = 0;
   if (cudaDeviceGetAttribute(&ok, cudaDevAttrMemoryPoolsSupported, dev) != cudaSuccess || !ok) return nullptr;
   cudaMemPoolProps props = {};
@@ -113,14 +124,26 @@ unsigned long long context_id() {
   return id;
 }
 
-cudaMemPool_t device_pool(bool plans) {
+unsigned long long primary_context_id(int *dev) {
   const unsigned long long id = context_id();
+  if (!id || cudaGetDevice(dev) != cudaSuccess || *dev < 0 || *dev >= kMaxDev) return 0;
+  std::lock_guard<std::mutex> lock(g_device_mutex);
+  DeviceEntry &e = g_devices[*dev];
+  if (e.primary != id) {
+    if (e.other == id) return 0;
+    (is_primary(*dev) ? e.primary : e.other) = id;
+  }
+  return e.primary == id ? id : 0;
+}
+
+cudaMemPool_t device_pool(bool plans) {
   int dev = 0;
-  if (!id || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) return nullptr;
-  std::lock_guard<std::mutex> lock(g_pool_mutex);
-  PoolEntry &e = g_pools[dev];
-  if (e.ctx != id) {  // first use, or the context was reset: its pool went with it
-    e.ctx = id;
+  const unsigned long long id = primary_context_id(&dev);
+  if (!id) return nullptr;  // a context of the application's own: plain allocations
+  std::lock_guard<std::mutex> lock(g_device_mutex);
+  DeviceEntry &e = g_devices[dev];
+  if (e.pools_of != id) {  // first use, or the primary context was reset: its pools went with it
+    e.pools_of = id;
     for (auto &p : e.pool) p = make_pool(dev);
   }
   return e.pool[plans ? 1 : 0];

@@ -67,6 +67,11 @@ cudaMemPool_t device_pool(bool plans);
 void trim_pools();
 // id of the current context, unique for the process's lifetime (0: no context is current)
 unsigned long long context_id();
+// the same if the current context is its device's primary one, else 0; *dev: the device.  What the library
+// keeps between calls is kept for primary contexts alone: a device has one at a time, so another id
+// means that the former one was reset and took its handles along, while contexts of the application's own
+// may come and go beside it (calls in them take and give back what they need).
+unsigned long long primary_context_id(int *dev);
 
 // Scratch of one call: allocated and freed in the order of `st`, so queued work may outlive it.
 struct ScratchBuf {
