@@ -34,11 +34,10 @@
 #include <algorithm>
 #include <cmath>
 #include <memory>
-#include <mutex>
-#include <vector>
 
 #include "dgp_common.cuh"
 #include "dgp_internal.h"
+#include "idle_shelf.h"
 
 namespace dgp {
 
@@ -952,6 +951,10 @@ struct LookaheadStreams {
     for (cudaStream_t q : {f, s, b, r})
       if (q) cudaStreamSynchronize(q);
   }
+  void abandon() {
+    for (cudaEvent_t *e : {&fork, &panel, &rest, &join, &step, &side, &diag, &below}) *e = nullptr;
+    for (cudaStream_t *q : {&f, &s, &b, &r}) *q = nullptr;
+  }
   ~LookaheadStreams() {
     wait();
     for (cudaEvent_t e : {fork, panel, rest, join, step, side, diag, below})
@@ -961,54 +964,26 @@ struct LookaheadStreams {
   }
 };
 
-// A set of streams on loan for one call: creating and destroying them took 0.5 ms of each.  At most
-// four idle sets are kept; a set made in a context that has been reset since is dropped (its
-// handles went with the context).
+// A set of streams on loan for one call: creating and destroying them took 0.5 ms of each.
 struct StreamLoan {
-  struct Idle {
-    unsigned long long ctx;
-    std::unique_ptr<LookaheadStreams> set;
-  };
-  static std::mutex &mutex() {
-    static std::mutex m;
-    return m;
+  static IdleShelf<LookaheadStreams> &shelf() {
+    static auto *s = new IdleShelf<LookaheadStreams>;  // (never destroyed: the driver may be gone by then)
+    return *s;
   }
-  static std::vector<Idle> &idle() {
-    static auto *v = new std::vector<Idle>;  // (never destroyed: the driver may be gone by then)
-    return *v;
-  }
+  int dev = 0;
   unsigned long long ctx = 0;
   std::unique_ptr<LookaheadStreams> set;
   bool clean = false;
   int take() {
-    ctx = context_id();
-    if (ctx) {
-      std::lock_guard<std::mutex> lock(mutex());
-      auto &v = idle();
-      for (size_t i = 0; i < v.size(); ++i)
-        if (v[i].ctx == ctx) {
-          set = std::move(v[i].set);
-          v.erase(v.begin() + i);
-          return DGP_OK;
-        }
-    }
+    ctx = primary_context_id(&dev);
+    if (ctx) set = shelf().take(dev, ctx);
+    if (set) return DGP_OK;
     set = std::make_unique<LookaheadStreams>();
     return set->create();
   }
   ~StreamLoan() {
-    if (!set) return;
-    if (!clean || !ctx) return;  // an error left work queued: the set's destructor waits for it
-    std::lock_guard<std::mutex> lock(mutex());
-    auto &v = idle();
-    if (v.size() >= 4) {
-      if (v.front().ctx != ctx) {
-        v.front().set.release();
-        v.erase(v.begin());
-      } else {
-        return;
-      }
-    }
-    v.push_back(Idle{ctx, std::move(set)});
+    // (an error left work queued: the set's destructor waits for it)
+    if (set && clean && ctx) shelf().put(dev, ctx, std::move(set));
   }
 };
 
