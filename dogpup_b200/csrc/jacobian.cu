@@ -426,20 +426,23 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
         const uint64_t bdesc0 = tc::sdesc_k_sw128(tc::smem_u32(sm + L.b_off + buf * L.nch * T2_BCH));
         for (int t = 0; t < L.ntile && ok; ++t, ++tl_idx) {
           const uint32_t slot = tl_idx % T2_NSLOT, use = tl_idx / T2_NSLOT;
-          if (use >= 1) ok = tc::mbar_wait(&tempty[slot], (use - 1) & 1);   // the epilogue has read it
+          if (use >= 1 && !tc::mbar_wait(&tempty[slot], (use - 1) & 1)) {   // the epilogue has read it
+            ok = false;
+            break;
+          }
           tc::fence_after_sync();
           const uint32_t d_tm = tmem + 64u * slot;
           // one wait per tile: on its last stage.  Every builder warp fills a tile's stages in
           // order and its arrival on a stage's barrier releases all of its earlier writes, so the
           // last stage's completion covers the tile's earlier stages too (an mbarrier wait right
           // after a burst of MMAs costs a few hundred cycles).
-          {
-            const int nst_tile = (L.nch + 1) / 2;
-            const uint32_t sl = st_idx + (uint32_t)nst_tile - 1u;
-            ok = tc::mbar_wait(&full[sl % T2_NST], (sl / T2_NST) & 1);
-            tc::fence_after_sync();
+          const uint32_t sl = st_idx + (uint32_t)((L.nch + 1) / 2) - 1u;
+          if (!tc::mbar_wait(&full[sl % T2_NST], (sl / T2_NST) & 1)) {
+            ok = false;
+            break;
           }
-          for (int c0 = 0; c0 < L.nch && ok; c0 += 2) {   // a stage = chunks c0, c0 + 1
+          tc::fence_after_sync();
+          for (int c0 = 0; c0 < L.nch; c0 += 2) {         // a stage = chunks c0, c0 + 1
             const uint32_t s = st_idx % T2_NST;
             for (int cc = 0; cc < 2 && c0 + cc < L.nch; ++cc) {
               const int c = c0 + cc;
@@ -456,7 +459,7 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
             tc::umma_commit(&empty[s]);
             ++st_idx;
           }
-          if (ok) tc::umma_commit(&tfull[slot]);
+          tc::umma_commit(&tfull[slot]);
         }
         if (ok) tc::umma_commit(&bempty[buf]);
       }

@@ -2,7 +2,8 @@
 // mbarriers with bounded waits, UMMA shared-memory and instruction
 // descriptors, tcgen05.mma issue / commit, tensor-memory loads.
 //
-// Every wait is bounded (kSpinLimit polls, 0.1 to 1 s): a kernel that times out
+// Every wait is bounded (kSpinLimit polls of ~4 us, 4.3 s measured on a barrier
+// that nothing arrives at): a kernel that times out
 // records an error flag and tears down instead of spinning for ever.  A poll
 // may suspend its warp for kSuspendNs: with the short default, waiting warps
 // took issue slots from the working ones (time-gated Jacobian, 25 warps per
