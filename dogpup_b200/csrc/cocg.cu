@@ -595,7 +595,7 @@ template <int VEC> int sweep_grids(FWork &w, int nf) {
 // workspace (allocated once per plan) and launch shapes
 int fused_setup(SolverPlan *S, FWork *out) {
   const int nsp = S->fnsp;
-  const int vec = nsp <= 8 ? 2 : 4;  // (at least two lanes per row: full warps down to 4 columns)
+  const int vec = nsp <= 8 ? 2 : 4;  // (two lanes per row or two halves of one: full warps down to 2 columns)
   if (!S->fscal.p) {
     S->drop_workspaces();
     const size_t vb = sizeof(float2) * (size_t)S->nf * S->n * nsp;
@@ -609,7 +609,7 @@ int fused_setup(SolverPlan *S, FWork *out) {
   }
   FWork w = fwork(S);
   w.vec = vec;
-    w.g = make_geo<float>(S->n, S->nf, nsp, vec, 16);
+  w.g = make_geo<float>(S->n, S->nf, nsp, vec, 16);
   w.g64 = make_geo<double>(S->n, S->nf, nsp, vec, 16);
   SolverPlan::Shape &sh = S->shape32;
   if (!sh.set) {

@@ -113,7 +113,7 @@ struct SolverPlan {
   int64_t bytes = 0;
   // ---- fused COCG (cocg.cu): the mixed solve unless a gather or tiled SpMM was asked for by name
   int32_t unfused = 0;
-  int32_t fnsp = 0;              // columns per harmonic, padded to a multiple of 4
+  int32_t fnsp = 0;              // columns per harmonic: 2, or padded to a multiple of 4
   std::vector<int32_t> h_harm;   // harmonic index of each batch slot
   double lam_lo = 0, lam_hi = 0; // 1^T K 1 / 1^T M 1 and max K_ii / M_ii at plan creation
   DevBuf fvec[4], fscal, fctl;   // x, p, q (also the right-hand side), T; per-column state; control block

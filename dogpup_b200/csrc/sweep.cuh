@@ -10,8 +10,8 @@
 //     a nonzero costs one shared-memory read (the record) instead of a global load or shuffles
 //     before its x gathers can start;
 //   - a row is spread over `lpr` lanes (any number up to 32, not only powers of two: 11 sources
-//     take 12 columns), four consecutive complex FP32 values per lane: one 32-byte load and eight
-//     packed FMAs per nonzero;
+//     take 12 columns; 1 or 2 sources: one lane, and a second one for half of the row's nonzeros),
+//     four consecutive complex FP32 values per lane: one 32-byte load and eight packed FMAs per nonzero;
 //   - blocks take chunks of up to 8 consecutive steps in harmonic-major order: a chunk's rows
 //     share most of their columns (Morton order) in L1, and the chunks in flight cover one or two
 //     harmonics, whose x planes fit L2.
@@ -82,6 +82,11 @@ __host__ __device__ inline Window window(int b, int e, int c0, int cap, bool liv
   w.first = (b > c0 ? b : c0) - c0;
   w.count = live ? (e < c0 + cap ? e : c0 + cap) - c0 - w.first : 0;
   return w;
+}
+// the lower or the upper half of a row's records
+__host__ __device__ inline void half_row(int &b, int &e, bool upper) {
+  const int mid = b + (e - b + 1) / 2;
+  (upper ? b : e) = mid;
 }
 // Place of the lane's u-th record.  A warp goes as far as its longest row; a lane without a u-th record
 // in this window is given the buffer's first one, so that every place lies below cap.
@@ -269,6 +274,9 @@ __device__ __forceinline__ void rows(const Geo &g, const int32_t *__restrict__ r
   // blocks 2167 / 2048 / 2581 (registers spill in the epilogues)
   constexpr int UNR = sizeof(R) == 4 ? 4 : 2;
   const int stride = g.cap * Tr<R>::REC;
+  // one lane per row (1 or 2 columns): lanes l and l + 16 take the halves of row l, added at the end
+  const bool split = VEC == 2 && g.lpr == 1;
+  const int row = split ? lane & 15 : rsub;
   auto bounds = [&](int step) {
     const int i = (step * WARPS + warp) * g.rpw + min(lane, g.rpw);
     return __ldg(rowptr + min(i, g.n));
@@ -281,9 +289,10 @@ __device__ __forceinline__ void rows(const Geo &g, const int32_t *__restrict__ r
   if (s0 + 1 < s1) rpn = bounds(s0 + 1);
   for (int step = s0; step < s1; ++step) {
     const int p0 = __shfl_sync(ALL, rp, 0), pe = __shfl_sync(ALL, rp, g.rpw);
-    const int b = __shfl_sync(ALL, rp, rsub), e = __shfl_sync(ALL, rp, rsub + 1);
-    const int i = (step * WARPS + warp) * g.rpw + rsub;
-    const bool valid = rsub < g.rpw && i < g.n;
+    int b = __shfl_sync(ALL, rp, row), e = __shfl_sync(ALL, rp, row + 1);
+    if (split) half_row(b, e, lane >= 16);
+    const int i = (step * WARPS + warp) * g.rpw + row;
+    const bool gather = row < g.rpw && i < g.n, valid = gather && rsub < g.rpw;
     unsigned char *buf = wbuf + cur * stride;
     pre(i, valid);
     int rpnn = 0;
@@ -303,7 +312,7 @@ __device__ __forceinline__ void rows(const Geo &g, const int32_t *__restrict__ r
 #pragma unroll
     for (int u = 0; u < UNR; ++u) Acc<R, VEC, PAD>::clear(z[u]);
     for (int c0 = p0;;) {
-      const Window win = window(b, e, c0, g.cap, valid && live);
+      const Window win = window(b, e, c0, g.cap, gather && live);
       const int m = __reduce_max_sync(ALL, win.count);
       int u0 = 0;
       auto block = [&](auto nu) {
@@ -330,6 +339,13 @@ __device__ __forceinline__ void rows(const Geo &g, const int32_t *__restrict__ r
     }
     C y[VEC];
     acc.result(om, y);
+    if (split) {
+#pragma unroll
+      for (int v = 0; v < VEC; ++v) {
+        y[v].x += __shfl_xor_sync(ALL, y[v].x, 16);
+        y[v].y += __shfl_xor_sync(ALL, y[v].y, 16);
+      }
+    }
     post(i, valid, y);
     __syncwarp();  // the buffer is free for the step after next
     rp = rpn;

@@ -65,3 +65,20 @@ def test_node_ids_behind_a_header(case, precision):  # noqa: F811
                                  api.make_opts(precision=precision, tol=1e-12 if precision == "fp64" else 1e-11))
         assert rep.n_not_converged == 0
         _check(case, nodes, w, X.cpu().numpy(), harm, np.ones(2), range(2))
+
+
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-12), ("mixed", 1e-11)])
+@pytest.mark.parametrize("ns,nf", [(1, 1), (1, 40), (2, 1), (2, 21)])
+def test_one_or_two_sources(case, precision, tol, ns, nf):  # noqa: F811
+    """Two columns per harmonic: a row's records in halves on two lanes; several levels and one."""
+    import torch
+    from dogpup_b200 import api
+    m, harm = case["m"], list(range(nf))
+    nodes = m.elem[[11, 500][:ns]].astype(np.int32)
+    w = np.random.default_rng(6).random((ns, 4))
+    S = api.Solver(case["fem"].rowptr, case["fem"].col, case["Kd"], case["Md"], DFC, nf, ns)
+    X, rep = S.solve_sources(torch.as_tensor(nodes, device="cuda"), torch.as_tensor(w, device="cuda"),
+                             torch.ones(nf, dtype=torch.complex128, device="cuda"),
+                             api.make_opts(precision=precision, tol=tol))
+    assert rep.n_not_converged == 0 and rep.max_rel_residual < 1e-10
+    _check(case, nodes, w, X.cpu().numpy(), harm, np.ones(nf), [0, nf // 2, nf - 1])

@@ -49,7 +49,7 @@ def matrix(request):
 
 
 @pytest.mark.parametrize("precision,tol,bar", [("mixed", 1e-11, 1e-6), ("fp64", 1e-12, 1e-8)])
-@pytest.mark.parametrize("ns", [1, 4, 8, 11, 16, 32, 128])
+@pytest.mark.parametrize("ns", [1, 2, 4, 8, 11, 16, 32, 128])
 def test_solution(matrix, ns, precision, tol, bar):
     import torch
     from dogpup_b200 import api
