@@ -195,7 +195,7 @@ template <int MODE> __device__ void decide(const DArgs &a, int state) {
   }
 }
 
-template <int VEC, int MODE> __global__ void __launch_bounds__(BS, 2) k_dsweep(const DArgs a) {
+template <int VEC, bool SPLIT, int MODE> __global__ void __launch_bounds__(BS, 2) k_dsweep(const DArgs a) {
   constexpr int NQ = nq_of<MODE>(), NQ1 = NQ ? NQ : 1;
   constexpr bool GATHER = MODE <= D_OMEGA, GRID = MODE == D_S || MODE == D_XRP || MODE == D_INIT;
   FCtl *ctl = a.ctl;
@@ -317,7 +317,7 @@ template <int VEC, int MODE> __global__ void __launch_bounds__(BS, 2) k_dsweep(c
       const Src<double> src{a.val + (int64_t)k * a.val_stride, a.col};
       const double om = a.omega ? a.omega[k] : 1.0;
       double2 w[VEC];
-      rows<double, VEC, true>(
+      rows<double, VEC, SPLIT, true>(
           g, a.rowptr, src, om, a.X + base, g.nsp, s0, s1, wbuf, lane, warp, rsub, live, VEC,
           [&](int i, bool valid) {
             if constexpr (MODE != D_STORE)
@@ -547,7 +547,7 @@ struct DWork {
   FCtl *ctl;
   double2 *x, *r, *p, *rhat, *v, *h, *T1, *z, *t;
   Geo g;
-  int vec, grid[7], grid_r;
+  int grid[7], grid_r;
   size_t sm[7], sm_r;
 };
 
@@ -562,26 +562,26 @@ size_t d_smem(const Geo &g, int mode) {
   return mode >= D_S ? std::max(b, sizeof(double) * (size_t)SMALL) : b;
 }
 
-template <int VEC, int MODE> int d_grid(DWork &w, int nf) {
+template <int VEC, bool SPLIT, int MODE> int d_grid(DWork &w, int nf) {
   w.sm[MODE] = d_smem(w.g, MODE);
-  DGP_TRY(allow_dyn_smem(k_dsweep<VEC, MODE>, w.sm[MODE]));
+  DGP_TRY(allow_dyn_smem(k_dsweep<VEC, SPLIT, MODE>, w.sm[MODE]));
   int occ = 0;
-  DGP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_dsweep<VEC, MODE>, BS, w.sm[MODE]));
+  DGP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_dsweep<VEC, SPLIT, MODE>, BS, w.sm[MODE]));
   w.grid[MODE] = (int)std::min<int64_t>((int64_t)std::max(1, occ) * sm_count(), (int64_t)w.g.steps * nf);
   return DGP_OK;
 }
-template <int VEC> int d_grids(DWork &w, int nf) {
-  DGP_TRY((d_grid<VEC, D_STORE>(w, nf)));
-  DGP_TRY((d_grid<VEC, D_V>(w, nf)));
-  DGP_TRY((d_grid<VEC, D_OMEGA>(w, nf)));
-  DGP_TRY((d_grid<VEC, D_S>(w, nf)));
-  DGP_TRY((d_grid<VEC, D_XRP>(w, nf)));
-  DGP_TRY((d_grid<VEC, D_P>(w, nf)));
-  DGP_TRY((d_grid<VEC, D_INIT>(w, nf)));
+template <int VEC, bool SPLIT> int d_grids(DWork &w, int nf) {
+  DGP_TRY((d_grid<VEC, SPLIT, D_STORE>(w, nf)));
+  DGP_TRY((d_grid<VEC, SPLIT, D_V>(w, nf)));
+  DGP_TRY((d_grid<VEC, SPLIT, D_OMEGA>(w, nf)));
+  DGP_TRY((d_grid<VEC, SPLIT, D_S>(w, nf)));
+  DGP_TRY((d_grid<VEC, SPLIT, D_XRP>(w, nf)));
+  DGP_TRY((d_grid<VEC, SPLIT, D_P>(w, nf)));
+  DGP_TRY((d_grid<VEC, SPLIT, D_INIT>(w, nf)));
   w.sm_r = stage_bytes<double>(w.g) + (size_t)w.g.nsp * (4 * 8 + WARPS * 8 + 4 * 4);
-  DGP_TRY(allow_dyn_smem(k_fresid<VEC>, w.sm_r));
+  DGP_TRY(allow_dyn_smem(k_fresid<VEC, SPLIT>, w.sm_r));
   int occ = 0;
-  DGP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fresid<VEC>, BS, w.sm_r));
+  DGP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fresid<VEC, SPLIT>, BS, w.sm_r));
   w.grid_r = (int)std::min<int64_t>((int64_t)std::max(1, occ) * sm_count(), (int64_t)w.g.steps * nf);
   return DGP_OK;
 }
@@ -590,11 +590,12 @@ int d_setup(SolverPlan *S, DWork *out) {
   DWork w{};
   const int nsp = S->fnsp, nf = S->nf;
   const int64_t C = (int64_t)nf * nsp;
-  w.vec = nsp <= 8 ? 2 : 4;
-  w.g = make_geo<double>(S->n, nf, nsp, w.vec, 16);
+  w.g = make_geo<double>(S->n, nf, nsp, nsp <= 8 ? 2 : 4, 16);
   SolverPlan::Shape &sh = S->shape64;
   if (!sh.set) {
-    DGP_TRY(w.vec == 2 ? d_grids<2>(w, nf) : d_grids<4>(w, nf));
+    int rc = DGP_OK;
+    with_shape(w.g, [&](auto v, auto split) { rc = d_grids<decltype(v)::value, decltype(split)::value>(w, nf); });
+    DGP_TRY(rc);
     std::copy(w.grid, w.grid + 7, sh.grid);
     std::copy(w.sm, w.sm + 7, sh.sm);
     sh.grid[7] = w.grid_r;
@@ -654,16 +655,16 @@ int d_setup(SolverPlan *S, DWork *out) {
   return DGP_OK;
 }
 
-template <int VEC> void d_launch(const DWork &w, int mode, const DArgs &a, cudaStream_t st) {
+template <int VEC, bool SPLIT> void d_launch(const DWork &w, int mode, const DArgs &a, cudaStream_t st) {
   const int g = w.grid[mode];
   switch (mode) {
-    case D_STORE: k_dsweep<VEC, D_STORE><<<g, BS, w.sm[mode], st>>>(a); break;
-    case D_V: k_dsweep<VEC, D_V><<<g, BS, w.sm[mode], st>>>(a); break;
-    case D_OMEGA: k_dsweep<VEC, D_OMEGA><<<g, BS, w.sm[mode], st>>>(a); break;
-    case D_S: k_dsweep<VEC, D_S><<<g, BS, w.sm[mode], st>>>(a); break;
-    case D_XRP: k_dsweep<VEC, D_XRP><<<g, BS, w.sm[mode], st>>>(a); break;
-    case D_P: k_dsweep<VEC, D_P><<<g, BS, w.sm[mode], st>>>(a); break;
-    default: k_dsweep<VEC, D_INIT><<<g, BS, w.sm[mode], st>>>(a); break;
+    case D_STORE: k_dsweep<VEC, SPLIT, D_STORE><<<g, BS, w.sm[mode], st>>>(a); break;
+    case D_V: k_dsweep<VEC, SPLIT, D_V><<<g, BS, w.sm[mode], st>>>(a); break;
+    case D_OMEGA: k_dsweep<VEC, SPLIT, D_OMEGA><<<g, BS, w.sm[mode], st>>>(a); break;
+    case D_S: k_dsweep<VEC, SPLIT, D_S><<<g, BS, w.sm[mode], st>>>(a); break;
+    case D_XRP: k_dsweep<VEC, SPLIT, D_XRP><<<g, BS, w.sm[mode], st>>>(a); break;
+    case D_P: k_dsweep<VEC, SPLIT, D_P><<<g, BS, w.sm[mode], st>>>(a); break;
+    default: k_dsweep<VEC, SPLIT, D_INIT><<<g, BS, w.sm[mode], st>>>(a); break;
   }
 }
 
@@ -688,7 +689,11 @@ struct Enqueue {
     base.v = w.v;
     base.rhat = w.rhat;
   }
-  void go(int mode, const DArgs &a) const { w.vec == 2 ? d_launch<2>(w, mode, a, st) : d_launch<4>(w, mode, a, st); }
+  void go(int mode, const DArgs &a) const {
+    with_shape(w.g, [&](auto v, auto split) {
+      d_launch<decltype(v)::value, decltype(split)::value>(w, mode, a, st);
+    });
+  }
   // op: 0 A, 1 G, 2 G^T
   void sweep(int mode, int op, const double2 *X, double2 *Y, const double2 *W) const {
     DArgs a = base;
@@ -822,8 +827,9 @@ int solve_fp64(SolverPlan *S, const double *d_B, const int32_t *d_nodes, const d
   r.ctl = w.ctl;
   r.list = w.d.c.rlist;
   r.nlist = nf;
-  if (w.vec == 2) k_fresid<2><<<w.grid_r, BS, w.sm_r, st>>>(r);
-  else k_fresid<4><<<w.grid_r, BS, w.sm_r, st>>>(r);
+  with_shape(w.g, [&](auto v, auto split) {
+    k_fresid<decltype(v)::value, decltype(split)::value><<<w.grid_r, BS, w.sm_r, st>>>(r);
+  });
   DGP_CHECK_LAUNCH();
   DGP_CUDA(cudaMemcpyAsync(h, w.ctl, sizeof(FCtl), cudaMemcpyDeviceToHost, st));
   DGP_CUDA(cudaStreamSynchronize(st));

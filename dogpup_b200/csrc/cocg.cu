@@ -137,7 +137,7 @@ __device__ void end_iteration(const FSweep &a, FCtl *ctl) {
   }
 }
 
-template <int VEC, int MODE> __global__ void __launch_bounds__(BS, 2) k_fsweep(const FSweep a) {
+template <int VEC, bool SPLIT, int MODE> __global__ void __launch_bounds__(BS, 2) k_fsweep(const FSweep a) {
   constexpr int NQ = MODE == F_A ? 2 : (MODE == F_G || MODE == F_G0) ? 3 : 0;
   constexpr int NQ1 = NQ ? NQ : 1;
   FCtl *ctl = a.ctl;
@@ -231,7 +231,7 @@ template <int VEC, int MODE> __global__ void __launch_bounds__(BS, 2) k_fsweep(c
     const float om = MODE == F_A ? a.omega[k] : 1.f;  // A: K + i w M; G: Re + i Im
     float2 e0[VEC], e1[VEC];
     const bool live = MODE == F_GT0 || (MODE == F_GT ? (act1 | act2) != 0 : act1 != 0);
-    rows<float, VEC>(
+    rows<float, VEC, SPLIT>(
         g, a.rowptr, src, om, X, g.nsp, s0, s1, wbuf, lane, warp, rsub, MODE == F_GT ? act1 != 0 : live, VEC,
         [&](int i, bool valid) {
           if (!valid || !live) return;
@@ -531,7 +531,7 @@ struct FWork {
   FCtl *ctl;
   float2 *x, *p, *q, *T;
   Geo g, g64;
-  int vec, grid[5], grid64;
+  int grid[5], grid64;
   size_t sm[5], sm64;
 };
 
@@ -571,23 +571,23 @@ FWork fwork(SolverPlan *S) {
   return w;
 }
 
-template <int VEC, int MODE> int sweep_grid(const FWork &w, int nf, int *grid) {
-  DGP_TRY(allow_dyn_smem(k_fsweep<VEC, MODE>, w.sm[MODE]));
+template <int VEC, bool SPLIT, int MODE> int sweep_grid(const FWork &w, int nf, int *grid) {
+  DGP_TRY(allow_dyn_smem(k_fsweep<VEC, SPLIT, MODE>, w.sm[MODE]));
   int occ = 0;
-  DGP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fsweep<VEC, MODE>, BS, w.sm[MODE]));
+  DGP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fsweep<VEC, SPLIT, MODE>, BS, w.sm[MODE]));
   *grid = (int)std::min<int64_t>((int64_t)std::max(1, occ) * sm_count(), (int64_t)w.g.steps * nf);
   return DGP_OK;
 }
 
-template <int VEC> int sweep_grids(FWork &w, int nf) {
-  DGP_TRY((sweep_grid<VEC, F_A>(w, nf, &w.grid[F_A])));
-  DGP_TRY((sweep_grid<VEC, F_G>(w, nf, &w.grid[F_G])));
-  DGP_TRY((sweep_grid<VEC, F_GT>(w, nf, &w.grid[F_GT])));
-  DGP_TRY((sweep_grid<VEC, F_G0>(w, nf, &w.grid[F_G0])));
-  DGP_TRY((sweep_grid<VEC, F_GT0>(w, nf, &w.grid[F_GT0])));
-  DGP_TRY(allow_dyn_smem(k_fresid<VEC>, w.sm64));
+template <int VEC, bool SPLIT> int sweep_grids(FWork &w, int nf) {
+  DGP_TRY((sweep_grid<VEC, SPLIT, F_A>(w, nf, &w.grid[F_A])));
+  DGP_TRY((sweep_grid<VEC, SPLIT, F_G>(w, nf, &w.grid[F_G])));
+  DGP_TRY((sweep_grid<VEC, SPLIT, F_GT>(w, nf, &w.grid[F_GT])));
+  DGP_TRY((sweep_grid<VEC, SPLIT, F_G0>(w, nf, &w.grid[F_G0])));
+  DGP_TRY((sweep_grid<VEC, SPLIT, F_GT0>(w, nf, &w.grid[F_GT0])));
+  DGP_TRY(allow_dyn_smem(k_fresid<VEC, SPLIT>, w.sm64));
   int occ = 0;
-  DGP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fresid<VEC>, BS, w.sm64));
+  DGP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fresid<VEC, SPLIT>, BS, w.sm64));
   w.grid64 = (int)std::min<int64_t>((int64_t)std::max(1, occ) * sm_count(), (int64_t)w.g64.steps * nf);
   return DGP_OK;
 }
@@ -608,7 +608,6 @@ int fused_setup(SolverPlan *S, FWork *out) {
     DGP_CUDA(cudaStreamSynchronize(cudaStreamPerThread));
   }
   FWork w = fwork(S);
-  w.vec = vec;
   w.g = make_geo<float>(S->n, S->nf, nsp, vec, 16);
   w.g64 = make_geo<double>(S->n, S->nf, nsp, vec, 16);
   SolverPlan::Shape &sh = S->shape32;
@@ -618,7 +617,9 @@ int fused_setup(SolverPlan *S, FWork *out) {
       w.sm[m] = stage_bytes<float>(w.g) + 16 * (size_t)nsp + 8 * (size_t)WARPS * nsp * nq;
     }
     w.sm64 = stage_bytes<double>(w.g64) + (size_t)nsp * (4 * 8 + WARPS * 8 + 4 * 4);
-    DGP_TRY(vec == 2 ? sweep_grids<2>(w, S->nf) : sweep_grids<4>(w, S->nf));
+    int rc = DGP_OK;
+    with_shape(w.g, [&](auto v, auto split) { rc = sweep_grids<decltype(v)::value, decltype(split)::value>(w, S->nf); });
+    DGP_TRY(rc);
     std::copy(w.grid, w.grid + 5, sh.grid);
     std::copy(w.sm, w.sm + 5, sh.sm);
     sh.grid[5] = w.grid64;
@@ -651,14 +652,14 @@ FSweep sweep_args(const SolverPlan *S, const FWork &w, int mode) {
   return a;
 }
 
-template <int VEC> void launch_sweep(const FWork &w, int mode, const FSweep &a, cudaStream_t st) {
+template <int VEC, bool SPLIT> void launch_sweep(const FWork &w, int mode, const FSweep &a, cudaStream_t st) {
   const dim3 g(w.grid[mode]);
   switch (mode) {
-    case F_A: k_fsweep<VEC, F_A><<<g, BS, w.sm[F_A], st>>>(a); break;
-    case F_G: k_fsweep<VEC, F_G><<<g, BS, w.sm[F_G], st>>>(a); break;
-    case F_GT: k_fsweep<VEC, F_GT><<<g, BS, w.sm[F_GT], st>>>(a); break;
-    case F_G0: k_fsweep<VEC, F_G0><<<g, BS, w.sm[F_G0], st>>>(a); break;
-    default: k_fsweep<VEC, F_GT0><<<g, BS, w.sm[F_GT0], st>>>(a); break;
+    case F_A: k_fsweep<VEC, SPLIT, F_A><<<g, BS, w.sm[F_A], st>>>(a); break;
+    case F_G: k_fsweep<VEC, SPLIT, F_G><<<g, BS, w.sm[F_G], st>>>(a); break;
+    case F_GT: k_fsweep<VEC, SPLIT, F_GT><<<g, BS, w.sm[F_GT], st>>>(a); break;
+    case F_G0: k_fsweep<VEC, SPLIT, F_G0><<<g, BS, w.sm[F_G0], st>>>(a); break;
+    default: k_fsweep<VEC, SPLIT, F_GT0><<<g, BS, w.sm[F_GT0], st>>>(a); break;
   }
 }
 
@@ -672,8 +673,9 @@ int fsweep(const SolverPlan *S, const FWork &w, int mode, cudaStream_t st, const
     b.patience = a.patience;
     b.check_every = a.check_every;
   }
-  if (w.vec == 2) launch_sweep<2>(w, mode, b, st);
-  else launch_sweep<4>(w, mode, b, st);
+  with_shape(w.g, [&](auto v, auto split) {
+    launch_sweep<decltype(v)::value, decltype(split)::value>(w, mode, b, st);
+  });
   DGP_CUDA(cudaGetLastError());
   return DGP_OK;
 }
@@ -700,8 +702,9 @@ int residual(SolverPlan *S, const FWork &w, int mode, int ns, const double *d_X,
   a.list = d_list;
   a.nlist = nlist;
   const unsigned grid = (unsigned)std::min<int64_t>(w.grid64, (int64_t)w.g64.steps * nlist);
-  if (w.vec == 2) k_fresid<2><<<grid, BS, w.sm64, st>>>(a);
-  else k_fresid<4><<<grid, BS, w.sm64, st>>>(a);
+  with_shape(w.g64, [&](auto v, auto split) {
+    k_fresid<decltype(v)::value, decltype(split)::value><<<grid, BS, w.sm64, st>>>(a);
+  });
   DGP_CHECK_LAUNCH();
   return DGP_OK;
 }

@@ -71,6 +71,13 @@ __device__ inline int compact_active(const FCols &c, int na) {
   return s_cnt;
 }
 
+// f(lane width, one lane per row) with the widths as constants: 2 columns, up to 8, more
+template <class F> inline void with_shape(const Geo &g, F f) {
+  if (g.lpr == 1) f(std::integral_constant<int, 2>(), std::true_type());
+  else if (g.nsp / g.lpr == 2) f(std::integral_constant<int, 2>(), std::false_type());
+  else f(std::integral_constant<int, 4>(), std::false_type());
+}
+
 struct FResid {
   Geo g;                    // FP64 mapping: column v * lpr + sub
   int ns, mode;             // mode 0: |b| only; 1: scaled residual to r32, oerr; 2: oerr only
@@ -90,7 +97,7 @@ struct FResid {
 
 // FP64 residual b - A_k X of the listed harmonics, written as FP32 scaled by 1 / |b|, with its
 // norm relative to |b| per column; b is dense or the point sources formed on the fly.
-template <int VEC> __global__ void __launch_bounds__(BS) k_fresid(const FResid a) {
+template <int VEC, bool SPLIT> __global__ void __launch_bounds__(BS) k_fresid(const FResid a) {
   const Geo &g = a.g;
   extern __shared__ __align__(16) unsigned char sm[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -198,7 +205,7 @@ template <int VEC> __global__ void __launch_bounds__(BS) k_fresid(const FResid a
       }
     };
     if (X) {
-      rows<double, VEC>(g, a.rowptr, src, a.omega[k], X, a.ns, s0, s1, wbuf, lane, warp, rsub, nv > 0, nv,
+      rows<double, VEC, SPLIT>(g, a.rowptr, src, a.omega[k], X, a.ns, s0, s1, wbuf, lane, warp, rsub, nv > 0, nv,
                               [](int, bool) {}, finish);
     } else {
       for (int step = s0; step < s1; ++step) {

@@ -74,23 +74,21 @@ template <class R> __host__ __device__ inline size_t stage_bytes(const Geo &g) {
 
 // A lane's records [b, e) in the staged window of cap records from c0: the first one's place in the
 // buffer, and how many there are (<= 0: none).
-struct Window {
-  int first, count;
-};
-__host__ __device__ inline Window window(int b, int e, int c0, int cap, bool live) {
-  Window w;
-  w.first = (b > c0 ? b : c0) - c0;
-  w.count = live ? (e < c0 + cap ? e : c0 + cap) - c0 - w.first : 0;
-  return w;
+__host__ __device__ inline int window_first(int b, int c0) { return max(b, c0) - c0; }
+__host__ __device__ inline int window_count(int e, int c0, int cap, int first, bool live) {
+  return live ? min(e, c0 + cap) - c0 - first : 0;
 }
 // the lower or the upper half of a row's records
 __host__ __device__ inline void half_row(int &b, int &e, bool upper) {
   const int mid = b + (e - b + 1) / 2;
   (upper ? b : e) = mid;
 }
-// Place of the lane's u-th record.  A warp goes as far as its longest row; a lane without a u-th record
-// in this window is given the buffer's first one, so that every place lies below cap.
-__host__ __device__ inline int place(const Window &w, int u) { return u < w.count ? w.first + u : 0; }
+// Place of the lane's u-th record.  A warp goes as far as its longest row.  A lane without a u-th record
+// in this window reads nothing in FP64 (Acc<double>::load leaves first: taking the place below as well
+// cost 2.5 %); in FP32 it is given the buffer's first record, so that every place read lies below cap.
+template <class R> __host__ __device__ inline int place(int first, int count, int u) {
+  return sizeof(R) == 8 || u < count ? first + u : 0;
+}
 
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
@@ -258,11 +256,13 @@ template <int VEC, bool PAD> struct Acc<double, VEC, PAD> {
 
 // Steps [s0, s1) of one harmonic for this warp.  X: the harmonic's plane at the lane's first
 // column, rows xs values apart; live: false skips the lane's gathers (all of its columns are
-// done); nv: columns of the lane that exist in X (FP64 only).  pre(i, valid) runs before the
+// done); nv: columns of the lane that exist in X (FP64 only).  SPLIT (g.lpr 1, 16 rows per warp): lanes l
+// and l + 16 take the halves of row l, added at the end (in its own instances: the 8-column ones took
+// 8 % longer in FP64 with the choice made at run time).  pre(i, valid) runs before the
 // gather of row i (its loads overlap it), post(i, valid, y) after.  wbuf: the warp's two staging
 // buffers.  Control flow is warp-uniform (the warp's longest row sets the trip counts, shorter
 // rows are predicated); lanes past the last row have valid = false.
-template <class R, int VEC, bool PAD = false, class Pre, class Post>
+template <class R, int VEC, bool SPLIT, bool PAD = false, class Pre, class Post>
 __device__ __forceinline__ void rows(const Geo &g, const int32_t *__restrict__ rowptr, const Src<R> &src, const R om,
                                      const typename Tr<R>::C *__restrict__ X, const int xs, const int s0, const int s1,
                                      unsigned char *wbuf, const int lane, const int warp, const int rsub,
@@ -274,9 +274,7 @@ __device__ __forceinline__ void rows(const Geo &g, const int32_t *__restrict__ r
   // blocks 2167 / 2048 / 2581 (registers spill in the epilogues)
   constexpr int UNR = sizeof(R) == 4 ? 4 : 2;
   const int stride = g.cap * Tr<R>::REC;
-  // one lane per row (1 or 2 columns): lanes l and l + 16 take the halves of row l, added at the end
-  const bool split = VEC == 2 && g.lpr == 1;
-  const int row = split ? lane & 15 : rsub;
+  const int row = SPLIT ? lane & 15 : rsub;
   auto bounds = [&](int step) {
     const int i = (step * WARPS + warp) * g.rpw + min(lane, g.rpw);
     return __ldg(rowptr + min(i, g.n));
@@ -290,9 +288,9 @@ __device__ __forceinline__ void rows(const Geo &g, const int32_t *__restrict__ r
   for (int step = s0; step < s1; ++step) {
     const int p0 = __shfl_sync(ALL, rp, 0), pe = __shfl_sync(ALL, rp, g.rpw);
     int b = __shfl_sync(ALL, rp, row), e = __shfl_sync(ALL, rp, row + 1);
-    if (split) half_row(b, e, lane >= 16);
+    if constexpr (SPLIT) half_row(b, e, lane >= 16);
     const int i = (step * WARPS + warp) * g.rpw + row;
-    const bool gather = row < g.rpw && i < g.n, valid = gather && rsub < g.rpw;
+    const bool gather = row < g.rpw && i < g.n, valid = SPLIT ? gather && lane < 16 : gather;
     unsigned char *buf = wbuf + cur * stride;
     pre(i, valid);
     int rpnn = 0;
@@ -312,14 +310,14 @@ __device__ __forceinline__ void rows(const Geo &g, const int32_t *__restrict__ r
 #pragma unroll
     for (int u = 0; u < UNR; ++u) Acc<R, VEC, PAD>::clear(z[u]);
     for (int c0 = p0;;) {
-      const Window win = window(b, e, c0, g.cap, gather && live);
-      const int m = __reduce_max_sync(ALL, win.count);
+      const int p = window_first(b, c0), cnt = window_count(e, c0, g.cap, p, gather && live);
+      const int m = __reduce_max_sync(ALL, cnt);
       int u0 = 0;
       auto block = [&](auto nu) {
         constexpr int N = decltype(nu)::value;
 #pragma unroll
         for (int u = 0; u < N; ++u)
-          acc.load(z[u], buf, g.cap, place(win, u0 + u), Xb, xb, g.lpr, nv, u0 + u < win.count);
+          acc.load(z[u], buf, g.cap, place<R>(p, cnt, u0 + u), Xb, xb, g.lpr, nv, u0 + u < cnt);
 #pragma unroll
         for (int u = 0; u < N; ++u) acc.add(z[u]);
         u0 += N;
@@ -339,7 +337,7 @@ __device__ __forceinline__ void rows(const Geo &g, const int32_t *__restrict__ r
     }
     C y[VEC];
     acc.result(om, y);
-    if (split) {
+    if constexpr (SPLIT) {
 #pragma unroll
       for (int v = 0; v < VEC; ++v) {
         y[v].x += __shfl_xor_sync(ALL, y[v].x, 16);

@@ -31,11 +31,17 @@ template <class R> int walk(const std::vector<int> &rp, int nsp) {
       for (int r = 0; r <= g.rpw; ++r) next[r] = bound(r);
       // a lane's row and records: one lane per row leaves lanes 16.. for the rows' second halves
       const bool split = g.lpr == 1;
+      struct Window {
+        int first, count;
+      };
       auto lane_window = [&](int lane, int c0) {
         const int r = split ? lane % 16 : lane / g.lpr;
         int b = bound(r), e = bound(r + 1);
         if (split) half_row(b, e, lane >= 16);
-        return window(b, e, c0, g.cap, r < g.rpw && r0 + r < n);
+        Window w;
+        w.first = window_first(b, c0);
+        w.count = window_count(e, c0, g.cap, w.first, r < g.rpw && r0 + r < n);
+        return w;
       };
       std::vector<char> seen(pe - p0 + 1, 0);
       for (int c0 = p0;;) {
@@ -45,7 +51,8 @@ template <class R> int walk(const std::vector<int> &rp, int nsp) {
           const int r = split ? lane % 16 : lane / g.lpr;
           const Window w = lane_window(lane, c0);
           for (int u = 0; u < m; ++u) {
-            const int q = place(w, u);
+            if (sizeof(R) == 8 && u >= w.count) continue;              // (not read)
+            const int q = place<R>(w.first, w.count, u);
             if (q < 0 || q >= g.cap) return 2;                         // outside the warp's buffer
             if (u < w.count) {
               if (c0 + q >= pe) return 3;                              // not staged
