@@ -607,7 +607,7 @@ int d_setup(SolverPlan *S, DWork *out) {
   DWork w{};
   const int nsp = S->fnsp, nf = S->nf;
   const int64_t C = (int64_t)nf * nsp;
-  w.g = make_geo<double>(S->n, nf, nsp, nsp <= 8 ? 2 : 4, 16);
+  w.g = make_geo<double>(S->n, nf, nsp, nsp <= 8 ? 2 : 4, std::max(S->nnz, S->nnzG));
   SolverPlan::Shape &sh = S->shape64;
   if (!sh.set) {
     int rc = DGP_OK;

@@ -608,8 +608,8 @@ int fused_setup(SolverPlan *S, FWork *out) {
     DGP_CUDA(cudaStreamSynchronize(cudaStreamPerThread));
   }
   FWork w = fwork(S);
-  w.g = make_geo<float>(S->n, S->nf, nsp, vec, 16);
-  w.g64 = make_geo<double>(S->n, S->nf, nsp, vec, 16);
+  w.g = make_geo<float>(S->n, S->nf, nsp, vec, std::max(S->nnz, S->nnzG));
+  w.g64 = make_geo<double>(S->n, S->nf, nsp, vec, std::max(S->nnz, S->nnzG));
   SolverPlan::Shape &sh = S->shape32;
   if (!sh.set) {
     for (int m = 0; m < 5; ++m) {

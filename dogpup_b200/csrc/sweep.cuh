@@ -55,15 +55,19 @@ struct Geo {
   int steps;       // steps per harmonic
 };
 
-// lanes per row, rows per warp and staging size; avg: records per row of the longest operator
-template <class R> inline Geo make_geo(int64_t n, int nf, int nsp, int vec, int avg) {
+// Lanes per row, rows per warp and staging size.  nnz: records of the operator with the most; runs of
+// average rows fit a buffer up to STAGE_MAX per block, which leaves room for two blocks and L1.
+constexpr size_t STAGE_MAX = 88 * 1024;
+template <class R> inline Geo make_geo(int64_t n, int nf, int nsp, int vec, int64_t nnz) {
   Geo g;
   g.n = (int)n;
   g.nf = nf;
   g.nsp = nsp;
   g.lpr = nsp / vec;
   g.rpw = 32 / g.lpr > 16 ? 16 : 32 / g.lpr;  // (row bounds travel in one register per lane: <= 31 rows)
-  g.cap = (avg * g.rpw + 16 + 3) & ~3;
+  const int64_t avg = ceil_div(nnz, n) > 16 ? ceil_div(nnz, n) : 16;
+  const int64_t most = STAGE_MAX / (WARPS * 2 * Tr<R>::REC), want = avg * g.rpw + 16 + 3;
+  g.cap = (int)(want < most ? want : most) & ~3;
   g.steps = (int)ceil_div(n, (int64_t)WARPS * g.rpw);
   return g;
 }

@@ -20,8 +20,8 @@ using namespace dgp::sweep;
 
 template <class R> int walk(const std::vector<int> &rp, int nsp) {
   const int n = (int)rp.size() - 1, vec = nsp <= 8 ? 2 : 4;
-  const Geo g = make_geo<R>(n, 1, nsp, vec, 16);
-  if (stage_bytes<R>(g) < (size_t)WARPS * 2 * g.cap * Tr<R>::REC) return 1;
+  const Geo g = make_geo<R>(n, 1, nsp, vec, rp[n]);
+  if (g.cap % 4 || stage_bytes<R>(g) > STAGE_MAX || stage_bytes<R>(g) < (size_t)WARPS * 2 * g.cap * Tr<R>::REC) return 1;
   for (int step = 0; step < g.steps; ++step)
     for (int warp = 0; warp < WARPS; ++warp) {
       const int r0 = (step * WARPS + warp) * g.rpw;
