@@ -294,16 +294,17 @@ __global__ void k_rytov_t(const double *__restrict__ rytov, int nm, int ng, floa
 //     to 13 % off the kernel's time);
 //   - a row of J (a gate's NS x ND entries) is put together in shared memory, 16-byte pieces in an
 //     order that spreads the banks, and leaves as one bulk copy, or through the Rytov division in
-//     consecutive 16-byte stores.
+//     consecutive 16-byte stores (other shapes: see EPI_DIRECT and EPI_WIDE).
 //
 // Persistent CTA (one per SM), warp-specialised, all hand-offs through mbarriers:
 //   warps 0-3   epilogue: per tile, tensor memory -> hi + lo halves, w_v (and Rytov) -> J
 //               (warp q reads accumulator lanes 32q.. = gate 4t+q of tile t, lane = source)
-//   warps 4-19  builders: A' stages tile by tile (lane = source, warp = gate within the tile x
-//               harmonic quarter of a chunk)
-//   warp 20     one thread issues the MMAs (tile by tile: every chunk of a tile, after which
+//   then        builders: A' stages tile by tile (lane = source, warp = gate within the tile x part of a
+//               chunk): 16 warps, a quarter of a chunk each, or 8 with a half up to 32 harmonics, where a
+//               tile is one stage and every warp's hand-over counts
+//   a warp      one thread issues the MMAs (tile by tile: every chunk of a tile, after which
 //               its accumulator is complete); tensor-memory allocation
-//   warps 21-24 feeders: sources and B'' of each voxel, ahead of the builders and MMAs that need
+//   4 warps     feeders: sources and B'' of each voxel, ahead of the builders and MMAs that need
 //               them (lane = optode)
 // Bound by the chain of build, hand-over and MMAs through the three stages that tensor memory has
 // room for: at 7.4 ms, without the MMAs the kernel took 5.1, without the builders' stores 6.6,
@@ -317,8 +318,8 @@ __global__ void k_rytov_t(const double *__restrict__ rytov, int nm, int ng, floa
 // a few hundred cycles on B200).  Every mbarrier
 // wait is bounded: a timeout sets err, raises the abort flag that every role polls, and the
 // MMA thread waits (bounded) for all of its MMAs before the tensor memory is freed.
-constexpr int T2_EPI = 4, T2_BLD = 16, T2_FD = 4;   // epilogue, A' builder, feeder warps
-constexpr int T2_THREADS = 32 * (T2_EPI + T2_BLD + 1 + T2_FD);
+constexpr int T2_EPI = 4, T2_FD = 4;               // epilogue and feeder warps
+constexpr int t2_threads(int bld) { return 32 * (T2_EPI + bld + 1 + T2_FD); }
 constexpr int T2_NSLOT = 2;                        // accumulator slots (64 columns each)
 constexpr int T2_NST = 3;                          // A' stages in tensor memory (2 chunks, 128 columns each)
 constexpr uint32_t T2_ACOL = 64u * T2_NSLOT;       // first A' column
@@ -362,7 +363,22 @@ __device__ inline void swap_if(bool p, float4 &x, float4 &y) {
   y = p ? t : y;
 }
 
-__global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const float2 *__restrict__ C /*[ng][nf]*/,
+// How the epilogue leaves J (one instance each: with all three in one kernel every one was 5 to 20 %
+// slower).  Kernel times at 27,949 nodes, us: former kernel (eight builders, EPI_WIDE) / sixteen builders
+// and EPI_ROWS for all / now:
+//   EPI_ROWS    full rows, nd % 4 == 0: put together in shared memory, for the Rytov division in 16-byte
+//               pieces, or past 16 harmonics as one bulk copy; 16 x 16 x 32 x 10: 774 / 741 / 694,
+//               with Rytov 2,039 / 865 / 798; 24 x 24 x 32 x 20: 1,186 / 1,284 / 1,113
+//   EPI_DIRECT  by halves of a row straight to J: full rows up to 16 harmonics, nd % 4 == 0 (32 x 32 x 16 x 20:
+//               906 / 1,122 / 853; 20 x 20 x 9 x 12: 573 / 732 / 506), and selected links without Rytov
+//               (8 x 8 x 13 x 24: 1,299 / 1,291 / 1,126); past 32 harmonics whatever is not EPI_ROWS
+//               (there is no room for EPI_WIDE's registers: 1,104 bytes of spills)
+//   EPI_WIDE    a whole row in registers, the slot free before the first store: full rows with nd % 4 != 0
+//               (5 x 30 x 13 x 7: 435 / 508 / 394) and selected links with Rytov (8 x 8 x 13 x 24: 2,042 / 2,190 /
+//               1,904).  15 x 31 x 20 x 16 without Rytov stays 6 % behind (1,138 / 1,317 / 1,213).
+enum { EPI_ROWS = 0, EPI_DIRECT = 1, EPI_WIDE = 2 };
+template <int T2_BLD, int NC, int EPI>
+__global__ void __launch_bounds__(t2_threads(T2_BLD), 1) k_jacobian_tg_tc(JArgs a, const float2 *__restrict__ C /*[ng][nf]*/,
                                                                  const float *__restrict__ ryt /*[ng][nm]*/, int dense,
                                                                  float *__restrict__ Jtg, int *err) {
   extern __shared__ __align__(1024) unsigned char t2_raw[];
@@ -376,6 +392,7 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
   int *lk = reinterpret_cast<int *>(sm + L.l_off);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   constexpr unsigned FULL = 0xffffffffu;
+  constexpr int T2_THREADS = t2_threads(T2_BLD), NH = 64 / T2_BLD;   // harmonics of a chunk per builder
   volatile int *abort_v = &abort_flag;
 
   if (tid == 0) {
@@ -546,12 +563,12 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
         break;
       }
       const float2 *fs = reinterpret_cast<const float2 *>(sm + L.f_off) + buf * 32 * L.nkp + s;
-      float pr[4][4], pi[4][4];
+      float pr[NC][NH], pi[NC][NH];
 #pragma unroll
-      for (int c = 0; c < 4; ++c)
+      for (int c = 0; c < NC; ++c)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 y = c < L.nch ? fs[32 * (16 * c + 4 * part + j)] : make_float2(0.f, 0.f);
+        for (int j = 0; j < NH; ++j) {
+          const float2 y = c < L.nch ? fs[32 * (16 * c + NH * part + j)] : make_float2(0.f, 0.f);
           pr[c][j] = y.x;
           pi[c][j] = y.y;
         }
@@ -559,7 +576,7 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
       if (lane == 0) tc::mbar_arrive(&sempty[buf]);
       for (int t = 0; t < L.ntile && !fail; ++t) {
 #pragma unroll
-        for (int c0 = 0; c0 < 4; c0 += 2) {             // a stage = chunks c0, c0 + 1
+        for (int c0 = 0; c0 < NC; c0 += 2) {            // a stage = chunks c0, c0 + 1
           if (c0 >= L.nch || fail) break;
           const uint32_t si = st_idx % T2_NST;
           if (st_idx >= T2_NST && !__all_sync(FULL, tc::mbar_wait(&empty[si], ((st_idx / T2_NST) - 1) & 1))) {
@@ -570,11 +587,11 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
 #pragma unroll
           for (int cc = 0; cc < 2; ++cc) {
             const int c = c0 + cc;
-            if (c >= L.nch) break;
-            const float2 *cg = Ct + (4 * t + gl) * L.nkp + 16 * c + 4 * part;
-            float hr[4], lr[4], hm[4], lm[4];
+            if (c >= NC || c >= L.nch) break;
+            const float2 *cg = Ct + (4 * t + gl) * L.nkp + 16 * c + NH * part;
+            float hr[NH], lr[NH], hm[NH], lm[NH];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < NH; ++j) {
               const float2 q = cg[j];
               const float qr = q.x * pr[c][j] - q.y * pi[c][j], qi = -(q.x * pi[c][j] + q.y * pr[c][j]);
               // hi = x with the 13 low mantissa bits cleared (a TF32 value), lo = x - hi (exact);
@@ -584,9 +601,9 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
               hm[j] = __uint_as_float(__float_as_uint(qi) & 0xffffe000u);
               lm[j] = qi - hm[j];
             }
-            // row gl * 32 + s = lane s of this warp's quadrant; chunk cc of the stage: K' = 4 part + j
-            // (real), 16 + 4 part + j (imaginary); lo 64 columns after hi
-            const uint32_t tq = tmem + ((uint32_t)(32 * gl) << 16) + T2_ACOL + 128u * si + 32u * cc + 4u * part;
+            // row gl * 32 + s = lane s of this warp's quadrant; chunk cc of the stage: K' = NH part + j
+            // (real), 16 + NH part + j (imaginary); lo 64 columns after hi
+            const uint32_t tq = tmem + ((uint32_t)(32 * gl) << 16) + T2_ACOL + 128u * si + 32u * cc + (uint32_t)NH * part;
             tc::tmem_st(tq, hr);
             tc::tmem_st(tq + 16u, hm);
             tc::tmem_st(tq + 64u, lr);
@@ -625,8 +642,30 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
         tc::fence_after_sync();
         const int g = 4 * t + gl;
         float *row = Jtg + ((int64_t)v * a.ng + g) * a.nm;
+        if constexpr (EPI == EPI_WIDE) {
+          uint32_t r[32], q[32];
+          const uint32_t ta = tmem + ((uint32_t)(32 * warp) << 16) + 64u * slot;
+          tc::tmem_ld32(ta, r);                          // (A_hi + A_lo) B_hi
+          tc::tmem_ld32(ta + 32u, q);                    // (A_hi + A_lo) B_lo
+          tc::fence_before_sync();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(&tempty[slot]);
+          if (g < a.ng && s < a.ns) {
+#pragma unroll
+            for (int d = 0; d < 32; ++d) {
+              if (d >= a.nd) break;
+              const int m = dense ? s * a.nd + d : lk[s * 32 + d];
+              if (m < 0) continue;
+              float val = wv * (__uint_as_float(r[d]) + __uint_as_float(q[d]));
+              if (ryt) val = val / ryt[(int64_t)g * a.nm + m];
+              row[m] = val;
+            }
+          }
+          __syncwarp();                                  // converged again for the next wait
+          continue;
+        }
         unsigned char *ob = sm + L.o_off + 4096 * (2 * warp + (tl_idx & 1u));
-        if (dense == 2) {                                // the copy before the last has left this buffer
+        if constexpr (EPI == EPI_ROWS) {                 // the copy before the last has left this buffer
           if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
           __syncwarp();
         }
@@ -642,7 +681,7 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(&tempty[slot]);
           }
-          if (dense == 2) {                              // m = s nd + d, nd a multiple of 4
+          if (EPI == EPI_ROWS || dense == 2) {           // m = s nd + d, nd a multiple of 4
             float4 x[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i)
@@ -650,6 +689,14 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
                                  wv * (__uint_as_float(r[4 * i + 1]) + __uint_as_float(q[4 * i + 1])),
                                  wv * (__uint_as_float(r[4 * i + 2]) + __uint_as_float(q[4 * i + 2])),
                                  wv * (__uint_as_float(r[4 * i + 3]) + __uint_as_float(q[4 * i + 3])));
+            if constexpr (EPI == EPI_DIRECT) {
+              if (g < a.ng && s < a.ns)
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                  if (16 * h + 4 * i < a.nd) *reinterpret_cast<float4 *>(row + s * a.nd + 16 * h + 4 * i) = x[i];
+              __syncwarp();
+              continue;
+            }
             // lane s stores its four 16-byte pieces in the order i ^ (s % 4): rows are 128 bytes apart
             swap_if(lane & 1, x[0], x[1]);
             swap_if(lane & 1, x[2], x[3]);
@@ -675,7 +722,7 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
           }
           __syncwarp();                                  // converged again for the next load
         }
-        if (dense == 2 && g < a.ng) {
+        if (EPI == EPI_ROWS && g < a.ng) {
           if (ryt) {
             for (int m = 4 * lane; m < a.nm; m += 128) {
               float4 x = *reinterpret_cast<const float4 *>(ob + 4 * m);
@@ -694,7 +741,7 @@ __global__ void __launch_bounds__(T2_THREADS, 1) k_jacobian_tg_tc(JArgs a, const
           __syncwarp();
         }
         // a group per tile, empty or not: the wait above counts them
-        if (dense == 2 && lane == 0) asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        if (EPI == EPI_ROWS && lane == 0) asm volatile("cp.async.bulk.commit_group;" ::: "memory");
       }
     }
     if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // no copy outlives the kernel
@@ -1213,10 +1260,26 @@ int jacobian_run(int mode, const int32_t *prow, const int32_t *pcol, const doubl
     ScratchBuf flag;
     DGP_TRY(flag.alloc(sizeof(int), st));
     DGP_CUDA(cudaMemsetAsync(flag.p, 0, sizeof(int), st));
-    DGP_TRY(allow_dyn_smem(k_jacobian_tg_tc, smem_tc));
     const int gtc = (int)std::min<int64_t>(nv, (int64_t)sm_count());
-    k_jacobian_tg_tc<<<gtc, T2_THREADS, smem_tc, st>>>(a, ctab.as<float2>(), ryt.as<float>(), dense, (float *)out,
-                                                       flag.as<int>());
+    int arc = DGP_OK;
+    auto go = [&](auto bld, auto nc, auto epi) {
+      constexpr int BLD_ = decltype(bld)::value, NC_ = decltype(nc)::value, EPI_ = decltype(epi)::value;
+      arc = allow_dyn_smem(k_jacobian_tg_tc<BLD_, NC_, EPI_>, smem_tc);
+      if (arc == DGP_OK)
+        k_jacobian_tg_tc<BLD_, NC_, EPI_><<<gtc, t2_threads(BLD_), smem_tc, st>>>(
+            a, ctab.as<float2>(), ryt.as<float>(), dense, (float *)out, flag.as<int>());
+    };
+    using std::integral_constant;
+    auto by_epi = [&](auto bld, auto nc) {
+      constexpr int NC_ = decltype(nc)::value;
+      if (dense == 2 && (rytov || NC_ > 1)) go(bld, nc, integral_constant<int, EPI_ROWS>());
+      else if (NC_ > 2 || (dense != 1 && !rytov)) go(bld, nc, integral_constant<int, EPI_DIRECT>());
+      else if constexpr (NC_ <= 2) go(bld, nc, integral_constant<int, EPI_WIDE>());
+    };
+    if (tl.nch > 2) by_epi(integral_constant<int, 16>(), integral_constant<int, 4>());
+    else if (tl.nch == 2) by_epi(integral_constant<int, 8>(), integral_constant<int, 2>());
+    else by_epi(integral_constant<int, 8>(), integral_constant<int, 1>());
+    DGP_TRY(arc);
     DGP_CHECK_LAUNCH();
     int h = 0;
     DGP_CUDA(cudaMemcpyAsync(&h, flag.p, sizeof(int), cudaMemcpyDeviceToHost, st));

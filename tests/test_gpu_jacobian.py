@@ -393,3 +393,37 @@ def test_tg_jacobian_tensor_core_rows(ns, nd, nf, ng, nn, use_rytov):
     mag = np.einsum("gk,kvm->vgm", np.abs(C), np.abs(a))
     scale = wts[:, None, None] / (ryt.T[None] if use_rytov else 1.0)
     assert (np.abs(J.cpu().numpy() - scale * J0) <= 400 * 2.0 ** -23 * np.sqrt(2) * scale * mag).all()
+
+
+@pytest.mark.parametrize("rytov", [False, True])
+@pytest.mark.parametrize("ns,nd,nf,ng", [(32, 32, 16, 9), (5, 30, 13, 7), (32, 32, 32, 5), (7, 12, 17, 6), (15, 31, 33, 4),
+                                         (8, 20, 48, 3)])
+@pytest.mark.parametrize("links", ["full", "some"])
+def test_tg_tensor_cores_harmonic_chunks_and_row_forms(ns, nd, nf, ng, links, rytov):
+    """One, two, three and four chunks of 16 harmonics; full rows of J whose length is and is not a multiple
+    of four, selected links; with and without the Rytov division: every instance of the kernel, against
+    64-bit sums.  Bound, relative to the sum of the terms' absolute values: operands keep 2^-22 of their size
+    and are formed with a few FP32 roundings (1e-6); the accumulator is cut to FP32 after each of the nf / 2
+    MMA steps of K = 8 for the hi and lo parts (2^-23 each, taken twice)."""
+    import torch
+    from dogpup_b200 import api
+    rng = np.random.default_rng(ns * 100 + nf)
+    nn, nt = 301, 64
+    cplx = lambda *s: rng.standard_normal(s) + 1j * rng.standard_normal(s)  # noqa: E731
+    phi, phiA, fpsf, gate = cplx(nf, nn, ns), cplx(nf, nn, nd), cplx(nf) + 3, cplx(ng, nf) / nt
+    link = np.stack(np.meshgrid(np.arange(ns), np.arange(nd), indexing="ij"), -1).reshape(-1, 2)
+    if links == "some":
+        link = link[rng.permutation(len(link))[:max(3, len(link) // 3)]]
+    data = rng.uniform(0.5, 2.0, (len(link), ng))
+    w = rng.uniform(0.5, 1.5, nn)
+    dev = lambda a: torch.as_tensor(a, device="cuda")  # noqa: E731
+    J = api.jacobian_tg(api.Basis(nn=nn, w=w), dev(phi), dev(phiA), dev(fpsf), dev(link.astype(np.int32)), dev(gate), nt,
+                        dev(data) if rytov else None).cpu().numpy()
+    h = np.where(np.arange(nf) == 0, 0.5, 1.0)
+    C = -2.0 * nt * h * np.conj(gate) / fpsf
+    a = phi[:, :, link[:, 0]] * phiA[:, :, link[:, 1]]
+    ref = np.einsum("gk,kvm->vgm", C, a).real * w[:, None, None]
+    size = np.einsum("gk,kvm->vgm", np.abs(C), np.abs(a)) * w[:, None, None]
+    if rytov:
+        ref, size = ref / data.T, size / data.T
+    assert (np.abs(J - ref) <= (1e-6 + 1.2e-7 * nf) * size).all(), (np.abs(J - ref) / size).max()
