@@ -39,6 +39,7 @@ _SIGS = {
     "dgp_version": (C.c_int, []),
     "dgp_kernel_launches": (I64, []),
     "dgp_device_allocations": (I64, []),
+    "dgp_trim_memory": (C.c_int, []),
     "dgp_smv_mex": (C.c_int, [P, P, P, P, P, P, P, P, P, C.c_int, C.c_int, C.c_int, P]),
     "dgp_fsaimv_mex": (C.c_int, [P, P, P, P, P, P, P, P, C.c_int, C.c_int, C.c_int, C.c_int, P]),
     "dgp_fsaip_mex": (C.c_int, [P, P, P, P, P, P, P, P, C.c_int, C.c_int, P]),

@@ -31,6 +31,11 @@ def as_real(t: torch.Tensor) -> torch.Tensor:
     return torch.view_as_real(t) if t.is_complex() else t
 
 
+def trim_memory():
+    """Give the device memory that the library keeps between calls back to the driver (dgp_trim_memory)."""
+    check(lib.dgp_trim_memory())
+
+
 class Fem:
     """Device FEM topology + assembly plan (``prepare_mesh``/``gen_fwdmat``, dMesh.m:945-1235)."""
 

@@ -2,6 +2,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <cstring>
@@ -150,12 +151,18 @@ cudaMemPool_t device_pool(bool plans) {
 }
 
 void trim_pools() {
-  for (bool plans : {false, true}) {
-    cudaMemPool_t pool = device_pool(plans);
-    if (!pool) continue;
-    cudaDeviceSynchronize();
-    cudaMemPoolTrimTo(pool, 0);
+  int dev = 0;
+  const unsigned long long id = primary_context_id(&dev);
+  if (!id) return;
+  cudaMemPool_t pool[2] = {nullptr, nullptr};
+  {
+    std::lock_guard<std::mutex> lock(g_device_mutex);
+    if (g_devices[dev].pools_of == id) std::copy(g_devices[dev].pool, g_devices[dev].pool + 2, pool);
   }
+  if (!pool[0] && !pool[1]) return;
+  cudaDeviceSynchronize();  // frees that are still queued
+  for (cudaMemPool_t p : pool)
+    if (p) cudaMemPoolTrimTo(p, 0);
 }
 
 // which: 0 cudaMalloc, 1 the scratch pool, 2 the plan pool, in the order of st; sets *pooled
@@ -327,6 +334,13 @@ int dgp_version(void) { return 10000; }
 int64_t dgp_kernel_launches(void) { return launch_count(); }
 
 int64_t dgp_device_allocations(void) { return g_device_allocs.load(std::memory_order_relaxed); }
+
+int dgp_trim_memory(void) {
+  DGP_GUARD([] {
+    trim_pools();
+    return DGP_OK;
+  }());
+}
 
 // ------------------------------------------------------------ mex layouts
 int dgp_smv_mex(double *d_out_real, double *d_out_imag, const double *d_x_real, const double *d_x_imag,

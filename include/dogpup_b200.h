@@ -58,10 +58,15 @@ int dgp_version(void);
 /* Number of kernels this library has launched in the process so far
  * (kernels inside its CUDA graphs included). */
 int64_t dgp_kernel_launches(void);
-/* Number of device allocations (cudaMalloc calls, failed ones included) this
+/* Number of device allocations (from a pool or the driver, failed ones included) this
  * library's own code has made in the process so far; allocations made inside
  * cuBLAS are not counted. */
 int64_t dgp_device_allocations(void);
+/* Gives the device memory that the library keeps between calls (up to 1/64 of
+ * the device's for scratch and as much for plans, in the current device's
+ * primary context) back to the driver, for another allocator of the process to
+ * use.  Waits for the device; plans and their results stay as they are. */
+int dgp_trim_memory(void);
 
 /* ====================================================================== *
  *  Drop-in host functions of the reference mex sources.  Same names,

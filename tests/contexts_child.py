@@ -2,7 +2,7 @@
 context of the application's own, in turn, as a program does that embeds the library beside its own driver
 API code.  No torch is loaded.
 
-    python contexts_child.py      -> one JSON line on stdout
+    python contexts_child.py alternate | trim     -> one JSON line on stdout
 """
 import ctypes as C
 import json
@@ -13,6 +13,7 @@ import numpy as np
 
 sys.path.insert(0, str(Path(__file__).resolve().parent.parent))
 
+from dogpup_b200 import _lib  # noqa: E402
 from dogpup_b200._lib import lib  # noqa: E402  (loads libdogpup_b200.so)
 
 U64, VP, SZ = C.c_uint64, C.c_void_p, C.c_size_t
@@ -67,12 +68,59 @@ def lm_update(jt, y):
     return x
 
 
+def matrix(n=20000, band=12):
+    """A diagonally dominant banded K and M in CSR form."""
+    cols = np.arange(n)[:, None] + np.arange(-band, band + 1)
+    keep = (cols >= 0) & (cols < n)
+    rp = np.concatenate([[0], np.cumsum(keep.sum(1))]).astype(np.int32)
+    off = np.broadcast_to(np.abs(np.arange(-band, band + 1)), cols.shape)
+    k = np.where(off == 0, 2.0 * band + 1.0, -1.0 / np.maximum(off, 1))
+    return rp, cols[keep].astype(np.int32), k[keep], np.where(off == 0, 1.0, 0.0)[keep]
+
+
+def plan_and_solve(nf=16, ns=16):
+    """A solver plan in the current context and its first solve; (handle, buffers)."""
+    rp, col, K, M = matrix()
+    n = len(rp) - 1
+    bufs = [up(rp), up(col), up(K), up(M)]
+    h = VP()
+    ck(lib.dgp_solver_create(C.byref(h), *[VP(b.value) for b in bufs[:2]], n, len(col), *[VP(b.value) for b in bufs[2:]],
+                             0.1, nf, ns, None, None), "dgp_solver_create")
+    nodes, w = np.arange(4 * ns, dtype=np.int32) * 300, np.full(4 * ns, 0.25)
+    fpsf = np.tile([1.0, 0.0], nf)
+    bufs += [up(nodes), up(w), up(fpsf), up(np.zeros(2 * nf * n * ns))]
+    opts, rep = _lib.default_opts(), _lib.SolveReport()
+    opts.precision, opts.tol = _lib.PREC_MIXED, 1e-8
+    ck(lib.dgp_solve_sources(h, *[VP(b.value) for b in bufs[4:7]], ns, VP(bufs[7].value), C.byref(opts), C.byref(rep),
+                             None), "dgp_solve_sources")
+    for b in bufs:
+        ck(cu.cuMemFree_v2(b), "cuMemFree")
+    return h
+
+
+def trim(prim):
+    """Free memory before a plan, with it, after it is destroyed, and after the trim."""
+    ck(cu.cuCtxSetCurrent(prim), "cuCtxSetCurrent")
+    ck(lib.dgp_solver_destroy(plan_and_solve()), "dgp_solver_destroy")   # modules loaded, pools made
+    ck(lib.dgp_trim_memory(), "dgp_trim_memory")
+    free = [free_bytes()]
+    h = plan_and_solve()
+    free.append(free_bytes())
+    ck(lib.dgp_solver_destroy(h), "dgp_solver_destroy")
+    free.append(free_bytes())
+    ck(lib.dgp_trim_memory(), "dgp_trim_memory")
+    return free + [free_bytes()]
+
+
 def main():
     ck(cu.cuInit(0), "cuInit")
     dev, prim, own = C.c_int(), VP(), VP()
     ck(cu.cuDeviceGet(C.byref(dev), 0), "cuDeviceGet")
     ck(cu.cuDevicePrimaryCtxRetain(C.byref(prim), dev), "cuDevicePrimaryCtxRetain")
     ck(cu.cuCtxCreate_v2(C.byref(own), 0, dev), "cuCtxCreate")
+    if sys.argv[1] == "trim":
+        print(json.dumps({"free": trim(prim)}))
+        return
     rng = np.random.default_rng(1)
     jt, y = rng.standard_normal((2500, 1500)).astype(np.float32), rng.standard_normal(1500)
     xs, free = [], []
