@@ -2244,6 +2244,7 @@ void SolverPlan::drop_workspaces() {
 }
 
 SolverPlan::~SolverPlan() {
+  const PrimaryScope scope(rowptr.dev);
   if (busy) cudaDeviceSynchronize();  // a call that ended early may have left work on the buffers
   drop_workspaces();
   for (auto &e : poll_ev)

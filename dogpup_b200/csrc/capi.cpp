@@ -45,6 +45,7 @@ namespace {
 // driver entry points fetched through the runtime (no link against libcuda)
 struct Driver {
   CUresult (*ctx_current)(CUcontext *) = nullptr;
+  CUresult (*ctx_set)(CUcontext) = nullptr;
   CUresult (*ctx_id)(CUcontext, unsigned long long *) = nullptr;
   CUresult (*primary_state)(CUdevice, unsigned *, int *) = nullptr;
   CUresult (*primary_retain)(CUcontext *, CUdevice) = nullptr;
@@ -64,6 +65,7 @@ const Driver &driver() {
         cudaGetLastError();
     };
     get("cuCtxGetCurrent", &d.ctx_current);
+    get("cuCtxSetCurrent", &d.ctx_set);
     get("cuCtxGetId", &d.ctx_id);
     get("cuDevicePrimaryCtxGetState", &d.primary_state);
     get("cuDevicePrimaryCtxRetain", &d.primary_retain);
@@ -221,18 +223,39 @@ int DevBuf::alloc_plan(size_t n) {
   release();
   DGP_TRY(device_alloc(&p, n, cudaStreamPerThread, 2, &pooled));
   bytes = n ? n : 16;
-  // any stream may use it from here on
-  if (pooled) DGP_CUDA(cudaStreamSynchronize(cudaStreamPerThread));
+  if (pooled) {
+    DGP_CUDA(cudaGetDevice(&dev));
+    DGP_CUDA(cudaStreamSynchronize(cudaStreamPerThread));  // any stream may use it from here on
+  }
   return DGP_OK;
 }
 
+PrimaryScope::PrimaryScope(int dev) {
+  int cur = -1;
+  if (dev < 0 || (primary_context_id(&cur) && cur == dev)) return;
+  CUcontext c = nullptr;
+  const Driver &d = driver();
+  if (!d.ctx_set || d.ctx_current(&c) != CUDA_SUCCESS) return;
+  back = c;
+  switched = cudaSetDevice(dev) == cudaSuccess;
+  if (!switched) cudaGetLastError();
+}
+
+PrimaryScope::~PrimaryScope() {
+  if (switched) driver().ctx_set(static_cast<CUcontext>(back));
+}
+
 void DevBuf::release() {
-  if (p) {
-    if (pooled) cudaFreeAsync(p, cudaStreamPerThread);
-    else cudaFree(p);
+  if (p && pooled) {
+    PrimaryScope scope(dev);
+    if (cudaFreeAsync(p, cudaStreamPerThread) != cudaSuccess) cudaGetLastError();
+  } else if (p) {
+    cudaFree(p);
   }
   p = nullptr;
   bytes = 0;
+  pooled = false;
+  dev = -1;
 }
 
 int sm_count() {

@@ -87,12 +87,24 @@ struct ScratchBuf {
   template <class T> T *as() const { return static_cast<T *>(p); }
 };
 
+// Makes dev's primary context current for its lifetime, and then the one before again (dev < 0: nothing):
+// a plan may be destroyed while another device or a context of the application's own is current, and
+// pooled memory is freed in the order of a stream of its own context.
+struct PrimaryScope {
+  void *back = nullptr;
+  bool switched = false;
+  explicit PrimaryScope(int dev);
+  PrimaryScope(const PrimaryScope &) = delete;
+  ~PrimaryScope();
+};
+
 // Device buffer owned by a plan; freed in the destructor.  alloc_plan takes it from the library's
 // pool: its owner frees it only when no work on it is queued any more.
 struct DevBuf {
   void *p = nullptr;
   size_t bytes = 0;
   bool pooled = false;
+  int dev = -1;  // pooled: the device whose primary context it belongs to
   DevBuf() = default;
   DevBuf(const DevBuf &) = delete;
   DevBuf &operator=(const DevBuf &) = delete;

@@ -2,7 +2,7 @@
 context of the application's own, in turn, as a program does that embeds the library beside its own driver
 API code.  No torch is loaded.
 
-    python contexts_child.py alternate | trim     -> one JSON line on stdout
+    python contexts_child.py alternate | trim | destroy     -> one JSON line on stdout
 """
 import ctypes as C
 import json
@@ -23,6 +23,7 @@ cu.cuDeviceGet.argtypes = [C.POINTER(C.c_int), C.c_int]
 cu.cuCtxCreate_v2.argtypes = [C.POINTER(VP), C.c_uint, C.c_int]
 cu.cuCtxDestroy_v2.argtypes = [VP]
 cu.cuCtxSetCurrent.argtypes = [VP]
+cu.cuCtxGetCurrent.argtypes = [C.POINTER(VP)]
 cu.cuDevicePrimaryCtxRetain.argtypes = [C.POINTER(VP), C.c_int]
 cu.cuMemAlloc_v2.argtypes = [C.POINTER(U64), SZ]
 cu.cuMemFree_v2.argtypes = [U64]
@@ -98,15 +99,20 @@ def plan_and_solve(nf=16, ns=16):
     return h
 
 
-def trim(prim):
-    """Free memory before a plan, with it, after it is destroyed, and after the trim."""
+def trim(prim, destroy_in):
+    """Free memory before a plan, with it, after it is destroyed (in the given context), and after the trim."""
     ck(cu.cuCtxSetCurrent(prim), "cuCtxSetCurrent")
     ck(lib.dgp_solver_destroy(plan_and_solve()), "dgp_solver_destroy")   # modules loaded, pools made
     ck(lib.dgp_trim_memory(), "dgp_trim_memory")
     free = [free_bytes()]
     h = plan_and_solve()
     free.append(free_bytes())
+    ck(cu.cuCtxSetCurrent(destroy_in), "cuCtxSetCurrent")
     ck(lib.dgp_solver_destroy(h), "dgp_solver_destroy")
+    cur = VP()
+    ck(cu.cuCtxGetCurrent(C.byref(cur)), "cuCtxGetCurrent")
+    assert cur.value == destroy_in.value
+    ck(cu.cuCtxSetCurrent(prim), "cuCtxSetCurrent")
     free.append(free_bytes())
     ck(lib.dgp_trim_memory(), "dgp_trim_memory")
     return free + [free_bytes()]
@@ -118,8 +124,8 @@ def main():
     ck(cu.cuDeviceGet(C.byref(dev), 0), "cuDeviceGet")
     ck(cu.cuDevicePrimaryCtxRetain(C.byref(prim), dev), "cuDevicePrimaryCtxRetain")
     ck(cu.cuCtxCreate_v2(C.byref(own), 0, dev), "cuCtxCreate")
-    if sys.argv[1] == "trim":
-        print(json.dumps({"free": trim(prim)}))
+    if sys.argv[1] != "alternate":
+        print(json.dumps({"free": trim(prim, own if sys.argv[1] == "destroy" else prim)}))
         return
     rng = np.random.default_rng(1)
     jt, y = rng.standard_normal((2500, 1500)).astype(np.float32), rng.standard_normal(1500)

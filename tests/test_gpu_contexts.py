@@ -26,9 +26,11 @@ def test_alternating_contexts_keep_one_pool():
     assert max(out["free"][1:]) - min(out["free"][1:]) <= 2 ** 21, out["free"]
 
 
-def test_trim_gives_a_destroyed_plans_memory_back():
-    """The library keeps a destroyed plan's memory for the next one; after a trim the device has as much free
-    as before the plan, to within one 2 MB page."""
-    before, plan, destroyed, trimmed = _child("trim")["free"]
+@pytest.mark.parametrize("mode", ["trim", "destroy"])
+def test_trim_gives_a_destroyed_plans_memory_back(mode):
+    """A plan destroyed in its own context, and while another one is current (which stays so).  The library
+    keeps a destroyed plan's memory for the next one; after a trim the device has as much free as before the
+    plan, to within one 2 MB page."""
+    before, plan, destroyed, trimmed = _child(mode)["free"]
     assert before - plan > 2 ** 27 and before - destroyed > 2 ** 27
     assert before - trimmed <= 2 ** 21
