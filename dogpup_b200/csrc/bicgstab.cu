@@ -1870,38 +1870,49 @@ void spmm_go(const SolverPlan *S, const Layout &L, size_t smem, cudaStream_t st,
   k_spmm<R, VEC, MODE, Op, 0><<<grid_of(L), BS, smem, st>>>(L, op, X, Y, W, cols, ctl);
 }
 
-// one BiCGSTAB iteration (dMesh.m:1295-1340) enqueued on st: KERNELS_PER_ITER launches
-// lane widths: plain SpMM sweeps VS, SpMM sweeps with dot products VD, vector updates 2
-constexpr int VU = 2;
+// Lane widths: plain SpMM sweeps VS, SpMM sweeps with dot products VD, vector updates 2 -- and 4 past
+// 64 padded sources, where 2 would take more lanes per row than a warp has.
+int vu_of(const SolverPlan *S) { return S->nsp > 64 ? 4 : 2; }
+template <class F> void with_vu(const SolverPlan *S, F f) {
+  if (vu_of(S) == 4) f(std::integral_constant<int, 4>());
+  else f(std::integral_constant<int, 2>());
+}
 
 // one BiCGSTAB iteration (dMesh.m:1295-1340) enqueued on st: KERNELS_PER_ITER launches
 // one complex-FP32 iteration with the tiled SpMM (same kernel sequence as enqueue_iteration)
 void enqueue_iteration_tiled(const SolverPlan *S, const Vecs<float> &V, const Work &W, cudaStream_t st) {
-  const Layout Lu = layouts_for(S, VU).L, Lud = layouts_for(S, VU).Ld;
+  const Layout Lu = layouts_for(S, vu_of(S)).L, Lud = layouts_for(S, vu_of(S)).Ld;
   Ctl *ctl = W.ctl;
   tspmm<0>(S, 1, V.p, V.T1, nullptr, W.cols, ctl, st);
   tspmm<0>(S, 2, V.T1, V.h, nullptr, W.cols, ctl, st);
   tspmm<1>(S, 0, V.h, V.v, V.rhat, W.cols, ctl, st);
   k_stage_alpha<<<1, 1024, 0, st>>>(W.cols, ctl);
-  k_update_s<float, VU><<<grid_of(Lud), BS, red_smem(Lud, 1), st>>>(Lud, V.r, V.v, V.s, W.cols, ctl);
+  with_vu(S, [&](auto u) {
+    k_update_s<float, decltype(u)::value><<<grid_of(Lud), BS, red_smem(Lud, 1), st>>>(
+        Lud, V.r, V.v, V.s, W.cols, ctl);
+  });
   k_stage_check_s<<<1, 1024, 0, st>>>(W.cols, ctl);
   tspmm<0>(S, 1, V.s, V.T1, nullptr, W.cols, ctl, st);
   tspmm<0>(S, 2, V.T1, V.z, nullptr, W.cols, ctl, st);
   tspmm<0>(S, 0, V.z, V.t, nullptr, W.cols, ctl, st);
   tspmm<2>(S, 1, V.t, nullptr, V.T1, W.cols, ctl, st);
   k_stage_omega<<<1, 1024, 0, st>>>(W.cols, ctl);
-  k_update_xrp<float, VU><<<grid_of(Lud), BS, red_smem(Lud, 2), st>>>(Lud, V.x, V.h, V.z, V.r, V.s, V.t, V.p, V.v,
-                                                                      V.rhat, W.cols, ctl);
+  with_vu(S, [&](auto u) {
+    k_update_xrp<float, decltype(u)::value><<<grid_of(Lud), BS, red_smem(Lud, 2), st>>>(
+        Lud, V.x, V.h, V.z, V.r, V.s, V.t, V.p, V.v, V.rhat, W.cols, ctl);
+  });
   k_stage_check_r<<<1, 1024, 0, st>>>(W.cols, ctl);
   k_stage_count<<<1, 1024, 0, st>>>(W.cols, ctl);
-  k_update_p<float, VU><<<grid_of(Lu), BS, 0, st>>>(Lu, V.r, V.p, W.cols, ctl);
+  with_vu(S, [&](auto u) {
+    k_update_p<float, decltype(u)::value><<<grid_of(Lu), BS, 0, st>>>(Lu, V.r, V.p, W.cols, ctl);
+  });
 }
 
 template <class R, int VS, int VD, class OpA, class OpG>
 void enqueue_iteration(const SolverPlan *S, const OpA &A, const OpG &G, const OpG &GT, const Vecs<R> &V,
                        const Work &W, cudaStream_t st) {
   const Layout Ls = spmm_layouts(S, VS, sizeof(R) == 4).L, Lsd = spmm_layouts(S, VD, sizeof(R) == 4).Ld;
-  const Layout Lu = layouts_for(S, VU).L, Lud = layouts_for(S, VU).Ld;
+  const Layout Lu = layouts_for(S, vu_of(S)).L, Lud = layouts_for(S, vu_of(S)).Ld;
   Ctl *ctl = W.ctl;
   if constexpr (sizeof(R) == 4) {
     if (S->tiled) {
@@ -1916,7 +1927,9 @@ void enqueue_iteration(const SolverPlan *S, const OpA &A, const OpG &G, const Op
   spmm_go<R, VD, 1>(S, Lsd, red_smem(Lsd, 1), st, A, V.h, V.v, V.rhat, W.cols, ctl);
   k_stage_alpha<<<1, 1024, 0, st>>>(W.cols, ctl);
   // s = r - alpha v ; ||s||                                     (:1306-1308)
-  k_update_s<R, VU><<<grid_of(Lud), BS, red_smem(Lud, 1), st>>>(Lud, V.r, V.v, V.s, W.cols, ctl);
+  with_vu(S, [&](auto u) {
+    k_update_s<R, decltype(u)::value><<<grid_of(Lud), BS, red_smem(Lud, 1), st>>>(Lud, V.r, V.v, V.s, W.cols, ctl);
+  });
   k_stage_check_s<<<1, 1024, 0, st>>>(W.cols, ctl);
   // Gs = G s ; z = G^T Gs ; t = A z ; (G t).Gs, (G t).(G t)     (:1315-1325)
   spmm_go<R, VS, 0>(S, Ls, 0, st, G, V.s, V.T1, nullptr, W.cols, ctl);
@@ -1925,12 +1938,16 @@ void enqueue_iteration(const SolverPlan *S, const OpA &A, const OpG &G, const Op
   spmm_go<R, VD, 2>(S, Lsd, red_smem(Lsd, 2), st, G, V.t, nullptr, V.T1, W.cols, ctl);
   k_stage_omega<<<1, 1024, 0, st>>>(W.cols, ctl);
   // x += alpha h + om z ; r = s - om t ; p -= om v ; ||r|| ; r0^.r   (:1305, :1327-1337)
-  k_update_xrp<R, VU><<<grid_of(Lud), BS, red_smem(Lud, 2), st>>>(Lud, V.x, V.h, V.z, V.r, V.s, V.t, V.p, V.v,
-                                                                  V.rhat, W.cols, ctl);
+  with_vu(S, [&](auto u) {
+    k_update_xrp<R, decltype(u)::value><<<grid_of(Lud), BS, red_smem(Lud, 2), st>>>(
+        Lud, V.x, V.h, V.z, V.r, V.s, V.t, V.p, V.v, V.rhat, W.cols, ctl);
+  });
   k_stage_check_r<<<1, 1024, 0, st>>>(W.cols, ctl);
   k_stage_count<<<1, 1024, 0, st>>>(W.cols, ctl);
   // p = r + beta p                                              (:1340)
-  k_update_p<R, VU><<<grid_of(Lu), BS, 0, st>>>(Lu, V.r, V.p, W.cols, ctl);
+  with_vu(S, [&](auto u) {
+    k_update_p<R, decltype(u)::value><<<grid_of(Lu), BS, 0, st>>>(Lu, V.r, V.p, W.cols, ctl);
+  });
 }
 
 // COCG preconditioner step: T1 = G r ; z = G^T T1 ; acc[D1] = r.z ; rho, beta.  The gather
@@ -1960,9 +1977,11 @@ void enqueue_cocg_precond(const SolverPlan *S, const OpG &G, const OpG &GT, cons
 template <class R, int VS, int VD, class OpG>
 void enqueue_cocg_start(const SolverPlan *S, const OpG &G, const OpG &GT, const Vecs<R> &V, const Work &W,
                         cudaStream_t st) {
-  const Layout Lu = layouts_for(S, VU).L;
+  const Layout Lu = layouts_for(S, vu_of(S)).L;
   enqueue_cocg_precond<R, VS, VD>(S, G, GT, V, W, 1, st);
-  k_update_p<R, VU><<<grid_of(Lu), BS, 0, st>>>(Lu, V.z, V.p, W.cols, W.ctl);
+  with_vu(S, [&](auto u) {
+    k_update_p<R, decltype(u)::value><<<grid_of(Lu), BS, 0, st>>>(Lu, V.z, V.p, W.cols, W.ctl);
+  });
 }
 
 // one preconditioned COCG iteration (conjugate-orthogonal CG for the complex-symmetric A_k with
@@ -1972,7 +1991,7 @@ void enqueue_cocg_start(const SolverPlan *S, const OpG &G, const OpG &GT, const 
 template <class R, int VS, int VD, class OpA, class OpG>
 void enqueue_cocg(const SolverPlan *S, const OpA &A, const OpG &G, const OpG &GT, const Vecs<R> &V, const Work &W,
                   cudaStream_t st) {
-  const Layout Lu = layouts_for(S, VU).L, Lud = layouts_for(S, VU).Ld;
+  const Layout Lu = layouts_for(S, vu_of(S)).L, Lud = layouts_for(S, vu_of(S)).Ld;
   Ctl *ctl = W.ctl;
   bool done = false;
   if constexpr (sizeof(R) == 4) {
@@ -1986,10 +2005,14 @@ void enqueue_cocg(const SolverPlan *S, const OpA &A, const OpG &G, const OpG &GT
     spmm_go<R, VD, 1>(S, Lsd, red_smem(Lsd, 1), st, A, V.p, V.v, V.p, W.cols, ctl);
   }
   k_cocg_alpha<<<1, 1024, 0, st>>>(W.cols, ctl);
-  k_update_r<R, VU><<<grid_of(Lud), BS, red_smem(Lud, 1), st>>>(Lud, V.r, V.v, W.cols, ctl);
+  with_vu(S, [&](auto u) {
+    k_update_r<R, decltype(u)::value><<<grid_of(Lud), BS, red_smem(Lud, 1), st>>>(Lud, V.r, V.v, W.cols, ctl);
+  });
   k_cocg_check<<<1, 1024, 0, st>>>(W.cols, ctl);
   enqueue_cocg_precond<R, VS, VD>(S, G, GT, V, W, 0, st);
-  k_update_px<R, VU><<<grid_of(Lu), BS, 0, st>>>(Lu, V.x, V.p, V.z, W.cols, ctl);
+  with_vu(S, [&](auto u) {
+    k_update_px<R, decltype(u)::value><<<grid_of(Lu), BS, 0, st>>>(Lu, V.x, V.p, V.z, W.cols, ctl);
+  });
   k_cocg_count<<<1, 1024, 0, st>>>(W.cols, ctl);
 }
 
@@ -2382,7 +2405,7 @@ static int solve_mixed(SolverPlan *S, const double *d_B, const int32_t *d_nodes,
     // against tol after each inner solve.  The stall guard of run_iterations ends inner solves
     // that stop making progress in FP32.
     DGP_TRY(set_ctl(W.ctl, o.inner_tol, inner_maxit, DGP_STOP_PER_COLUMN, st, S->h_ctl));
-    launch_init<float, VU>(layouts_for(S, VU).Ld, V, W, st);
+    with_vu(S, [&](auto u) { launch_init<float, decltype(u)::value>(layouts_for(S, vu_of(S)).Ld, V, W, st); });
     DGP_CHECK_LAUNCH();
     k_stage_init<<<1, 1024, 0, st>>>(W.cols, W.ctl, S->nsp, ns, ref > 0 ? W.outer_err : nullptr, o.tol);
     DGP_CHECK_LAUNCH();
@@ -2488,20 +2511,33 @@ template <int VEC>
 void profile_launch(int which, const SolverPlan *S, const OpA32 &A, const OpG32 &G, const Vecs<float> &V,
                     const Work &W, const Ctl *ctl, cudaStream_t st) {
   const Layout L = spmm_layouts(S, VEC, true).L, Ld = spmm_layouts(S, VEC, true).Ld;
-  const Layout Lu = layouts_for(S, VU).L, Lud = layouts_for(S, VU).Ld;
+  const Layout Lu = layouts_for(S, vu_of(S)).L, Lud = layouts_for(S, vu_of(S)).Ld;
   switch (which) {
     case 0: spmm_go<float, VEC, 0>(S, L, 0, st, A, V.z, V.x, nullptr, W.cols, ctl); break;
     case 1: spmm_go<float, VEC, 0>(S, L, 0, st, G, V.p, V.T1, nullptr, W.cols, ctl); break;
     case 4: spmm_go<float, VEC, 1>(S, Ld, red_smem(Ld, 1), st, A, V.p, V.v, V.p, W.cols, ctl); break;
     case 5: spmm_go<float, VEC, 3>(S, Ld, red_smem(Ld, 1), st, G, V.r, V.T1, nullptr, W.cols, ctl); break;
-    case 6: k_update_r<float, VU><<<grid_of(Lud), BS, red_smem(Lud, 1), st>>>(Lud, V.r, V.v, W.cols, ctl); break;
-    case 7: k_update_px<float, VU><<<grid_of(Lu), BS, 0, st>>>(Lu, V.x, V.p, V.z, W.cols, ctl); break;
+    case 6:
+      with_vu(S, [&](auto u) {
+        k_update_r<float, decltype(u)::value><<<grid_of(Lud), BS, red_smem(Lud, 1), st>>>(Lud, V.r, V.v, W.cols, ctl);
+      });
+      break;
+    case 7:
+      with_vu(S, [&](auto u) {
+        k_update_px<float, decltype(u)::value><<<grid_of(Lu), BS, 0, st>>>(Lu, V.x, V.p, V.z, W.cols, ctl);
+      });
+      break;
     case 2:
-      k_update_xrp<float, VU><<<grid_of(Lud), BS, red_smem(Lud, 2), st>>>(Lud, V.x, V.h, V.z, V.r, V.s, V.t, V.p,
-                                                                          V.v, V.rhat, W.cols, ctl);
+      with_vu(S, [&](auto u) {
+        k_update_xrp<float, decltype(u)::value><<<grid_of(Lud), BS, red_smem(Lud, 2), st>>>(
+            Lud, V.x, V.h, V.z, V.r, V.s, V.t, V.p, V.v, V.rhat, W.cols, ctl);
+      });
       break;
     default:
-      k_update_s<float, VU><<<grid_of(Lud), BS, red_smem(Lud, 1), st>>>(Lud, V.r, V.v, V.s, W.cols, ctl);
+      with_vu(S, [&](auto u) {
+        k_update_s<float, decltype(u)::value><<<grid_of(Lud), BS, red_smem(Lud, 1), st>>>(
+            Lud, V.r, V.v, V.s, W.cols, ctl);
+      });
       break;
   }
 }

@@ -469,3 +469,34 @@ def test_solver_fp64_per_column_skips_finished_harmonics(small_case, gpu_case, t
     err = np.linalg.norm(np.transpose(X.cpu().numpy(), (1, 2, 0)) - xd, axis=0) / np.linalg.norm(xd, axis=0)
     assert err.max() < 1e-8, err.max()
     assert (status.cpu().numpy() == 0).all()
+
+
+@pytest.mark.parametrize("ns", [64, 65, 128])
+def test_unfused_solves_past_64_sources(small_case, gpu_case, torch, ns):
+    """BiCGSTAB inner solves, COCG at a launch shape set by hand, the autotuner and the kernel timings take
+    every source count that a plan does."""
+    from dogpup_b200 import api
+    import scipy.sparse.linalg as sla
+    m, K, M, dfc, harm = small_case["mesh"], small_case["K"], small_case["M"], 0.003, [0, 9]
+    rng = np.random.default_rng(ns)
+    nodes = m.elem[rng.choice(m.ne, ns, replace=False)].astype(np.int32)
+    w = rng.random((ns, 4))
+    S = api.Solver(gpu_case["fem"].rowptr, gpu_case["fem"].col, gpu_case["K"], gpu_case["M"], dfc, 2, ns, harmonics=harm)
+    src = [torch.as_tensor(a, device="cuda") for a in (nodes, w, np.ones(2, dtype=complex))]
+    B = np.zeros((m.nn, ns), dtype=complex)
+    for s in range(ns):
+        B[nodes[s], s] = w[s]
+    ref = [sla.splu((K + 1j * h * dfc * M).tocsc()).solve(B) for h in harm]
+
+    def check(precision):
+        X, rep = S.solve_sources(*src, api.make_opts(precision=precision, tol=1e-10))
+        assert rep.n_not_converged == 0
+        for x, x0 in zip(X.cpu().numpy(), ref):
+            assert (np.linalg.norm(x - x0, axis=0) <= 1e-6 * np.linalg.norm(x0, axis=0)).all()
+
+    check("mixed_bicgstab")
+    S.autotune()
+    check("mixed_bicgstab")
+    S.set_spmm(False, 4, 64)
+    check("mixed")
+    assert all(S.profile_kernel(q, 1)[0] > 0 for q in range(8))
