@@ -1738,9 +1738,8 @@ int tiled_setup(SolverPlan *S, cudaStream_t st) {
   }
 }
 
-template <class R> struct Vecs {
-  using C = typename CT<R>::C;
-  C *x, *r, *rhat, *p, *v, *h, *s, *T1, *z, *t;
+struct Vecs {
+  float2 *x, *r, *rhat, *p, *v, *h, *s, *T1, *z, *t;
 };
 
 struct Work {
@@ -1778,11 +1777,10 @@ size_t scal_bytes(int64_t C) { return (sizeof(double) * 5 + sizeof(double2) * (4
 // BiCGSTAB all NVEC_ALL; a slot that is not allocated yet views as NULL
 constexpr int NVEC_COCG = 7, NVEC_ALL = 10;
 
-template <class R> Vecs<R> vec_views(SolverPlan *S) {
-  using C = typename CT<R>::C;
-  Vecs<R> V;
-  C **slots[NVEC_ALL] = {&V.x, &V.r, &V.rhat, &V.p, &V.v, &V.T1, &V.z, &V.h, &V.s, &V.t};
-  for (int q = 0; q < NVEC_ALL; ++q) *slots[q] = S->vec[q].as<C>();
+Vecs vec_views(SolverPlan *S) {
+  Vecs V;
+  float2 **slots[NVEC_ALL] = {&V.x, &V.r, &V.rhat, &V.p, &V.v, &V.T1, &V.z, &V.h, &V.s, &V.t};
+  for (int q = 0; q < NVEC_ALL; ++q) *slots[q] = S->vec[q].as<float2>();
   return V;
 }
 
@@ -1790,18 +1788,17 @@ template <class R> Vecs<R> vec_views(SolverPlan *S) {
 // reallocates everything; more vectors for the same precision are added without moving the
 // existing ones (graphs captured on them stay valid).  The mixed solve with the COCG inner
 // solver needs 7 of the 10 vectors (70 instead of 100 GB at 153k nodes x 64 x 128).
-int ensure_workspace(SolverPlan *S, int prec, int nvec = NVEC_ALL) {
+int ensure_workspace(SolverPlan *S, int nvec) {
   const int64_t C = (int64_t)S->nf * S->nsp;
-  const size_t esz = prec == DGP_PREC_FP64 ? sizeof(double2) : sizeof(float2);
-  const size_t vb = esz * (size_t)C * S->n;
-  if (S->ws_prec != prec) {
+  const size_t vb = sizeof(float2) * (size_t)C * S->n;
+  if (S->ws_prec != DGP_PREC_MIXED) {
     S->drop_workspaces();
     DGP_TRY(S->scal.alloc_plan(scal_bytes(C)));
     DGP_TRY(S->status.alloc_plan(sizeof(int) * C));
     DGP_TRY(S->ctl.alloc_plan(sizeof(Ctl)));
     DGP_CUDA(cudaMemsetAsync(S->scal.p, 0, scal_bytes(C), cudaStreamPerThread));
     DGP_CUDA(cudaStreamSynchronize(cudaStreamPerThread));
-    S->ws_prec = prec;
+    S->ws_prec = DGP_PREC_MIXED;
     S->ws_cols = C;
   }
   for (int q = 0; q < nvec; ++q)
@@ -1829,9 +1826,9 @@ Layouts layouts_for(const SolverPlan *S, int vec, int rows = 64) {
 // SpMM layouts: rows per block from the autotuner when it has run; the complex-FP32 dot
 // sweeps take tune_dot (default 4) times those rows per block and at most 32 rows per
 // lane, the bound of their FP32 per-lane partial sums
-Layouts spmm_layouts(const SolverPlan *S, int vec, bool fp32) {
-  Layouts x = layouts_for(S, vec, (fp32 && S->tune_rows) ? S->tune_rows : 64);
-  if (fp32) x.Ld.ipb = std::max(x.L.ipb, std::min(x.L.ipb * (S->tune_dot ? S->tune_dot : 4), 32));
+Layouts spmm_layouts(const SolverPlan *S, int vec) {
+  Layouts x = layouts_for(S, vec, S->tune_rows ? S->tune_rows : 64);
+  x.Ld.ipb = std::max(x.L.ipb, std::min(x.L.ipb * (S->tune_dot ? S->tune_dot : 4), 32));
   return x;
 }
 
@@ -1847,30 +1844,27 @@ inline int vec_for(const SolverPlan *S, bool fp32) {
 
 dim3 grid_of(const Layout &L) { return dim3((unsigned)ceil_div(L.n, L.rows_per_block()), (unsigned)L.nf); }
 
-// k_spmm launch with the plan's gather kind (complex FP32: S->tune_kind; FP64: kind 0)
-template <class R, int VEC, int MODE, class Op>
-void spmm_go(const SolverPlan *S, const Layout &L, size_t smem, cudaStream_t st, const Op &op,
-             const typename CT<R>::C *X, typename CT<R>::C *Y, const typename CT<R>::C *W, const Cols &cols,
-             const Ctl *ctl) {
-  if constexpr (sizeof(R) == 4) {
-    switch (S->tune_kind) {
-      case 1: k_spmm<R, VEC, MODE, Op, 1><<<grid_of(L), BS, smem, st>>>(L, op, X, Y, W, cols, ctl); return;
-      case 2: k_spmm<R, VEC, MODE, Op, 2><<<grid_of(L), BS, smem, st>>>(L, op, X, Y, W, cols, ctl); return;
-      case 3: k_spmm<R, VEC, MODE, Op, 3><<<grid_of(L), BS, smem, st>>>(L, op, X, Y, W, cols, ctl); return;
-      case 4:                                           // harmonic pairs for A; kind 0 for G, G^T
-        if constexpr (std::is_same<Op, OpA32>::value) {
-          const dim3 g((unsigned)ceil_div(L.n, L.rows_per_block()), (unsigned)ceil_div(L.nf, 2));
-          k_spmm_pair<VEC, MODE><<<g, BS, smem, st>>>(L, op, X, Y, W, cols, ctl);
-          return;
-        }
-        break;
-      default: break;
-    }
+// k_spmm launch with the plan's gather kind
+template <int VEC, int MODE, class Op>
+void spmm_go(const SolverPlan *S, const Layout &L, size_t smem, cudaStream_t st, const Op &op, const float2 *X,
+             float2 *Y, const float2 *W, const Cols &cols, const Ctl *ctl) {
+  switch (S->tune_kind) {
+    case 1: k_spmm<float, VEC, MODE, Op, 1><<<grid_of(L), BS, smem, st>>>(L, op, X, Y, W, cols, ctl); return;
+    case 2: k_spmm<float, VEC, MODE, Op, 2><<<grid_of(L), BS, smem, st>>>(L, op, X, Y, W, cols, ctl); return;
+    case 3: k_spmm<float, VEC, MODE, Op, 3><<<grid_of(L), BS, smem, st>>>(L, op, X, Y, W, cols, ctl); return;
+    case 4:                                             // harmonic pairs for A; kind 0 for G, G^T
+      if constexpr (std::is_same<Op, OpA32>::value) {
+        const dim3 g((unsigned)ceil_div(L.n, L.rows_per_block()), (unsigned)ceil_div(L.nf, 2));
+        k_spmm_pair<VEC, MODE><<<g, BS, smem, st>>>(L, op, X, Y, W, cols, ctl);
+        return;
+      }
+      break;
+    default: break;
   }
-  k_spmm<R, VEC, MODE, Op, 0><<<grid_of(L), BS, smem, st>>>(L, op, X, Y, W, cols, ctl);
+  k_spmm<float, VEC, MODE, Op, 0><<<grid_of(L), BS, smem, st>>>(L, op, X, Y, W, cols, ctl);
 }
 
-// Lane widths: plain SpMM sweeps VS, SpMM sweeps with dot products VD, vector updates 2 -- and 4 past
+// Lane widths: SpMM sweeps VS, vector updates 2 -- and 4 past
 // 64 padded sources, where 2 would take more lanes per row than a warp has.
 int vu_of(const SolverPlan *S) { return S->nsp > 64 ? 4 : 2; }
 template <class F> void with_vu(const SolverPlan *S, F f) {
@@ -1880,7 +1874,7 @@ template <class F> void with_vu(const SolverPlan *S, F f) {
 
 // one BiCGSTAB iteration (dMesh.m:1295-1340) enqueued on st: KERNELS_PER_ITER launches
 // one complex-FP32 iteration with the tiled SpMM (same kernel sequence as enqueue_iteration)
-void enqueue_iteration_tiled(const SolverPlan *S, const Vecs<float> &V, const Work &W, cudaStream_t st) {
+void enqueue_iteration_tiled(const SolverPlan *S, const Vecs &V, const Work &W, cudaStream_t st) {
   const Layout Lu = layouts_for(S, vu_of(S)).L, Lud = layouts_for(S, vu_of(S)).Ld;
   Ctl *ctl = W.ctl;
   tspmm<0>(S, 1, V.p, V.T1, nullptr, W.cols, ctl, st);
@@ -1908,79 +1902,72 @@ void enqueue_iteration_tiled(const SolverPlan *S, const Vecs<float> &V, const Wo
   });
 }
 
-template <class R, int VS, int VD, class OpA, class OpG>
-void enqueue_iteration(const SolverPlan *S, const OpA &A, const OpG &G, const OpG &GT, const Vecs<R> &V,
+template <int VS, class OpA, class OpG>
+void enqueue_iteration(const SolverPlan *S, const OpA &A, const OpG &G, const OpG &GT, const Vecs &V,
                        const Work &W, cudaStream_t st) {
-  const Layout Ls = spmm_layouts(S, VS, sizeof(R) == 4).L, Lsd = spmm_layouts(S, VD, sizeof(R) == 4).Ld;
+  const Layout Ls = spmm_layouts(S, VS).L, Lsd = spmm_layouts(S, VS).Ld;
   const Layout Lu = layouts_for(S, vu_of(S)).L, Lud = layouts_for(S, vu_of(S)).Ld;
   Ctl *ctl = W.ctl;
-  if constexpr (sizeof(R) == 4) {
-    if (S->tiled) {
-      enqueue_iteration_tiled(S, V, W, st);
-      return;
-    }
+  if (S->tiled) {
+    enqueue_iteration_tiled(S, V, W, st);
+    return;
   }
   // T1 = G p ; h = G^T T1                                       (:1295-1296)
-  spmm_go<R, VS, 0>(S, Ls, 0, st, G, V.p, V.T1, nullptr, W.cols, ctl);
-  spmm_go<R, VS, 0>(S, Ls, 0, st, GT, V.T1, V.h, nullptr, W.cols, ctl);
+  spmm_go<VS, 0>(S, Ls, 0, st, G, V.p, V.T1, nullptr, W.cols, ctl);
+  spmm_go<VS, 0>(S, Ls, 0, st, GT, V.T1, V.h, nullptr, W.cols, ctl);
   // v = A h, d1 = v.r0^                                         (:1301, :1304)
-  spmm_go<R, VD, 1>(S, Lsd, red_smem(Lsd, 1), st, A, V.h, V.v, V.rhat, W.cols, ctl);
+  spmm_go<VS, 1>(S, Lsd, red_smem(Lsd, 1), st, A, V.h, V.v, V.rhat, W.cols, ctl);
   k_stage_alpha<<<1, 1024, 0, st>>>(W.cols, ctl);
   // s = r - alpha v ; ||s||                                     (:1306-1308)
   with_vu(S, [&](auto u) {
-    k_update_s<R, decltype(u)::value><<<grid_of(Lud), BS, red_smem(Lud, 1), st>>>(Lud, V.r, V.v, V.s, W.cols, ctl);
+    k_update_s<float, decltype(u)::value><<<grid_of(Lud), BS, red_smem(Lud, 1), st>>>(Lud, V.r, V.v, V.s, W.cols, ctl);
   });
   k_stage_check_s<<<1, 1024, 0, st>>>(W.cols, ctl);
   // Gs = G s ; z = G^T Gs ; t = A z ; (G t).Gs, (G t).(G t)     (:1315-1325)
-  spmm_go<R, VS, 0>(S, Ls, 0, st, G, V.s, V.T1, nullptr, W.cols, ctl);
-  spmm_go<R, VS, 0>(S, Ls, 0, st, GT, V.T1, V.z, nullptr, W.cols, ctl);
-  spmm_go<R, VS, 0>(S, Ls, 0, st, A, V.z, V.t, nullptr, W.cols, ctl);
-  spmm_go<R, VD, 2>(S, Lsd, red_smem(Lsd, 2), st, G, V.t, nullptr, V.T1, W.cols, ctl);
+  spmm_go<VS, 0>(S, Ls, 0, st, G, V.s, V.T1, nullptr, W.cols, ctl);
+  spmm_go<VS, 0>(S, Ls, 0, st, GT, V.T1, V.z, nullptr, W.cols, ctl);
+  spmm_go<VS, 0>(S, Ls, 0, st, A, V.z, V.t, nullptr, W.cols, ctl);
+  spmm_go<VS, 2>(S, Lsd, red_smem(Lsd, 2), st, G, V.t, nullptr, V.T1, W.cols, ctl);
   k_stage_omega<<<1, 1024, 0, st>>>(W.cols, ctl);
   // x += alpha h + om z ; r = s - om t ; p -= om v ; ||r|| ; r0^.r   (:1305, :1327-1337)
   with_vu(S, [&](auto u) {
-    k_update_xrp<R, decltype(u)::value><<<grid_of(Lud), BS, red_smem(Lud, 2), st>>>(
+    k_update_xrp<float, decltype(u)::value><<<grid_of(Lud), BS, red_smem(Lud, 2), st>>>(
         Lud, V.x, V.h, V.z, V.r, V.s, V.t, V.p, V.v, V.rhat, W.cols, ctl);
   });
   k_stage_check_r<<<1, 1024, 0, st>>>(W.cols, ctl);
   k_stage_count<<<1, 1024, 0, st>>>(W.cols, ctl);
   // p = r + beta p                                              (:1340)
   with_vu(S, [&](auto u) {
-    k_update_p<R, decltype(u)::value><<<grid_of(Lu), BS, 0, st>>>(Lu, V.r, V.p, W.cols, ctl);
+    k_update_p<float, decltype(u)::value><<<grid_of(Lu), BS, 0, st>>>(Lu, V.r, V.p, W.cols, ctl);
   });
 }
 
 // COCG preconditioner step: T1 = G r ; z = G^T T1 ; acc[D1] = r.z ; rho, beta.  The gather
 // path takes r.z = r^T G^T G r as T1.T1 in the G sweep (no second read of r); the tiled path
 // takes it as r.z in the G^T sweep.
-template <class R, int VS, int VD, class OpG>
-void enqueue_cocg_precond(const SolverPlan *S, const OpG &G, const OpG &GT, const Vecs<R> &V, const Work &W,
+template <int VS, class OpG>
+void enqueue_cocg_precond(const SolverPlan *S, const OpG &G, const OpG &GT, const Vecs &V, const Work &W,
                           int first, cudaStream_t st) {
   Ctl *ctl = W.ctl;
-  bool done = false;
-  if constexpr (sizeof(R) == 4) {
-    if (S->tiled) {
-      tspmm<0>(S, 1, V.r, V.T1, nullptr, W.cols, ctl, st);
-      tspmm<1>(S, 2, V.T1, V.z, V.r, W.cols, ctl, st);
-      done = true;
-    }
-  }
-  if (!done) {
-    const Layout Ls = spmm_layouts(S, VS, sizeof(R) == 4).L, Lsd = spmm_layouts(S, VD, sizeof(R) == 4).Ld;
-    spmm_go<R, VD, 3>(S, Lsd, red_smem(Lsd, 1), st, G, V.r, V.T1, nullptr, W.cols, ctl);
-    spmm_go<R, VS, 0>(S, Ls, 0, st, GT, V.T1, V.z, nullptr, W.cols, ctl);
+  if (S->tiled) {
+    tspmm<0>(S, 1, V.r, V.T1, nullptr, W.cols, ctl, st);
+    tspmm<1>(S, 2, V.T1, V.z, V.r, W.cols, ctl, st);
+  } else {
+    const Layout Ls = spmm_layouts(S, VS).L, Lsd = spmm_layouts(S, VS).Ld;
+    spmm_go<VS, 3>(S, Lsd, red_smem(Lsd, 1), st, G, V.r, V.T1, nullptr, W.cols, ctl);
+    spmm_go<VS, 0>(S, Ls, 0, st, GT, V.T1, V.z, nullptr, W.cols, ctl);
   }
   k_cocg_rho<<<1, 1024, 0, st>>>(W.cols, ctl, first);
 }
 
 // COCG start after k_stage_init: z0 = G^T G r0, rho = r0.z0, p = z0 (p holds r0 from k_init, finite)
-template <class R, int VS, int VD, class OpG>
-void enqueue_cocg_start(const SolverPlan *S, const OpG &G, const OpG &GT, const Vecs<R> &V, const Work &W,
+template <int VS, class OpG>
+void enqueue_cocg_start(const SolverPlan *S, const OpG &G, const OpG &GT, const Vecs &V, const Work &W,
                         cudaStream_t st) {
   const Layout Lu = layouts_for(S, vu_of(S)).L;
-  enqueue_cocg_precond<R, VS, VD>(S, G, GT, V, W, 1, st);
+  enqueue_cocg_precond<VS>(S, G, GT, V, W, 1, st);
   with_vu(S, [&](auto u) {
-    k_update_p<R, decltype(u)::value><<<grid_of(Lu), BS, 0, st>>>(Lu, V.z, V.p, W.cols, W.ctl);
+    k_update_p<float, decltype(u)::value><<<grid_of(Lu), BS, 0, st>>>(Lu, V.z, V.p, W.cols, W.ctl);
   });
 }
 
@@ -1988,64 +1975,49 @@ void enqueue_cocg_start(const SolverPlan *S, const OpG &G, const OpG &GT, const 
 // the complex-symmetric FSAI preconditioner G^T G), KERNELS_PER_ITER_COCG launches:
 //   q = A p, p.q ; alpha = rho/(p.q) ; r -= alpha q, ||r|| ; stop checks ;
 //   z = G^T G r, rho' = r.z, beta = rho'/rho ; x += alpha p, p = z + beta p ; count
-template <class R, int VS, int VD, class OpA, class OpG>
-void enqueue_cocg(const SolverPlan *S, const OpA &A, const OpG &G, const OpG &GT, const Vecs<R> &V, const Work &W,
+template <int VS, class OpA, class OpG>
+void enqueue_cocg(const SolverPlan *S, const OpA &A, const OpG &G, const OpG &GT, const Vecs &V, const Work &W,
                   cudaStream_t st) {
   const Layout Lu = layouts_for(S, vu_of(S)).L, Lud = layouts_for(S, vu_of(S)).Ld;
   Ctl *ctl = W.ctl;
-  bool done = false;
-  if constexpr (sizeof(R) == 4) {
-    if (S->tiled) {
-      tspmm<1>(S, 0, V.p, V.v, V.p, W.cols, ctl, st);
-      done = true;
-    }
-  }
-  if (!done) {
-    const Layout Lsd = spmm_layouts(S, VD, sizeof(R) == 4).Ld;
-    spmm_go<R, VD, 1>(S, Lsd, red_smem(Lsd, 1), st, A, V.p, V.v, V.p, W.cols, ctl);
+  if (S->tiled) {
+    tspmm<1>(S, 0, V.p, V.v, V.p, W.cols, ctl, st);
+  } else {
+    const Layout Lsd = spmm_layouts(S, VS).Ld;
+    spmm_go<VS, 1>(S, Lsd, red_smem(Lsd, 1), st, A, V.p, V.v, V.p, W.cols, ctl);
   }
   k_cocg_alpha<<<1, 1024, 0, st>>>(W.cols, ctl);
   with_vu(S, [&](auto u) {
-    k_update_r<R, decltype(u)::value><<<grid_of(Lud), BS, red_smem(Lud, 1), st>>>(Lud, V.r, V.v, W.cols, ctl);
+    k_update_r<float, decltype(u)::value><<<grid_of(Lud), BS, red_smem(Lud, 1), st>>>(Lud, V.r, V.v, W.cols, ctl);
   });
   k_cocg_check<<<1, 1024, 0, st>>>(W.cols, ctl);
-  enqueue_cocg_precond<R, VS, VD>(S, G, GT, V, W, 0, st);
+  enqueue_cocg_precond<VS>(S, G, GT, V, W, 0, st);
   with_vu(S, [&](auto u) {
-    k_update_px<R, decltype(u)::value><<<grid_of(Lu), BS, 0, st>>>(Lu, V.x, V.p, V.z, W.cols, ctl);
+    k_update_px<float, decltype(u)::value><<<grid_of(Lu), BS, 0, st>>>(Lu, V.x, V.p, V.z, W.cols, ctl);
   });
   k_cocg_count<<<1, 1024, 0, st>>>(W.cols, ctl);
 }
 
 enum { ENQ_BICGSTAB = 0, ENQ_COCG = 1, ENQ_COCG_START = 2 };
 
-template <class R, int VS>
-int enqueue_for(SolverPlan *S, const Vecs<R> &V, const Work &W, cudaStream_t st, int what = ENQ_BICGSTAB) {
-  // lane width of the SpMM sweeps with dot products: the FP32 sweeps keep their
-  // partials in FP32 and afford the plain sweeps' width; FP64 ones cap at 4
-  constexpr int VD = sizeof(R) == 4 ? VS : (VS < 4 ? VS : 4);
-  const int32_t *rp = S->rowptr.as<int32_t>();
-  if constexpr (sizeof(R) == 4) {
-    OpA32 A{rp, S->RecA32.as<Rec32>(), (const float *)(S->omega.as<char>() + sizeof(double) * S->nf)};
-    OpG32 G{S->P.rowptr.as<int32_t>(), S->RecG32.as<Rec32>(), S->nnzG};
-    OpG32 GT{S->P.rowptrT.as<int32_t>(), S->RecGT32.as<Rec32>(), S->nnzG};
-    if (what == ENQ_COCG) enqueue_cocg<R, VS, VD>(S, A, G, GT, V, W, st);
-    else if (what == ENQ_COCG_START) enqueue_cocg_start<R, VS, VD>(S, G, GT, V, W, st);
-    else enqueue_iteration<R, VS, VD>(S, A, G, GT, V, W, st);
-  }
+template <int VS>
+int enqueue_for(SolverPlan *S, const Vecs &V, const Work &W, cudaStream_t st, int what) {
+  OpA32 A{S->rowptr.as<int32_t>(), S->RecA32.as<Rec32>(), (const float *)(S->omega.as<char>() + sizeof(double) * S->nf)};
+  OpG32 G{S->P.rowptr.as<int32_t>(), S->RecG32.as<Rec32>(), S->nnzG};
+  OpG32 GT{S->P.rowptrT.as<int32_t>(), S->RecGT32.as<Rec32>(), S->nnzG};
+  if (what == ENQ_COCG) enqueue_cocg<VS>(S, A, G, GT, V, W, st);
+  else if (what == ENQ_COCG_START) enqueue_cocg_start<VS>(S, G, GT, V, W, st);
+  else enqueue_iteration<VS>(S, A, G, GT, V, W, st);
   DGP_CUDA(cudaGetLastError());
   return DGP_OK;
 }
 
-// run BiCGSTAB iterations (graph-captured blocks) until the control block says done
 // dispatch of enqueue_for on the plan's lane width
-template <class R>
-int enqueue_vec(SolverPlan *S, const Vecs<R> &V, const Work &W, cudaStream_t st, int what) {
-  switch (vec_for(S, sizeof(R) == 4)) {
-    case 2: return enqueue_for<R, 2>(S, V, W, st, what);
-    case 4: return enqueue_for<R, 4>(S, V, W, st, what);
-    default:
-      if constexpr (sizeof(R) == 4) return enqueue_for<R, 8>(S, V, W, st, what);
-      return DGP_OK;
+int enqueue_vec(SolverPlan *S, const Vecs &V, const Work &W, cudaStream_t st, int what) {
+  switch (vec_for(S, true)) {
+    case 2: return enqueue_for<2>(S, V, W, st, what);
+    case 4: return enqueue_for<4>(S, V, W, st, what);
+    default: return enqueue_for<8>(S, V, W, st, what);
   }
 }
 
@@ -2075,10 +2047,9 @@ __global__ void k_loop_cond(cudaGraphConditionalHandle h, Ctl *ctl, int stall_gu
 // Device-driven form of run_iterations: ONE graph launch whose WHILE node replays blocks of
 // check_every iterations until k_loop_cond clears the condition; the host waits once for the
 // control block.
-template <class R>
-int run_iterations_device(SolverPlan *S, const Vecs<R> &V, const Work &W, int check_every, cudaStream_t st,
+int run_iterations_device(SolverPlan *S, const Vecs &V, const Work &W, int check_every, cudaStream_t st,
                           int *iters_out, bool stall_guard, bool cocg) {
-  const int gi = 3 + (sizeof(R) == 4 ? (cocg ? 2 : 1) : 0);
+  const int gi = 2 + (cocg ? 1 : 0);
   const int per_iter = cocg ? KERNELS_PER_ITER_COCG : KERNELS_PER_ITER;
   const int patience = std::max(3, 40 / check_every);
   if (!S->graph[gi] || S->graph_iters[gi] != check_every) {
@@ -2108,7 +2079,7 @@ int run_iterations_device(SolverPlan *S, const Vecs<R> &V, const Work &W, int ch
     int rc = DGP_OK;
     if (e == cudaSuccess) {
       for (int q = 0; q < check_every && rc == DGP_OK; ++q)
-        rc = enqueue_vec<R>(S, V, W, cs, cocg ? ENQ_COCG : ENQ_BICGSTAB);
+        rc = enqueue_vec(S, V, W, cs, cocg ? ENQ_COCG : ENQ_BICGSTAB);
       k_loop_cond<<<1, 32, 0, cs>>>(h, W.ctl, stall_guard ? 1 : 0, patience, check_every);
       cudaGraph_t out = nullptr;
       e = cudaStreamEndCapture(cs, &out);
@@ -2129,13 +2100,13 @@ int run_iterations_device(SolverPlan *S, const Vecs<R> &V, const Work &W, int ch
   return DGP_OK;
 }
 
-template <class R>
-int run_iterations(SolverPlan *S, const Vecs<R> &V, const Work &W, int check_every, int maxit, cudaStream_t st,
+// Iterations (graph-captured blocks) until the control block says done.
+int run_iterations(SolverPlan *S, const Vecs &V, const Work &W, int check_every, int maxit, cudaStream_t st,
                    int *iters_out, bool stall_guard = false, bool cocg = false) {
-  const int gi = sizeof(R) == 4 ? (cocg ? 2 : 1) : 0;
+  const int gi = cocg ? 1 : 0;
   const int per_iter = cocg ? KERNELS_PER_ITER_COCG : KERNELS_PER_ITER;
   if (check_every < 1) check_every = 1;
-  if (S->device_loop) return run_iterations_device<R>(S, V, W, check_every, st, iters_out, stall_guard, cocg);
+  if (S->device_loop) return run_iterations_device(S, V, W, check_every, st, iters_out, stall_guard, cocg);
   if (!S->graph[gi] || S->graph_iters[gi] != check_every) {
     if (S->graph[gi]) {
       cudaGraphExecDestroy(S->graph[gi]);
@@ -2147,7 +2118,7 @@ int run_iterations(SolverPlan *S, const Vecs<R> &V, const Work &W, int check_eve
     DGP_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
     int rc = DGP_OK;
     for (int q = 0; q < check_every && rc == DGP_OK; ++q)
-      rc = enqueue_vec<R>(S, V, W, cs, cocg ? ENQ_COCG : ENQ_BICGSTAB);
+      rc = enqueue_vec(S, V, W, cs, cocg ? ENQ_COCG : ENQ_BICGSTAB);
     cudaError_t e = cudaStreamEndCapture(cs, &g);
     cudaStreamDestroy(cs);
     if (rc != DGP_OK) return rc;
@@ -2224,9 +2195,9 @@ int set_ctl(Ctl *d, double tol, int maxit, int stop_rule, cudaStream_t st, void 
   return DGP_OK;
 }
 
-template <class R, int VEC>
-void launch_init(const Layout &Ld, const Vecs<R> &V, const Work &W, cudaStream_t st) {
-  k_init<R, VEC><<<grid_of(Ld), BS, red_smem(Ld, 2), st>>>(Ld, V.x, V.r, V.rhat, V.p, W.cols);
+template <int VEC>
+void launch_init(const Layout &Ld, const Vecs &V, const Work &W, cudaStream_t st) {
+  k_init<float, VEC><<<grid_of(Ld), BS, red_smem(Ld, 2), st>>>(Ld, V.x, V.r, V.rhat, V.p, W.cols);
 }
 
 // FP64 residual sweep b - A x with the solver's lane layout for its source count
@@ -2251,8 +2222,7 @@ void launch_residual(SolverPlan *S, int ns, const double *d_X, const double *d_B
 }  // namespace
 
 void SolverPlan::drop_workspaces() {
-  for (cudaGraphExec_t *g : {graph, graph + 1, graph + 2, graph + 3, graph + 4, graph + 5, fgraph, fgraph + 1, dgraph,
-                             dgraph + 1})
+  for (cudaGraphExec_t *g : {graph, graph + 1, graph + 2, graph + 3, fgraph, fgraph + 1, dgraph, dgraph + 1})
     if (*g) {
       cudaGraphExecDestroy(*g);
       *g = nullptr;
@@ -2380,9 +2350,9 @@ static int solve_mixed(SolverPlan *S, const double *d_B, const int32_t *d_nodes,
                        const double *d_fpsf, double *d_X, int ns, const dgp_solve_opts &o, dgp_solve_report *rep,
                        cudaStream_t st) {
   const bool cocg = o.precision == DGP_PREC_MIXED;
-  DGP_TRY(ensure_workspace(S, DGP_PREC_MIXED, cocg ? NVEC_COCG : NVEC_ALL));
+  DGP_TRY(ensure_workspace(S, cocg ? NVEC_COCG : NVEC_ALL));
   Work W = work_views(S);
-  Vecs<float> V = vec_views<float>(S);
+  Vecs V = vec_views(S);
   const int vec = vec_for(S, true);
   const Layouts LL = layouts_for(S, vec);
   DGP_CUDA(cudaMemsetAsync(d_X, 0, sizeof(double2) * (size_t)S->nf * S->n * ns, st));
@@ -2405,16 +2375,16 @@ static int solve_mixed(SolverPlan *S, const double *d_B, const int32_t *d_nodes,
     // against tol after each inner solve.  The stall guard of run_iterations ends inner solves
     // that stop making progress in FP32.
     DGP_TRY(set_ctl(W.ctl, o.inner_tol, inner_maxit, DGP_STOP_PER_COLUMN, st, S->h_ctl));
-    with_vu(S, [&](auto u) { launch_init<float, decltype(u)::value>(layouts_for(S, vu_of(S)).Ld, V, W, st); });
+    with_vu(S, [&](auto u) { launch_init<decltype(u)::value>(layouts_for(S, vu_of(S)).Ld, V, W, st); });
     DGP_CHECK_LAUNCH();
     k_stage_init<<<1, 1024, 0, st>>>(W.cols, W.ctl, S->nsp, ns, ref > 0 ? W.outer_err : nullptr, o.tol);
     DGP_CHECK_LAUNCH();
     if (cocg) {
-      DGP_TRY(enqueue_vec<float>(S, V, W, st, ENQ_COCG_START));
+      DGP_TRY(enqueue_vec(S, V, W, st, ENQ_COCG_START));
       count_launches(3);
     }
     int it = 0;
-    DGP_TRY(run_iterations<float>(S, V, W, o.check_every, inner_maxit, st, &it, true, cocg));
+    DGP_TRY(run_iterations(S, V, W, o.check_every, inner_maxit, st, &it, true, cocg));
     total_iters += it;
     refinements += 1;
     // X += x32 ; r = b - A X in FP64
@@ -2508,15 +2478,15 @@ __global__ void k_all_active(Cols c) {
 }
 
 template <int VEC>
-void profile_launch(int which, const SolverPlan *S, const OpA32 &A, const OpG32 &G, const Vecs<float> &V,
+void profile_launch(int which, const SolverPlan *S, const OpA32 &A, const OpG32 &G, const Vecs &V,
                     const Work &W, const Ctl *ctl, cudaStream_t st) {
-  const Layout L = spmm_layouts(S, VEC, true).L, Ld = spmm_layouts(S, VEC, true).Ld;
+  const Layout L = spmm_layouts(S, VEC).L, Ld = spmm_layouts(S, VEC).Ld;
   const Layout Lu = layouts_for(S, vu_of(S)).L, Lud = layouts_for(S, vu_of(S)).Ld;
   switch (which) {
-    case 0: spmm_go<float, VEC, 0>(S, L, 0, st, A, V.z, V.x, nullptr, W.cols, ctl); break;
-    case 1: spmm_go<float, VEC, 0>(S, L, 0, st, G, V.p, V.T1, nullptr, W.cols, ctl); break;
-    case 4: spmm_go<float, VEC, 1>(S, Ld, red_smem(Ld, 1), st, A, V.p, V.v, V.p, W.cols, ctl); break;
-    case 5: spmm_go<float, VEC, 3>(S, Ld, red_smem(Ld, 1), st, G, V.r, V.T1, nullptr, W.cols, ctl); break;
+    case 0: spmm_go<VEC, 0>(S, L, 0, st, A, V.z, V.x, nullptr, W.cols, ctl); break;
+    case 1: spmm_go<VEC, 0>(S, L, 0, st, G, V.p, V.T1, nullptr, W.cols, ctl); break;
+    case 4: spmm_go<VEC, 1>(S, Ld, red_smem(Ld, 1), st, A, V.p, V.v, V.p, W.cols, ctl); break;
+    case 5: spmm_go<VEC, 3>(S, Ld, red_smem(Ld, 1), st, G, V.r, V.T1, nullptr, W.cols, ctl); break;
     case 6:
       with_vu(S, [&](auto u) {
         k_update_r<float, decltype(u)::value><<<grid_of(Lud), BS, red_smem(Lud, 1), st>>>(Lud, V.r, V.v, W.cols, ctl);
@@ -2555,9 +2525,9 @@ int solver_profile(SolverPlan *S, int which, int reps, float *ms, double *bytes,
     call.done();
     return DGP_OK;
   }
-  DGP_TRY(ensure_workspace(S, DGP_PREC_MIXED, NVEC_COCG));
-  if (which == 2 || which == 3) DGP_TRY(ensure_workspace(S, DGP_PREC_MIXED, NVEC_ALL));  // BiCGSTAB updates
-  Vecs<float> V = vec_views<float>(S);
+  DGP_TRY(ensure_workspace(S, NVEC_COCG));
+  if (which == 2 || which == 3) DGP_TRY(ensure_workspace(S, NVEC_ALL));  // BiCGSTAB updates
+  Vecs V = vec_views(S);
   Work W = work_views(S);
   W.cols.hact = nullptr;  // timing / checking runs sweep every harmonic
   ScratchBuf dctl;
@@ -2618,22 +2588,22 @@ int solver_profile(SolverPlan *S, int which, int reps, float *ms, double *bytes,
 namespace {
 // the complex-FP32 SpMM sweeps of one iteration (enqueue_iteration's 7 SpMM launches)
 template <int VEC>
-void spmm_set(const SolverPlan *S, const OpA32 &A, const OpG32 &G, const OpG32 &GT, const Vecs<float> &V,
+void spmm_set(const SolverPlan *S, const OpA32 &A, const OpG32 &G, const OpG32 &GT, const Vecs &V,
               const Work &W, const Ctl *ctl, cudaStream_t st) {
-  const Layouts LL = spmm_layouts(S, VEC, true);
+  const Layouts LL = spmm_layouts(S, VEC);
   const Layout Ls = LL.L, Lsd = LL.Ld;
   // scratch vectors from the first NVEC_COCG slots only (x, r and r^ stand in for h, s and t)
-  spmm_go<float, VEC, 0>(S, Ls, 0, st, G, V.p, V.T1, nullptr, W.cols, ctl);
-  spmm_go<float, VEC, 0>(S, Ls, 0, st, GT, V.T1, V.x, nullptr, W.cols, ctl);
-  spmm_go<float, VEC, 1>(S, Lsd, red_smem(Lsd, 1), st, A, V.x, V.v, V.rhat, W.cols, ctl);
-  spmm_go<float, VEC, 0>(S, Ls, 0, st, G, V.r, V.T1, nullptr, W.cols, ctl);
-  spmm_go<float, VEC, 0>(S, Ls, 0, st, GT, V.T1, V.z, nullptr, W.cols, ctl);
-  spmm_go<float, VEC, 0>(S, Ls, 0, st, A, V.z, V.rhat, nullptr, W.cols, ctl);
-  spmm_go<float, VEC, 2>(S, Lsd, red_smem(Lsd, 2), st, G, V.rhat, nullptr, V.T1, W.cols, ctl);
+  spmm_go<VEC, 0>(S, Ls, 0, st, G, V.p, V.T1, nullptr, W.cols, ctl);
+  spmm_go<VEC, 0>(S, Ls, 0, st, GT, V.T1, V.x, nullptr, W.cols, ctl);
+  spmm_go<VEC, 1>(S, Lsd, red_smem(Lsd, 1), st, A, V.x, V.v, V.rhat, W.cols, ctl);
+  spmm_go<VEC, 0>(S, Ls, 0, st, G, V.r, V.T1, nullptr, W.cols, ctl);
+  spmm_go<VEC, 0>(S, Ls, 0, st, GT, V.T1, V.z, nullptr, W.cols, ctl);
+  spmm_go<VEC, 0>(S, Ls, 0, st, A, V.z, V.rhat, nullptr, W.cols, ctl);
+  spmm_go<VEC, 2>(S, Lsd, red_smem(Lsd, 2), st, G, V.rhat, nullptr, V.T1, W.cols, ctl);
 }
 }  // namespace
 
-void tspmm_set(const SolverPlan *S, const Vecs<float> &V, const Work &W, const Ctl *ctl, cudaStream_t st) {
+void tspmm_set(const SolverPlan *S, const Vecs &V, const Work &W, const Ctl *ctl, cudaStream_t st) {
   tspmm<0>(S, 1, V.p, V.T1, nullptr, W.cols, ctl, st);
   tspmm<0>(S, 2, V.T1, V.x, nullptr, W.cols, ctl, st);
   tspmm<1>(S, 0, V.x, V.v, V.rhat, W.cols, ctl, st);
@@ -2683,8 +2653,8 @@ int solver_autotune(SolverPlan *S, int32_t *tiled_out, int32_t *vec_out, int32_t
                     cudaStream_t st) {
   PlanCall call(S);
   DGP_TRY(tiled_setup(S, st));
-  DGP_TRY(ensure_workspace(S, DGP_PREC_MIXED, NVEC_COCG));
-  Vecs<float> V = vec_views<float>(S);
+  DGP_TRY(ensure_workspace(S, NVEC_COCG));
+  Vecs V = vec_views(S);
   Work W = work_views(S);
   W.cols.hact = nullptr;  // timing / checking runs sweep every harmonic
   ScratchBuf dctl;
@@ -2715,7 +2685,7 @@ int solver_autotune(SolverPlan *S, int32_t *tiled_out, int32_t *vec_out, int32_t
       S->tune_vec = vec;
       S->tune_rows = rows;
       S->tune_kind = kind;
-      const int ipb = spmm_layouts(S, vec, true).L.ipb;
+      const int ipb = spmm_layouts(S, vec).L.ipb;
       if (ipb == last_ipb) continue;  // same launch shape as the previous candidate
       last_ipb = ipb;
       auto run = [&]() {
@@ -2872,8 +2842,8 @@ int solver_check_spmm(SolverPlan *S, double *max_rel, cudaStream_t st) {
   PlanCall call(S);
   DGP_TRY(tiled_setup(S, st));
   DGP_REQUIRE(S->tiled_ok, "check_spmm: the tiled SpMM does not fit this plan");
-  DGP_TRY(ensure_workspace(S, DGP_PREC_MIXED, NVEC_COCG));
-  Vecs<float> V = vec_views<float>(S);
+  DGP_TRY(ensure_workspace(S, NVEC_COCG));
+  Vecs V = vec_views(S);
   Work W = work_views(S);
   W.cols.hact = nullptr;  // timing / checking runs sweep every harmonic
   ScratchBuf dctl, dm;

@@ -97,10 +97,10 @@ struct SolverPlan {
   DevBuf status;                 // per-column status
   void *h_ctl = nullptr;         // pinned mirrors of the control block (two)
   cudaEvent_t poll_ev[2] = {nullptr, nullptr};  // the two mirrors' copy-done events
-  // blocks of iterations captured as graphs -- [0..2]: FP64 BiCGSTAB, FP32 BiCGSTAB, FP32 COCG
-  // (replayed and polled by the host); [3..5]: the same inside a device-driven WHILE loop
-  cudaGraphExec_t graph[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-  int graph_iters[6] = {0, 0, 0, 0, 0, 0};
+  // blocks of iterations of the unfused solves captured as graphs -- [0], [1]: BiCGSTAB, COCG (replayed
+  // and polled by the host); [2], [3]: the same inside a device-driven WHILE loop
+  cudaGraphExec_t graph[4] = {nullptr, nullptr, nullptr, nullptr};
+  int graph_iters[4] = {0, 0, 0, 0};
   int32_t device_loop = 1;       // 1: an inner solve is one graph launch (WHILE node), 0: host polling
   // SpMM launch shape of the complex-FP32 sweeps chosen by solver_autotune (0 = built-in default)
   int32_t tune_vec = 0, tune_rows = 0;
