@@ -909,8 +909,8 @@ def run_ours(a, rank, world, local_rank):
              2: "k_update_xrp<float>", 3: "k_update_s<float>",
              4: a1, 5: f"k_spmm<float,{sv},3,OpG32,{gk}> (T = G r, T.T)",
              6: "k_update_r<float>", 7: "k_update_px<float>",
-             8: "k_fsweep<4,0> (q = A p, p.q)", 9: "k_fsweep<4,1> (T -= alpha G q, T.T)",
-             10: "k_fsweep<4,2> (x += alpha p, p = G^T T + beta p)"}
+             8: "k_fsweep<4,false,0> (q = A p, p.q)", 9: "k_fsweep<4,false,1> (T -= alpha G q, T.T)",
+             10: "k_fsweep<4,false,2> (x += alpha p, p = G^T T + beta p)"}
     prof = {q: solver.profile_kernel(q, 5) for q in per_iter}
     dom = max(prof, key=lambda q: prof[q][0] * per_iter[q])
     pk = json.load(open(ROOT / "MEASURED_PEAKS.json")) if (ROOT / "MEASURED_PEAKS.json").exists() else {}
@@ -930,7 +930,7 @@ def run_ours(a, rank, world, local_rank):
             "frac": round(ach / peak, 4), "traffic": traffic, "traffic_bytes_per_launch": traffic_bytes,
             "algorithmic_bytes_per_launch": prof[dom][1],
             "traffic_note": ("GB/s of DRAM traffic (read + write) per launch: ncu capture of this kernel on the "
-                             "20,497-node x 32-harmonic case scaled by nodes x harmonics") if traffic else None,
+                             f"{47034 if dom >= 8 else 20497:,}-node x 32-harmonic case scaled by nodes x harmonics") if traffic else None,
             "peak_source": "measured" if pk else "fallback",
             "per_kernel_ms": {names[q]: round(prof[q][0], 3) for q in prof},
             "per_kernel_gbs": {names[q]: round(prof[q][1] / (prof[q][0] * 1e-3) / 1e9, 1) for q in prof}}

@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(GTHREADS, GBN == 64 ? 2 : 1) k_dgemm_nt(Gemm g
 // of depth 128 is 15 us of one SM's FP64 tensor pipe, a 32-row strip a quarter of that.  The
 // strip is loaded whole, the other operand in 32-column chunks through two buffers (108 KB: fits
 // beside a trailing-update CTA).  8 warps of 16 rows x 32 columns; a warp skips the chunks and
-// columns that the triangles leave empty.  Step chain per block at n = 10,240: 27 + 20 -> 9 + 8 us.
+// columns that the triangles leave empty.  Step chain per block at n = 10,240: 27 + 20 -> 9 + 12 us.
 constexpr int SR = 32, SK = 32, SLD = SK + 4, SALD = CB + 4;
 constexpr int STRIP_SMEM = (int)sizeof(double) * (SR * SALD + 2 * CB * SLD);
 struct Strip {
